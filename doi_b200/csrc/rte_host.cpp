@@ -313,9 +313,11 @@ struct rte_ctx {
   int* d_perm = nullptr;
   double *d_mut = nullptr, *d_mus = nullptr;
   float* d_mutf = nullptr;
+  double* d_mutc = nullptr;     // mu_t in column order
+  float* d_mutfc = nullptr;
   double *d_W = nullptr, *d_Wn = nullptr, *d_sum = nullptr, *d_part = nullptr, *d_mom = nullptr;
   double *d_aux1 = nullptr, *d_aux2 = nullptr, *d_aux3 = nullptr, *d_aux4 = nullptr;  // real-basis staging
-  float* d_Wf = nullptr;
+  void* d_Wf = nullptr;         // source rows of the pair kernels in slot order (one right-hand side; FP32 or FP64)
   float* d_K = nullptr;
   double* d_K64 = nullptr;      // FP64 pair kernel (FP64 contexts in RTE_KERNEL_STORE mode)
   bool K_valid = false;
@@ -324,8 +326,10 @@ struct rte_ctx {
   double* d_img = nullptr;  // trans, ref (complex)
   bool medium_set = false;
   int max_split = 8;
-  std::vector<std::array<int, 4>> splits;  // (kernel key, S, chunk, tile) of each planned launch shape
-  size_t Kld = 0;
+  std::vector<std::array<int, 3>> splits;  // (kernel key, S, chunk) of each planned launch shape
+  void* d_slab = nullptr;       // recompute workspace: pair-kernel rows of slab_cols source columns
+  size_t slab_bytes = 0;
+  int slab_cols = 0;
   double* d_selfp = nullptr;    // self-voxel term [N][nb][C]
   int* d_self_idx = nullptr;    // voxel -> distinct mu_t
   double* d_self_lut = nullptr; // [ndistinct][C][C]
@@ -335,12 +339,12 @@ struct rte_ctx {
   int* d_islot = nullptr;       // voxel -> slot
   float4* d_slot_xyz = nullptr; // slot -> (x, y, z, voxel)
   int* d_err = nullptr;         // bounded-wait failure flag of the pair kernels
-  int cpad = 0;                 // FP32 source row length (nb = 1)
-  int cstride = 0;              // FP32 stride of one right-hand side within a row (multiple of 4: 16-byte loads)
+  void* d_tab[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // angle rows [FP64][transposed] (rte_column.cu)
+  double tab_kappa[2][2] = {{0, 0}, {0, 0}};  // the modulation their phases belong to
   // batched solves (several sources on one medium): buffers for up to bcap right-hand sides
   int bcap = 0;
   double *d_bW = nullptr, *d_bWn = nullptr, *d_bsum = nullptr, *d_bres = nullptr, *d_bball = nullptr;
-  float* d_bWf = nullptr;
+  void* d_bWf = nullptr;
   size_t part_cap = 0, selfp_cap = 0;
   // detectors and gradient
   double* d_h = nullptr;        // [6][C] face flux weights
@@ -485,7 +489,7 @@ static void free_all(rte_ctx* c) {
                 c->d_bW, c->d_bWn, c->d_bsum, c->d_bres, c->d_bball, c->d_bWf, c->d_h, c->d_S, c->d_out,
                 c->d_e, c->d_lam, c->d_y, c->d_gt, c->d_gs, c->d_J, c->d_rho, c->d_dlut, c->d_fball, c->d_q, c->d_bq,
                 c->d_Qbp, c->d_mask, c->d_dmut, c->d_dmus, c->d_mut_self, c->d_mus_src, c->d_T, c->d_cidx, c->d_cval, c->d_self_lut_im,
-                c->d_fball_im};
+                c->d_fball_im, c->d_mutc, c->d_mutfc, c->d_slab, c->d_tab[0][0], c->d_tab[0][1], c->d_tab[1][0], c->d_tab[1][1]};
   for (void* p : ps)
     if (p) cudaFree(p);
   if (c->ev0) cudaEventDestroy(c->ev0);
@@ -493,24 +497,19 @@ static void free_all(rte_ctx* c) {
   if (c->st) cudaStreamDestroy(c->st);
 }
 
-// destination order: Morton (z-order) over (x, y, z) so that a warp's 32 destinations form a
-// compact brick (coherent path walks, shared cache lines of mu_t).
-static std::vector<int> morton_perm(int nx, int ny, int nz) {
-  auto spread = [](uint64_t v) {
-    uint64_t r = 0;
-    for (int b = 0; b < 21; b++) r |= ((v >> b) & 1ull) << (3 * b);
-    return r;
-  };
-  std::vector<std::pair<uint64_t, int>> keys;
-  keys.reserve((size_t)nx * ny * nz);
-  for (int i = 0; i < nz; i++)
-    for (int j = 0; j < ny; j++)
-      for (int k = 0; k < nx; k++)
-        keys.push_back({spread(k) | (spread(j) << 1) | (spread(i) << 2), (i * ny + j) * nx + k});
-  std::sort(keys.begin(), keys.end());
-  std::vector<int> p(keys.size());
-  for (size_t q = 0; q < keys.size(); q++) p[q] = keys[q].second;
+// Column order (x, y columns, z fastest): the order of the column kernels, which take one column of sources
+// against the destinations of a few columns at a time (rte_column.cu).
+static std::vector<int> column_perm(int nx, int ny, int nz) {
+  std::vector<int> p((size_t)nx * ny * nz);
+  size_t q = 0;
+  for (int col = 0; col < nx * ny; col++)
+    for (int i = 0; i < nz; i++) p[q++] = i * nx * ny + col;
   return p;
+}
+
+// Layout of the column kernels' source and angle rows in the context's precision.
+static ColDims col_dims(const rte_ctx* c) {
+  return rte_col_dims(c->C, c->L, c->nz, c->precision == RTE_PREC_FP64 ? 1 : 0, c->kappa != 0.0 ? 1 : 0);
 }
 
 extern "C" {
@@ -586,6 +585,8 @@ int rte_create(const rte_config* cfg, rte_ctx** out) {
   if (rc == RTE_OK) cu(dalloc(c, &c->d_mut, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_mus, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_mutf, c->N), "alloc");
+  if (rc == RTE_OK) cu(dalloc(c, &c->d_mutc, c->N), "alloc");
+  if (rc == RTE_OK) cu(dalloc(c, &c->d_mutfc, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_W, NC), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_Wn, NC), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_sum, NC), "alloc");
@@ -598,10 +599,13 @@ int rte_create(const rte_config* cfg, rte_ctx** out) {
   c->part_cap = NC * c->max_split;
   c->selfp_cap = NC;
   if (rc == RTE_OK) cu(dalloc(c, &c->d_self_idx, c->N), "alloc");
-  c->cstride = (c->C + 3) / 4 * 4;
-  c->cpad = (c->cstride + 3) / 4 * 4;
-  if (rc == RTE_OK) cu(dalloc(c, &c->d_Wf, (size_t)c->N * c->cpad), "alloc");
-  if (rc == RTE_OK) cu(cudaMemset(c->d_Wf, 0, sizeof(float) * (size_t)c->N * c->cpad), "memset");
+  {  // room for FP64 rows in either precision (rte_fisher runs FP64 solves in mixed contexts)
+    const size_t nrow = (size_t)c->N * rte_col_dims(c->C, c->L, c->nz, 1, 0).pitch;
+    double* rows = nullptr;
+    if (rc == RTE_OK) cu(dalloc(c, &rows, nrow), "alloc");
+    c->d_Wf = rows;
+    if (rc == RTE_OK) cu(cudaMemset(c->d_Wf, 0, sizeof(double) * nrow), "memset");
+  }
   if (rc == RTE_OK) cu(dalloc(c, &c->d_islot, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_slot_xyz, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_err, 1), "alloc");
@@ -613,7 +617,7 @@ int rte_create(const rte_config* cfg, rte_ctx** out) {
   if (rc == RTE_OK) cu(dalloc(c, &c->d_fball, npix), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_q, NC), "alloc");
   if (rc == RTE_OK) {
-    std::vector<int> p = morton_perm(c->nx, c->ny, c->nz);
+    std::vector<int> p = column_perm(c->nx, c->ny, c->nz);
     std::vector<int> inv(c->N);
     std::vector<float4> xyz(c->N);
     for (int q = 0; q < c->N; q++) {
@@ -780,7 +784,8 @@ static int build_self_lut(rte_ctx* c) {
 // mu_t, mu_s (and the FP32 mu_t) from device arrays; the pair kernel becomes stale.
 static int medium_from_device(rte_ctx* c, const double* d_mua, const double* d_mus) {
   CUDA_TRY(c, cudaMemsetAsync(c->d_red + 6, 0, sizeof(double), c->st));
-  CUDA_TRY(c, (c->launches++, rte_launch_medium(d_mua, d_mus, c->d_mut, c->d_mus, c->d_mutf, c->N, c->d_red + 6, c->st)));
+  CUDA_TRY(c, (c->launches++, rte_launch_medium(d_mua, d_mus, c->d_mut, c->d_mus, c->d_mutf, c->d_mutc, c->d_mutfc,
+                                                   c->d_islot, c->N, c->d_red + 6, c->st)));
   double mumax = 0.0;
   CUDA_TRY(c, cudaMemcpyAsync(&mumax, c->d_red + 6, sizeof(double), cudaMemcpyDeviceToHost, c->st));
   CUDA_TRY(c, cudaStreamSynchronize(c->st));
@@ -870,48 +875,87 @@ static void scatter_factors(const rte_ctx* c, int flag, double* s) {
   }
 }
 
-// The stored pair kernel: FP32 for the mixed method (store or automatic mode), FP64 for the FP64
-// method when RTE_KERNEL_STORE asks for it (automatic FP64 contexts keep recomputing: the plain method).
+// Cells of the pair kernel over `rows` source slots (whole blocks of destinations, kmat_index).
+static size_t kernel_cells(const rte_ctx* c, size_t rows) {
+  const ColDims d = col_dims(c);
+  const size_t np = (size_t)c->nx * c->ny * d.nzp, kb = 32 * (size_t)d.group;
+  return (np + kb - 1) / kb * kb * rows;
+}
+
+// Workspace of the forms that recompute the pair kernel: slabs of source columns, at most this much at a time.
+static const size_t kSlabBytes = 1ull << 30;
+
+// Arguments of the pair-kernel precompute for source columns [col0, col1) into K.
+static StoreArgs store_args(const rte_ctx* c, void* K, size_t ld, int col0, int col1) {
+  StoreArgs a;
+  memset(&a, 0, sizeof a);
+  const ColDims d = col_dims(c);
+  a.N = c->N;
+  a.nx = c->nx;
+  a.ny = c->ny;
+  a.nz = c->nz;
+  a.dx = c->dx;
+  a.dy = c->dy;
+  a.dz = c->dz;
+  a.prop_thresh = c->prop_thresh;
+  a.kscale = c->dV / c->cm;
+  a.mu = c->precision == RTE_PREC_FP64 ? (const void*)c->d_mutc : (const void*)c->d_mutfc;
+  a.K = K;
+  a.Kld = ld;
+  a.nzp = d.nzp;
+  a.group = d.group;
+  a.col0 = col0;
+  a.col1 = col1;
+  return a;
+}
+
+// The stored pair kernel: FP32 for the mixed method (store or automatic mode), FP64 for the FP64 method when
+// RTE_KERNEL_STORE asks for it, or in automatic mode when it is no larger than the recompute workspace.
+// *stored = false: the kernel is recomputed in every application, a slab of source columns at a time (the
+// workspace is allocated here).
 static int ensure_pair_kernel(rte_ctx* c, bool* stored) {
   *stored = false;
   const bool f64 = c->precision == RTE_PREC_FP64;
-  if (c->kernel_mode == RTE_KERNEL_RECOMPUTE || (f64 && c->kernel_mode != RTE_KERNEL_STORE)) return RTE_OK;
-  const size_t ld = ((size_t)c->N + 31) / 32 * 32;  // 128-byte rows
-  const size_t need = f64 ? (size_t)c->N * ld * sizeof(double)
-                          : ((size_t)c->N + RTE_KBLK - 1) / RTE_KBLK * RTE_KBLK * ld * sizeof(float);
-  if (f64 ? !c->d_K64 : !c->d_K) {
+  const size_t esize = f64 ? sizeof(double) : sizeof(float);
+  const size_t cells = kernel_cells(c, c->N), need = cells * esize;
+  bool keep = c->kernel_mode == RTE_KERNEL_STORE || (c->kernel_mode == RTE_KERNEL_AUTO && (!f64 || need <= kSlabBytes));
+  if (keep && (f64 ? !c->d_K64 : !c->d_K)) {
     size_t fr = 0, tot = 0;
     CUDA_TRY(c, cudaMemGetInfo(&fr, &tot));
     if (need + (1ull << 30) > fr) {
       if (c->kernel_mode == RTE_KERNEL_STORE)
         return fail(c, RTE_ERR_NOMEM, "pair kernel needs %.1f GB, %.1f GB free", need / 1e9, fr / 1e9);
-      return RTE_OK;  // auto: recompute
+      keep = false;  // auto: recompute
+    } else if (f64) {
+      CUDA_TRY(c, dalloc(c, &c->d_K64, cells));
+    } else {
+      CUDA_TRY(c, dalloc(c, &c->d_K, cells));
     }
-    if (f64)
-      CUDA_TRY(c, dalloc(c, &c->d_K64, (size_t)c->N * ld));
-    else  // whole 128-destination blocks of ld source rows (kmat_index)
-      CUDA_TRY(c, dalloc(c, &c->d_K, ((size_t)c->N + RTE_KBLK - 1) / RTE_KBLK * RTE_KBLK * ld));
-    c->Kld = ld;
+  }
+  if (!keep) {
+    const int ncol = c->nx * c->ny;
+    const size_t per_col = kernel_cells(c, c->nz) * esize;
+    int cols = (int)std::max<size_t>(1, std::min<size_t>(ncol, kSlabBytes / per_col));
+    if (cols > c->nx && cols < ncol) cols = cols / c->nx * c->nx;  // whole rows of columns
+    const size_t bytes = per_col * cols;
+    if (bytes > c->slab_bytes) {
+      if (c->capturing) return fail(c, RTE_ERR_STATE, "the kernel workspace must exist before a graph is recorded");
+      if (c->d_slab) {
+        cudaFree(c->d_slab);
+        c->bytes -= c->slab_bytes;
+        c->d_slab = nullptr;
+        c->slab_bytes = 0;
+      }
+      unsigned char* m = nullptr;
+      CUDA_TRY(c, dalloc(c, &m, bytes));
+      c->d_slab = m;
+      c->slab_bytes = bytes;
+    }
+    c->slab_cols = cols;
+    return RTE_OK;
   }
   if (!c->K_valid || c->capture_store) {
-    PairArgs a;
-    memset(&a, 0, sizeof a);
-    a.N = c->N;
-    a.nx = c->nx;
-    a.ny = c->ny;
-    a.nz = c->nz;
-    a.Cfull = c->C;
-    a.dx = c->dx;
-    a.dy = c->dy;
-    a.dz = c->dz;
-    a.prop_thresh = c->prop_thresh;
-    a.kscale = c->dV / c->cm;
-    a.perm = c->d_perm;
-    a.mut = c->d_mut;
-    a.mutf = c->d_mutf;
-    a.Kmat = c->d_K;
-    a.Kmat64 = c->d_K64;
-    a.Kld = c->Kld;
+    const StoreArgs a = store_args(c, f64 ? (void*)c->d_K64 : (void*)c->d_K, c->N, 0, c->nx * c->ny);
     if (c->capturing) {
       CUDA_TRY(c, rte_launch_store_kernel(a, c->st, f64 ? 1 : 0));
     } else {
@@ -932,102 +976,132 @@ static int ensure_pair_kernel(rte_ctx* c, bool* stored) {
   return RTE_OK;
 }
 
-// Split-K plan: the number of source chunks S so that tiles x S CTAs fill whole waves of the
-// kernel's resident CTAs (a partial last wave idles SMs).
 static int check_kernel_err(rte_ctx* c);
-
-// Pair-kernel arguments for nb right-hand sides split S ways (chunk sources per split).
-static PairArgs pair_args(const rte_ctx* c, const double* in64, const float* in32, int nb, int S, int chunk) {
-  PairArgs a;
-  memset(&a, 0, sizeof a);
-  a.N = c->N;
-  a.nx = c->nx;
-  a.ny = c->ny;
-  a.nz = c->nz;
-  a.Cfull = c->C;
-  a.dx = c->dx;
-  a.dy = c->dy;
-  a.dz = c->dz;
-  a.prop_thresh = c->prop_thresh;
-  a.kscale = c->dV / c->cm;
-  a.perm = c->d_perm;
-  a.mut = c->d_mut;
-  a.mutf = c->d_mutf;
-  a.Win = in64;
-  a.Winf = in32;
-  a.Kmat = c->d_K;
-  a.Kmat64 = c->d_K64;
-  a.Kld = c->Kld;
-  a.part = c->d_part;
-  a.partf = reinterpret_cast<float*>(c->d_part);
-  a.chunk = chunk;
-  a.nsplit = S;
-  a.nb = nb;
-  a.slot_xyz = c->d_slot_xyz;
-  a.cstride = (c->C + 3) / 4 * 4;
-  a.cpad = (nb * a.cstride + 3) / 4 * 4;
-  a.err = c->d_err;
-  a.kappa = c->kappa;
-  a.transpose = c->transpose ? 1 : 0;
-  return a;
-}
 
 static inline int split_chunk(int N, int S) {
   return ((N + S - 1) / S + RTE_PAIR_TS - 1) / RTE_PAIR_TS * RTE_PAIR_TS;
 }
 
-// Split-K autotuner.  The pair kernel's grid is (destination tiles) x S source chunks; the best S
-// balances wave quantisation on the 148 SMs against the partial-sum traffic of the epilogue and
-// depends on N, the order, the right-hand-side count and the kernel variant.  Candidates are the
-// splits whose occupancy-model wave fill is within 25% of the best; each is launched on the
-// context's own buffers and timed with CUDA events (best of two), and the winner is kept for the
-// process (every context of that shape on that device reuses it).  RTE_AUTOTUNE=0 keeps the
-// occupancy model's choice; RTE_NSPLIT forces a split.
+// Angle rows of the column kernels in the context's precision (and for the transposed table model).
+static int ensure_col_table(rte_ctx* c) {
+  const int f = c->precision == RTE_PREC_FP64 ? 1 : 0, tr = c->transpose ? 1 : 0;
+  void** p = &c->d_tab[f][tr];
+  if (*p && c->tab_kappa[f][tr] == c->kappa) return RTE_OK;
+  if (c->capturing) return fail(c, RTE_ERR_STATE, "angle rows must exist before a graph is recorded");
+  const ColDims d = col_dims(c);
+  const size_t esize = f ? sizeof(double) : sizeof(float);
+  if (!*p) {  // room for the phases of a modulated context
+    const size_t row = rte_col_dims(c->C, c->L, c->nz, f, 1).row;
+    unsigned char* m = nullptr;
+    CUDA_TRY(c, dalloc(c, &m, (size_t)(2 * c->nx - 1) * (2 * c->ny - 1) * row * esize));
+    *p = m;
+  }
+  ColTabArgs a;
+  memset(&a, 0, sizeof a);
+  a.nx = c->nx;
+  a.ny = c->ny;
+  a.nz = c->nz;
+  a.nzp = d.nzp;
+  a.L = c->L;
+  a.dx = c->dx;
+  a.dy = c->dy;
+  a.dz = c->dz;
+  a.kappa = c->kappa;
+  a.table = c->model == RTE_MODEL_FIM ? 1 : 0;
+  a.transpose = tr;
+  a.row = d.row;
+  a.azn = d.azn;
+  a.csn = d.csn;
+  a.nk = d.nk;
+  a.pho = d.pho;
+  a.tg = d.tg;
+  a.cls = d.cls;
+  CUDA_TRY(c, (c->launches++, rte_launch_col_table(a, *p, f, c->st)));
+  c->tab_kappa[f][tr] = c->kappa;
+  return RTE_OK;
+}
+
+// Column-kernel arguments for nb right-hand sides: source columns [col0, col1) in chunks, pair-kernel rows K from
+// column col0 (ld source rows), chunk sums from slice split0.
+static ColArgs col_args(const rte_ctx* c, int nb, const void* K, size_t ld, int col0, int col1, int chunk, int split0) {
+  ColArgs a;
+  memset(&a, 0, sizeof a);
+  const int f = c->precision == RTE_PREC_FP64 ? 1 : 0;
+  const ColDims d = col_dims(c);
+  a.N = c->N;
+  a.nx = c->nx;
+  a.ny = c->ny;
+  a.nz = c->nz;
+  a.Cfull = c->C;
+  a.nzp = d.nzp;
+  a.group = d.group;
+  a.nrhs = c->kappa != 0.0 ? nb / 2 : nb;
+  a.W = nb == 1 ? c->d_Wf : c->d_bWf;
+  a.pitch = d.pitch;
+  a.K = K;
+  a.Kld = ld;
+  a.kslot0 = col0 * c->nz;
+  a.tab = c->d_tab[f][c->transpose ? 1 : 0];
+  a.row = d.row;
+  a.azn = d.azn;
+  a.csn = d.csn;
+  a.cls = d.cls;
+  a.pho = d.pho;
+  a.part = c->d_part;
+  a.vstride = nb * c->C;
+  a.col0 = col0;
+  a.col1 = col1;
+  a.chunk = chunk;
+  a.nsplit = (col1 - col0 + chunk - 1) / chunk;
+  a.split0 = split0;
+  a.err = c->d_err;
+  return a;
+}
+
+static cudaError_t launch_columns(const rte_ctx* c, const ColArgs& a, int LA) {
+  return rte_launch_column(a, LA, c->precision == RTE_PREC_FP64 ? 1 : 0, c->kappa != 0.0 ? 1 : 0, c->st);
+}
+
+// Launch-plan autotuner of the column kernels.  The grid is (tiles of 128 threads' destinations x right-hand
+// sides) x (chunks of source columns); more chunks fill the SMs' last wave better and cost chunk sums.
+// Candidates are the chunk sizes that a model of waves and chunk-sum traffic ranks best; in mixed precision on
+// 4096 voxels and more each is launched on the context's own buffers and timed with CUDA events (best of two),
+// and the fastest is kept for the process (every context of that shape on that device reuses it).
+// RTE_AUTOTUNE=0 keeps the model's choice; RTE_NSPLIT forces a split.
 namespace {
-using TuneKey = std::tuple<int, int, int, int, int, int, int>;  // device, N, LA, stored, nb, precision, table
+using TuneKey = std::tuple<int, int, int, int, int, int, int, int, int>;  // device, grid, LA, nb, precision, cplx, columns
 std::mutex g_tune_mu;
-std::map<TuneKey, std::pair<int, int>> g_tuned;  // (S, tile)
-struct Plan {
-  double fill;  // wave fill of the occupancy model
-  int S, tile;
-};
+std::map<TuneKey, int> g_tuned;  // source columns per chunk
 }  // namespace
 
-// Launch-plan autotuner: each candidate (split S, source tile) is launched on the context's own buffers
-// and timed with CUDA events (best of two); the fastest is kept for the process.
-static int tune_split(rte_ctx* c, int LA, int stored, int nb, const std::vector<Plan>& cands, int* S_best,
-                      int* tile_best) {
-  const int table = c->model == RTE_MODEL_FIM ? 1 : 0;
-  const double* in64 = nb == 1 ? c->d_W : c->d_bW;
-  const float* in32 = nb == 1 ? c->d_Wf : c->d_bWf;
-  if (!in64 || (c->precision == RTE_PREC_MIXED && !in32)) return RTE_OK;
+static int tune_chunk(rte_ctx* c, int LA, int nb, const void* K, size_t ld, int cols, const std::vector<int>& cands,
+                      double part_us, int* best_chunk) {
   cudaEvent_t e0, e1;
   CUDA_TRY(c, cudaEventCreate(&e0));
   CUDA_TRY(c, cudaEventCreate(&e1));
-  double best = 1e30;
+  float best = 1e30f;
   cudaError_t err = cudaSuccess;
   // each launch is checked with cudaGetLastError: clear what an earlier call of this thread left there
   // (a failure handled where it happened, or one inside a library), so it is not read as a launch's
   (void)cudaGetLastError();
-  for (const auto& cand : cands) {
-    PairArgs a = pair_args(c, in64, in32, nb, cand.S, split_chunk(c->N, cand.S));
-    a.tile = cand.tile;
+  for (int chunk : cands) {
+    const ColArgs a = col_args(c, nb, K, ld, 0, cols, chunk, 0);
     float t = 1e30f;
     for (int rep = 0; rep < 2 && err == cudaSuccess; rep++) {
       cudaEventRecord(e0, c->st);
-      err = rte_launch_pair(a, LA, c->precision, table, stored, c->st);
+      err = launch_columns(c, a, LA);
       cudaEventRecord(e1, c->st);
       if (err == cudaSuccess) err = cudaEventSynchronize(e1);
       float ms = 0;
       if (err == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
-      if (rep == 1 || cands.size() == 1) t = std::min(t, ms);
+      if (rep == 1) t = ms;
     }
     c->launches += 2;
     if (err != cudaSuccess) break;
+    t += (float)(a.nsplit * part_us * 1e-3);  // the chunk sums' share of the epilogue
     if (t < best) {
       best = t;
-      *S_best = cand.S;
-      *tile_best = cand.tile;
+      *best_chunk = chunk;
     }
   }
   cudaEventDestroy(e0);
@@ -1036,122 +1110,129 @@ static int tune_split(rte_ctx* c, int LA, int stored, int nb, const std::vector<
   return check_kernel_err(c);
 }
 
-// The tile-staged stored-kernel launch (mixed precision, exact directions, real right-hand sides: see
-// k_pair_mixed_tk) keeps each CTA's FP32 sums in registers over its whole source chunk; chunks of at most
-// kTkChunk sources keep those sums short (the epilogue adds the chunks in FP64): 33^3 L=5 error against
-// FP64 3.9e-6 with chunks of ~4,500 sources, see the bench line's fp64_rel_err for the capped chunks.
-static const int kTkChunk = 1024;
-static bool tk_kernel(const rte_ctx* c, int stored, int cplx) {
-  return c->precision == RTE_PREC_MIXED && stored && c->model != RTE_MODEL_FIM && !cplx;
-}
-// The recomputed four-right-hand-side kernel at L >= 6 (k_pair_mixed_grp: two thread groups sharing the
-// path walks) leaves FP32 chunk sums as well.
-static bool grp_kernel(const rte_ctx* c, int stored, int cplx, int nb, int LA) {
-  return c->precision == RTE_PREC_MIXED && !stored && c->model != RTE_MODEL_FIM && !cplx && nb == 4 && LA >= 6;
-}
+// The FP32 sums of a chunk are sums over one column of sources at a time, added over at most this many columns
+// (the epilogue adds the chunks in FP64).
+static const int kChunkColumns = 128;
 
 template <class T>
 static int grow(rte_ctx* c, T** p, size_t& cap, size_t n);
 
-static int plan_split(rte_ctx* c, int LA, int stored, int nb, int* S_out, int* chunk_out, int* tile_out = nullptr) {
-  const int cplx = c->kappa != 0.0 ? 1 : 0;
-  const int key = (((LA * 2 + stored) * 8 + nb) * 2 + (c->precision == RTE_PREC_MIXED ? 1 : 0)) * 2 + cplx;
+// Chunk size for launches over `cols` source columns of K (ld rows); total: the chunk sums of one application.
+static int plan_columns(rte_ctx* c, int LA, int nb, const void* K, size_t ld, int cols, int* chunk_out, int* total_out) {
+  const int cplx = c->kappa != 0.0 ? 1 : 0, f = c->precision == RTE_PREC_FP64 ? 1 : 0;
+  int rc = ensure_col_table(c);
+  if (rc) return rc;
+  const int ncol = c->nx * c->ny;
+  auto total = [&](int chunk) {  // slices over all slabs of `cols` columns
+    const int full = ncol / cols, rest = ncol % cols;
+    return full * ((cols + chunk - 1) / chunk) + (rest + chunk - 1) / chunk;
+  };
+  const int key = (((LA * 8 + nb) * 2 + f) * 2 + cplx) * 2 + (cols == ncol ? 1 : 0);
   for (auto& e : c->splits)
-    if (e[0] == key) {
-      *S_out = e[1];
+    if (e[0] == key && e[1] == cols) {
       *chunk_out = e[2];
-      if (tile_out) *tile_out = e[3];
+      *total_out = total(e[2]);
       return RTE_OK;
     }
-  const int table = c->model == RTE_MODEL_FIM ? 1 : 0;
-  const int cpad = (nb * ((c->C + 3) / 4 * 4) + 3) / 4 * 4;
-  int sms = 0;
+  int sms = 0, occ = 0;
   CUDA_TRY(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
-  const int tiles = (c->N + RTE_PAIR_THREADS - 1) / RTE_PAIR_THREADS;
-  const bool tk = tk_kernel(c, stored, cplx);
-  const bool chunked = tk || grp_kernel(c, stored, cplx, nb, LA);  // FP32 chunk sums, chunks capped
-  const int Smin = chunked ? (c->N + kTkChunk - 1) / kTkChunk : 1;
-  const int Smax = chunked ? Smin + c->max_split : c->max_split;
-  if (chunked) {  // partial sums of Smax chunks (before any capture: plan_split runs ahead of graph recording)
-    int rc = grow(c, &c->d_part, c->part_cap, (size_t)c->N * c->C * nb * Smax);
-    if (rc) return rc;
+  CUDA_TRY(c, rte_launch_column(col_args(c, nb, K, ld, 0, cols, cols, 0), LA, f, cplx, c->st, &occ));
+  const ColDims d = col_dims(c);
+  const int rhs = cplx ? nb / 2 : nb, group = cplx ? 1 : d.group;
+  const long long tiles = (long long)((ncol * d.nzp + 128 * group - 1) / (128 * group)) * rhs;
+  const long long slots = (long long)std::max(occ, 1) * sms;
+  const int cap = f ? cols : std::min(cols, kChunkColumns);
+  // a wave of resident CTAs takes (chunk + one column of start-up) x the SM's time per column at ~0.6 of the FMA
+  // rate; chunk sums are written and read once more each (us)
+  const double col_us = (f ? 2.0 : 1.0) * (cplx ? 2 : 1) * occ * (double)group * c->nz * (4 * LA + 15.0) / (1.9e3 * 0.6);
+  const double part_us = (double)c->N * c->C * nb * (f ? 8 : 4) * 2 / 5e6;
+  std::vector<std::pair<double, int>> rank;
+  for (int chunk = 1, last = 0; chunk <= cap; chunk++) {
+    const int S = (cols + chunk - 1) / chunk;
+    if (S == last) continue;  // the smallest chunk of each split count
+    last = S;
+    const double waves = ceil((double)tiles * S / (double)slots);
+    rank.push_back({waves * (chunk + 1) * col_us + S * part_us, chunk});
   }
-  // occupancy-model candidates: (wave fill, S, tile) for each source tile the kernel offers
-  std::vector<Plan> fills;
-  Plan model{-1.0, Smin, 0};
-  for (int tile = 0; tile < (tk ? 2 : 1); tile++) {
-    int occ = 0;
-    CUDA_TRY(c, rte_pair_occupancy(LA, c->precision, table, stored, nb, cpad, &occ, cplx, tile));
-    const long long slots = (long long)std::max(occ, 1) * sms;
-    double best = -1.0;
-    int bestS = Smin;
-    for (int S = Smin; S <= Smax; S++) {
-      const int Sreal = (c->N + split_chunk(c->N, S) - 1) / split_chunk(c->N, S);
-      if (Sreal != S) continue;
-      const double waves = (double)tiles * S / (double)slots;
-      const double eff = waves / ceil(waves);
-      fills.push_back({eff, S, tile});
-      // prefer the smallest S within 3% of the best fill, and at least one full wave when possible
-      if (eff > best + 0.03 || (best < 0.97 && eff > best)) {
-        best = eff;
-        bestS = S;
-      }
-    }
-    if (tile == 0) model = {best, bestS, 0};
-  }
-  int bestS = model.S, bestTile = 0;
+  std::sort(rank.begin(), rank.end());
+  if (rank.size() > 4) rank.resize(4);
+  int chunk = rank[0].second;
   const char* forced = getenv("RTE_NSPLIT");
   const char* at = getenv("RTE_AUTOTUNE");
-  const bool tune = !forced && !(at && at[0] == '0') && !c->capturing && c->precision == RTE_PREC_MIXED &&
-                    c->N >= 4096;
-  if (forced) {
-    bestS = std::max(Smin, std::min(Smax, atoi(forced)));
-  } else if (tune) {
-    const TuneKey tk_key{c->cfg.device, c->N, LA, stored, nb, c->precision, table + 2 * cplx};
-    bool have = false;
-    {
-      std::lock_guard<std::mutex> lk(g_tune_mu);
-      auto it = g_tuned.find(tk_key);
-      if (it != g_tuned.end() && it->second.first <= Smax && it->second.first >= Smin) {
-        bestS = it->second.first;
-        bestTile = it->second.second;
-        have = true;
-      }
-    }
-    if (!have) {
-      // per tile: the splits whose wave fill is within 25% of that tile's best, the four best of them
-      std::vector<Plan> cands;
-      for (int tile = 0; tile < (tk ? 2 : 1); tile++) {
-        double best = 0.0;
-        for (auto& f : fills)
-          if (f.tile == tile) best = std::max(best, f.fill);
-        std::vector<Plan> mine;
-        for (auto& f : fills)
-          if (f.tile == tile && f.fill >= 0.75 * best) mine.push_back(f);
-        std::sort(mine.begin(), mine.end(), [](const Plan& x, const Plan& y) {
-          return x.fill > y.fill || (x.fill == y.fill && x.S < y.S);
-        });
-        if (mine.size() > 4) mine.resize(4);
-        cands.insert(cands.end(), mine.begin(), mine.end());
-      }
-      int rc = tune_split(c, LA, stored, nb, cands, &bestS, &bestTile);
-      if (rc) return rc;
-      std::lock_guard<std::mutex> lk(g_tune_mu);
-      g_tuned[tk_key] = {bestS, bestTile};
+  const bool tune = !forced && !(at && at[0] == '0') && !c->capturing && !f && c->N >= 4096 && rank.size() > 1;
+  if (forced) chunk = std::max(1, std::min(cap, (cols + std::max(1, atoi(forced)) - 1) / std::max(1, atoi(forced))));
+  const TuneKey tk{c->cfg.device, c->nx, c->ny, c->nz, LA, nb, c->precision, cplx, cols};
+  bool have = false;
+  if (tune) {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    auto it = g_tuned.find(tk);
+    if (it != g_tuned.end()) {
+      chunk = it->second;
+      have = true;
     }
   }
-  const int chunk = split_chunk(c->N, bestS);
-  const int S = (c->N + chunk - 1) / chunk;
-  c->splits.push_back({key, S, chunk, bestTile});
-  *S_out = S;
+  int smax = total(chunk);
+  if (tune && !have)
+    for (auto& r : rank) smax = std::max(smax, (cols + r.second - 1) / r.second);
+  // chunk sums (before any capture: plans are made ahead of graph recording)
+  size_t cells = (size_t)c->N * c->C * nb * smax;
+  rc = grow(c, &c->d_part, c->part_cap, f ? cells : (cells + 1) / 2);
+  if (rc) return rc;
+  if (tune && !have) {
+    std::vector<int> cands;
+    for (auto& r : rank) cands.push_back(r.second);
+    rc = tune_chunk(c, LA, nb, K, ld, cols, cands, part_us / 2, &chunk);
+    if (rc) return rc;
+    {
+      std::lock_guard<std::mutex> lk(g_tune_mu);
+      g_tuned[tk] = chunk;
+    }
+    cells = (size_t)c->N * c->C * nb * total(chunk);
+    rc = grow(c, &c->d_part, c->part_cap, f ? cells : (cells + 1) / 2);
+    if (rc) return rc;
+  }
+  c->splits.push_back({key, cols, chunk});
   *chunk_out = chunk;
-  if (tile_out) *tile_out = bestTile;
+  *total_out = total(chunk);
   return RTE_OK;
 }
 
-// One term on the real basis for nb right-hand sides (layout [N][nb][C]): out = [D] A in.
-// in64 is FP64 (and in32 its FP32 copy for the mixed kernels).  sum != null accumulates the result;
-// d_red receives the norms.
+// Off-diagonal operator on the rows of rows_of(c, nb): chunk sums into d_part, *S of them.
+static int pair_term(rte_ctx* c, int LA, int nb, int* S) {
+  bool stored = false;
+  int rc = ensure_pair_kernel(c, &stored), chunk = 1;
+  if (rc) return rc;
+  const int f = c->precision == RTE_PREC_FP64 ? 1 : 0, ncol = c->nx * c->ny;
+  if (stored) {
+    const void* K = f ? (const void*)c->d_K64 : (const void*)c->d_K;
+    rc = plan_columns(c, LA, nb, K, c->N, ncol, &chunk, S);
+    if (rc) return rc;
+    ProfScope ps(c, 0);
+    CUDA_TRY(c, launch_columns(c, col_args(c, nb, K, c->N, 0, ncol, chunk, 0), LA));
+    return RTE_OK;
+  }
+  const int cols = c->slab_cols;
+  rc = plan_columns(c, LA, nb, c->d_slab, (size_t)cols * c->nz, cols, &chunk, S);
+  if (rc) return rc;
+  for (int c0 = 0, s0 = 0; c0 < ncol; c0 += cols) {
+    const int c1 = std::min(ncol, c0 + cols);
+    const size_t ld = (size_t)cols * c->nz;
+    {
+      ProfScope ps(c, 1);
+      CUDA_TRY(c, rte_launch_store_kernel(store_args(c, c->d_slab, ld, c0, c1), c->st, f));
+    }
+    ProfScope ps(c, 0);
+    const ColArgs a = col_args(c, nb, c->d_slab, ld, c0, c1, chunk, s0);
+    CUDA_TRY(c, launch_columns(c, a, LA));
+    s0 += a.nsplit;
+  }
+  return RTE_OK;
+}
+
+// One term on the real basis for nb right-hand sides (layout [N][nb][C]): out = [D] A in.  The pair kernels
+// read `in` as rows in slot order (rows_of): rows_ready says that they hold it already, keep_rows that they
+// are to hold `out` afterwards (the next term's input).  sum != null accumulates the result; d_red receives
+// the norms.
 static const int kMaxBatch = 4;  // right-hand sides of one batched solve
 
 // Uniform media in automatic kernel mode take the convolution path (rte_fft.cpp), outside graph
@@ -1184,11 +1265,13 @@ static int ensure_fft(rte_ctx* c) {
   return RTE_OK;
 }
 
-static int apply_term(rte_ctx* c, const double* in64, const float* in32, double* out, float* out32, double* sum,
-                      int flag, int flag_scat, int nb = 1) {
+static void* rows_of(const rte_ctx* c, int nb) { return nb == 1 ? c->d_Wf : c->d_bWf; }
+
+static int apply_term(rte_ctx* c, const double* in64, double* out, double* sum, int flag, int flag_scat, int nb = 1,
+                      bool rows_ready = false, bool keep_rows = false) {
   const int LA = flag ? c->L : 0;
-  int S = 1, chunk = c->N;
-  bool f32part = false;  // the tile-staged kernel leaves FP32 chunk sums
+  int S = 1;
+  bool f32part = false;  // FP32 chunk sums
   int rc;
   if (fft_active(c)) {
     rc = ensure_fft(c);
@@ -1196,18 +1279,12 @@ static int apply_term(rte_ctx* c, const double* in64, const float* in32, double*
     ProfScope ps(c, 0);
     CUDA_TRY(c, (c->launches += 5, rte_fft_apply(c->fft, in64, nb * c->C, c->C, LA, nb, c->d_part, c->st)));
   } else {
-    bool stored = false;
-    rc = ensure_pair_kernel(c, &stored);
+    if (!rows_ready)
+      CUDA_TRY(c, (c->launches++, rte_launch_rows(in64, rows_of(c, nb), c->d_islot, c->N, nb, col_dims(c).pitch, c->C,
+                                                  c->precision == RTE_PREC_FP64 ? 1 : 0, c->st)));
+    rc = pair_term(c, LA, nb, &S);
     if (rc) return rc;
-    int tile = 0;
-    rc = plan_split(c, LA, stored ? 1 : 0, nb, &S, &chunk, &tile);
-    if (rc) return rc;
-    PairArgs a = pair_args(c, in64, in32, nb, S, chunk);
-    a.tile = tile;
-    f32part = tk_kernel(c, stored ? 1 : 0, c->kappa != 0.0 ? 1 : 0) ||
-              grp_kernel(c, stored ? 1 : 0, c->kappa != 0.0 ? 1 : 0, nb, LA);
-    ProfScope ps(c, 0);
-    CUDA_TRY(c, rte_launch_pair(a, LA, c->precision, c->model == RTE_MODEL_FIM ? 1 : 0, stored ? 1 : 0, c->st));
+    f32part = c->precision == RTE_PREC_MIXED;
   }
   SelfArgs sa;
   memset(&sa, 0, sizeof sa);
@@ -1248,10 +1325,10 @@ static int apply_term(rte_ctx* c, const double* in64, const float* in32, double*
   e.flag_scat = flag_scat;
   scatter_factors(c, flag, e.scat);
   e.Wout = out;
-  e.Woutf = out32;
+  e.rows = keep_rows && !fft_active(c) ? rows_of(c, nb) : nullptr;
+  e.rows64 = c->precision == RTE_PREC_FP64 ? 1 : 0;
   e.islot = c->d_islot;
-  e.cstride = (c->C + 3) / 4 * 4;
-  e.cpad = (nb * e.cstride + 3) / 4 * 4;
+  e.pitch = col_dims(c).pitch;
   e.sum = sum;
   e.red = c->d_red;
   e.cplx = c->kappa != 0.0 ? 1 : 0;
@@ -1287,7 +1364,6 @@ static int neumann_real(rte_ctx* c, const double* W0, const double* S0, double* 
   double rel = 0.0;
   if (flag) {
     CUDA_TRY(c, cudaMemcpyAsync(c->d_W, W0, NC * sizeof(double), cudaMemcpyDeviceToDevice, c->st));
-    if (mixed) CUDA_TRY(c, (c->launches++, rte_launch_to_f32_slots(c->d_W, c->d_Wf, c->d_islot, c->N, c->C, c->cpad, c->C, c->cstride, c->st)));
     const int flag_l = c->cfg.g != 0.0 ? 1 : 0;  // neumann.cu:74-79
     const int rule = force_terms >= 0 ? RTE_STOP_FIXED : stop->rule;
     const int maxt = force_terms >= 0 ? force_terms : (rule == RTE_STOP_REFERENCE ? 10000 : stop->max_terms);
@@ -1320,7 +1396,7 @@ static int neumann_real(rte_ctx* c, const double* W0, const double* S0, double* 
         break;
       }
       n++;
-      int rc = apply_term(c, c->d_W, c->d_Wf, c->d_Wn, mixed ? c->d_Wf : nullptr, c->d_sum, flag_l, 1);
+      int rc = apply_term(c, c->d_W, c->d_Wn, c->d_sum, flag_l, 1, 1, terms > 0, true);
       if (rc) return rc;
       std::swap(c->d_W, c->d_Wn);
       terms++;
@@ -1333,12 +1409,7 @@ static int neumann_real(rte_ctx* c, const double* W0, const double* S0, double* 
     }
   }
   // final A on the running sum (no scatter), neumann.cu:95-118
-  float* in32 = nullptr;
-  if (mixed) {
-    CUDA_TRY(c, (c->launches++, rte_launch_to_f32_slots(c->d_sum, c->d_Wf, c->d_islot, c->N, c->C, c->cpad, c->C, c->cstride, c->st)));
-    in32 = c->d_Wf;
-  }
-  int rc = apply_term(c, c->d_sum, in32, res, nullptr, nullptr, 1, 0);
+  int rc = apply_term(c, c->d_sum, res, nullptr, 1, 0);
   if (rc) return rc;
   rc = check_kernel_err(c);
   if (rc) return rc;
@@ -1397,14 +1468,10 @@ static int download_pair(rte_ctx* c, const double* d_pair, rte_cplx* h) {
 // (row pairs); A * sum to d_bres.  Stop rules as neumann_real (the reference rule on the real parts
 // of the complex-basis layer sums, as StopIteration takes creal, Kernels_selfsub.c:1184-1220).
 static int neumann_cplx(rte_ctx* c, int flag, const rte_stop* stop, int* nterms, double* last_rel) {
-  const int vs = 2 * c->C, cp = (2 * c->cstride + 3) / 4 * 4;
   const bool mixed = c->precision == RTE_PREC_MIXED;
   int terms = 0;
   double rel = 0.0;
   if (flag) {
-    if (mixed)
-      CUDA_TRY(c, (c->launches++, rte_launch_to_f32_slots(c->d_bW, c->d_bWf, c->d_islot, c->N, vs, cp, c->C,
-                                                          c->cstride, c->st)));
     const int flag_l = c->cfg.g != 0.0 ? 1 : 0;
     const int rule = stop->rule;
     const int maxt = rule == RTE_STOP_REFERENCE ? 10000 : stop->max_terms;
@@ -1437,7 +1504,7 @@ static int neumann_cplx(rte_ctx* c, int flag, const rte_stop* stop, int* nterms,
         break;
       }
       n++;
-      int rc = apply_term(c, c->d_bW, c->d_bWf, c->d_bWn, mixed ? c->d_bWf : nullptr, c->d_bsum, flag_l, 1, 2);
+      int rc = apply_term(c, c->d_bW, c->d_bWn, c->d_bsum, flag_l, 1, 2, terms > 0, true);
       if (rc) return rc;
       std::swap(c->d_bW, c->d_bWn);
       terms++;
@@ -1449,10 +1516,7 @@ static int neumann_cplx(rte_ctx* c, int flag, const rte_stop* stop, int* nterms,
       }
     }
   }
-  if (mixed)
-    CUDA_TRY(c, (c->launches++, rte_launch_to_f32_slots(c->d_bsum, c->d_bWf, c->d_islot, c->N, vs, cp, c->C,
-                                                        c->cstride, c->st)));
-  int rc = apply_term(c, c->d_bsum, c->d_bWf, c->d_bres, nullptr, nullptr, 1, 0, 2);
+  int rc = apply_term(c, c->d_bsum, c->d_bres, nullptr, 1, 0, 2);
   if (!rc) rc = check_kernel_err(c);
   if (rc) return rc;
   if (nterms) *nterms = terms;
@@ -1506,10 +1570,7 @@ extern "C" int rte_prop_abs(rte_ctx* c, const rte_cplx* in, rte_cplx* out, int f
     int rc = ensure_batch(c, 2);
     if (!rc) rc = upload_pair(c, in, c->d_bW);
     if (rc) return rc;
-    if (c->precision == RTE_PREC_MIXED)
-      CUDA_TRY(c, (c->launches++, rte_launch_to_f32_slots(c->d_bW, c->d_bWf, c->d_islot, c->N, 2 * c->C,
-                                                          (2 * c->cstride + 3) / 4 * 4, c->C, c->cstride, c->st)));
-    rc = apply_term(c, c->d_bW, c->d_bWf, c->d_bres, nullptr, nullptr, flag, flag_scat, 2);
+    rc = apply_term(c, c->d_bW, c->d_bres, nullptr, flag, flag_scat, 2);
     if (!rc) rc = check_kernel_err(c);
     if (rc) return rc;
     return download_pair(c, c->d_bres, out);
@@ -1520,12 +1581,10 @@ extern "C" int rte_prop_abs(rte_ctx* c, const rte_cplx* in, rte_cplx* out, int f
   const size_t NC = (size_t)c->N * c->C;
   const bool mixed = c->precision == RTE_PREC_MIXED;
   // part 1 -> d_W, part 2 -> d_sum (both scratch here)
-  if (mixed) CUDA_TRY(c, (c->launches++, rte_launch_to_f32_slots(c->d_aux1, c->d_Wf, c->d_islot, c->N, c->C, c->cpad, c->C, c->cstride, c->st)));
-  rc = apply_term(c, c->d_aux1, c->d_Wf, c->d_W, nullptr, nullptr, flag, flag_scat);
+  rc = apply_term(c, c->d_aux1, c->d_W, nullptr, flag, flag_scat);
   if (rc) return rc;
   if (has2) {
-    if (mixed) CUDA_TRY(c, (c->launches++, rte_launch_to_f32_slots(c->d_aux2, c->d_Wf, c->d_islot, c->N, c->C, c->cpad, c->C, c->cstride, c->st)));
-    rc = apply_term(c, c->d_aux2, c->d_Wf, c->d_sum, nullptr, nullptr, flag, flag_scat);
+    rc = apply_term(c, c->d_aux2, c->d_sum, nullptr, flag, flag_scat);
     if (rc) return rc;
   }
   rc = check_kernel_err(c);
@@ -1548,11 +1607,8 @@ extern "C" int rte_prop_abs_adjoint(rte_ctx* c, const rte_cplx* in, rte_cplx* ou
   double* res[2] = {c->d_W, c->d_sum};
   for (int k = 0; k < (has2 ? 2 : 1) && !rc; k++) {
     if (!table) CUDA_TRY(c, (c->launches++, rte_launch_parity(parts[k], c->N, c->L, c->C, c->st)));
-    if (mixed)
-      CUDA_TRY(c, (c->launches++, rte_launch_to_f32_slots(parts[k], c->d_Wf, c->d_islot, c->N, c->C, c->cpad, c->C,
-                                                          c->cstride, c->st)));
     c->transpose = table;
-    rc = apply_term(c, parts[k], c->d_Wf, res[k], nullptr, nullptr, flag, 0);
+    rc = apply_term(c, parts[k], res[k], nullptr, flag, 0);
     c->transpose = false;
     if (!rc && !table) CUDA_TRY(c, (c->launches++, rte_launch_parity(res[k], c->N, c->L, c->C, c->st)));
   }
@@ -1871,16 +1927,13 @@ extern "C" int rte_images(rte_ctx* c, const rte_cplx* out, const rte_source* s, 
 // First term and initial running sum of the series for beams (xi) and point sources (q):
 // W0 = xi + D A q, S0 = xi + q + D A q (the point's uncollided field enters through the final A).
 // xi (in d_xi) becomes S0; W0 goes to d_w0.  nb right-hand sides interleaved ([N][nb][C]).
-static int series_start(rte_ctx* c, double* d_xi, double* d_q, double* d_w0, int nb, float* d_f32, int cpad) {
+static int series_start(rte_ctx* c, double* d_xi, double* d_q, double* d_w0, int nb) {
   const size_t n = (size_t)c->N * nb * c->C;
   if (!c->has_point) {
     CUDA_TRY(c, cudaMemcpyAsync(d_w0, d_xi, n * sizeof(double), cudaMemcpyDeviceToDevice, c->st));
     return RTE_OK;
   }
-  if (c->precision == RTE_PREC_MIXED)
-    CUDA_TRY(c, (c->launches++, rte_launch_to_f32_slots(d_q, d_f32, c->d_islot, c->N, nb * c->C, cpad, c->C,
-                                                        c->cstride, c->st)));
-  int rc = apply_term(c, d_q, d_f32, d_w0, nullptr, nullptr, 1, 1, nb);
+  int rc = apply_term(c, d_q, d_w0, nullptr, 1, 1, nb);
   if (rc) return rc;
   CUDA_TRY(c, (c->launches++, rte_launch_axpy(d_w0, d_xi, 1.0, n, c->st)));  // W0 = xi + DAq
   CUDA_TRY(c, cudaMemcpyAsync(d_xi, d_w0, n * sizeof(double), cudaMemcpyDeviceToDevice, c->st));
@@ -1901,7 +1954,7 @@ static int forward_cplx(rte_ctx* c, const rte_source* s, const rte_stop* stop, r
   c->has_point = false;
   rc = launch_source(c, s, c->d_bsum, 2 * c->C, c->d_bball, false, c->d_bq, c->d_bball + npix);
   // W0 -> d_bW, S0 -> d_bsum
-  if (!rc) rc = series_start(c, c->d_bsum, c->d_bq, c->d_bW, 2, c->d_bWf, (2 * c->cstride + 3) / 4 * 4);
+  if (!rc) rc = series_start(c, c->d_bsum, c->d_bq, c->d_bW, 2);
   if (!rc) rc = neumann_cplx(c, 1, stop, terms, rel);
   if (!rc && (trans || ref))
     rc = run_images(c, c->d_bres, s, true, trans, ref, 2 * c->C, c->d_bball, c->d_bres + c->C, c->d_bball + npix);
@@ -1953,7 +2006,7 @@ extern "C" int rte_forward(rte_ctx* c, const rte_source* s, const rte_stop* stop
   int rc = RTE_OK;
   if (s->kind == RTE_SRC_POINT) CUDA_TRY(c, cudaMemsetAsync(c->d_q, 0, (size_t)c->N * c->C * sizeof(double), c->st));
   rc = launch_source(c, s, c->d_aux1, 0, nullptr, true, c->d_q);
-  if (!rc) rc = series_start(c, c->d_aux1, c->d_q, c->d_aux3, 1, c->d_Wf, c->cpad);
+  if (!rc) rc = series_start(c, c->d_aux1, c->d_q, c->d_aux3, 1);
   if (!rc) rc = neumann_real(c, c->d_aux3, c->d_aux1, c->d_aux2, 1, stop, -1, &terms, &rel);
   if (!rc && (trans || ref)) rc = run_images(c, c->d_aux2, s, true, trans, ref);
   if (!rc) CUDA_TRY(c, cudaEventRecord(t1, c->st));
@@ -2088,9 +2141,14 @@ static int ensure_batch(rte_ctx* c, int nb) {
   CUDA_TRY(c, dalloc(c, &c->d_bq, NC * nb));
   if (c->d_bWf) cudaFree(c->d_bWf);
   c->d_bWf = nullptr;
-  const int cp = (nb * c->cstride + 3) / 4 * 4;
-  CUDA_TRY(c, dalloc(c, &c->d_bWf, (size_t)c->N * cp));
-  CUDA_TRY(c, cudaMemset(c->d_bWf, 0, sizeof(float) * (size_t)c->N * cp));
+  {  // FP32 rows of nb right-hand sides, or FP64 rows of a complex pair
+    const size_t pf = nb * rte_col_dims(c->C, c->L, c->nz, 0, 0).pitch * sizeof(float),
+                 pd = 2 * rte_col_dims(c->C, c->L, c->nz, 1, 0).pitch * sizeof(double);
+    unsigned char* rows = nullptr;
+    CUDA_TRY(c, dalloc(c, &rows, (size_t)c->N * std::max(pf, pd)));
+    c->d_bWf = rows;
+    CUDA_TRY(c, cudaMemset(c->d_bWf, 0, (size_t)c->N * std::max(pf, pd)));
+  }
   c->bcap = nb;
   return RTE_OK;
 }
@@ -2100,13 +2158,11 @@ static int ensure_batch(rte_ctx* c, int nb) {
 // right-hand sides).
 static int series_batch(rte_ctx* c, int nb, const rte_stop* stop, int* terms_out, double* rel_out) {
   const int vs = nb * c->C;
-  const int cp = (nb * c->cstride + 3) / 4 * 4;
-  CUDA_TRY(c, (c->launches++, rte_launch_to_f32_slots(c->d_bW, c->d_bWf, c->d_islot, c->N, vs, cp, c->C, c->cstride, c->st)));
   const int flag_l = c->cfg.g != 0.0 ? 1 : 0;
   int terms = 0;
   double rel = 0.0;
   while (terms < stop->max_terms) {
-    int rc = apply_term(c, c->d_bW, c->d_bWf, c->d_bWn, c->d_bWf, c->d_bsum, flag_l, 1, nb);
+    int rc = apply_term(c, c->d_bW, c->d_bWn, c->d_bsum, flag_l, 1, nb, terms > 0, true);
     if (rc) return rc;
     std::swap(c->d_bW, c->d_bWn);
     terms++;
@@ -2118,8 +2174,7 @@ static int series_batch(rte_ctx* c, int nb, const rte_stop* stop, int* terms_out
       if (rel < stop->tol) break;
     }
   }
-  CUDA_TRY(c, (c->launches++, rte_launch_to_f32_slots(c->d_bsum, c->d_bWf, c->d_islot, c->N, vs, cp, c->C, c->cstride, c->st)));
-  int rc = apply_term(c, c->d_bsum, c->d_bWf, c->d_bres, nullptr, nullptr, 1, 0, nb);
+  int rc = apply_term(c, c->d_bsum, c->d_bres, nullptr, 1, 0, nb);
   if (!rc) rc = check_kernel_err(c);
   if (terms_out) *terms_out = terms;
   if (rel_out) *rel_out = rel;
@@ -2134,23 +2189,6 @@ extern "C" int rte_forward_batch(rte_ctx* c, int nsrc, const rte_source* srcs, c
   if (stop->rule == RTE_STOP_REFERENCE)
     return fail(c, RTE_ERR_UNSUPPORTED, "batched solves take a fixed or relative-L2 stop rule");
   const size_t NC = (size_t)c->N * c->C, np = (size_t)c->nx * c->ny;
-  // four right-hand sides of 49-64 coefficients exceed one thread's registers: at L >= 6 the recomputed
-  // path integrals take k_pair_mixed_grp (two thread groups of two sharing the walks), the other forms
-  // run two batches of two
-  const bool grp = c->kernel_mode == RTE_KERNEL_RECOMPUTE && c->model != RTE_MODEL_FIM && c->kappa == 0.0;
-  if (c->L >= 6 && nsrc > 2 && c->precision == RTE_PREC_MIXED && !grp) {
-    rte_report r1, r2;
-    int rc = rte_forward_batch(c, 2, srcs, stop, W_out, trans, ref, &r1);
-    if (!rc)
-      rc = rte_forward_batch(c, nsrc - 2, srcs + 2, stop, W_out ? W_out + 2 * NC : nullptr, trans ? trans + 2 * np : nullptr,
-                             ref ? ref + 2 * np : nullptr, &r2);
-    if (rc) return rc;
-    if (rep) {
-      *rep = r2;
-      rep->ms_device = r1.ms_device + r2.ms_device;
-    }
-    return RTE_OK;
-  }
   bool modulated = c->kappa != 0.0;
   for (int b = 0; b < nsrc; b++) modulated = modulated || srcs[b].modulation != 0.0;
   if (c->precision != RTE_PREC_MIXED || nsrc == 1 || modulated) {  // one source at a time
@@ -2173,7 +2211,6 @@ extern "C" int rte_forward_batch(rte_ctx* c, int nsrc, const rte_source* srcs, c
   int rc = ensure_batch(c, nb);
   if (rc) return rc;
   const int vs = nb * c->C;
-  const int cp = (nb * c->cstride + 3) / 4 * 4;
   cudaEvent_t t0, t1;
   CUDA_TRY(c, cudaEventCreate(&t0));
   CUDA_TRY(c, cudaEventCreate(&t1));
@@ -2187,7 +2224,7 @@ extern "C" int rte_forward_batch(rte_ctx* c, int nsrc, const rte_source* srcs, c
     rc = launch_source(c, &srcs[b], c->d_bsum + b * c->C, vs, c->d_bball + b * npix, false, c->d_bq + b * c->C);
   if (rc) return rc;
   // W0 -> d_bW, S0 -> d_bsum
-  rc = series_start(c, c->d_bsum, c->d_bq, c->d_bW, nb, c->d_bWf, cp);
+  rc = series_start(c, c->d_bsum, c->d_bq, c->d_bW, nb);
   if (rc) return rc;
   int terms = 0;
   double rel = 0.0;
@@ -2351,7 +2388,7 @@ static int forward_with_flux(rte_ctx* c, const rte_source* s, const rte_stop* st
   c->has_point = false;
   if (s->kind == RTE_SRC_POINT) CUDA_TRY(c, cudaMemsetAsync(c->d_q, 0, NC * sizeof(double), c->st));
   int rc = launch_source(c, s, c->d_aux1, 0, nullptr, true, c->d_q);
-  if (!rc) rc = series_start(c, c->d_aux1, c->d_q, c->d_aux3, 1, c->d_Wf, c->cpad);
+  if (!rc) rc = series_start(c, c->d_aux1, c->d_q, c->d_aux3, 1);
   if (rc) return rc;
   rc = neumann_real(c, c->d_aux3, c->d_aux1, c->d_out, 1, stop, -1, terms, nullptr);
   if (rc) return rc;
@@ -2434,7 +2471,9 @@ static BpArgs bp_args(rte_ctx* c, bool accumulate) {
   bp.S = c->d_S;
   bp.Kmat = c->K_valid && c->d_K ? c->d_K : nullptr;
   bp.Kmat64 = c->K_valid && c->d_K64 ? c->d_K64 : nullptr;
-  bp.Kld = ((size_t)c->N + 31) / 32 * 32;
+  bp.Kld = c->N;
+  bp.nzp = col_dims(c).nzp;
+  bp.group = col_dims(c).group;
   bp.g = c->d_gt;
   bp.Q = c->d_Qbp;
   bp.accumulate = accumulate ? 1 : 0;
@@ -2472,11 +2511,8 @@ static int adjoint_series(rte_ctx* c, const rte_stop* stop, int terms) {
   const bool table = c->model == RTE_MODEL_FIM;
   CUDA_TRY(c, cudaMemcpyAsync(c->d_aux3, c->d_e, NC * sizeof(double), cudaMemcpyDeviceToDevice, c->st));
   if (!table) CUDA_TRY(c, (c->launches++, rte_launch_parity(c->d_aux3, c->N, c->L, c->C, c->st)));
-  if (c->precision == RTE_PREC_MIXED)
-    CUDA_TRY(c, (c->launches++, rte_launch_to_f32_slots(c->d_aux3, c->d_Wf, c->d_islot, c->N, c->C, c->cpad, c->C,
-                                                        c->cstride, c->st)));
   c->transpose = table;
-  int rc = apply_term(c, c->d_aux3, c->d_Wf, c->d_aux4, nullptr, nullptr, 1, 1);
+  int rc = apply_term(c, c->d_aux3, c->d_aux4, nullptr, 1, 1);
   if (!rc) {
     CUDA_TRY(c, (c->launches++, rte_launch_axpy(c->d_aux3, c->d_aux4, 1.0, NC, c->st)));
     rc = neumann_real(c, c->d_aux4, c->d_aux3, c->d_lam, 1, stop, std::max(terms - 1, 0), nullptr, nullptr);
@@ -2702,7 +2738,7 @@ extern "C" int rte_image_gradient(rte_ctx* c, const rte_source* s, const rte_sto
   if (s->kind == RTE_SRC_CPU) {  // several columns: the flux path takes single-column sources
     c->has_point = false;
     rc = launch_source(c, s, c->d_aux1, 0, nullptr, true, c->d_q);
-    if (!rc) rc = series_start(c, c->d_aux1, c->d_q, c->d_aux3, 1, c->d_Wf, c->cpad);
+    if (!rc) rc = series_start(c, c->d_aux1, c->d_q, c->d_aux3, 1);
     if (!rc) rc = neumann_real(c, c->d_aux3, c->d_aux1, c->d_out, 1, stop, -1, &terms, nullptr);
     if (!rc) CUDA_TRY(c, cudaMemcpyAsync(c->d_S, c->d_sum, NC * sizeof(double), cudaMemcpyDeviceToDevice, c->st));
   } else {
@@ -2770,10 +2806,10 @@ static std::vector<uintptr_t> graph_signature(const rte_ctx* c, int nb) {
   const double* W = nb == 1 ? c->d_W : c->d_bW;
   const double* Wn = nb == 1 ? c->d_Wn : c->d_bWn;
   return {u(std::min(W, Wn)), u(std::max(W, Wn)), u(nb == 1 ? c->d_sum : c->d_bsum),
-          u(nb == 1 ? c->d_aux2 : c->d_bres), u(nb == 1 ? (const void*)c->d_Wf : (const void*)c->d_bWf),
+          u(nb == 1 ? c->d_aux2 : c->d_bres), u(nb == 1 ? c->d_Wf : c->d_bWf),
           u(c->d_part), u(c->d_selfp), u(c->d_self_idx), u(c->d_self_lut), u(c->d_mom), (uintptr_t)c->K,
-          (uintptr_t)c->self_lut_ok, u(c->d_K), u(c->d_K64), (uintptr_t)c->Kld, u(c->d_mut), u(c->d_mutf), u(c->d_mus),
-          u(c->d_red), u(c->d_err), (uintptr_t)c->bcap, (uintptr_t)(fft_eligible(c) && !c->fft_graph_failed),
+          (uintptr_t)c->self_lut_ok, u(c->d_K), u(c->d_K64), u(c->d_slab), u(c->d_mut), u(c->d_mutf), u(c->d_mus),
+          u(c->d_tab[0][0]), u(c->d_tab[1][0]), u(c->d_red), u(c->d_err), (uintptr_t)c->bcap, (uintptr_t)(fft_eligible(c) && !c->fft_graph_failed),
           rte_fft_signature(c->fft)};
 }
 
@@ -2785,12 +2821,10 @@ static int run_series_graph(rte_ctx* c, int nb, int nterms, double** d_res) {
   const int gi = nb;
   const size_t NC = (size_t)c->N * c->C;
   const int vs = nb * c->C;
-  const int cp = (nb * c->cstride + 3) / 4 * 4;
   double* W = nb == 1 ? c->d_W : c->d_bW;
   double* Wn = nb == 1 ? c->d_Wn : c->d_bWn;
   double* sum = nb == 1 ? c->d_sum : c->d_bsum;
   double* res = nb == 1 ? c->d_aux2 : c->d_bres;
-  float* Wf = nb == 1 ? c->d_Wf : c->d_bWf;
   const int flag_l = c->cfg.g != 0.0 ? 1 : 0;
   if (graph_stale(c, nb, nterms)) {
     if (c->graph[gi]) {
@@ -2808,10 +2842,11 @@ static int run_series_graph(rte_ctx* c, int nb, int nterms, double** d_res) {
     } else {
       rc = ensure_pair_kernel(c, &stored);
       if (rc) return rc;
-      int S, chunk;
-      rc = plan_split(c, 0, stored ? 1 : 0, nb, &S, &chunk);
-      if (!rc) rc = plan_split(c, c->L, stored ? 1 : 0, nb, &S, &chunk);
-      if (!rc && flag_l == 0) rc = plan_split(c, 0, stored ? 1 : 0, nb, &S, &chunk);
+      const void* K = stored ? (c->precision == RTE_PREC_FP64 ? (const void*)c->d_K64 : (const void*)c->d_K) : c->d_slab;
+      const int cols = stored ? c->nx * c->ny : c->slab_cols;
+      int chunk, S;
+      rc = plan_columns(c, c->L, nb, K, (size_t)cols * c->nz, cols, &chunk, &S);
+      if (!rc && flag_l == 0) rc = plan_columns(c, 0, nb, K, (size_t)cols * c->nz, cols, &chunk, &S);
     }
     if (rc) return rc;
     c->fft_in_graph[gi] = use_fft;
@@ -2828,21 +2863,19 @@ static int run_series_graph(rte_ctx* c, int nb, int nterms, double** d_res) {
       rc = ensure_pair_kernel(c, &stored);
       c->capture_store = false;
     }
-    cudaError_t e = rte_launch_to_f32_slots(W, Wf, c->d_islot, c->N, vs, cp, c->C, c->cstride, c->st);
-    if (e == cudaSuccess) {
+    if (!rc) {
       double *w = W, *wn = Wn;
       for (int t = 0; t < nterms && !rc; t++) {
-        rc = apply_term(c, w, Wf, wn, Wf, sum, flag_l, 1, nb);
+        rc = apply_term(c, w, wn, sum, flag_l, 1, nb, t > 0, true);
         std::swap(w, wn);
       }
-      if (!rc) e = rte_launch_to_f32_slots(sum, Wf, c->d_islot, c->N, vs, cp, c->C, c->cstride, c->st);
-      if (!rc && e == cudaSuccess) rc = apply_term(c, sum, Wf, res, nullptr, nullptr, 1, 0, nb);
+      if (!rc) rc = apply_term(c, sum, res, nullptr, 1, 0, nb);
     }
     cudaError_t e2 = cudaStreamEndCapture(c->st, &g);
     c->capturing = false;
     c->fft_capture_ready = false;
     c->profiling = prof;
-    if ((rc || e != cudaSuccess || e2 != cudaSuccess) && use_fft) {
+    if ((rc || e2 != cudaSuccess) && use_fft) {
       // the transforms could not be recorded: record the pair kernels instead from now on
       if (g) cudaGraphDestroy(g);
       cudaGetLastError();
@@ -2853,8 +2886,7 @@ static int run_series_graph(rte_ctx* c, int nb, int nterms, double** d_res) {
       if (g) cudaGraphDestroy(g);
       return rc;
     }
-    if (e != cudaSuccess || e2 != cudaSuccess)
-      return fail(c, RTE_ERR_DEVICE, "graph capture: %s", cudaGetErrorString(e != cudaSuccess ? e : e2));
+    if (e2 != cudaSuccess) return fail(c, RTE_ERR_DEVICE, "graph capture: %s", cudaGetErrorString(e2));
     cudaError_t e3 = cudaGraphInstantiate(&c->graph[gi], g, 0);
     cudaGraphDestroy(g);
     if (e3 != cudaSuccess) return fail(c, RTE_ERR_DEVICE, "graph instantiate: %s", cudaGetErrorString(e3));
@@ -2894,7 +2926,6 @@ static int forward_graph(rte_ctx* c, int nsrc, const rte_source* srcs, int nterm
   const size_t NC = (size_t)c->N * c->C, np = (size_t)c->nx * c->ny;
   const size_t npix = 2 * (np + (size_t)c->nz * c->nx + (size_t)c->nz * c->ny);
   const int vs = nb * c->C;
-  const int cp = (nb * c->cstride + 3) / 4 * 4;
   if (!c->ev_graph[0]) {
     CUDA_TRY(c, cudaEventCreate(&c->ev_graph[0]));
     CUDA_TRY(c, cudaEventCreate(&c->ev_graph[1]));
@@ -2922,7 +2953,7 @@ static int forward_graph(rte_ctx* c, int nsrc, const rte_source* srcs, int nterm
   c->has_point = false;
   for (int b = 0; b < nsrc && !rc; b++)
     rc = launch_source(c, &srcs[b], S0 + b * c->C, vs, fb + b * npix, false, q + b * c->C);
-  if (!rc) rc = series_start(c, S0, q, W0, nb, nb == 1 ? c->d_Wf : c->d_bWf, cp);
+  if (!rc) rc = series_start(c, S0, q, W0, nb);
   if (!rc) rc = run_series_graph(c, nb, nterms, &dres);
   for (int b = 0; b < nsrc && !rc && (trans || ref); b++)
     rc = run_images(c, dres + b * c->C, &srcs[b], true, trans ? trans + b * np : nullptr,
@@ -2943,19 +2974,6 @@ extern "C" int rte_forward_graph(rte_ctx* c, int nsrc, const rte_source* srcs, i
   if (c->kappa != 0.0) return unsupported_modulated(c, "graph replay");
   for (int b = 0; b < nsrc; b++)
     if (srcs[b].modulation != 0.0) return unsupported_modulated(c, "graph replay");
-  if (c->L >= 6 && nsrc > 2 && c->precision == RTE_PREC_MIXED) {  // as rte_forward_batch: two graphs of two
-    const size_t np = (size_t)c->nx * c->ny;
-    rte_report r1, r2;
-    int rc = rte_forward_graph(c, 2, srcs, nterms, trans, ref, &r1);
-    if (!rc) rc = rte_forward_graph(c, nsrc - 2, srcs + 2, nterms, trans ? trans + 2 * np : nullptr,
-                                    ref ? ref + 2 * np : nullptr, &r2);
-    if (rc) return rc;
-    if (rep) {
-      *rep = r2;
-      rep->ms_device = r1.ms_device + r2.ms_device;
-    }
-    return RTE_OK;
-  }
   CUDA_TRY(c, cudaSetDevice(c->cfg.device));
   float ms = 0;
   int rc = forward_graph(c, nsrc, srcs, nterms, trans, ref, &ms);
@@ -2981,7 +2999,7 @@ static int forward_to_out(rte_ctx* c, const rte_source* s, const rte_stop* stop,
   c->has_point = false;
   if (s->kind == RTE_SRC_POINT) CUDA_TRY(c, cudaMemsetAsync(c->d_q, 0, (size_t)c->N * c->C * sizeof(double), c->st));
   rc = launch_source(c, s, c->d_aux1, 0, nullptr, true, c->d_q);
-  if (!rc) rc = series_start(c, c->d_aux1, c->d_q, c->d_aux3, 1, c->d_Wf, c->cpad);
+  if (!rc) rc = series_start(c, c->d_aux1, c->d_q, c->d_aux3, 1);
   if (!rc) rc = neumann_real(c, c->d_aux3, c->d_aux1, c->d_out, 1, stop, -1, nullptr, nullptr);
   if (!rc) rc = run_images(c, c->d_out, s, true, trans, ref);
   return rc;
@@ -3123,7 +3141,27 @@ static int tangent_dA(rte_ctx* c, const double* d_in, double* d_outT, const std:
   CUDA_TRY(c, cudaMemcpyAsync(c->d_dmut, dmut.data(), sizeof(double) * c->N, cudaMemcpyHostToDevice, c->st));
   const int tiles = (c->N + RTE_PAIR_THREADS - 1) / RTE_PAIR_THREADS;
   const int S = std::max(1, std::min(c->max_split, (4 * 148 + tiles - 1) / tiles));
-  PairArgs a = pair_args(c, d_in, nullptr, 1, S, split_chunk(c->N, S));
+  PairArgs a;
+  memset(&a, 0, sizeof a);
+  a.N = c->N;
+  a.nx = c->nx;
+  a.ny = c->ny;
+  a.nz = c->nz;
+  a.Cfull = c->C;
+  a.dx = c->dx;
+  a.dy = c->dy;
+  a.dz = c->dz;
+  a.prop_thresh = c->prop_thresh;
+  a.kscale = c->dV / c->cm;
+  a.perm = c->d_perm;
+  a.mut = c->d_mut;
+  a.mutf = c->d_mutf;
+  a.Kld = c->N;
+  a.nzp = col_dims(c).nzp;
+  a.group = col_dims(c).group;
+  a.Win = d_in;
+  a.part = c->d_part;
+  a.chunk = split_chunk(c->N, S);
   a.nsplit = (c->N + a.chunk - 1) / a.chunk;
   a.Kmat = c->K_valid && c->d_K ? c->d_K : nullptr;
   a.Kmat64 = c->K_valid && c->d_K64 ? c->d_K64 : nullptr;
@@ -3193,12 +3231,8 @@ extern "C" int rte_fisher(rte_ctx* c, int nsrc, const rte_source* srcs, const rt
   const size_t npix = 2 * (np + (size_t)c->nz * c->nx + (size_t)c->nz * c->ny);
   const int nb = d->nbins;
   const size_t NB2 = (size_t)6 * nb * nb;
-  // tangent series run together: four at L <= 5 (the widest pair-kernel batch whose accumulators fit in
-  // registers) and, with the path integrals recomputed, at L >= 6 (k_pair_mixed_grp: two thread groups
-  // of two sharing each pair's walk); two otherwise.  The pair walk (and at L <= 5 the SH recurrence) of
-  // every pair serves the whole group.
-  const bool recompute = c->kernel_mode == RTE_KERNEL_RECOMPUTE && c->model != RTE_MODEL_FIM;
-  const int nbt = c->precision == RTE_PREC_MIXED ? (c->L <= 5 || recompute ? 4 : 2) : 1;
+  // tangent series run together: each pair-kernel value streamed or recomputed serves the whole group
+  const int nbt = c->precision == RTE_PREC_MIXED ? 4 : 1;
   if (nbt > 1) {
     rc = ensure_batch(c, nbt);
     if (rc) return rc;

@@ -9,49 +9,88 @@
 #define RTE_PAIR_TS 64        // source voxels staged in shared memory per step
 #define RTE_MAX_MOM 48        // self-term power-series terms
 
-// Stored FP32 pair kernel layout: blocks of 128 destination slots, each block [source slot][128
-// destinations] with ld (>= N) source rows.  The kernel values of a run of consecutive sources for one
-// pair-kernel CTA's 128 destinations are then one contiguous block (a single bulk copy).
-#define RTE_KBLK 128
-__host__ __device__ inline size_t kmat_index(size_t s, size_t d, size_t ld) {
-  return ((d / RTE_KBLK) * ld + s) * RTE_KBLK + (d % RTE_KBLK);
+// Stored pair kernel layout.  Sources in column order (slot = (y * nx + x) * nz + z), destinations in the same
+// order with every column padded to nzp positions, a whole number of groups (one thread's destinations, see
+// rte_column.cu).  A block holds the 32 * group positions of one warp of the column kernels, [source slot]
+// [32 * group] with ld source rows, each row destination-major (the 32 lanes' first destinations, their
+// second, ...): a warp's values of a run of sources are one contiguous block.
+__host__ __device__ inline size_t kmat_index(size_t s, size_t p, size_t ld, int group) {
+  const size_t kb = 32 * (size_t)group, o = p % kb;
+  return (p / kb * ld + s) * kb + o % group * 32 + o / group;
 }
+// destination position of a slot
+__host__ __device__ inline int kmat_pos(int slot, int nz, int nzp) { return slot / nz * nzp + slot % nz; }
+// Destinations per thread of the column kernels.  Three at L <= 5, where four CTAs per SM still fit (33^3 L=5 launch:
+// 2 per thread 2.93 ms, 3 2.41, 4 at two CTAs 3.11; FP64: 1 7.0 ms, 2 9.3, 3 5.6), two above.
+#define RTE_COL_G(L) ((L) <= 5 ? 3 : 2)
 
 struct PairArgs {
   int N, nx, ny, nz, Cfull;
   double dx, dy, dz;
   double prop_thresh;
   double kscale;        // dV / cm folded into the pair kernel
-  const int* perm;      // destination slot -> voxel index (spatially compact order)
+  const int* perm;      // slot -> voxel index (column order)
+  const int* islot;     // voxel -> slot
   const double* mut;    // mu_t per voxel, FP64
   const float* mutf;    // mu_t per voxel, FP32
-  const double* Win;    // current term, real basis, N x Cfull, FP64
-  const float* Winf;    // current term, FP32 copy in slot order, coefficient c times N_c (sh_eval_monic)
-  float* Kmat;          // stored pair kernel K(source slot, destination slot), blocked (kmat_index, ld = Kld)
-  double* Kmat64;       // FP64 stored kernel (FP64 method), row-major [source slot][destination slot], stride Kld
+  float* Kmat;          // FP32 pair kernel, blocked (kmat_index, ld = Kld, columns padded to nzp)
+  double* Kmat64;       // FP64 pair kernel, same layout
   size_t Kld;
-  double* part;         // split-K partial sums, [S][N][Cfull], indexed by voxel
-  float* partf;         // FP32 partial sums in the same layout (tile-staged kernel: raw chunk sums, no N_c)
-  int chunk;            // source voxels per blockIdx.y
-  int nsplit;           // S
-  int nb;               // right-hand sides sharing the medium (mixed kernels), layout [N][nb][Cfull]
-  const float4* slot_xyz;  // per slot: (x, y, z) voxel coordinates as exact floats, w = voxel index
-  int cpad;             // FP32 source row length in floats: nb*cstride rounded up to a multiple of 4
-  int cstride;          // FP32 row stride of one right-hand side: Cfull rounded up to a multiple of 4
-  int* err;             // set to 1 when a bounded wait runs out (kernel result invalid)
-  // tangent pass (k_pair_tangent): derivative of mu_t along a parameter direction, and the voxel
-  // bounding box of its support (pairs whose segment misses the box have no path derivative)
+  int nzp, group;
+  // tangent pass (k_pair_tangent): current term N x Cfull, sums over `chunk` sources per blockIdx.y, derivative
+  // of mu_t along a parameter direction, and the voxel bounding box of its support (pairs whose segment misses
+  // the box have no path derivative)
+  const double* Win;
+  double* part;         // partial sums [S][N][Cfull], indexed by voxel
+  int chunk, nsplit;
   const double* dmut;
   int box_lo[3], box_hi[3];  // (x, y, z) voxel indices
-  const int* islot;          // voxel -> slot (row of the stored kernel)
-  // intensity modulation: mu_t has the uniform imaginary part kappa, so every pair kernel gains the
-  // phase exp(-i kappa |r - r'|); the right-hand sides are complex, (real, imaginary) pairs of rows
-  double kappa;
-  // transposed operator of the table model: each pair's table direction is snapped from the reverse
-  // displacement (source minus destination).  Snapping does not commute with negation, so for the
-  // FisherInfo_IO table A^T != P A P; with exact SH the parity form is used instead.
-  int transpose;
-  int tile;  // staged stored-kernel launch: 0 = 32-source tiles, 1 = 64-source tiles (autotuned)
+};
+
+// Pair-kernel precompute (rte_store.cu): rows of the source columns [col0, col1), destinations all.
+struct StoreArgs {
+  int N, nx, ny, nz;
+  double dx, dy, dz, prop_thresh, kscale;
+  const void* mu;     // mu_t in column order (T)
+  void* K;            // T, row 0 is the first source of col0 (kmat_index with ld = Kld)
+  size_t Kld;
+  int nzp, group;
+  int col0, col1;
+  int npair, zb, group_ch;  // set by the launcher: column pairs per chunk, z block, chunks that share their lists
+};
+
+// Column form of the pair operator (rte_column.cu): sources and destinations in column order, one CTA per
+// 128 threads' destinations, right-hand side and chunk of source columns.
+struct ColArgs {
+  int N, nx, ny, nz, Cfull;
+  int nzp, group;     // destination positions per column, destinations per thread (ColDims)
+  int nrhs;           // right-hand sides of this launch (1 for a complex pair)
+  const void* W;      // source rows [nrhs][N][pitch] (T, slot order), coefficient c times N_c
+  int pitch;
+  const void* K;      // pair kernel (T), rows from source slot kslot0 (kmat_index with ld = Kld)
+  size_t Kld;
+  int kslot0;
+  const void* tab;    // angle rows (rte_launch_col_table)
+  int row, azn, csn, cls, pho;
+  void* part;         // chunk sums [S][N][vstride]: FP32 raw, or FP64 with N_c applied
+  int vstride;
+  int split0;         // first chunk-sum slice
+  int col0, col1;     // source columns [col0, col1), `chunk` columns per blockIdx.y
+  int chunk, nsplit;
+  int* err;
+  int tz, ncd;        // set by the launcher: sources per run, destination columns per CTA at most
+};
+struct ColDims {
+  int pitch;                        // source rows
+  int group, nzp;                   // destinations per thread, destination positions per column
+  int row, azn, csn, nk, pho;       // angle rows: entries of csn values in tg residue classes of cls
+  int tg, cls;
+};
+struct ColTabArgs {
+  int nx, ny, nz, nzp, L;
+  double dx, dy, dz, kappa;
+  int table, transpose;
+  int row, azn, csn, nk, pho, tg, cls;
 };
 
 struct EpiArgs {
@@ -63,9 +102,10 @@ struct EpiArgs {
   int flag_scat;
   double scat[RTE_MAX_L + 1];  // per-l scatter factor (times mu_s of the voxel)
   double* Wout;         // FP64 result (may alias nothing else)
-  float* Woutf;         // FP32 copy in slot order (times N_c), rows of cpad floats (may be null)
+  void* rows;           // copy [nb][N][pitch] in slot order (times N_c) for the next pair launch (may be null)
+  int rows64;           // rows are FP64 (else FP32)
   const int* islot;     // voxel -> slot
-  int cpad, cstride;
+  int pitch;
   double* sum;          // running sum (null = do not accumulate)
   double* red;          // [0] ||Wout||^2 [1] ||sum||^2 [2] stop-layer sum of Wout [3] of sum
   int cplx;             // right-hand sides are (real, imaginary) pairs: odd ones are imaginary parts
@@ -150,6 +190,7 @@ struct BpArgs {
   const float* Kmat;   // stored pair kernel (null: recompute the path integral)
   const double* Kmat64;  // FP64 stored pair kernel (FP64 contexts in stored-kernel mode)
   size_t Kld;
+  int nzp, group;      // layout of the stored kernel (ColDims)
   double* g;           // gradient w.r.t. mu_t, accumulated [N]
   int use_smem;        // per-CTA private accumulator of N entries in shared memory (set by the launcher)
   void* Q;             // per unordered pair weight [source slot][destination slot] (row stride Kld), T
@@ -203,8 +244,9 @@ cudaError_t rte_launch_grad_local(const GradLocalArgs& a, cudaStream_t st);
 // message returned by rte_last_error(NULL) on this thread
 __attribute__((visibility("hidden"))) void rte_set_global_error(const char* msg);
 cudaError_t rte_launch_source(const SrcArgs& a, cudaStream_t st);
+// mutc / mutfc: mu_t in column order (islot), FP64 and FP32
 cudaError_t rte_launch_medium(const double* mua, const double* mus, double* mut, double* mus_out, float* mutf,
-                              int N, double* red_max, cudaStream_t st);
+                              double* mutc, float* mutfc, const int* islot, int N, double* red_max, cudaStream_t st);
 cudaError_t rte_launch_fma_peak(int fp64, int iters, float* sink, cudaStream_t st, int blocks);
 cudaError_t rte_upload_sh_tables(const ShTables& t);
 // Uniform-medium convolution path (rte_fft.cpp): grid, padded grid, spacing, coupling distance,
@@ -234,11 +276,8 @@ void rte_fft_destroy(FftState* s);
 // host copies: the recurrence tables and the real SH R_c at a unit direction (index l*l + l + m)
 ShTables make_sh_tables();
 void sh_real_host(const ShTables& t, int L, double x, double y, double z, double* R);
-cudaError_t rte_launch_pair(const PairArgs& a, int LA, int precision, int table, int stored, cudaStream_t st);
-// fp64 = 1: FP64 path sums and exp into a.Kmat64; else FP32 into a.Kmat
-cudaError_t rte_launch_store_kernel(const PairArgs& a, cudaStream_t st, int fp64 = 0);
-cudaError_t rte_pair_occupancy(int LA, int precision, int table, int stored, int nb, int cpad, int* blocks_per_sm,
-                               int cplx = 0, int tile = 0);
+cudaError_t rte_launch_pair_fp64(const PairArgs& a, int LA, cudaStream_t st);
+cudaError_t rte_launch_store_kernel(const StoreArgs& a, cudaStream_t st, int fp64);
 cudaError_t rte_launch_epilogue(const EpiArgs& a, int LA, cudaStream_t st);
 cudaError_t rte_launch_images(const ImgArgs& a, cudaStream_t st);
 cudaError_t rte_launch_self(const SelfArgs& a, cudaStream_t st);
@@ -249,9 +288,12 @@ cudaError_t rte_launch_to_cplx(const double* u1, const double* u2, double* cplx,
                                cudaStream_t st, int ustride = 0);
 cudaError_t rte_launch_layer_sums(const double* W, const double* S, int N, int nx, int ny, int nz, int Cfull,
                                   double* red, cudaStream_t st, int cplx = 0);
-cudaError_t rte_launch_f64_to_f32(const double* a, float* b, size_t n, cudaStream_t st);
-// FP64 [N][vstride] (voxel order) -> FP32 [slot][cpad] (slot order), coefficient c scaled by the monic
-// SH normalisation N_c that the mixed pair kernels factor out of their per-pair recurrence
-cudaError_t rte_launch_to_f32_slots(const double* a, float* b, const int* islot, int N, int vstride, int cpad,
-                                    int Cfull, int cstride, cudaStream_t st);
+// FP64 [N][vstride] (voxel order) -> source rows of the pair kernels in slot order (FP32, or FP64),
+// coefficient c times the monic SH normalisation N_c
+cudaError_t rte_launch_rows(const double* w, void* rows, const int* islot, int N, int nb, int pitch, int Cfull,
+                            int fp64, cudaStream_t st);
+ColDims rte_col_dims(int C, int L, int nz, int fp64, int cplx);
+cudaError_t rte_launch_col_table(const ColTabArgs& a, void* tab, int fp64, cudaStream_t st);
+// launches, or with occ != null only reports the CTAs per SM
+cudaError_t rte_launch_column(const ColArgs& a, int LA, int fp64, int cplx, cudaStream_t st, int* occ = nullptr);
 }

@@ -1,4 +1,5 @@
-// rte_kernels.cu -- sm_100a kernels of the Neumann-series RTE term W <- D A W.
+// rte_kernels.cu -- sm_100a kernels of the Neumann-series RTE term W <- D A W: epilogue, self-voxel term, sources,
+// images, detectors, tangent and adjoint passes, the uniform-medium convolution.
 //
 // The attenuation operator A of the reference (FisherInfo_IO/src/kernels.cu:151-418,
 // compute_diagonal_abs + compute_propabs + scale_dist_dev, and prop_scat_dev for D) is
@@ -8,11 +9,9 @@
 //            + (dV/cm) sum_c' Dself_cc'(mu_t(r)) W[r,c'],
 //   w = (r - r')/|r - r'|,  k = exp(-tau(r,r')) dV / (cm |r - r'|^2),
 //
-// then D multiplies coefficient (l,m) by scat[l] * mu_s(r).  One CUDA thread owns one
-// destination voxel and streams all source voxels through shared memory (the warp
-// reads the same source at the same time, so source data is a shared-memory
-// broadcast).  The source range is split over blockIdx.y (split-K); the epilogue
-// kernel adds the partial sums in a fixed order, so results are deterministic.
+// then D multiplies coefficient (l,m) by scat[l] * mu_s(r).  The sum over pairs is in rte_column.cu, k in
+// rte_store.cu; the pair sums arrive here as chunk sums that the epilogue adds in a fixed order, so results are
+// deterministic.
 //
 // Path integrals follow mu_int (FisherInfo_IO/src/kernels.cu:50-148): a Siddon walk
 // between voxel centres whose axis crossings are ordered here with exact integer
@@ -27,23 +26,8 @@
 
 #include <type_traits>
 
+#include "rte_device.cuh"
 #include "rte_internal.h"
-
-// Packed FP32 pairs (sm_100 f32x2 arithmetic): two FP32 FMAs per instruction.
-typedef unsigned long long f2_t;
-__device__ __forceinline__ f2_t f2_pack(float lo, float hi) {
-  f2_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void f2_unpack(f2_t v, float& lo, float& hi) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
-}
-__device__ __forceinline__ f2_t f2_fma(f2_t a, f2_t b, f2_t c) {
-  f2_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
 
 struct ScatTab {
   double v[RTE_MAX_L + 1];
@@ -77,39 +61,6 @@ template <> __device__ __forceinline__ double shQ0<double>(int i) { return c_sh.
 template <> __device__ __forceinline__ float shA<float>(int i) { return c_shAf[i]; }
 template <> __device__ __forceinline__ float shB<float>(int i) { return c_shBf[i]; }
 template <> __device__ __forceinline__ float shQ0<float>(int i) { return c_shQ0f[i]; }
-
-// Compile-time copies of the SH recurrence coefficients (the same formulas as the host tables in
-// rte_host.cpp), so the unrolled FP32 recurrence multiplies by immediates and the l = m+1 steps
-// carry no B term.
-struct ShConstTab {
-  double A[64], B[64], Q0[RTE_MAX_L + 1];
-};
-constexpr double c_sqrt(double x) {
-  double r = x > 1.0 ? x : 1.0;
-  for (int i = 0; i < 80; ++i) r = 0.5 * (r + x / r);
-  return r;
-}
-constexpr double c_knorm(int l, int m) {
-  double f = 1.0;
-  for (int i = l - m + 1; i <= l + m; ++i) f *= (double)i;
-  const double k = c_sqrt((2.0 * l + 1.0) / (4.0 * 3.14159265358979323846) / f);
-  return m > 0 ? k * c_sqrt(2.0) : k;
-}
-constexpr ShConstTab make_sh_const() {
-  ShConstTab t{};
-  for (int m = 0; m <= RTE_MAX_L; ++m) {
-    double dfact = 1.0;
-    for (int i = 2 * m - 1; i > 0; i -= 2) dfact *= (double)i;
-    t.Q0[m] = c_knorm(m, m) * ((m & 1) ? -1.0 : 1.0) * dfact;
-    for (int l = m + 1; l <= RTE_MAX_L; ++l) {
-      const int id = l * (l + 1) / 2 + m;
-      t.A[id] = c_knorm(l, m) * (2.0 * l - 1.0) / ((double)(l - m) * c_knorm(l - 1, m));
-      t.B[id] = (l - 2 >= m) ? c_knorm(l, m) * (double)(l + m - 1) / ((double)(l - m) * c_knorm(l - 2, m)) : 0.0;
-    }
-  }
-  return t;
-}
-__device__ constexpr ShConstTab kShConst = make_sh_const();
 
 // Real orthonormal SH R_lm at the unit direction (x, y, z), index l*l + l + m.
 // R_l0 = q_l^0(z), R_l,+m = q_l^m(z) Re((x+iy)^m), R_l,-m = q_l^m(z) Im((x+iy)^m), with the
@@ -161,33 +112,6 @@ __device__ __forceinline__ void sh_eval(T x, T y, T z, T* R) {
   }
 }
 
-// Monic form of the same recurrence for the mixed pair kernel.  With q_l^m = s_lm u_l^m, s_mm = Q0[m]
-// and s_lm = A_lm s_{l-1,m}, the polynomials u satisfy u_l = z u_{l-1} - beta_lm u_{l-2} (beta_lm =
-// B_lm s_{l-2,m} / s_lm), so R_c = N_c U_c with U_{l,+-m} = u_l^m Re/Im((x+iy)^m) and N_c = s_lm.
-// The kernel carries U instead of R: the factors N_c are applied once per source row (the FP32 copy
-// of W holds N_c W_c) and once per destination (the partial sums), not per pair, and a recurrence
-// step costs two operations instead of three.
-struct MonicTab {
-  double beta[64];  // index l*(l+1)/2 + m
-  double N[64];     // index l*l + l + m
-};
-constexpr MonicTab make_monic() {
-  MonicTab t{};
-  const ShConstTab q = make_sh_const();
-  for (int m = 0; m <= RTE_MAX_L; ++m) {
-    double s[RTE_MAX_L + 1] = {};
-    s[m] = q.Q0[m];
-    for (int l = m + 1; l <= RTE_MAX_L; ++l) s[l] = q.A[l * (l + 1) / 2 + m] * s[l - 1];
-    for (int l = m; l <= RTE_MAX_L; ++l) {
-      if (l >= m + 2) t.beta[l * (l + 1) / 2 + m] = q.B[l * (l + 1) / 2 + m] * s[l - 2] / s[l];
-      t.N[l * l + l + m] = s[l];
-      t.N[l * l + l - m] = s[l];
-    }
-  }
-  return t;
-}
-__device__ constexpr MonicTab kMonic = make_monic();
-
 // The monic recurrence, each coefficient handed to emit(index, value) as it is made (the index is a
 // compile-time constant once the loops unroll).
 template <int L, typename T, typename Emit>
@@ -236,175 +160,54 @@ __device__ __forceinline__ void sh_monic_recurrence(T x, T y, T z, Emit emit) {
   }
 }
 
-template <int L, typename T>
-__device__ __forceinline__ void sh_eval_monic(T x, T y, T z, T* U) {
-  sh_monic_recurrence<L, T>(x, y, z, [&](int c, T v) { U[c] = v; });
-}
-
-// Direction snapped to the reference's 100x100 SH table cell (FisherInfo_IO/src/defines.h:53-56
-// and kernels.cu:326-333: theta = acos(dz/dist), phi = atan2(dy,dx) NOT wrapped to [0,2pi), so a
-// negative phi index reads the previous theta row of the flat table).
-__device__ __forceinline__ void table_direction(double ddx, double ddy, double ddz, double dist, double& ux,
-                                                double& uy, double& uz) {
-  double theta = acos(ddz / dist);
-  double phi = atan2(ddy, ddx);
-  int ti = (int)rintf((float)((100 - 1) * (theta) / (M_PI)));
-  int pj = (int)rintf((float)((100 - 1) * (phi) / (2 * M_PI)));
-  int off = ti * 100 + pj;
-  if (off < 0) off = 0;
-  int tq = off / 100, pq = off - tq * 100;
-  double th = (tq * M_PI) / (100 - 1);
-  double ph = (pq * 2.0 * M_PI) / (100 - 1);
-  double st, ct, sp, cp;
-  sincos(th, &st, &ct);
-  sincos(ph, &sp, &cp);
-  ux = st * cp;
-  uy = st * sp;
-  uz = ct;
-}
-
 #include "rte_walk.cuh"
 
 // ---------------------------------------------------------------------------------------------
-// Plain FP64 method: every pair recomputed in FP64 (path integral, SH, projections).  CPLX: one
-// complex right-hand side stored as (real, imaginary) rows per voxel, and the pair kernel carries the
-// modulation phase exp(-i kappa |r - r'|) (complex mu_t = mu_t + i kappa, uniform imaginary part).
-// STORED: the pair kernel exp(-tau) dV/(cm r^2) is read from the FP64 matrix Kmat64[source slot]
-// [destination slot] instead of walking the path; sources are then visited in slot order, so the
-// warp's 32 destinations read one contiguous 256-byte run of K per source.
-template <int LA, bool TABLE, bool CPLX, bool STORED = false>
+// Plain FP64 pair operator with exact directions, every path integral walked: for callers without room for
+// kernel or angle tables (rte_noalloc.cu).  One thread per destination voxel, sources streamed through shared
+// memory (the warp reads the same source at the same time); `chunk` sources per blockIdx.y.
+template <int LA>
 __global__ void __launch_bounds__(RTE_PAIR_THREADS) k_pair_fp64(PairArgs a) {
-  constexpr int C = (LA + 1) * (LA + 1);
-  constexpr int NP = CPLX ? 2 : 1;        // rows per voxel
-  constexpr int TS = RTE_PAIR_TS / NP;    // sources per shared-memory tile
-  __shared__ double sW[TS * NP * C];
-  __shared__ int sxyz[STORED ? TS : 1][3];  // source coordinates (slot order)
+  constexpr int C = (LA + 1) * (LA + 1), TS = RTE_PAIR_TS;
+  __shared__ double sW[TS * C];
   const int tid = threadIdx.x;
   const int slot = blockIdx.x * RTE_PAIR_THREADS + tid;
   const bool act = slot < a.N;
   const int r = act ? a.perm[slot] : 0;
   const int plane = a.nx * a.ny;
   const int i = r / plane, j = (r / a.nx) % a.ny, k = r % a.nx;
-  const int vs = NP * a.Cfull;
-  double acc[NP][C];
+  double acc[C];
 #pragma unroll
-  for (int p = 0; p < NP; ++p)
-#pragma unroll
-    for (int c = 0; c < C; ++c) acc[p][c] = 0.0;
+  for (int c = 0; c < C; ++c) acc[c] = 0.0;
   const int sb = blockIdx.y * a.chunk;
   const int se = min(a.N, sb + a.chunk);
   for (int s0 = sb; s0 < se; s0 += TS) {
     const int ns = min(TS, se - s0);
     __syncthreads();
-    for (int q = tid; q < ns * NP * C; q += RTE_PAIR_THREADS) {
-      const int sv = q / (NP * C), e = q - sv * NP * C, p = e / C, c = e - p * C;
-      const int src = STORED ? a.perm[s0 + sv] : s0 + sv;
-      sW[q] = a.Win[(size_t)src * vs + (size_t)p * a.Cfull + c];
-    }
-    if (STORED && tid < ns) {
-      const int v = a.perm[s0 + tid];
-      sxyz[tid][0] = v % a.nx;
-      sxyz[tid][1] = (v / a.nx) % a.ny;
-      sxyz[tid][2] = v / plane;
+    for (int q = tid; q < ns * C; q += RTE_PAIR_THREADS) {
+      const int sv = q / C, c = q - sv * C;
+      sW[q] = a.Win[(size_t)(s0 + sv) * a.Cfull + c];
     }
     __syncthreads();
     if (!act) continue;
-    if constexpr (STORED) {
-      const double* Kcol = a.Kmat64 + (size_t)s0 * a.Kld + slot;
-      double knext = __ldg(Kcol);
-      for (int sv = 0; sv < ns; ++sv) {
-        const double kk = knext;
-        if (sv + 1 < ns) knext = __ldg(Kcol + (size_t)(sv + 1) * a.Kld);
-        if (kk == 0.0) continue;  // the diagonal and pairs beyond the coupling distance
-        const double ddx = (double)(k - sxyz[sv][0]) * a.dx, ddy = (double)(j - sxyz[sv][1]) * a.dy,
-                     ddz = (double)(i - sxyz[sv][2]) * a.dz;
-        const double dist = sqrt(ddx * ddx + ddy * ddy + ddz * ddz);
-        double ux, uy, uz;
-        if (TABLE) {
-          // A^T: snap(source - destination), negated in integers so that a zero component stays +0.0 (the
-          // table's unwrapped phi index depends on atan2's sign of zero) -- the forward kernel's exact bits
-          const int sg = a.transpose ? -1 : 1;
-          table_direction((double)(sg * (k - sxyz[sv][0])) * a.dx, (double)(sg * (j - sxyz[sv][1])) * a.dy,
-                          (double)(sg * (i - sxyz[sv][2])) * a.dz, dist, ux, uy, uz);
-        } else {
-          const double inv = 1.0 / dist;
-          ux = ddx * inv;
-          uy = ddy * inv;
-          uz = ddz * inv;
-        }
-        double R[C];
-        sh_eval<LA, double>(ux, uy, uz, R);
-        double S[NP];
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          S[p] = 0.0;
-#pragma unroll
-          for (int c = 0; c < C; ++c) S[p] = fma(R[c], sW[(sv * NP + p) * C + c], S[p]);
-        }
-        if (CPLX) {
-          double sn, cs;
-          sincos(a.kappa * dist, &sn, &cs);
-          const double t0 = kk * (cs * S[0] + sn * S[NP - 1]), t1 = kk * (cs * S[NP - 1] - sn * S[0]);
-#pragma unroll
-          for (int c = 0; c < C; ++c) {
-            acc[0][c] = fma(R[c], t0, acc[0][c]);
-            acc[NP - 1][c] = fma(R[c], t1, acc[NP - 1][c]);
-          }
-        } else {
-          const double t = kk * S[0];
-#pragma unroll
-          for (int c = 0; c < C; ++c) acc[0][c] = fma(R[c], t, acc[0][c]);
-        }
-      }
-      continue;
-    }
     int kp = s0 % a.nx, jp = (s0 / a.nx) % a.ny, ip = s0 / plane;
     for (int sv = 0; sv < ns; ++sv) {
-      const int rp = s0 + sv;
-      if (rp != r) {
+      if (s0 + sv != r) {
         const double ddx = (double)(k - kp) * a.dx, ddy = (double)(j - jp) * a.dy, ddz = (double)(i - ip) * a.dz;
         const double d2 = ddx * ddx + ddy * ddy + ddz * ddz;
         const double dist = sqrt(d2);
         if (dist < a.prop_thresh) {
-          double ux, uy, uz;
-          if (TABLE) {
-            // A^T: snap(source - destination), negated in integers (a zero component stays +0.0)
-            const int sg = a.transpose ? -1 : 1;
-            table_direction((double)(sg * (k - kp)) * a.dx, (double)(sg * (j - jp)) * a.dy,
-                            (double)(sg * (i - ip)) * a.dz, dist, ux, uy, uz);
-          } else {
-            const double inv = 1.0 / dist;
-            ux = ddx * inv;
-            uy = ddy * inv;
-            uz = ddz * inv;
-          }
+          const double inv = 1.0 / dist;
           double R[C];
-          sh_eval<LA, double>(ux, uy, uz, R);
-          double S[NP];
+          sh_eval<LA, double>(ddx * inv, ddy * inv, ddz * inv, R);
+          double S = 0.0;
 #pragma unroll
-          for (int p = 0; p < NP; ++p) {
-            S[p] = 0.0;
-#pragma unroll
-            for (int c = 0; c < C; ++c) S[p] = fma(R[c], sW[(sv * NP + p) * C + c], S[p]);
-          }
+          for (int c = 0; c < C; ++c) S = fma(R[c], sW[sv * C + c], S);
           int Q;
           const double ps = path_sum<double, double>(i, j, k, ip, jp, kp, a.mut, a.nx, plane, Q);
-          const double tau = ps * dist / (double)Q;
-          const double kk = exp(-tau) * a.kscale / d2;
-          if (CPLX) {  // kk exp(-i kappa dist) (S0 + i S1)
-            double sn, cs;
-            sincos(a.kappa * dist, &sn, &cs);
-            const double t0 = kk * (cs * S[0] + sn * S[NP - 1]), t1 = kk * (cs * S[NP - 1] - sn * S[0]);
+          const double t = exp(-ps * dist / (double)Q) * a.kscale / d2 * S;
 #pragma unroll
-            for (int c = 0; c < C; ++c) {
-              acc[0][c] = fma(R[c], t0, acc[0][c]);
-              acc[NP - 1][c] = fma(R[c], t1, acc[NP - 1][c]);
-            }
-          } else {
-            const double t = kk * S[0];
-#pragma unroll
-            for (int c = 0; c < C; ++c) acc[0][c] = fma(R[c], t, acc[0][c]);
-          }
+          for (int c = 0; c < C; ++c) acc[c] = fma(R[c], t, acc[c]);
         }
       }
       if (++kp == a.nx) {
@@ -417,11 +220,9 @@ __global__ void __launch_bounds__(RTE_PAIR_THREADS) k_pair_fp64(PairArgs a) {
     }
   }
   if (act) {
-    double* o = a.part + ((size_t)blockIdx.y * a.N + r) * vs;
+    double* o = a.part + ((size_t)blockIdx.y * a.N + r) * a.Cfull;
 #pragma unroll
-    for (int p = 0; p < NP; ++p)
-#pragma unroll
-      for (int c = 0; c < C; ++c) o[(size_t)p * a.Cfull + c] = acc[p][c];
+    for (int c = 0; c < C; ++c) o[c] = acc[c];
   }
 }
 
@@ -507,9 +308,9 @@ __global__ void __launch_bounds__(RTE_PAIR_THREADS) k_pair_tangent(PairArgs a) {
             const T dtau = dps * dist / (T)Q;
             T kk;
             if (a.Kmat64) {
-              kk = (T)__ldg(a.Kmat64 + (size_t)a.islot[rp] * a.Kld + slot);
+              kk = (T)__ldg(a.Kmat64 + kmat_index(a.islot[rp], kmat_pos(slot, a.nz, a.nzp), a.Kld, a.group));
             } else if (a.Kmat) {
-              kk = (T)__ldg(a.Kmat + kmat_index(a.islot[rp], slot, a.Kld));
+              kk = (T)__ldg(a.Kmat + kmat_index(a.islot[rp], kmat_pos(slot, a.nz, a.nzp), a.Kld, a.group));
             } else {
               int Q2;
               const T ps = path_sum<T, double>(i, j, k, ip, jp, kp, a.mut, a.nx, plane, Q2);
@@ -575,650 +376,7 @@ __global__ void k_strided_add(double* dst, const double* a, int astride, const d
   dst[t] = a[(size_t)r * astride + c] + b[t];
 }
 
-// ---------------------------------------------------------------------------------------------
-// Mixed precision: path integrals, SH and projections in FP32 (SH in FP64 for l >= 7).  NB right-
-// hand sides that share the medium are propagated together: the direction, its SH and the pair
-// kernel are computed once per pair and used NB times.  Sources are visited in slot order (the
-// same spatially compact order as the destinations).  The FP32 source coefficients are kept in
-// slot order with rows of CP floats, so a 64-source tile (and its coordinates) is one contiguous
-// block: one thread issues two TMA bulk copies (cp.async.bulk, completion on an mbarrier) per tile
-// into a double buffer, overlapping the next tile's copy with this tile's arithmetic.  Sums: FP32
-// over one tile in registers (projections split over four accumulators), FP32 across tiles in
-// shared memory, FP64 across the split-K chunks in the epilogue.  STORED reads the precomputed
-// pair kernel K[source slot][destination slot] (FP32); otherwise the path is walked in FP32.
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
-      "l"(src), "r"(bytes), "r"(smem_u32(bar))
-      : "memory");
-}
-// bounded wait on an mbarrier phase; false when the limit ran out
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (int it = 0; it < (1 << 22); ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
-// shared memory: [2][TS] float4 | [2][TS][cpad] float | [NB*C][T] float | 2 mbarriers (TS sources per tile)
-struct MixedLayout {
-  size_t off_w, off_acc, off_bar, bytes;
-  __host__ __device__ MixedLayout(int cpad, int nbc, int ts = RTE_PAIR_TS) {
-    off_w = sizeof(float4) * 2 * ts;
-    off_acc = off_w + sizeof(float) * 2 * ts * (size_t)cpad;
-    off_bar = (off_acc + sizeof(float) * (size_t)nbc * RTE_PAIR_THREADS + 15) / 16 * 16;
-    bytes = off_bar + 2 * sizeof(uint64_t);
-  }
-};
-
-// CPLX (NB = 2): the two right-hand sides are the real and imaginary parts of one complex one and the
-// pair kernel carries the modulation phase exp(-i kappa |r - r'|).  L = 7 with one right-hand side runs
-// under a three-CTA register bound (168 registers, k_pair_mixed_3): 33^3 launch 38.3 -> 33.9 ms (the
-// same bound made L = 6 slower, so it applies to L = 7 alone).
-template <int LA, bool TABLE, bool STORED, int NB, bool CPLX>
-__device__ __forceinline__ void pair_mixed_body(const PairArgs& a) {
-  static_assert(!CPLX || NB == 2, "a complex right-hand side is a (real, imaginary) pair");
-  // wide rows (NB * C >= 128: 4 RHS at L = 5, 2 RHS at L = 7): 32-source tiles, so that two CTAs (their
-  // register limit) fit the shared memory
-  constexpr int C = (LA + 1) * (LA + 1), TS = NB * C >= 128 ? 32 : RTE_PAIR_TS, T = RTE_PAIR_THREADS;
-  const int CP = a.cpad;  // FP32 source row: nb * Cfull floats, padded to a multiple of 4
-  const MixedLayout Sh(CP, NB * C, TS);
-  typedef typename std::conditional<(LA >= 7), double, float>::type ShT;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float4* sP = reinterpret_cast<float4*>(smem_raw);
-  float* sW = reinterpret_cast<float*>(smem_raw + Sh.off_w);
-  float* sAcc = reinterpret_cast<float*>(smem_raw + Sh.off_acc);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + Sh.off_bar);
-  const int tid = threadIdx.x;
-  const int slot = blockIdx.x * T + tid;
-  const bool act = slot < a.N;
-  const float4 me = a.slot_xyz[act ? slot : 0];
-  const int r = __float_as_int(me.w);
-  const int plane = a.nx * a.ny;
-  const int i = (int)me.z, j = (int)me.y, k = (int)me.x;
-  const float dxf = (float)a.dx, dyf = (float)a.dy, dzf = (float)a.dz;
-  const float kscalef = (float)a.kscale;
-  const float thr = (float)a.prop_thresh;
-#pragma unroll
-  for (int q = 0; q < NB * C; ++q) sAcc[q * T + tid] = 0.f;
-  const int sb = blockIdx.y * a.chunk;
-  const int se = min(a.N, sb + a.chunk);
-  const int ntile = (se - sb + TS - 1) / TS;
-  if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  auto issue = [&](int t) {  // tile t -> buffer t & 1 (one thread)
-    const int s0 = sb + t * TS;
-    const int ns = min(TS, se - s0);
-    const int b = t & 1;
-    const uint32_t bw = (uint32_t)(ns * CP * sizeof(float)), bp = (uint32_t)(ns * sizeof(float4));
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(&bar[b], bw + bp);
-    bulk_g2s(sW + b * TS * CP, a.Winf + (size_t)s0 * CP, bw, &bar[b]);
-    bulk_g2s(sP + b * TS, a.slot_xyz + s0, bp, &bar[b]);
-  };
-  if (tid == 0 && ntile > 0) issue(0);
-  constexpr int C2 = (C + 1) / 2;  // coefficient pairs (packed f32x2 arithmetic)
-  const int CS = a.cstride;        // FP32 row stride of one right-hand side (even)
-  f2_t acc[NB][C2];
-  for (int t = 0; t < ntile; ++t) {
-    if (tid == 0 && t + 1 < ntile) issue(t + 1);
-    const bool ok = mbar_wait(&bar[t & 1], (uint32_t)((t >> 1) & 1));
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) atomicExch(a.err, 1);
-      return;
-    }
-    const int s0 = sb + t * TS;
-    const int ns = min(TS, se - s0);
-    const float4* P = sP + (t & 1) * TS;
-    const float* Wt = sW + (t & 1) * TS * CP;
-    if (act) {
-#pragma unroll
-      for (int b = 0; b < NB; ++b)
-#pragma unroll
-        for (int c = 0; c < C2; ++c) acc[b][c] = 0ull;
-      const float* Kcol = STORED ? a.Kmat + kmat_index(s0, slot, a.Kld) : nullptr;  // next source: +RTE_KBLK
-      float k0 = 0.f, k1 = 0.f;
-      if (STORED) {
-        k0 = __ldg(Kcol);
-        if (ns > 1) k1 = __ldg(Kcol + RTE_KBLK);
-      }
-      // stored kernel with exact SH: no per-pair branch (the diagonal and pairs beyond the coupling
-      // distance carry k = 0), so two sources' SH recurrences can interleave
-      constexpr bool FLAT = STORED && !TABLE;
-      constexpr int UNR = FLAT ? 3 : 1;
-#pragma unroll UNR
-      for (int sv = 0; sv < ns; ++sv) {
-        float kk = 0.f;
-        if (STORED) {
-          kk = k0;
-          k0 = k1;
-          if (sv + 2 < ns) k1 = __ldg(Kcol + (size_t)(sv + 2) * RTE_KBLK);
-        }
-        const float4 q = P[sv];
-        const float ddx = (me.x - q.x) * dxf, ddy = (me.y - q.y) * dyf, ddz = (me.z - q.z) * dzf;
-        const float d2 = fmaf(ddx, ddx, fmaf(ddy, ddy, ddz * ddz));
-        bool live;
-        float dist = 0.f;
-        if (STORED) {
-          live = FLAT || kk != 0.f;
-        } else {
-          dist = sqrtf(d2);
-          live = d2 > 0.f && dist < thr;
-        }
-        if (live) {
-          ShT R[C];
-          if (TABLE) {
-            // A^T: snap(source - destination), negated in integers (a zero component stays +0.0)
-            const int sg = a.transpose ? -1 : 1;
-            const double ex = (double)(sg * (k - (int)q.x)) * a.dx, ey = (double)(sg * (j - (int)q.y)) * a.dy,
-                         ez = (double)(sg * (i - (int)q.z)) * a.dz;
-            double ux, uy, uz;
-            table_direction(ex, ey, ez, sqrt(ex * ex + ey * ey + ez * ez), ux, uy, uz);
-            sh_eval_monic<LA, ShT>((ShT)ux, (ShT)uy, (ShT)uz, R);  // A^T: snap(source - destination)
-          } else {
-            const float inv = FLAT ? (d2 > 0.f ? rsqrtf(d2) : 0.f) : rsqrtf(d2);
-            sh_eval_monic<LA, ShT>((ShT)(ddx * inv), (ShT)(ddy * inv), (ShT)(ddz * inv), R);
-          }
-          if (!STORED) {
-            int Q;
-            const float ps = path_sum<float, float>(i, j, k, (int)q.z, (int)q.y, (int)q.x, a.mutf, a.nx, plane, Q);
-            kk = __expf(-ps * dist / (float)Q) * kscalef / d2;
-          }
-          f2_t R2[C2];
-#pragma unroll
-          for (int c = 0; c < C2; ++c) R2[c] = f2_pack((float)R[2 * c], 2 * c + 1 < C ? (float)R[2 * c + 1] : 0.f);
-          if constexpr (CPLX) {
-            float Sv[2];
-#pragma unroll
-            for (int b = 0; b < 2; ++b) {
-              const f2_t* w = reinterpret_cast<const f2_t*>(Wt + sv * CP + b * CS);
-              f2_t Sa = 0ull, Sb = 0ull;
-#pragma unroll
-              for (int c = 0; c < C2; c += 2) {
-                Sa = f2_fma(R2[c], w[c], Sa);
-                if (c + 1 < C2) Sb = f2_fma(R2[c + 1], w[c + 1], Sb);
-              }
-              float a0, a1, b0, b1;
-              f2_unpack(Sa, a0, a1);
-              f2_unpack(Sb, b0, b1);
-              Sv[b] = (a0 + a1) + (b0 + b1);
-            }
-            float sn, cs;
-            sincosf((float)a.kappa * sqrtf(d2), &sn, &cs);
-            const float t0 = kk * (cs * Sv[0] + sn * Sv[1]), t1 = kk * (cs * Sv[1] - sn * Sv[0]);
-            const f2_t T0 = f2_pack(t0, t0), T1 = f2_pack(t1, t1);
-#pragma unroll
-            for (int c = 0; c < C2; ++c) {
-              acc[0][c] = f2_fma(R2[c], T0, acc[0][c]);
-              acc[NB - 1][c] = f2_fma(R2[c], T1, acc[NB - 1][c]);
-            }
-          } else {
-#pragma unroll
-          for (int b = 0; b < NB; ++b) {
-            const f2_t* w = reinterpret_cast<const f2_t*>(Wt + sv * CP + b * CS);
-            f2_t Sa = 0ull, Sb = 0ull;
-#pragma unroll
-            for (int c = 0; c < C2; c += 2) {
-              Sa = f2_fma(R2[c], w[c], Sa);
-              if (c + 1 < C2) Sb = f2_fma(R2[c + 1], w[c + 1], Sb);
-            }
-            float a0, a1, b0, b1;
-            f2_unpack(Sa, a0, a1);
-            f2_unpack(Sb, b0, b1);
-            const float tb = kk * ((a0 + a1) + (b0 + b1));
-            const f2_t T2 = f2_pack(tb, tb);
-#pragma unroll
-            for (int c = 0; c < C2; ++c) acc[b][c] = f2_fma(R2[c], T2, acc[b][c]);
-          }
-          }
-        }
-      }
-#pragma unroll
-      for (int b = 0; b < NB; ++b)
-#pragma unroll
-        for (int c = 0; c < C2; ++c) {
-          float lo, hi;
-          f2_unpack(acc[b][c], lo, hi);
-          sAcc[(b * C + 2 * c) * T + tid] += lo;
-          if (2 * c + 1 < C) sAcc[(b * C + 2 * c + 1) * T + tid] += hi;
-        }
-    }
-    __syncthreads();  // buffer t & 1 is free for tile t + 2
-  }
-  if (act) {
-    const int vstride = NB * a.Cfull;
-    double* o = a.part + ((size_t)blockIdx.y * a.N + r) * vstride;
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-#pragma unroll
-      for (int c = 0; c < C; ++c) o[b * a.Cfull + c] = (double)sAcc[(b * C + c) * T + tid] * kMonic.N[c];
-  }
-}
-
-// Stored pair kernel with exact directions (the benchmark's form): the kernel values of each 32-source
-// tile for the CTA's 128 destinations are one contiguous block of the blocked K layout (kmat_index) and
-// arrive by bulk copy on the same mbarrier as the tile's FP32 rows and coordinates, so the pair loop
-// reads K from shared memory instead of waiting on a global load per source.  The FP32 accumulators stay
-// in registers across the chunk's tiles (the chunks are summed in FP64 by the epilogue), which frees the
-// shared-memory accumulator and leaves room for the K tiles.
-// The source tile size TS (32 or 64) is chosen per shape by the autotuner (PairArgs::tile).
-struct TkLayout {
-  size_t off_w, off_k, off_bar, bytes;
-  __host__ __device__ TkLayout(int cpad, int ts) {
-    off_w = sizeof(float4) * 2 * ts;
-    off_k = off_w + sizeof(float) * 2 * ts * (size_t)cpad;  // cpad is a multiple of 4: 16-byte aligned
-    off_bar = off_k + sizeof(float) * 2 * ts * RTE_KBLK;
-    bytes = off_bar + 2 * sizeof(uint64_t);
-  }
-};
-
-template <int LA, int NB, int TS>
-__global__ void __launch_bounds__(RTE_PAIR_THREADS) k_pair_mixed_tk(PairArgs a) {
-  static_assert(RTE_PAIR_THREADS == RTE_KBLK, "one K block per CTA");
-  constexpr int C = (LA + 1) * (LA + 1), T = RTE_PAIR_THREADS;
-  typedef typename std::conditional<(LA >= 7), double, float>::type ShT;
-  // 16-byte source-row loads, except for wide L = 7 rows where the extra registers cost more than the
-  // loads save (33^3 L=7, 2 RHS: 30.1 -> 33.8 ms per launch with them)
-  constexpr bool V4 = LA < 7 || NB == 1;
-  const int CP = a.cpad;
-  const TkLayout Sh(CP, TS);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float4* sP = reinterpret_cast<float4*>(smem_raw);
-  float* sW = reinterpret_cast<float*>(smem_raw + Sh.off_w);
-  float* sK = reinterpret_cast<float*>(smem_raw + Sh.off_k);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + Sh.off_bar);
-  const int tid = threadIdx.x;
-  const int slot = blockIdx.x * T + tid;
-  const bool act = slot < a.N;
-  const float4 me = a.slot_xyz[act ? slot : 0];
-  const int r = __float_as_int(me.w);
-  const float dxf = (float)a.dx, dyf = (float)a.dy, dzf = (float)a.dz;
-  const int sb = blockIdx.y * a.chunk;
-  const int se = min(a.N, sb + a.chunk);
-  const int ntile = (se - sb + TS - 1) / TS;
-  if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  const float* Kblk = a.Kmat + kmat_index(0, (size_t)blockIdx.x * T, a.Kld);  // this CTA's destination block
-  auto issue = [&](int t) {  // tile t -> buffer t & 1 (one thread)
-    const int s0 = sb + t * TS;
-    const int ns = min(TS, se - s0);
-    const int b = t & 1;
-    const uint32_t bw = (uint32_t)(ns * CP * sizeof(float)), bp = (uint32_t)(ns * sizeof(float4)),
-                   bk = (uint32_t)(ns * RTE_KBLK * sizeof(float));
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(&bar[b], bw + bp + bk);
-    bulk_g2s(sW + b * TS * CP, a.Winf + (size_t)s0 * CP, bw, &bar[b]);
-    bulk_g2s(sP + b * TS, a.slot_xyz + s0, bp, &bar[b]);
-    bulk_g2s(sK + b * TS * RTE_KBLK, Kblk + (size_t)s0 * RTE_KBLK, bk, &bar[b]);
-  };
-  if (tid == 0 && ntile > 0) issue(0);
-  constexpr int C2 = (C + 1) / 2;  // coefficient pairs (packed f32x2 arithmetic)
-  const int CS = a.cstride;        // FP32 row stride of one right-hand side (a multiple of 4)
-  f2_t acc[NB][C2];
-#pragma unroll
-  for (int b = 0; b < NB; ++b)
-#pragma unroll
-    for (int c = 0; c < C2; ++c) acc[b][c] = 0ull;
-  for (int t = 0; t < ntile; ++t) {
-    if (tid == 0 && t + 1 < ntile) issue(t + 1);
-    const bool ok = mbar_wait(&bar[t & 1], (uint32_t)((t >> 1) & 1));
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) atomicExch(a.err, 1);
-      return;
-    }
-    const int ns = min(TS, se - (sb + t * TS));
-    const float4* P = sP + (t & 1) * TS;
-    const float* Wt = sW + (t & 1) * TS * CP;
-    const float* Kt = sK + (t & 1) * TS * RTE_KBLK + tid;
-    if (act) {
-      // no per-pair branch: the diagonal and pairs beyond the coupling distance carry K = 0
-#pragma unroll 4
-      for (int sv = 0; sv < ns; ++sv) {
-        const float kk = Kt[sv * RTE_KBLK];
-        const float4 q = P[sv];
-        const float ddx = (me.x - q.x) * dxf, ddy = (me.y - q.y) * dyf, ddz = (me.z - q.z) * dzf;
-        const float d2 = fmaf(ddx, ddx, fmaf(ddy, ddy, ddz * ddz));
-        const float inv = d2 > 0.f ? rsqrtf(d2) : 0.f;
-        ShT R[C];
-        sh_eval_monic<LA, ShT>((ShT)(ddx * inv), (ShT)(ddy * inv), (ShT)(ddz * inv), R);
-        f2_t R2[C2];
-#pragma unroll
-        for (int c = 0; c < C2; ++c) R2[c] = f2_pack((float)R[2 * c], 2 * c + 1 < C ? (float)R[2 * c + 1] : 0.f);
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-          // broadcast loads of the source row (CS and CP are multiples of 4 floats; the padding beyond C
-          // is zero)
-          f2_t Sa = 0ull, Sb = 0ull;
-          if constexpr (V4) {
-            const float4* w4 = reinterpret_cast<const float4*>(Wt + sv * CP + b * CS);
-#pragma unroll
-            for (int c = 0; c < C2; c += 2) {
-              const float4 v = w4[c / 2];
-              Sa = f2_fma(R2[c], f2_pack(v.x, v.y), Sa);
-              if (c + 1 < C2) Sb = f2_fma(R2[c + 1], f2_pack(v.z, v.w), Sb);
-            }
-          } else {
-            const f2_t* w = reinterpret_cast<const f2_t*>(Wt + sv * CP + b * CS);
-#pragma unroll
-            for (int c = 0; c < C2; c += 2) {
-              Sa = f2_fma(R2[c], w[c], Sa);
-              if (c + 1 < C2) Sb = f2_fma(R2[c + 1], w[c + 1], Sb);
-            }
-          }
-          float a0, a1, b0, b1;
-          f2_unpack(Sa, a0, a1);
-          f2_unpack(Sb, b0, b1);
-          const float tb = kk * ((a0 + a1) + (b0 + b1));
-          const f2_t T2 = f2_pack(tb, tb);
-#pragma unroll
-          for (int c = 0; c < C2; ++c) acc[b][c] = f2_fma(R2[c], T2, acc[b][c]);
-        }
-      }
-    }
-    __syncthreads();  // buffer t & 1 is free for tile t + 2
-  }
-  if (act) {  // the chunk's FP32 sums as they are (the epilogue applies N_c after adding the chunks in FP64)
-    const int vstride = NB * a.Cfull;
-    float* o = a.partf + ((size_t)blockIdx.y * a.N + r) * vstride;
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-#pragma unroll
-      for (int c = 0; c < C2; ++c) {
-        float lo, hi;
-        f2_unpack(acc[b][c], lo, hi);
-        o[b * a.Cfull + 2 * c] = lo;
-        if (2 * c + 1 < C) o[b * a.Cfull + 2 * c + 1] = hi;
-      }
-  }
-}
-
-// Recomputed pair kernel for four right-hand sides at L >= 6 (exact directions, real rows), where four
-// right-hand sides' FP32 sums no longer fit one thread's registers: 256 threads per CTA, the 128
-// destinations of a K block twice over, thread group g = tid / 128 holding right-hand sides 2g and
-// 2g + 1.  The path walks are shared: the kernel values of the CTA's 128 destinations x a 32-source tile
-// go to shared memory, each group walking half of the tile's sources, so every pair is walked once for
-// the four right-hand sides instead of once per pair of them.  The walks for tile t + 1 are interleaved
-// with the projections of tile t (one walk after every second source), so each thread's instruction
-// stream mixes the integer walk with the FMA work as the one-group kernels do.  FP32 sums stay in
-// registers over the source chunk (FP32 chunk partials, as k_pair_mixed_tk).
-struct GrpLayout {
-  size_t off_w, off_k, off_bar, bytes;
-  __host__ __device__ GrpLayout(int cpad, int ts) {
-    off_w = sizeof(float4) * 2 * ts;
-    off_k = off_w + sizeof(float) * 2 * ts * (size_t)cpad;  // cpad is a multiple of 4: 16-byte aligned
-    off_bar = off_k + sizeof(float) * 2 * ts * RTE_KBLK;
-    bytes = off_bar + 2 * sizeof(uint64_t);
-  }
-};
-#define RTE_GRP_THREADS (2 * RTE_KBLK)
-#define RTE_GRP_TS 32
-
-template <int LA>
-__global__ void __launch_bounds__(RTE_GRP_THREADS, 1) k_pair_mixed_grp(PairArgs a) {
-  constexpr int C = (LA + 1) * (LA + 1), C2 = (C + 1) / 2, TS = RTE_GRP_TS, NBG = 2, HALF = TS / 2;
-  typedef typename std::conditional<(LA >= 7), double, float>::type ShT;
-  constexpr bool V4 = LA < 7;  // 16-byte row loads (the one-group rule for two right-hand sides)
-  const int CP = a.cpad;
-  const GrpLayout Sh(CP, TS);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float4* sP = reinterpret_cast<float4*>(smem_raw);
-  float* sW = reinterpret_cast<float*>(smem_raw + Sh.off_w);
-  float* sK = reinterpret_cast<float*>(smem_raw + Sh.off_k);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + Sh.off_bar);
-  const int tid = threadIdx.x;
-  const int d = tid & (RTE_KBLK - 1), g = tid / RTE_KBLK;
-  const int slot = blockIdx.x * RTE_KBLK + d;
-  const bool act = slot < a.N;
-  const float4 me = a.slot_xyz[act ? slot : 0];
-  const int r = __float_as_int(me.w);
-  const int plane = a.nx * a.ny;
-  const int i = (int)me.z, j = (int)me.y, k = (int)me.x;
-  const float dxf = (float)a.dx, dyf = (float)a.dy, dzf = (float)a.dz;
-  const float kscalef = (float)a.kscale, thr = (float)a.prop_thresh;
-  const int sb = blockIdx.y * a.chunk;
-  const int se = min(a.N, sb + a.chunk);
-  const int ntile = (se - sb + TS - 1) / TS;
-  if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  auto issue = [&](int t) {  // source rows and coordinates of tile t -> buffer t & 1 (one thread)
-    const int s0 = sb + t * TS;
-    const int ns = min(TS, se - s0);
-    const int b = t & 1;
-    const uint32_t bw = (uint32_t)(ns * CP * sizeof(float)), bp = (uint32_t)(ns * sizeof(float4));
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(&bar[b], bw + bp);
-    bulk_g2s(sW + b * TS * CP, a.Winf + (size_t)s0 * CP, bw, &bar[b]);
-    bulk_g2s(sP + b * TS, a.slot_xyz + s0, bp, &bar[b]);
-  };
-  // the pair kernel exp(-tau) dV/(cm r^2) of this destination and source q, as the one-group kernels
-  // recompute it (0 on the diagonal and beyond the coupling distance)
-  auto kval = [&](const float4 q) -> float {
-    const float ddx = (me.x - q.x) * dxf, ddy = (me.y - q.y) * dyf, ddz = (me.z - q.z) * dzf;
-    const float d2 = fmaf(ddx, ddx, fmaf(ddy, ddy, ddz * ddz));
-    const float dist = sqrtf(d2);
-    if (!(d2 > 0.f && dist < thr)) return 0.f;
-    int Q;
-    const float ps = path_sum<float, float>(i, j, k, (int)q.z, (int)q.y, (int)q.x, a.mutf, a.nx, plane, Q);
-    return __expf(-ps * dist / (float)Q) * kscalef / d2;
-  };
-  f2_t acc[NBG][C2];
-#pragma unroll
-  for (int b = 0; b < NBG; ++b)
-#pragma unroll
-    for (int c = 0; c < C2; ++c) acc[b][c] = 0ull;
-  if (ntile > 0) {
-    if (tid == 0) issue(0);
-    const bool ok = mbar_wait(&bar[0], 0u);
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) atomicExch(a.err, 1);
-      return;
-    }
-    if (tid == 0 && ntile > 1) issue(1);
-    const int ns0 = min(TS, se - sb);
-    if (act)
-      for (int h = 0; h < HALF; ++h) {
-        const int sv = g * HALF + h;
-        if (sv < ns0) sK[sv * RTE_KBLK + d] = kval(sP[sv]);
-      }
-    __syncthreads();
-  }
-  const int CS = a.cstride;  // FP32 row stride of one right-hand side (a multiple of 4)
-  for (int t = 0; t < ntile; ++t) {
-    const bool has_next = t + 1 < ntile;
-    bool ok = true;
-    if (has_next) ok = mbar_wait(&bar[(t + 1) & 1], (uint32_t)(((t + 1) >> 1) & 1));
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) atomicExch(a.err, 1);
-      return;
-    }
-    const int ns = min(TS, se - (sb + t * TS));
-    const int nsn = has_next ? min(TS, se - (sb + (t + 1) * TS)) : 0;
-    const float4* P = sP + (t & 1) * TS;
-    const float* Wt = sW + (t & 1) * TS * CP + 2 * g * CS;  // this group's two right-hand sides
-    const float* Kt = sK + (t & 1) * TS * RTE_KBLK + d;
-    const float4* Pn = sP + ((t + 1) & 1) * TS;
-    float* Kn = sK + ((t + 1) & 1) * TS * RTE_KBLK + d;
-    if (act) {
-      for (int sv = 0; sv < ns; ++sv) {
-        const float kk = Kt[sv * RTE_KBLK];
-        const float4 q = P[sv];
-        const float ddx = (me.x - q.x) * dxf, ddy = (me.y - q.y) * dyf, ddz = (me.z - q.z) * dzf;
-        const float d2 = fmaf(ddx, ddx, fmaf(ddy, ddy, ddz * ddz));
-        const float inv = d2 > 0.f ? rsqrtf(d2) : 0.f;
-        ShT R[C];
-        sh_eval_monic<LA, ShT>((ShT)(ddx * inv), (ShT)(ddy * inv), (ShT)(ddz * inv), R);
-        f2_t R2[C2];
-#pragma unroll
-        for (int c = 0; c < C2; ++c) R2[c] = f2_pack((float)R[2 * c], 2 * c + 1 < C ? (float)R[2 * c + 1] : 0.f);
-#pragma unroll
-        for (int b = 0; b < NBG; ++b) {
-          f2_t Sa = 0ull, Sb = 0ull;
-          if constexpr (V4) {
-            const float4* w4 = reinterpret_cast<const float4*>(Wt + sv * CP + b * CS);
-#pragma unroll
-            for (int c = 0; c < C2; c += 2) {
-              const float4 v = w4[c / 2];
-              Sa = f2_fma(R2[c], f2_pack(v.x, v.y), Sa);
-              if (c + 1 < C2) Sb = f2_fma(R2[c + 1], f2_pack(v.z, v.w), Sb);
-            }
-          } else {
-            const f2_t* w = reinterpret_cast<const f2_t*>(Wt + sv * CP + b * CS);
-#pragma unroll
-            for (int c = 0; c < C2; c += 2) {
-              Sa = f2_fma(R2[c], w[c], Sa);
-              if (c + 1 < C2) Sb = f2_fma(R2[c + 1], w[c + 1], Sb);
-            }
-          }
-          float a0, a1, b0, b1;
-          f2_unpack(Sa, a0, a1);
-          f2_unpack(Sb, b0, b1);
-          const float tb = kk * ((a0 + a1) + (b0 + b1));
-          const f2_t T2 = f2_pack(tb, tb);
-#pragma unroll
-          for (int c = 0; c < C2; ++c) acc[b][c] = f2_fma(R2[c], T2, acc[b][c]);
-        }
-        if ((sv & 1) == 0) {  // one walk of the next tile after every second source
-          const int svn = g * HALF + (sv >> 1);
-          if (svn < nsn) Kn[svn * RTE_KBLK] = kval(Pn[svn]);
-        }
-      }
-      // a short last tile leaves walks of the next tile undone only when there is no next tile
-    }
-    __syncthreads();  // tile t's buffers are free, tile t + 1's kernel values complete
-    if (tid == 0 && t + 2 < ntile) issue(t + 2);
-  }
-  if (act) {  // the chunk's FP32 sums (the epilogue applies N_c after adding the chunks in FP64)
-    const int vstride = 2 * NBG * a.Cfull;
-    float* o = a.partf + ((size_t)blockIdx.y * a.N + r) * vstride + (size_t)(NBG * g) * a.Cfull;
-#pragma unroll
-    for (int b = 0; b < NBG; ++b)
-#pragma unroll
-      for (int c = 0; c < C2; ++c) {
-        float lo, hi;
-        f2_unpack(acc[b][c], lo, hi);
-        o[b * a.Cfull + 2 * c] = lo;
-        if (2 * c + 1 < C) o[b * a.Cfull + 2 * c + 1] = hi;
-      }
-  }
-}
-
-// Launch wrappers.  k_pair_mixed_3 carries a 3-CTA register bound and is used for L = 7 with one
-// right-hand side only; an explicit minimum-block count on the others makes ptxas take more registers
-// (L = 5, 2 RHS: 218 instead of 164, two CTAs per SM instead of three, 13.2 -> 17.0 ms per launch).
-template <int LA, bool TABLE, bool STORED, int NB, bool CPLX>
-__global__ void __launch_bounds__(RTE_PAIR_THREADS) k_pair_mixed(PairArgs a) {
-  pair_mixed_body<LA, TABLE, STORED, NB, CPLX>(a);
-}
-template <int LA, bool TABLE, bool STORED, int NB, bool CPLX>
-__global__ void __launch_bounds__(RTE_PAIR_THREADS, 3) k_pair_mixed_3(PairArgs a) {
-  pair_mixed_body<LA, TABLE, STORED, NB, CPLX>(a);
-}
-
-// Pair-kernel precompute K[s][d] = exp(-tau) dV/(cm |r_d - r_s|^2) over destination slots d and
-// source slots s (0 on the diagonal and beyond propThresh), path sums in FP32 (T = float, into Kmat)
-// or FP64 (T = double, into Kmat64, for the FP64 method).  K is symmetric: one CTA computes a 64x64
-// tile with source tile index <= destination tile index into shared memory and writes it and its
-// transpose with coalesced stores (a diagonal tile once).
-#define RTE_KT 64
-template <typename T>
-__global__ void __launch_bounds__(RTE_KT) k_store_kernel(PairArgs a) {
-  constexpr bool F64 = std::is_same<T, double>::value;
-  __shared__ T tile[RTE_KT][RTE_KT + 1];
-  __shared__ int sxyz[RTE_KT][3];
-  const int ntile = (a.N + RTE_KT - 1) / RTE_KT;
-  // linear CTA index -> (bs, bd) with bs <= bd, row-major over the upper triangle
-  long long t = blockIdx.x;
-  int bd = (int)((sqrt(8.0 * (double)t + 1.0) - 1.0) / 2.0);
-  while ((long long)(bd + 1) * (bd + 2) / 2 <= t) ++bd;
-  while ((long long)bd * (bd + 1) / 2 > t) --bd;
-  const int bs = (int)(t - (long long)bd * (bd + 1) / 2);
-  if (bd >= ntile) return;
-  const int tid = threadIdx.x;
-  const int plane = a.nx * a.ny;
-  const int s0 = bs * RTE_KT, d0 = bd * RTE_KT;
-  {
-    const int sl = s0 + tid;
-    const int v = sl < a.N ? a.perm[sl] : 0;
-    sxyz[tid][0] = v % a.nx;
-    sxyz[tid][1] = (v / a.nx) % a.ny;
-    sxyz[tid][2] = v / plane;
-  }
-  __syncthreads();
-  const int d = d0 + tid;
-  if (d < a.N) {
-    const int r = a.perm[d];
-    const int k = r % a.nx, j = (r / a.nx) % a.ny, i = r / plane;
-    const T dxf = (T)a.dx, dyf = (T)a.dy, dzf = (T)a.dz;
-    const T kscalef = (T)a.kscale, thr = (T)a.prop_thresh;
-    for (int q = 0; q < RTE_KT; ++q) {
-      T kk = T(0);
-      if (s0 + q < a.N) {
-        const int kp = sxyz[q][0], jp = sxyz[q][1], ip = sxyz[q][2];
-        const T ddx = (T)(k - kp) * dxf, ddy = (T)(j - jp) * dyf, ddz = (T)(i - ip) * dzf;
-        const T d2 = fma(ddx, ddx, fma(ddy, ddy, ddz * ddz));
-        const T dist = sqrt(d2);
-        if (d2 > T(0) && dist < thr) {
-          int Q;
-          if constexpr (F64) {
-            const double ps = path_sum<double, double>(i, j, k, ip, jp, kp, a.mut, a.nx, plane, Q);
-            kk = exp(-ps * dist / (double)Q) * kscalef / d2;
-          } else {
-            const float ps = path_sum<float, float>(i, j, k, ip, jp, kp, a.mutf, a.nx, plane, Q);
-            kk = __expf(-ps * dist / (float)Q) * kscalef / d2;
-          }
-        }
-      }
-      tile[tid][q] = kk;  // [destination][source]
-    }
-  }
-  __syncthreads();
-  // K(s, d): FP64 row-major [source slot][destination slot]; FP32 in 128-destination blocks
-  // (kmat_index).  Either way the 64 destinations of a tile row are contiguous (d0 is a multiple of 64).
-  auto at = [&](size_t sl, size_t d) -> T& {
-    if constexpr (F64)
-      return a.Kmat64[sl * a.Kld + d];
-    else
-      return a.Kmat[kmat_index(sl, d, a.Kld)];
-  };
-  for (int q = 0; q < RTE_KT; ++q) {
-    const int sl = s0 + q;
-    if (sl < a.N && d0 + tid < a.N) at(sl, d0 + tid) = tile[tid][q];
-  }
-  if (bs != bd) {
-    // K(d, s): the destination slots of this tile acting as sources
-    for (int q = 0; q < RTE_KT; ++q) {
-      const int dl = d0 + q;
-      if (dl < a.N && s0 + tid < a.N) at(dl, s0 + tid) = tile[q][tid];
-    }
-  }
-}
+#define RTE_KT 64  // slots per side of a back-projection tile
 
 // Weight of real coefficient c in the reference stop rule's layer sum, sum over m of Re(w_lm) in the
 // complex basis (dist.cu:1143-1152): for a real function R_l0 + sqrt2 R_l,m (even m > 0); for the
@@ -1262,8 +420,14 @@ __global__ void __launch_bounds__(256) k_epilogue(EpiArgs a, int Cact) {
       if (a.flag_scat) x *= a.scat[l] * a.mus[r];
     }
     a.Wout[t] = x;
-    // the mixed pair kernels read N_c W_c (monic SH, sh_eval_monic)
-    if (a.Woutf) a.Woutf[(size_t)a.islot[r] * a.cpad + (size_t)b * a.cstride + c] = (float)(x * kMonic.N[c]);
+    // the pair kernels read N_c W_c (monic SH, sh_eval_monic)
+    if (a.rows) {
+      const size_t o = ((size_t)b * a.N + a.islot[r]) * a.pitch + c;
+      if (a.rows64)
+        static_cast<double*>(a.rows)[o] = x * kMonic.N[c];
+      else
+        static_cast<float*>(a.rows)[o] = (float)(x * kMonic.N[c]);
+    }
     w2 += x * x;
     double sv = 0.0;
     if (a.sum) {
@@ -1500,16 +664,18 @@ __global__ void k_source(SrcArgs a) {
   if (a.fball_im) a.fball_im[off[ef] + p] = bi;
 }
 
-// mu_t = mu_a + mu_s (FP64 and FP32 copies), mu_s copy, and max(mu_t) into red_max (>= 0 values,
+// mu_t = mu_a + mu_s (FP64 and FP32 copies, in voxel and column order), mu_s copy, and max(mu_t) into red_max (>= 0 values,
 // so the bit pattern orders like the value).
-__global__ void k_medium(const double* mua, const double* mus, double* mut, double* mus_out, float* mutf, int N,
-                         double* red_max) {
+__global__ void k_medium(const double* mua, const double* mus, double* mut, double* mus_out, float* mutf, double* mutc,
+                         float* mutfc, const int* islot, int N, double* red_max) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   double m = 0.0;
   if (r < N) {
     m = mua[r] + mus[r];
     mut[r] = m;
     mutf[r] = (float)m;
+    mutc[islot[r]] = m;
+    mutfc[islot[r]] = (float)m;
     if (mus_out != mus) mus_out[r] = mus[r];
   }
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -1803,9 +969,9 @@ __global__ void __launch_bounds__(RTE_KT) k_bp_weights(BpArgs a) {
     if (d2 > T(0) && dist < thr) {
       T kk;
       if (a.Kmat64) {
-        kk = (T)__ldg(a.Kmat64 + (size_t)sl * a.Kld + d);
+        kk = (T)__ldg(a.Kmat64 + kmat_index(sl, kmat_pos(d, a.nz, a.nzp), a.Kld, a.group));
       } else if (a.Kmat) {
-        kk = (T)__ldg(a.Kmat + kmat_index(sl, d, a.Kld));
+        kk = (T)__ldg(a.Kmat + kmat_index(sl, kmat_pos(d, a.nz, a.nzp), a.Kld, a.group));
       } else {
         int Q0;
         const T ps = path_sum<T, double>(i, j, k, ip, jp, kp, a.mut, a.nx, plane, Q0);
@@ -1829,7 +995,7 @@ __global__ void __launch_bounds__(RTE_KT) k_bp_weights(BpArgs a) {
       }
       w = kk * (a1 * b1 + a2 * b2);
     }
-    const size_t idx = (size_t)sl * a.Kld + d;
+    const size_t idx = (size_t)sl * ((a.N + 31) / 32 * 32) + d;
     Qp[idx] = a.accumulate ? Qp[idx] + w : w;
   }
 }
@@ -1874,7 +1040,7 @@ __global__ void __launch_bounds__(RTE_BPW_THREADS) k_bp_walk(BpArgs a) {
       for (int q = 0; q < qend; ++q) {
         const int sl = s0 + q;
         if (sl >= a.N) break;
-        const T w = Qp[(size_t)sl * a.Kld + d];
+        const T w = Qp[(size_t)sl * ((a.N + 31) / 32 * 32) + d];
         if (w == T(0)) continue;
         const int kp = gx[q * 3 + 0], jp = gx[q * 3 + 1], ip = gx[q * 3 + 2];
         const T ddx = (T)(k - kp) * (T)a.dx, ddy = (T)(j - jp) * (T)a.dy, ddz = (T)(i - ip) * (T)a.dz;
@@ -2044,20 +1210,6 @@ __global__ void k_layer_sums(const double* W, const double* S, int N, int nx, in
   }
 }
 
-__global__ void k_to_f32_slots(const double* a, float* b, const int* islot, int N, int vstride, int cpad,
-                               int Cfull, int cstride) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (long long)N * vstride) return;
-  const int r = (int)(t / vstride), e = (int)(t % vstride);
-  const int rhs = e / Cfull, c = e - rhs * Cfull;
-  b[(size_t)islot[r] * cpad + (size_t)rhs * cstride + c] = (float)(a[t] * kMonic.N[c]);  // N_c W_c, see sh_eval_monic
-}
-
-__global__ void k_f64_to_f32(const double* a, float* b, size_t n) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = (float)a[i];
-}
-
 // ---------------------------------------------------------------------------------------------
 // launchers
 
@@ -2076,115 +1228,19 @@ static cudaError_t allow_smem(const void* kern, size_t smem) {
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
 }
 
-template <int LA, bool TABLE, bool STORED, int NB, bool CPLX = false>
-static cudaError_t launch_mixed(const PairArgs& a, cudaStream_t st, int* occ) {
-  if constexpr (!STORED && !TABLE && !CPLX && NB == 4 && LA >= 6) {  // shared walks, two groups of two
-    const size_t smem = GrpLayout(a.cpad, RTE_GRP_TS).bytes;
-    void (*kern)(PairArgs) = k_pair_mixed_grp<LA>;
-    cudaError_t e = allow_smem((const void*)kern, smem);
-    if (e != cudaSuccess) return e;
-    if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, RTE_GRP_THREADS, smem);
-    dim3 grid((a.N + RTE_KBLK - 1) / RTE_KBLK, a.nsplit);
-    kern<<<grid, RTE_GRP_THREADS, smem, st>>>(a);
-    return cudaGetLastError();
-  }
-  if constexpr (STORED && !TABLE && !CPLX) {  // K tiles staged with the source rows, 32 or 64 sources a tile
-    const int ts = a.tile ? 64 : 32;
-    const size_t smem = TkLayout(a.cpad, ts).bytes;
-    void (*kern)(PairArgs) = a.tile ? k_pair_mixed_tk<LA, NB, 64> : k_pair_mixed_tk<LA, NB, 32>;
-    cudaError_t e = allow_smem((const void*)kern, smem);
-    if (e != cudaSuccess) return e;
-    if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, RTE_PAIR_THREADS, smem);
-    dim3 grid((a.N + RTE_PAIR_THREADS - 1) / RTE_PAIR_THREADS, a.nsplit);
-    kern<<<grid, RTE_PAIR_THREADS, smem, st>>>(a);
-    return cudaGetLastError();
-  }
-  const size_t smem = MixedLayout(a.cpad, NB * (LA + 1) * (LA + 1), NB * (LA + 1) * (LA + 1) >= 128 ? 32 : RTE_PAIR_TS).bytes;
-  void (*kern)(PairArgs);
-  if constexpr (LA == 7 && NB == 1)
-    kern = k_pair_mixed_3<LA, TABLE, STORED, NB, CPLX>;
-  else
-    kern = k_pair_mixed<LA, TABLE, STORED, NB, CPLX>;
-  cudaError_t e = allow_smem((const void*)kern, smem);
-  if (e != cudaSuccess) return e;
-  if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, RTE_PAIR_THREADS, smem);
+cudaError_t rte_launch_pair_fp64(const PairArgs& a, int LA, cudaStream_t st) {
   dim3 grid((a.N + RTE_PAIR_THREADS - 1) / RTE_PAIR_THREADS, a.nsplit);
-  kern<<<grid, RTE_PAIR_THREADS, smem, st>>>(a);
-  return cudaGetLastError();
-}
-
-template <int LA, int NB>
-static cudaError_t launch_mixed_nb(const PairArgs& a, int table, int stored, cudaStream_t st, int* occ) {
-  if (table)
-    return stored ? launch_mixed<LA, true, true, NB>(a, st, occ) : launch_mixed<LA, true, false, NB>(a, st, occ);
-  return stored ? launch_mixed<LA, false, true, NB>(a, st, occ) : launch_mixed<LA, false, false, NB>(a, st, occ);
-}
-
-template <int LA>
-static cudaError_t launch_pair_LA(const PairArgs& a, int precision, int table, int stored, int nb, cudaStream_t st,
-                                  int* occ) {
-  if (a.kappa != 0.0) {  // one complex right-hand side (exact SH only)
-    if (table || nb != 2) return cudaErrorInvalidValue;
-    if (precision == 0) {
-      void (*kern)(PairArgs) = stored ? k_pair_fp64<LA, false, true, true> : k_pair_fp64<LA, false, true>;
-      if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, RTE_PAIR_THREADS, 0);
-      dim3 grid((a.N + RTE_PAIR_THREADS - 1) / RTE_PAIR_THREADS, a.nsplit);
-      kern<<<grid, RTE_PAIR_THREADS, 0, st>>>(a);
-      return cudaGetLastError();
-    }
-    return stored ? launch_mixed<LA, false, true, 2, true>(a, st, occ) : launch_mixed<LA, false, false, 2, true>(a, st, occ);
-  }
-  if (precision == 0) {
-    void (*kern)(PairArgs) = stored ? (table ? k_pair_fp64<LA, true, false, true> : k_pair_fp64<LA, false, false, true>)
-                                    : (table ? k_pair_fp64<LA, true, false> : k_pair_fp64<LA, false, false>);
-    if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, RTE_PAIR_THREADS, 0);
-    dim3 grid((a.N + RTE_PAIR_THREADS - 1) / RTE_PAIR_THREADS, a.nsplit);
-    kern<<<grid, RTE_PAIR_THREADS, 0, st>>>(a);
-    return cudaGetLastError();
-  }
-  switch (nb) {
-    case 1: return launch_mixed_nb<LA, 1>(a, table, stored, st, occ);
-    case 2: return launch_mixed_nb<LA, 2>(a, table, stored, st, occ);
-    case 4: return launch_mixed_nb<LA, 4>(a, table, stored, st, occ);
-  }
-  return cudaErrorInvalidValue;
-}
-
-static cudaError_t pair_dispatch(const PairArgs& a, int LA, int precision, int table, int stored, int nb,
-                                 cudaStream_t st, int* occ) {
   switch (LA) {
-    case 0: return launch_pair_LA<0>(a, precision, table, stored, nb, st, occ);
-    case 1: return launch_pair_LA<1>(a, precision, table, stored, nb, st, occ);
-    case 2: return launch_pair_LA<2>(a, precision, table, stored, nb, st, occ);
-    case 3: return launch_pair_LA<3>(a, precision, table, stored, nb, st, occ);
-    case 4: return launch_pair_LA<4>(a, precision, table, stored, nb, st, occ);
-    case 5: return launch_pair_LA<5>(a, precision, table, stored, nb, st, occ);
-    case 6: return launch_pair_LA<6>(a, precision, table, stored, nb, st, occ);
-    case 7: return launch_pair_LA<7>(a, precision, table, stored, nb, st, occ);
+    case 0: k_pair_fp64<0><<<grid, RTE_PAIR_THREADS, 0, st>>>(a); break;
+    case 1: k_pair_fp64<1><<<grid, RTE_PAIR_THREADS, 0, st>>>(a); break;
+    case 2: k_pair_fp64<2><<<grid, RTE_PAIR_THREADS, 0, st>>>(a); break;
+    case 3: k_pair_fp64<3><<<grid, RTE_PAIR_THREADS, 0, st>>>(a); break;
+    case 4: k_pair_fp64<4><<<grid, RTE_PAIR_THREADS, 0, st>>>(a); break;
+    case 5: k_pair_fp64<5><<<grid, RTE_PAIR_THREADS, 0, st>>>(a); break;
+    case 6: k_pair_fp64<6><<<grid, RTE_PAIR_THREADS, 0, st>>>(a); break;
+    case 7: k_pair_fp64<7><<<grid, RTE_PAIR_THREADS, 0, st>>>(a); break;
+    default: return cudaErrorInvalidValue;
   }
-  return cudaErrorInvalidValue;
-}
-
-cudaError_t rte_launch_pair(const PairArgs& a, int LA, int precision, int table, int stored, cudaStream_t st) {
-  return pair_dispatch(a, LA, precision, table, stored, a.nb > 0 ? a.nb : 1, st, nullptr);
-}
-
-cudaError_t rte_pair_occupancy(int LA, int precision, int table, int stored, int nb, int cpad, int* blocks_per_sm,
-                               int cplx, int tile) {
-  PairArgs dummy;
-  memset(&dummy, 0, sizeof dummy);
-  dummy.cpad = cpad;
-  dummy.kappa = cplx ? 1.0 : 0.0;
-  dummy.tile = tile;
-  return pair_dispatch(dummy, LA, precision, table, stored, nb, nullptr, blocks_per_sm);
-}
-
-cudaError_t rte_launch_store_kernel(const PairArgs& a, cudaStream_t st, int fp64) {
-  const long long nt = (a.N + RTE_KT - 1) / RTE_KT;
-  if (fp64)
-    k_store_kernel<double><<<(unsigned)(nt * (nt + 1) / 2), RTE_KT, 0, st>>>(a);
-  else
-    k_store_kernel<float><<<(unsigned)(nt * (nt + 1) / 2), RTE_KT, 0, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -2241,8 +1297,8 @@ cudaError_t rte_launch_source(const SrcArgs& a, cudaStream_t st) {
 }
 
 cudaError_t rte_launch_medium(const double* mua, const double* mus, double* mut, double* mus_out, float* mutf,
-                              int N, double* red_max, cudaStream_t st) {
-  k_medium<<<(N + 127) / 128, 128, 0, st>>>(mua, mus, mut, mus_out, mutf, N, red_max);
+                              double* mutc, float* mutfc, const int* islot, int N, double* red_max, cudaStream_t st) {
+  k_medium<<<(N + 127) / 128, 128, 0, st>>>(mua, mus, mut, mus_out, mutf, mutc, mutfc, islot, N, red_max);
   return cudaGetLastError();
 }
 
@@ -2255,18 +1311,6 @@ cudaError_t rte_launch_fma_peak(int fp64, int iters, float* sink, cudaStream_t s
     k_fma_peak<double><<<blocks, 256, 0, st>>>(iters, sink);
   else
     k_fma_peak<float><<<blocks, 256, 0, st>>>(iters, sink);
-  return cudaGetLastError();
-}
-
-cudaError_t rte_launch_to_f32_slots(const double* a, float* b, const int* islot, int N, int vstride, int cpad,
-                                    int Cfull, int cstride, cudaStream_t st) {
-  const long long n = (long long)N * vstride;
-  k_to_f32_slots<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a, b, islot, N, vstride, cpad, Cfull, cstride);
-  return cudaGetLastError();
-}
-
-cudaError_t rte_launch_f64_to_f32(const double* a, float* b, size_t n, cudaStream_t st) {
-  k_f64_to_f32<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a, b, n);
   return cudaGetLastError();
 }
 

@@ -129,7 +129,7 @@ extern "C" int rte_attenuate_noalloc(int nx, int ny, int nz, double dx, double d
     a.part = part;
     a.chunk = chunk;
     a.nsplit = S;
-    e = rte_launch_pair(a, nL, 0, 0, 0, st);
+    e = rte_launch_pair_fp64(a, nL, st);
     if (e != cudaSuccess) break;
     // partial sums -> output coefficients (the epilogue with no self term and no scatter)
     EpiArgs ep;

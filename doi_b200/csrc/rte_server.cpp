@@ -69,10 +69,13 @@ size_t estimate_bytes(const ShapeKey& k, int nsrc) {
   const size_t N = (size_t)k.n * k.n * k.n, C = (size_t)(k.L + 1) * (k.L + 1);
   const size_t nb = nsrc == 1 ? 1 : (nsrc <= 2 ? 2 : 4);
   size_t b = 8 * N * C * (24 + 14 * nb) + (64ull << 20);
-  if (k.prec == RTE_PREC_MIXED) {
-    b += 4 * ((N + 127) / 128 * 128) * ((N + 31) / 32 * 32);  // stored pair kernel (128-destination blocks)
-    b += 8 * N * C * nb * ((N + 1023) / 1024 + 8);            // partial sums of 1024-source chunks
-  }
+  // pair kernel: destination columns padded to whole groups (FP64: stored or recomputed in a 1 GB workspace), and
+  // the angle rows of every column displacement
+  const size_t nzp = k.n + 2, cells = N * ((size_t)k.n * k.n * nzp + 96);
+  const size_t row = 16 + (k.n + nzp + 3) * (k.L >= 7 ? 14 : 4);
+  b += k.prec == RTE_PREC_MIXED ? 4 * cells : std::min<size_t>(8 * cells, 1ull << 30);
+  b += (2 * (size_t)k.n) * (2 * (size_t)k.n) * row * 8;
+  if (k.prec == RTE_PREC_MIXED) b += 8 * N * C * nb * ((N + 1023) / 1024 + 8);  // chunk sums
   return b;
 }
 

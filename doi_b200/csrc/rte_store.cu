@@ -1,0 +1,335 @@
+// rte_store.cu -- the pair kernel K(r, r') = exp(-tau(r, r')) dV / (cm |r - r'|^2), tau the path integral of mu_t
+// between the voxel centres (FisherInfo_IO/src/kernels.cu:50-148 walks it per pair; rte_walk.cuh does).
+//
+// The voxels a path crosses and its lengths in them depend on the displacement alone, so a CTA takes all pairs of
+// columns at one column displacement (dx, dy), up to `npair` of them, and for every |dz| makes the list of
+// (voxel offset, length) once: the crossings of the three axes are arithmetic progressions, so each crossing's
+// rank, offset and length follow in closed form and the list is made in parallel.  A pair's integral is then one
+// load and one fused multiply-add per voxel crossed, the lanes of a warp taking pairs of the same |dz|.  Lengths
+// are integers over Q = 2 max(|dx|,1) max(|dy|,1) max(|dz|,1) and the sum runs in walking order from the
+// destination, as path_sum's.  The results of a column pair collect in shared memory and go out as runs of
+// destinations per source row; over all sources K is symmetric, so half of the displacements are computed and
+// written both ways.  mu_t is read from shared memory (in column order) when it fits, else through L1.
+//
+// Bound: instruction issue of the path sums (one add, one load, one multiply-add per voxel crossed) and the barriers
+// between lists, sums and write-out.  33^3 FP32: 22.8 ms by a walk per pair (70 % ALU) -> 9.2; FP64 35.3 -> 21;
+// 41^3 FP32: 96 -> 52.
+#include <cuda_runtime.h>
+#include <math.h>
+#include <stdint.h>
+#include <string.h>
+
+#include <algorithm>
+#include <type_traits>
+
+#include "rte_internal.h"
+
+namespace {
+
+constexpr int ST_THREADS = 512;
+// path sums per lane, of E column pairs: one list entry serves them all (33^3 FP32, mu_t in shared memory: 4 per lane
+// 10.1 ms, 6 9.2; 41^3 through L1: 4 50 ms, 6 55)
+template <typename T, bool STAGE>
+__host__ __device__ constexpr int st_e() {
+  return sizeof(T) == 4 && STAGE ? 6 : 4;
+}
+constexpr int ST_CAP = 3072;               // list entries per batch (one list has at most 3 * 1023 + 1)
+
+// A voxel of a path: its column offset and z steps from the destination (the sign of z is the pair's), and the
+// length in it.  The packed form holds column offsets of grids below 2^21 voxels.
+template <typename T, bool PACK>
+struct Entry;
+template <>
+struct __align__(8) Entry<float, true> {
+  int code;
+  float len;
+  __device__ void set(int oc, int oz) { code = oc * 1024 + oz; }
+  __device__ int oc() const { return code >> 10; }
+  __device__ int oz() const { return code & 1023; }
+};
+template <>
+struct __align__(16) Entry<float, false> {
+  int c, z;
+  float len, pad;
+  __device__ void set(int oc, int oz) { c = oc, z = oz; }
+  __device__ int oc() const { return c; }
+  __device__ int oz() const { return z; }
+};
+template <>
+struct __align__(16) Entry<double, false> {
+  int c, z;
+  double len;
+  __device__ void set(int oc, int oz) { c = oc, z = oz; }
+  __device__ int oc() const { return c; }
+  __device__ int oz() const { return z; }
+};
+
+// entries | tile [npair][zb][zb | 1] | per list: f1, f2 | per pair and z: kernel offset of the destination and of the
+// source column's position | per list: start | per pair: destination, source column | mu_t
+template <typename T, bool PACK>
+struct StLayout {
+  size_t off_tile, off_f, off_o, off_s, off_c, off_mu, bytes;
+  __host__ __device__ StLayout(int npair, int zb, int nz, int n_mu) {
+    off_tile = sizeof(Entry<T, PACK>) * ST_CAP;
+    off_f = (off_tile + sizeof(T) * npair * zb * (zb | 1) + 15) / 16 * 16;
+    off_o = off_f + sizeof(T) * 2 * nz;
+    off_s = off_o + sizeof(size_t) * 2 * npair * zb;
+    off_c = off_s + sizeof(int) * nz;
+    off_mu = (off_c + sizeof(int) * (2 * npair + 1) + 15) / 16 * 16;
+    bytes = off_mu + sizeof(T) * n_mu;
+  }
+};
+
+template <typename T, bool STAGE, bool PACK, int G>
+__global__ void __launch_bounds__(ST_THREADS, STAGE ? 1 : 2) k_store_lists(StoreArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int nx = a.nx, ny = a.ny, nz = a.nz, tid = threadIdx.x, wid = tid / 32, lane = tid % 32;
+  const StLayout<T, PACK> Sh(a.npair, a.zb, nz, STAGE ? a.N : 0);
+  Entry<T, PACK>* ent = reinterpret_cast<Entry<T, PACK>*>(smem_raw);
+  T* tile = reinterpret_cast<T*>(smem_raw + Sh.off_tile);
+  T* lf = reinterpret_cast<T*>(smem_raw + Sh.off_f);       // per |dz|: log2(e) dist / Q (exp2 argument), dV / (cm dist^2)
+  size_t* so = reinterpret_cast<size_t*>(smem_raw + Sh.off_o);
+  int* ls = reinterpret_cast<int*>(smem_raw + Sh.off_s);   // per |dz|: first entry
+  int* cols = reinterpret_cast<int*>(smem_raw + Sh.off_c);  // [npair] destination, [npair] source columns, count
+  T* smu = reinterpret_cast<T*>(smem_raw + Sh.off_mu);
+  constexpr int E = st_e<T, STAGE>();
+  const T* gmu = static_cast<const T*>(a.mu);
+  if constexpr (STAGE)
+    for (int q = tid; q < a.N; q += ST_THREADS) smu[q] = gmu[q];
+  const bool whole = a.col0 == 0 && a.col1 == nx * ny;
+  const int noff = whole ? (2 * nx - 1) * (ny - 1) + nx : (2 * nx - 1) * (2 * ny - 1);
+  const int y0 = a.col0 / nx, y1 = (a.col1 - 1) / nx;  // source rows
+  const int maxch = (nx * (y1 - y0 + 1) + a.npair - 1) / a.npair, ngrp = (maxch + a.group_ch - 1) / a.group_ch;
+  const int zb = a.zb, nblk = (nz + zb - 1) / zb, pitch = zb | 1;
+  const T dxf = (T)a.dx, dyf = (T)a.dy, dzf = (T)a.dz, thr = (T)a.prop_thresh;
+  for (long long w = blockIdx.x; w < (long long)noff * ngrp; w += gridDim.x) {
+    // neighbouring CTAs take neighbouring dx: their runs of destinations meet in L2
+    const int off = (int)(w % noff), ch0 = (int)(w / noff) * a.group_ch;
+    int dx, dy;  // destination minus source column
+    if (whole) {  // dy = 0, dx >= 0, then dy > 0
+      dy = off < nx ? 0 : (off - nx) / (2 * nx - 1) + 1;
+      dx = off < nx ? off : (off - nx) % (2 * nx - 1) - (nx - 1);
+    } else {
+      dy = off / (2 * nx - 1) - (ny - 1);
+      dx = off % (2 * nx - 1) - (nx - 1);
+    }
+    const int xa = max(0, -dx), wx = nx - abs(dx), ya = max(y0, -dy), yb = min(y1, ny - 1 - max(dy, 0));
+    const int np = wx * (yb - ya + 1);  // source columns xa.., ya.. of this displacement
+    if (yb < ya || ch0 * a.npair >= np) continue;
+    const int Dx = abs(dx), Dy = abs(dy), sxy = Dx + Dy;
+    const int mx = max(Dx, 1), my = max(Dy, 1);
+    const int stx = dx > 0 ? -nz : nz, sty = dy > 0 ? -nx * nz : nx * nz;  // steps towards the source
+    // one batch holds all lists of the displacement (ordinary grids): made once for the group's chunks
+    const bool once = nblk == 1 && nz * (sxy + 1) + nz * (nz - 1) / 2 <= ST_CAP;
+    for (int ch = ch0; ch < ch0 + a.group_ch && ch * a.npair < np; ++ch)
+    for (int bb = 0; bb < nblk * nblk; ++bb) {
+      // destination z in [d0, d1), source z in [s0, s1)
+      const int d0 = bb / nblk * zb, d1 = min(nz, d0 + zb), s0 = bb % nblk * zb, s1 = min(nz, s0 + zb);
+      const int amin = max(0, max(d0 - s1 + 1, s0 - d1 + 1)), amax = max(d1 - 1 - s0, s1 - 1 - d0);
+      __syncthreads();  // the previous tile, lists and columns are done with (and mu_t is staged)
+      if (wid == 0) {  // the chunk's column pairs, those of the slab's columns
+        const int pr = ch * a.npair + lane;
+        int cs = -1, cd = 0;
+        if (lane < a.npair && pr < np) {
+          const int xs = xa + pr % wx, ys = ya + pr / wx;
+          cs = ys * nx + xs;
+          cd = (ys + dy) * nx + xs + dx;
+          if (cs < a.col0 || cs >= a.col1) cs = -1;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, cs >= 0);
+        if (cs >= 0) {
+          const int n = __popc(m & ((1u << lane) - 1));
+          cols[n] = cd;
+          cols[a.npair + n] = cs;
+        }
+        if (lane == 0) cols[2 * a.npair] = __popc(m);
+      }
+      for (int a0 = amin; a0 <= amax;) {
+        int a1 = a0, total = 0;  // lists a0 .. a1 - 1 of this batch
+        while (a1 <= amax && total + sxy + a1 + 1 <= ST_CAP) total += sxy + a1++ + 1;
+        if (a0 > amin) __syncthreads();
+        if (!once || ch == ch0)
+        for (int da = a0 + wid; da < a1; da += ST_THREADS / 32) {
+          const int mz = max(da, 1), hx = my * mz, hy = mx * mz, hz = mx * my, Q = 2 * mx * hx;
+          const int first = (da - a0) * (sxy + 1) + (da * (da - 1) - a0 * (a0 - 1)) / 2, S = sxy + da;
+          if (lane == 0) {
+            ls[da] = first;
+            const T ex = (T)Dx * dxf, ey = (T)Dy * dyf, ez = (T)da * dzf;
+            const T d2 = fma(ex, ex, fma(ey, ey, ez * ez));
+            const double x = Dx * a.dx, y = Dy * a.dy, z = da * a.dz, r2 = x * x + y * y + z * z;
+            lf[2 * da] = (T)(-1.4426950408889634 * sqrt(r2) / (double)Q);
+            lf[2 * da + 1] = d2 > T(0) && sqrt(d2) < thr ? (T)(a.kscale / r2) : T(0);
+          }
+          // crossing n of an axis lies at (2 n + 1) h; ties step z, then y, then x
+          auto before = [](int t, int h, int D, bool ties) { return D ? (t + h - (ties ? 0 : 1)) / (2 * h) : 0; };
+          for (int e = lane; e <= S; e += 32) {
+            int t, cx, cy, cz;  // this crossing, and the crossings of each axis that precede it
+            if (e == S) {
+              t = Q, cx = Dx, cy = Dy, cz = da;
+            } else if (e < Dx) {
+              t = (2 * e + 1) * hx, cx = e, cy = before(t, hy, Dy, true), cz = before(t, hz, da, true);
+            } else if (e < sxy) {
+              t = (2 * (e - Dx) + 1) * hy, cy = e - Dx, cx = before(t, hx, Dx, false), cz = before(t, hz, da, true);
+            } else {
+              t = (2 * (e - sxy) + 1) * hz, cz = e - sxy, cx = before(t, hx, Dx, false), cy = before(t, hy, Dy, false);
+            }
+            const int prev = max(max((2 * cx - 1) * hx, (2 * cy - 1) * hy), max((2 * cz - 1) * hz, 0));
+            Entry<T, PACK> v;
+            v.set(cx * stx + cy * sty, cz);
+            v.len = (T)(t - prev);
+            ent[first + cx + cy + cz] = v;
+          }
+        }
+        __syncthreads();
+        const int npv = cols[2 * a.npair], jq = a.npair / E;  // lane element: (one of jq pairs) x E, z, sign of dz
+        for (int ab = a0, rot = wid; ab < a1; ab += 32) {
+          // lane l holds list a1 - 1 - (ab - a0) - l, the longest first: the pairs of z at dz = +|dz| and -|dz| and its tasks of 32 elements
+          const int da_l = a1 - 1 - (ab - a0) - lane;
+          int pl_l = 0, np_l = 0, ml_l = 0, nm_l = 0;
+          if (da_l >= a0) {
+            pl_l = max(d0, s0 + da_l);
+            np_l = max(0, min(d1, s1 + da_l) - pl_l);
+            ml_l = max(d0, s0 - da_l);
+            nm_l = da_l > 0 ? max(0, min(d1, s1 - da_l) - ml_l) : 0;
+          }
+          int incl = (jq * (np_l + nm_l) + 31) / 32;
+          const int own = incl;
+#pragma unroll
+          for (int o = 1; o < 32; o *= 2) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+          }
+          const int ntask = __shfl_sync(0xffffffffu, incl, 31);
+          int task = rot;
+          for (; task < ntask; task += ST_THREADS / 32) {
+            const int l = __ffs(__ballot_sync(0xffffffffu, incl > task)) - 1, da = a1 - 1 - (ab - a0) - l;
+            const int f0 = (task - __shfl_sync(0xffffffffu, incl - own, l)) * 32;
+            const int pl = __shfl_sync(0xffffffffu, pl_l, l), np_ = __shfl_sync(0xffffffffu, np_l, l);
+            const int ml = __shfl_sync(0xffffffffu, ml_l, l), per = np_ + __shfl_sync(0xffffffffu, nm_l, l);
+            const bool live = f0 + lane < jq * per;
+            const int f = live ? f0 + lane : 0, js = f / per, r = f - js * per;
+            const bool plus = r < np_;
+            const int z = plus ? pl + r : ml + r - np_, sg = plus ? -1 : 1;
+            uint32_t base[E];
+            T acc[E];
+#pragma unroll
+            for (int q = 0; q < E; ++q) {
+              base[q] = (uint32_t)(cols[min(q * jq + js, npv - 1)] * nz + z);
+              if constexpr (STAGE) base[q] = (uint32_t)Sh.off_mu + base[q] * (uint32_t)sizeof(T);  // byte offset: one add per load
+              acc[q] = T(0);
+            }
+            const T f1 = lf[2 * da], f2 = lf[2 * da + 1];
+            if (f2 != T(0)) {
+              const Entry<T, PACK>* le = ent + ls[da];
+              const int S = sxy + da;
+#pragma unroll 2
+              for (int e = 0; e <= S; ++e) {
+                const Entry<T, PACK> v = le[e];
+                const uint32_t at = (uint32_t)(v.oc() + sg * v.oz()) * (STAGE ? (uint32_t)sizeof(T) : 1u);
+#pragma unroll
+                for (int q = 0; q < E; ++q) {
+                  T mu;
+                  if constexpr (STAGE)
+                    mu = *reinterpret_cast<const T*>(smem_raw + (base[q] + at));
+                  else
+                    mu = __ldg(gmu + (base[q] + at));
+                  acc[q] = fma(mu, v.len, acc[q]);
+                }
+              }
+            }
+            if (!live) continue;
+            T* to = tile + (js * zb + (z + sg * da - s0)) * pitch + z - d0;  // [pair][source z][destination z]
+#pragma unroll
+            for (int q = 0; q < E; ++q) {
+              T k;
+              if constexpr (std::is_same<T, float>::value)
+                k = exp2f(acc[q] * f1) * f2;
+              else
+                k = exp2(acc[q] * f1) * f2;
+              to[q * jq * zb * pitch] = k;
+            }
+          }
+          rot = task - ntask;
+        }
+        a0 = a1;
+      }
+      __syncthreads();
+      // out: the source column's rows, and (all sources) the destination column's rows of the transpose
+      T* K = static_cast<T*>(a.K);
+      constexpr unsigned KB = 32 * G;
+      const unsigned nd = d1 - d0, ns = s1 - s0, md = ((1u << 20) + nd - 1) / nd, ms = ((1u << 20) + ns - 1) / ns;
+      const int npv = cols[2 * a.npair], src0 = a.col0 * nz;
+      for (unsigned e = tid; e < 2 * npv * (unsigned)zb; e += ST_THREADS) {  // kmat_index(0, position of column and z)
+        const unsigned jj = e / zb, zz = e - jj * zb, side = jj >= (unsigned)npv;
+        const int col = side ? cols[a.npair + jj - npv] : cols[jj];
+        const unsigned p = (unsigned)(col * a.nzp + (side ? s0 : d0)) + zz, o = p % KB;
+        so[(side * a.npair + (side ? jj - npv : jj)) * zb + zz] = (size_t)(p / KB) * a.Kld * KB + o % G * 32 + o / G;
+      }
+      __syncthreads();
+      for (unsigned e = tid; e < nd * ns; e += ST_THREADS) {
+        const unsigned zs = (e * md) >> 20, zd = e - zs * nd;  // e < 48^2
+        for (int j = 0; j < npv; ++j)
+          K[so[j * zb + zd] + (size_t)(unsigned)(cols[a.npair + j] * nz + s0 - src0 + (int)zs) * KB] =
+              tile[(j * zb + zs) * pitch + zd];
+      }
+      if (whole)
+        for (unsigned e = tid; e < nd * ns; e += ST_THREADS) {
+          const unsigned zd = (e * ms) >> 20, zs = e - zd * ns;
+          for (int j = 0; j < npv; ++j)
+            if (cols[j] != cols[a.npair + j])
+              K[so[(a.npair + j) * zb + zs] + (size_t)(unsigned)(cols[j] * nz + d0 + (int)zd) * KB] =
+                  tile[(j * zb + zs) * pitch + zd];
+        }
+    }
+  }
+}
+
+template <typename T, bool STAGE, bool PACK, int G>
+cudaError_t launch(StoreArgs a, int cap, int sms, cudaStream_t st) {
+  void (*kern)(StoreArgs) = k_store_lists<T, STAGE, PACK, G>;
+  typedef StLayout<T, PACK> Layout;
+  const int nblk = (a.nz + 47) / 48;
+  a.zb = (a.nz + nblk - 1) / nblk;
+  const size_t budget = STAGE && Layout(8, a.zb, a.nz, a.N).bytes > 110 * 1024 ? (size_t)cap : (size_t)110 * 1024;
+  constexpr int E = st_e<T, STAGE>();
+  a.npair = E;
+  while (a.npair + E <= 16 && Layout(a.npair + E, a.zb, a.nz, STAGE ? a.N : 0).bytes <= budget) a.npair += E;
+  const size_t smem = Layout(a.npair, a.zb, a.nz, STAGE ? a.N : 0).bytes;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
+  if (e != cudaSuccess) return e;
+  int occ = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, ST_THREADS, smem);
+  if (e != cudaSuccess) return e;
+  if (occ < 1) return cudaErrorInvalidConfiguration;
+  // chunks of column pairs that share one set of lists: as many as leave a few groups for every CTA
+  const long long rows = (a.col1 - 1) / a.nx - a.col0 / a.nx + 1, maxch = (a.nx * rows + a.npair - 1) / a.npair;
+  const long long noff = a.col0 == 0 && a.col1 == a.nx * a.ny ? (2 * a.nx - 1) * (a.ny - 1) + a.nx
+                                                               : (2ll * a.nx - 1) * (2 * a.ny - 1);
+  a.group_ch = (int)std::max<long long>(1, std::min<long long>(8, maxch * noff / (16ll * occ * sms)));
+  kern<<<occ * sms, ST_THREADS, smem, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <int G>
+cudaError_t launch_G(const StoreArgs& a, int fp64, int cap, int sms, cudaStream_t st) {
+  // mu_t in shared memory when 48 KB and more remain for tiles beside the lists
+  const size_t es = fp64 ? sizeof(double) : sizeof(float);
+  const size_t lists = ST_CAP * (fp64 ? sizeof(Entry<double, false>) : sizeof(Entry<float, true>));
+  const bool stage = es * a.N + lists + 48 * 1024 <= (size_t)cap;
+  if (fp64) return stage ? launch<double, true, false, G>(a, cap, sms, st) : launch<double, false, false, G>(a, cap, sms, st);
+  if (stage) return launch<float, true, true, G>(a, cap, sms, st);
+  return a.N < (1 << 21) ? launch<float, false, true, G>(a, cap, sms, st) : launch<float, false, false, G>(a, cap, sms, st);
+}
+
+}  // namespace
+
+cudaError_t rte_launch_store_kernel(const StoreArgs& a, cudaStream_t st, int fp64) {
+  int dev = 0, cap = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  if (a.group == 3) return launch_G<3>(a, fp64, cap, sms, st);
+  if (a.group == 2) return launch_G<2>(a, fp64, cap, sms, st);
+  return cudaErrorInvalidValue;
+}

@@ -42,10 +42,12 @@ extern "C" {
 #define RTE_PREC_MIXED 1 /* FP32 path integrals + SH projection, FP64 sums and norms */
 
 #define RTE_KERNEL_AUTO 0      /* mixed precision: store the voxel-pair kernel when it fits, else recompute;
-                                  FP64: recompute (the plain method) */
+                                  FP64: recompute (the plain method), keeping the kernel while it is no
+                                  larger than the recompute workspace (1 GB) */
 #define RTE_KERNEL_STORE 1     /* store exp(-tau)/r^2 per voxel pair in HBM (FP32 for mixed precision,
                                   FP64 for the FP64 method: 8 N^2 bytes) */
-#define RTE_KERNEL_RECOMPUTE 2 /* recompute path integrals every term */
+#define RTE_KERNEL_RECOMPUTE 2 /* recompute path integrals every term, in a workspace of at most 1 GB or one
+                                  column of sources */
 
 #define RTE_SRC_COLUMN 0 /* collimated pencil on the z=0 face, column containing (pos_x,pos_y) */
 #define RTE_SRC_FIM 1    /* FisherInfo_IO rule: column x == nX/2.0 && y == nY/2.0 (even grids only) */
