@@ -169,9 +169,6 @@ __device__ __forceinline__ void for_each_u(F f) {
   }
 }
 
-__device__ __forceinline__ void cp16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
 // sources per stage of the kernel-value ring (a multiple of G), and its stages
 template <int G>
 __host__ __device__ constexpr int ring_rows() {
@@ -179,10 +176,10 @@ __host__ __device__ constexpr int ring_rows() {
 }
 template <int G>
 __host__ __device__ constexpr int ring_stages() {
-  return G == 3 ? 3 : 4;
+  return G == 3 ? 2 : 4;
 }
 
-// Shared memory (elements of T): [2][NB][tz][pitch] source rows | [2][ncd][azn] azimuth values | [ncd][polar]
+// Shared memory (elements of T): [NB][tz][pitch] source rows | [2][ncd][azn] azimuth values | [ncd][polar]
 // polar values | [ncd][tz][NB][nb_row] contracted sources | [4 warps][stages][rows][32 G] kernel values |
 // 2 + 4 * stages mbarriers | the tensor-memory address, (x, y) of the destination columns
 struct ColLayout {
@@ -190,7 +187,7 @@ struct ColLayout {
   size_t off_bar, off_xy, bytes;
   __host__ __device__ ColLayout(int tz, int pitch, int azn, int polar, int ncd, int nbr, int nb, int ring, int stages,
                                 int esize) {
-    off_a = 2 * nb * tz * pitch;
+    off_a = nb * tz * pitch;
     off_t = off_a + 2 * ncd * azn;
     off_b = off_t + ncd * polar;
     off_k = off_b + ncd * tz * nbr;
@@ -209,8 +206,7 @@ __host__ __device__ constexpr int tmem_cols() {
 }
 
 // One CTA: 128 threads of G consecutive destinations of a column each, against the source columns of its
-// chunk, one run of tz sources of a column at a time (rows by bulk copy, double-buffered; angle rows by 16-byte
-// asynchronous copies).  What bounds it is the FMA pipe and, close behind, the shared memory's 128 bytes per
+// chunk, one run of tz sources of a column at a time.  What bounds it is the FMA pipe and, close behind, the shared memory's 128 bytes per
 // cycle: a value read by every lane of a warp costs as much as 32 different ones, so the contracted source row
 // (2L+1 numbers) is read once for G destinations, and since their displacements to consecutive sources overlap,
 // one new trigonometric row per source serves all G.  The pair kernel is streamed by bulk copies, a ring of
@@ -218,12 +214,15 @@ __host__ __device__ constexpr int tmem_cols() {
 // every load (5.9 ms against 2.7 at 33^3 L=5).  The coefficient sums, touched once per source column, live in
 // tensor memory, which leaves the registers of four CTAs per SM.  CPLX: (real, imaginary) rows of one complex
 // right-hand side, the pair kernel times exp(-i kappa r) (phase tabulated beside the angles).
-// 33^3 L=5 launch, FP32, one right-hand side: 7.40 ms by per-pair spherical harmonics -> 2.40; four: 20.1 -> 9.4;
-// FP64: 24.7 -> 5.4.  Of the 2.4 ms, skipping phases one at a time: pair loop 1.15, contraction 0.25, angle rows
-// 0.2, the kernel stream 0.15, the rest expansion, start of runs and barriers.
+// 33^3 L=5 launch, FP32, one right-hand side: 7.40 ms by per-pair spherical harmonics -> 2.36; four: 20.1 -> 9.3;
+// FP64: 24.7 -> 4.3.  Of the 2.4 ms, skipping phases one at a time: pair loop 1.15, contraction 0.25, angle rows
+// 0.2, the kernel stream 0.15, the rest expansion, start of runs and barriers.  All copies are bulk copies by warp 0
+// and by each warp for its own ring (copies by all threads: 2.40, FP64 5.4); deeper rings and a fifth of the
+// registers less did not pay (ring of 3 stages 2.37, four CTAs with 3-row stages 2.50).
 template <int L, typename T, int G, bool CPLX, bool FULL>
 __device__ __forceinline__ void column_body(const ColArgs& a) {
   constexpr int C = (L + 1) * (L + 1), NT = nb_row<L>(), NB = CPLX ? 2 : 1, LL = L > 0 ? L : 1;
+  constexpr bool SUB = G == 1;  // one destination of each thread of the layout's groups
   constexpr bool F32 = std::is_same<T, float>::value;
   constexpr int U = ring_rows<G>(), NST = ring_stages<G>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -241,20 +240,19 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
   const int tid = threadIdx.x, nz = a.nz, ncol = a.nx * a.ny;
   const int tile = blockIdx.x / a.nrhs, rhs = CPLX ? 0 : blockIdx.x - tile * a.nrhs;
   const int p0 = tile * T_CTA * G, np = ncol * a.nzp;  // destination positions: columns padded to nzp
-  // destination columns of the CTA (a complex pair's CTA: those of the layout's blocks that its warps lie in)
-  const int pa = CPLX ? p0 / (32 * a.group) * 32 * a.group : p0;
-  const int pb = CPLX ? ((p0 + T_CTA - 1) / (32 * a.group) + 1) * 32 * a.group : p0 + T_CTA * G;
+  // destination columns of the CTA (SUB: those of the layout's blocks that its warps lie in)
+  const int pa = SUB ? p0 / (32 * a.group) * 32 * a.group : p0;
+  const int pb = SUB ? ((p0 + T_CTA - 1) / (32 * a.group) + 1) * 32 * a.group : p0 + T_CTA * G;
   const int c0 = pa / a.nzp, ncd = (min(pb, np) - 1) / a.nzp - c0 + 1;
-  // a complex pair's kernel (G = 1) takes one destination of each thread of the layout's groups
-  const int pw = tile * (T_CTA / 32) + wid, pt = CPLX ? (pw / a.group * 32 + lane) * a.group + pw % a.group : p0 + tid * G;
+  const int pw = tile * (T_CTA / 32) + wid, pt = SUB ? (pw / a.group * 32 + lane) * a.group + pw % a.group : p0 + tid * G;
   const int p = min(pt, np - G);
   const bool act = pt < np;
   const int cd = p / a.nzp, z = p - cd * a.nzp, j = cd - c0;
   const int cb = a.col0 + blockIdx.y * a.chunk, ce = min(a.col1, cb + a.chunk);
   const int nrun = (nz + a.tz - 1) / a.tz, ntile = max(ce - cb, 0) * nrun;
   if (tid == 0) {
-    mbar_init(&bar[0], 1);
-    mbar_init(&bar[1], 1);
+    mbar_init(&bar[0], 1);  // a run's source rows and azimuth values
+    mbar_init(&bar[1], 1);  // its polar values
     for (int q = 0; q < T_CTA / 32 * NST; ++q) mbar_init(&bar[2 + q], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -270,8 +268,8 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
   // kernel values of this warp's destinations: rows of 32 * group per source slot
   const int kb = 32 * a.group;
   const T* gK = static_cast<const T*>(a.K) +
-                ((size_t)(CPLX ? pw / a.group : pw) * a.Kld) * kb + (CPLX ? pw % a.group * 32 : 0);
-  const bool wact = (CPLX ? pw / a.group * kb : pw * kb) < np;  // warps beyond the last block have no rows
+                ((size_t)(SUB ? pw / a.group : pw) * a.Kld) * kb + (SUB ? pw % a.group * 32 : 0);
+  const bool wact = (SUB ? pw / a.group * kb : pw * kb) < np;  // warps beyond the last block have no rows
   // a run: sources z0 .. z0 + tz of column col; the runs of a column follow one another
   struct Run {
     int col, xs, ys, z0;
@@ -285,62 +283,65 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
     }
     return r;
   };
-  auto issue = [&](const Run& r, int b) {  // source rows -> buffer b (one thread)
-    const int ns = min(a.tz, nz - r.z0), s0 = r.col * nz + r.z0;
-    const uint32_t bw = (uint32_t)(ns * a.pitch * sizeof(T));
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_expect_tx(&bar[b], NB * bw);
-#pragma unroll
-    for (int q = 0; q < NB; ++q)
-      bulk_g2s(sW + (b * NB + q) * a.tz * a.pitch, gW + ((size_t)q * a.N + s0) * a.pitch, bw, &bar[b]);
-  };
-  // angle rows of a run's column against each destination column (a warp per row): the azimuth values into
-  // buffer b, a run ahead; the polar values into their single buffer, read after the contraction
-  const int az16 = a.azn * (int)sizeof(T) / 16, po16 = (a.row - a.azn) * (int)sizeof(T) / 16;
+  // Copies by warp 0.  A run's source rows (one buffer, free after its contraction) and azimuth values (buffer b)
+  // come while the previous run's pairs are summed, its polar values (one buffer) while it is contracted.
   auto angle_row = [&](const Run& r, int jj) {
     const int xd = sxy[jj] & 0xffff, yd = sxy[jj] >> 16;
     return gT + ((size_t)(yd - r.ys + a.ny - 1) * (2 * a.nx - 1) + (xd - r.xs + a.nx - 1)) * a.row;
   };
-  auto copy16 = [&](T* dst, const T* src, int n) {
-    for (int e = lane; e < n; e += 32)
-      cp16(reinterpret_cast<unsigned char*>(dst) + e * 16, reinterpret_cast<const unsigned char*>(src) + e * 16);
-  };
-  auto azimuths = [&](const Run& r, int b) {
-    for (int jj = wid; jj < ncd; jj += T_CTA / 32) copy16(sA + (b * a.ncd + jj) * a.azn, angle_row(r, jj), az16);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+  const uint32_t azb = (uint32_t)(a.azn * sizeof(T)), pob = (uint32_t)((a.row - a.azn) * sizeof(T));
+  auto rows = [&](const Run& r, int b) {
+    const int ns = min(a.tz, nz - r.z0), s0 = r.col * nz + r.z0;
+    const uint32_t bw = (uint32_t)(ns * a.pitch * sizeof(T));
+    if (lane == 0) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      mbar_expect_tx(&bar[0], NB * bw + ncd * azb);
+#pragma unroll
+      for (int q = 0; q < NB; ++q) bulk_g2s(sW + q * a.tz * a.pitch, gW + ((size_t)q * a.N + s0) * a.pitch, bw, &bar[0]);
+    }
+    __syncwarp();
+    if (azb > 0)
+      for (int jj = lane; jj < ncd; jj += 32) bulk_g2s(sA + (b * a.ncd + jj) * a.azn, angle_row(r, jj), azb, &bar[0]);
   };
   auto polars = [&](const Run& r) {
-    for (int jj = wid; jj < ncd; jj += T_CTA / 32)
-      copy16(sT + jj * (a.row - a.azn), angle_row(r, jj) + a.azn, po16);
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    if (lane == 0) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      mbar_expect_tx(&bar[1], ncd * pob);
+    }
+    __syncwarp();
+    for (int jj = lane; jj < ncd; jj += 32)
+      bulk_g2s(sT + jj * (a.row - a.azn), angle_row(r, jj) + a.azn, pob, &bar[1]);
   };
-  // Ring of kernel values: group g of up to U sources (groups do not cross runs) in stage g % NST.
-  int i_src = cb * nz, i_z = 0, i_run = 0, i_grp = 0;  // cursor of the next group to copy
-  const int src_end = ce * nz;
+  // Ring of kernel values: groups of up to U sources (groups do not cross runs), one per stage.
+  const T* k_src = gK + (size_t)(cb * nz - a.kslot0) * kb;  // cursor of the next group to copy
+  int k_rem = max(ce - cb, 0) * nz, k_z = 0, k_left = min(a.tz, nz), k_st = 0, k_fly = 0;
   auto next_group = [&]() {
-    if (i_src >= src_end) return;
-    const int rows = min(U, min(a.tz - i_run, nz - i_z)), st = i_grp % NST;
+    if (k_rem <= 0) return;
+    const int n = min(U, k_left);
     if (wact) {
-      const T* src = gK + (size_t)(i_src - a.kslot0) * kb;
-      T* dst = sK + st * U * 32 * G;
+      T* dst = sK + k_st * U * 32 * G;
       if (lane == 0) {
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        mbar_expect_tx(&kbar[st], (uint32_t)(rows * 32 * G * sizeof(T)));
-        if constexpr (!CPLX) bulk_g2s(dst, src, (uint32_t)(rows * 32 * G * sizeof(T)), &kbar[st]);
+        mbar_expect_tx(&kbar[k_st], (uint32_t)(n * 32 * G * sizeof(T)));
+        if constexpr (!SUB) bulk_g2s(dst, k_src, (uint32_t)(n * 32 * G * sizeof(T)), &kbar[k_st]);
       }
-      if constexpr (CPLX) {
+      if constexpr (SUB) {
         __syncwarp();
-        if (lane < rows) bulk_g2s(dst + lane * 32, src + (size_t)lane * kb, 32 * sizeof(T), &kbar[st]);
+        if (lane < n) bulk_g2s(dst + lane * 32, k_src + (size_t)lane * kb, 32 * sizeof(T), &kbar[k_st]);
       }
     }
-    i_src += rows;
-    i_z += rows;
-    i_run += rows;
-    if (i_z == nz) i_z = 0, i_run = 0;
-    if (i_run == a.tz) i_run = 0;
-    ++i_grp;
+    ++k_fly;
+    k_src += n * kb;
+    k_rem -= n;
+    k_left -= n;
+    if (k_left == 0) {  // the next run
+      k_z = k_z + a.tz < nz ? k_z + a.tz : 0;
+      k_left = min(a.tz, nz - k_z);
+    }
+    if (++k_st == NST) k_st = 0;
   };
-  int grp = 0;  // next group to use
+  int u_st = 0;  // stage of the next group to use, and its phase
+  uint32_t u_ph = 0;
   bool kok = true;
   {  // the destinations' coefficient sums live in tensor memory, one row of C values per destination
     uint32_t zero[C * W32];
@@ -352,32 +353,31 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
   }
   Run cur{cb, cb % a.nx, cb / a.nx, 0};
   if (ntile > 0) {
-    if (tid == 0) issue(cur, 0);
-    azimuths(cur, 0);
-    polars(cur);
+    if (wid == 0) {
+      rows(cur, 0);
+      polars(cur);
+    }
     for (int q = 0; q < NST; ++q) next_group();
   }
   const int nmag = ((1 << 22) + min(a.tz, nz) - 1) / min(a.tz, nz);  // q / tz = q * nmag >> 22 (q * tz < 2^22)
   for (int t = 0; t < ntile; ++t) {
     const int bf = t & 1;
     const Run nxt = after(cur);
-    if (t + 1 < ntile) {
-      if (tid == 0) issue(nxt, bf ^ 1);
-    }
-    // groups in flight: this run's azimuth and polar values; only the polar ones may still be under way
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
-    const bool ok = mbar_wait(&bar[bf], (uint32_t)((t >> 1) & 1));
+    const bool ok = mbar_wait(&bar[0], (uint32_t)bf);
     if (__syncthreads_or(!ok || !kok)) {
-      if (tid == 0) atomicExch(a.err, 1);
-      if (t + 1 < ntile) mbar_wait(&bar[bf ^ 1], (uint32_t)(((t + 1) >> 1) & 1));  // copies in flight
-      for (; wact && grp < i_grp; ++grp) mbar_wait(&kbar[grp % NST], (uint32_t)((grp / NST) & 1));
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      if (tid == 0) {
+        atomicExch(a.err, 1);
+        mbar_wait(&bar[1], (uint32_t)bf);  // copies in flight
+      }
+      for (; wact && k_fly > 0; --k_fly) {
+        mbar_wait(&kbar[u_st], u_ph);
+        if (++u_st == NST) u_st = 0, u_ph ^= 1;
+      }
       __syncthreads();
       if (wid == 0) tmem_free(*stm, TMC);
       return;
     }
     const int z0 = cur.z0, ns = min(a.tz, nz - z0);
-    const T* Wt = sW + bf * NB * a.tz * a.pitch;
     const T* At = sA + bf * a.ncd * a.azn;
     // contract the run's sources onto the destination columns' meridians, two columns per row read
     // (neighbouring threads take neighbouring sources: rows are an odd number of 16-byte units apart, so the
@@ -385,7 +385,7 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
     for (int q = tid; q < (ncd + 1) / 2 * NB * a.tz; q += T_CTA) {
       const int jb = (int)(((long long)q * nmag) >> 22), s = q - jb * a.tz, jp = jb / NB, b = jb - jp * NB;
       if (s >= ns) continue;
-      const T* w = Wt + (b * a.tz + s) * a.pitch;
+      const T* w = sW + (b * a.tz + s) * a.pitch;
       T row[C];
       if constexpr (F32) {
 #pragma unroll
@@ -419,13 +419,9 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
         }
       }
     }
-    if (t + 1 < ntile) {
-      azimuths(nxt, bf ^ 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");  // this run's polar values
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
     __syncthreads();
+    if (wid == 0 && t + 1 < ntile) rows(nxt, bf ^ 1);
+    kok = mbar_wait(&bar[1], (uint32_t)bf) && kok;
     const T* B = sB + j * a.tz * NB * NT;
     typedef typename std::conditional<F32, f2_t, double2>::type Pair;
     Pair tr[G][LL];  // p_k (signed) of destination i, source sb + u at slot (i - u) mod G
@@ -553,9 +549,11 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
       turn(ap[u % G], ((G - 1 - u) % G + G) % G);
       ap[u % G] -= a.csn;
     };
-    for (int sb = 0; sb < ns; sb += U, ++grp) {
-      if (wact) kok = mbar_wait(&kbar[grp % NST], (uint32_t)((grp / NST) & 1)) && kok;
-      const T* Kt = sK + grp % NST * U * 32 * G + lane;
+    for (int sb = 0; sb < ns; sb += U) {
+      if (wact) kok = mbar_wait(&kbar[u_st], u_ph) && kok;
+      const T* Kt = sK + u_st * U * 32 * G + lane;
+      if (++u_st == NST) u_st = 0, u_ph ^= 1;
+      --k_fly;
       if (sb + U <= ns)
         for_each_u<U>([&](auto uc) { step(uc, sb + decltype(uc)::value, Kt); });
       else
@@ -590,7 +588,7 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
     tmem_wait_st();
     cur = nxt;
     __syncthreads();  // the contracted sources and buffer bf are free for run t + 2
-    if (t + 1 < ntile) polars(cur);
+    if (wid == 0 && t + 1 < ntile) polars(cur);
   }
   if (!kok && lane == 0) atomicExch(a.err, 1);
 #pragma unroll
@@ -715,8 +713,8 @@ cudaError_t launch_one(ColArgs a, cudaStream_t st, int* occ) {
   if constexpr (L >= RTE_FULL_L && std::is_same<T, float>::value)
     if (a.nz <= RTE_FULL_NZ) kern = k_column<L, T, G, CPLX, true>;
   const int np = a.nx * a.ny * a.nzp;
-  // positions a CTA's columns span: its threads' destinations, or the layout blocks of a complex pair's warps
-  const int span = CPLX ? ((T_CTA / 32 + a.group - 2) / a.group + 1) * 32 * a.group : T_CTA * G;
+  // positions a CTA's columns span: its threads' destinations, or (G = 1) the layout blocks of its warps
+  const int span = G == 1 ? ((T_CTA / 32 + a.group - 2) / a.group + 1) * 32 * a.group : T_CTA * G;
   a.ncd = (span + a.nzp - 2) / a.nzp + 1;
   // the whole column as one run when two CTAs fit an SM's shared memory, else equal runs
   size_t smem = 0;
@@ -730,26 +728,31 @@ cudaError_t launch_one(ColArgs a, cudaStream_t st, int* occ) {
   if (e != cudaSuccess) return e;
   if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, T_CTA, smem);
   const int nblk = (np + 32 * a.group - 1) / (32 * a.group);  // layout blocks: a warp each, or `group` warps for G = 1
-  const int warps = CPLX ? nblk * a.group : nblk;
+  const int warps = G == 1 ? nblk * a.group : nblk;
   dim3 grid((unsigned)((warps + T_CTA / 32 - 1) / (T_CTA / 32)) * a.nrhs, a.nsplit);
   kern<<<grid, T_CTA, smem, st>>>(a);
   return cudaGetLastError();
 }
 
-// Destinations per thread: RTE_COL_G; a complex pair's kernel takes one on the same layout.  A launch of a lower
+// Destinations per thread: RTE_COL_G; a complex pair's kernel may take one on the same layout (RTE_COL_GC).  A launch of a lower
 // order than the context's (l = 0 passes of isotropic scatter) runs on its layout, so order 0 takes any of them.
-template <int L, int G>
+template <int L, int G, int GC, int GC64>
 cudaError_t launch_G(const ColArgs& a, int fp64, int cplx, cudaStream_t st, int* occ) {
-  if (cplx) return fp64 ? launch_one<L, double, 1, true>(a, st, occ) : launch_one<L, float, 1, true>(a, st, occ);
+  if (cplx) return fp64 ? launch_one<L, double, GC64, true>(a, st, occ) : launch_one<L, float, GC, true>(a, st, occ);
   return fp64 ? launch_one<L, double, G, false>(a, st, occ) : launch_one<L, float, G, false>(a, st, occ);
 }
 
 template <int L>
 cudaError_t launch_L(const ColArgs& a, int fp64, int cplx, cudaStream_t st, int* occ) {
   if constexpr (L == 0) {
-    if (a.group == RTE_COL_G(RTE_MAX_L)) return launch_G<0, RTE_COL_G(RTE_MAX_L)>(a, fp64, cplx, st, occ);
+    switch (a.tg) {
+      case 1: return launch_G<0, 2, 1, 1>(a, fp64, cplx, st, occ);
+      case 2: return launch_G<0, 2, 2, 2>(a, fp64, cplx, st, occ);
+      default: return launch_G<0, 3, 3, 3>(a, fp64, cplx, st, occ);
+    }
+  } else {
+    return launch_G<L, RTE_COL_G(L), RTE_COL_GC(L, 0), RTE_COL_GC(L, 1)>(a, fp64, cplx, st, occ);
   }
-  return launch_G<L, RTE_COL_G(L)>(a, fp64, cplx, st, occ);
 }
 
 }  // namespace
@@ -768,7 +771,7 @@ ColDims rte_col_dims(int C, int L, int nz, int fp64, int cplx) {
   d.nk = fp64 ? 1 : (full ? L : 2);
   d.pho = cplx ? 2 * d.nk : 0;
   d.csn = 2 * d.nk + (cplx ? (fp64 ? 2 : 4) : 0);
-  d.tg = cplx ? 1 : d.group;
+  d.tg = cplx ? RTE_COL_GC(L, fp64) : d.group;
   d.cls = (nz + d.nzp + d.tg - 1) / d.tg;
   d.row = (d.azn + d.tg * d.cls * d.csn + unit - 1) / unit * unit;
   return d;

@@ -1047,6 +1047,7 @@ static ColArgs col_args(const rte_ctx* c, int nb, const void* K, size_t ld, int 
   a.csn = d.csn;
   a.cls = d.cls;
   a.pho = d.pho;
+  a.tg = d.tg;
   a.part = c->d_part;
   a.vstride = nb * c->C;
   a.col0 = col0;
@@ -1138,7 +1139,7 @@ static int plan_columns(rte_ctx* c, int LA, int nb, const void* K, size_t ld, in
   CUDA_TRY(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
   CUDA_TRY(c, rte_launch_column(col_args(c, nb, K, ld, 0, cols, cols, 0), LA, f, cplx, c->st, &occ));
   const ColDims d = col_dims(c);
-  const int rhs = cplx ? nb / 2 : nb, group = cplx ? 1 : d.group;
+  const int rhs = cplx ? nb / 2 : nb, group = d.tg;
   const long long tiles = (long long)((ncol * d.nzp + 128 * group - 1) / (128 * group)) * rhs;
   const long long slots = (long long)std::max(occ, 1) * sms;
   const int cap = f ? cols : std::min(cols, kChunkColumns);
@@ -1155,11 +1156,11 @@ static int plan_columns(rte_ctx* c, int LA, int nb, const void* K, size_t ld, in
     rank.push_back({waves * (chunk + 1) * col_us + S * part_us, chunk});
   }
   std::sort(rank.begin(), rank.end());
-  if (rank.size() > 4) rank.resize(4);
+  if (rank.size() > 6) rank.resize(6);
   int chunk = rank[0].second;
   const char* forced = getenv("RTE_NSPLIT");
   const char* at = getenv("RTE_AUTOTUNE");
-  const bool tune = !forced && !(at && at[0] == '0') && !c->capturing && !f && c->N >= 4096 && rank.size() > 1;
+  const bool tune = !forced && !(at && at[0] == '0') && !c->capturing && c->N >= 1024 && rank.size() > 1;
   if (forced) chunk = std::max(1, std::min(cap, (cols + std::max(1, atoi(forced)) - 1) / std::max(1, atoi(forced))));
   const TuneKey tk{c->cfg.device, c->nx, c->ny, c->nz, LA, nb, c->precision, cplx, cols};
   bool have = false;

@@ -23,6 +23,8 @@ __host__ __device__ inline int kmat_pos(int slot, int nz, int nzp) { return slot
 // Destinations per thread of the column kernels.  Three at L <= 5, where four CTAs per SM still fit (33^3 L=5 launch:
 // 2 per thread 2.93 ms, 3 2.41, 4 at two CTAs 3.11; FP64: 1 7.0 ms, 2 9.3, 3 5.6), two above.
 #define RTE_COL_G(L) ((L) <= 5 ? 3 : 2)
+// ... of a complex pair's kernel: the same, or one where two sets of sums exceed the registers
+#define RTE_COL_GC(L, fp64) ((L) <= ((fp64) ? 3 : 5) ? RTE_COL_G(L) : 1)
 
 struct PairArgs {
   int N, nx, ny, nz, Cfull;
@@ -71,7 +73,7 @@ struct ColArgs {
   size_t Kld;
   int kslot0;
   const void* tab;    // angle rows (rte_launch_col_table)
-  int row, azn, csn, cls, pho;
+  int row, azn, csn, cls, pho, tg;
   void* part;         // chunk sums [S][N][vstride]: FP32 raw, or FP64 with N_c applied
   int vstride;
   int split0;         // first chunk-sum slice
