@@ -256,6 +256,7 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
     for (int q = 0; q < T_CTA / 32 * NST; ++q) mbar_init(&bar[2 + q], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  if (blockIdx.x == 0 && blockIdx.y == 0 && tid < 4 && a.red) a.red[tid] = 0.0;
   constexpr int TMC = tmem_cols<L, T, G, CPLX>(), W32 = sizeof(T) / 4;
   if (wid == 0) tmem_alloc(stm, TMC);
   tmem_fence_before();

@@ -330,7 +330,6 @@ struct rte_ctx {
   void* d_slab = nullptr;       // recompute workspace: pair-kernel rows of slab_cols source columns
   size_t slab_bytes = 0;
   int slab_cols = 0;
-  double* d_selfp = nullptr;    // self-voxel term [N][nb][C]
   int* d_self_idx = nullptr;    // voxel -> distinct mu_t
   double* d_self_lut = nullptr; // [ndistinct][C][C]
   bool self_lut_ok = false;
@@ -345,7 +344,7 @@ struct rte_ctx {
   int bcap = 0;
   double *d_bW = nullptr, *d_bWn = nullptr, *d_bsum = nullptr, *d_bres = nullptr, *d_bball = nullptr;
   void* d_bWf = nullptr;
-  size_t part_cap = 0, selfp_cap = 0;
+  size_t part_cap = 0;
   // detectors and gradient
   double* d_h = nullptr;        // [6][C] face flux weights
   double *d_S = nullptr, *d_out = nullptr, *d_e = nullptr, *d_lam = nullptr, *d_y = nullptr;
@@ -485,7 +484,7 @@ static void free_all(rte_ctx* c) {
   for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
   void* ps[] = {c->d_perm, c->d_mut, c->d_mus, c->d_mutf, c->d_W, c->d_Wn, c->d_sum, c->d_part, c->d_mom,
                 c->d_aux1, c->d_aux2, c->d_aux3, c->d_aux4, c->d_Wf, c->d_K, c->d_K64, c->d_cplx, c->d_red, c->d_img,
-                c->d_selfp, c->d_self_idx, c->d_self_lut, c->d_islot, c->d_slot_xyz, c->d_err,
+                c->d_self_idx, c->d_self_lut, c->d_islot, c->d_slot_xyz, c->d_err,
                 c->d_bW, c->d_bWn, c->d_bsum, c->d_bres, c->d_bball, c->d_bWf, c->d_h, c->d_S, c->d_out,
                 c->d_e, c->d_lam, c->d_y, c->d_gt, c->d_gs, c->d_J, c->d_rho, c->d_dlut, c->d_fball, c->d_q, c->d_bq,
                 c->d_Qbp, c->d_mask, c->d_dmut, c->d_dmus, c->d_mut_self, c->d_mus_src, c->d_T, c->d_cidx, c->d_cval, c->d_self_lut_im,
@@ -595,9 +594,7 @@ int rte_create(const rte_config* cfg, rte_ctx** out) {
   if (rc == RTE_OK) cu(dalloc(c, &c->d_aux3, NC), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_aux4, NC), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_part, NC * c->max_split), "alloc");
-  if (rc == RTE_OK) cu(dalloc(c, &c->d_selfp, NC), "alloc");
   c->part_cap = NC * c->max_split;
-  c->selfp_cap = NC;
   if (rc == RTE_OK) cu(dalloc(c, &c->d_self_idx, c->N), "alloc");
   {  // room for FP64 rows in either precision (rte_fisher runs FP64 solves in mixed contexts)
     const size_t nrow = (size_t)c->N * rte_col_dims(c->C, c->L, c->nz, 1, 0).pitch;
@@ -1056,6 +1053,7 @@ static ColArgs col_args(const rte_ctx* c, int nb, const void* K, size_t ld, int 
   a.nsplit = (col1 - col0 + chunk - 1) / chunk;
   a.split0 = split0;
   a.err = c->d_err;
+  a.red = c->d_red;
   return a;
 }
 
@@ -1266,6 +1264,22 @@ static int ensure_fft(rte_ctx* c) {
   return RTE_OK;
 }
 
+// Self-voxel term of the distribution W (lut: the caller's, D or its derivative).
+static SelfArgs self_args(const rte_ctx* c, const double* W) {
+  SelfArgs a;
+  memset(&a, 0, sizeof a);
+  a.K = c->K;
+  a.W = W;
+  a.mut = self_mut(c);
+  a.idx = c->self_lut_ok ? c->d_self_idx : nullptr;
+  a.mom = c->d_mom;
+  a.scale = c->dV / c->cm;
+  a.air_no_self = c->model == RTE_MODEL_FIM ? 1 : 0;
+  a.kappa = c->kappa;
+  a.lut_im = c->d_self_lut_im;
+  return a;
+}
+
 static void* rows_of(const rte_ctx* c, int nb) { return nb == 1 ? c->d_Wf : c->d_bWf; }
 
 static int apply_term(rte_ctx* c, const double* in64, double* out, double* sum, int flag, int flag_scat, int nb = 1,
@@ -1287,29 +1301,7 @@ static int apply_term(rte_ctx* c, const double* in64, double* out, double* sum, 
     if (rc) return rc;
     f32part = c->precision == RTE_PREC_MIXED;
   }
-  SelfArgs sa;
-  memset(&sa, 0, sizeof sa);
-  sa.N = c->N;
-  sa.nb = nb;
-  sa.Cfull = c->C;
-  sa.Cact = (LA + 1) * (LA + 1);
-  sa.K = c->K;
-  sa.W = in64;
-  sa.mut = self_mut(c);
-  sa.idx = c->self_lut_ok ? c->d_self_idx : nullptr;
-  sa.lut = c->d_self_lut;
-  sa.mom = c->d_mom;
-  sa.scale = c->dV / c->cm;
-  sa.air_no_self = c->model == RTE_MODEL_FIM ? 1 : 0;
-  sa.out = c->d_selfp;
-  sa.kappa = c->kappa;
-  sa.lut_im = c->d_self_lut_im;
   if (c->kappa != 0.0 && nb % 2) return fail(c, RTE_ERR_STATE, "a modulated term needs (real, imaginary) row pairs");
-  if (LA < c->L) CUDA_TRY(c, cudaMemsetAsync(c->d_selfp, 0, (size_t)c->N * nb * c->C * sizeof(double), c->st));
-  {
-    ProfScope ps(c, 2);
-    CUDA_TRY(c, rte_launch_self(sa, c->st));
-  }
   EpiArgs e;
   memset(&e, 0, sizeof e);
   e.N = c->N;
@@ -1321,7 +1313,8 @@ static int apply_term(rte_ctx* c, const double* in64, double* out, double* sum, 
   e.nb = nb;
   e.part = c->d_part;
   e.partf = f32part ? reinterpret_cast<const float*>(c->d_part) : nullptr;
-  e.selfp = c->d_selfp;
+  e.self = self_args(c, in64);
+  e.self.lut = c->d_self_lut;
   e.mus = c->d_mus;
   e.flag_scat = flag_scat;
   scatter_factors(c, flag, e.scat);
@@ -1333,7 +1326,8 @@ static int apply_term(rte_ctx* c, const double* in64, double* out, double* sum, 
   e.sum = sum;
   e.red = c->d_red;
   e.cplx = c->kappa != 0.0 ? 1 : 0;
-  CUDA_TRY(c, cudaMemsetAsync(c->d_red, 0, 4 * sizeof(double), c->st));
+  if (fft_active(c))  // the column kernels zero the norms
+    CUDA_TRY(c, cudaMemsetAsync(c->d_red, 0, 4 * sizeof(double), c->st));
   {
     ProfScope ps(c, 2);
     CUDA_TRY(c, rte_launch_epilogue(e, LA, c->st));
@@ -2125,7 +2119,6 @@ static int grow(rte_ctx* c, T** p, size_t& cap, size_t n) {
 static int ensure_batch(rte_ctx* c, int nb) {
   const size_t NC = (size_t)c->N * c->C;
   int rc = grow(c, &c->d_part, c->part_cap, NC * nb * c->max_split);
-  if (!rc) rc = grow(c, &c->d_selfp, c->selfp_cap, NC * nb);
   if (rc || nb <= c->bcap) return rc;
   double** bufs[] = {&c->d_bW, &c->d_bWn, &c->d_bsum, &c->d_bres};
   for (double** b : bufs) {
@@ -2808,7 +2801,7 @@ static std::vector<uintptr_t> graph_signature(const rte_ctx* c, int nb) {
   const double* Wn = nb == 1 ? c->d_Wn : c->d_bWn;
   return {u(std::min(W, Wn)), u(std::max(W, Wn)), u(nb == 1 ? c->d_sum : c->d_bsum),
           u(nb == 1 ? c->d_aux2 : c->d_bres), u(nb == 1 ? c->d_Wf : c->d_bWf),
-          u(c->d_part), u(c->d_selfp), u(c->d_self_idx), u(c->d_self_lut), u(c->d_mom), (uintptr_t)c->K,
+          u(c->d_part), u(c->d_self_idx), u(c->d_self_lut), u(c->d_mom), (uintptr_t)c->K,
           (uintptr_t)c->self_lut_ok, u(c->d_K), u(c->d_K64), u(c->d_slab), u(c->d_mut), u(c->d_mutf), u(c->d_mus),
           u(c->d_tab[0][0]), u(c->d_tab[1][0]), u(c->d_red), u(c->d_err), (uintptr_t)c->bcap, (uintptr_t)(fft_eligible(c) && !c->fft_graph_failed),
           rte_fft_signature(c->fft)};
@@ -3177,25 +3170,6 @@ static int tangent_dA(rte_ctx* c, const double* d_in, double* d_outT, const std:
     CUDA_TRY(c, (c->launches++, rte_launch_pair_tangent(a, c->L, c->precision == RTE_PREC_MIXED ? 0 : 1,
                                                          c->model == RTE_MODEL_FIM ? 1 : 0, c->st)));
   }
-  SelfArgs sa;
-  memset(&sa, 0, sizeof sa);
-  sa.N = c->N;
-  sa.nb = 1;
-  sa.Cfull = c->C;
-  sa.Cact = c->C;
-  sa.K = c->K;
-  sa.W = d_in;
-  sa.mut = c->d_mut;
-  sa.idx = c->self_lut_ok ? c->d_self_idx : nullptr;
-  sa.lut = c->d_self_lut;
-  sa.mom = c->d_mom;
-  sa.scale = c->dV / c->cm;
-  sa.air_no_self = c->model == RTE_MODEL_FIM ? 1 : 0;
-  sa.out = c->d_selfp;
-
-  sa.dmut = c->d_dmut;
-  sa.dlut = c->d_dlut;
-  CUDA_TRY(c, (c->launches++, rte_launch_self(sa, c->st)));
   EpiArgs e;
   memset(&e, 0, sizeof e);
   e.N = c->N;
@@ -3206,7 +3180,10 @@ static int tangent_dA(rte_ctx* c, const double* d_in, double* d_outT, const std:
   e.S = a.nsplit;
   e.nb = 1;
   e.part = c->d_part;
-  e.selfp = c->d_selfp;
+  e.self = self_args(c, d_in);
+  e.self.mut = c->d_mut;
+  e.self.lut = c->d_dlut;
+  e.self.dmut = c->d_dmut;
   e.mus = c->d_mus;
   e.flag_scat = 0;
   e.Wout = d_outT;

@@ -80,6 +80,7 @@ struct ColArgs {
   int col0, col1;     // source columns [col0, col1), `chunk` columns per blockIdx.y
   int chunk, nsplit;
   int* err;
+  double* red;        // the epilogue's four norms, zeroed here for it
   int tz, ncd;        // set by the launcher: sources per run, destination columns per CTA at most
 };
 struct ColDims {
@@ -95,11 +96,30 @@ struct ColTabArgs {
   int row, azn, csn, nk, pho, tg, cls;
 };
 
+// Self-voxel term of the epilogue: scale * D(mu_t(r)) W[r], D symmetric, from a table of the medium's distinct mu_t
+// or the power series; W null: none.
+struct SelfArgs {
+  int K;
+  const double* W;      // [N][nb][Cfull]
+  const double* mut;
+  const int* idx;       // voxel -> row of lut (null: power series)
+  const double* lut;    // [ndistinct][Cfull][Cfull]
+  const double* mom;    // [K][Cfull][Cfull]
+  double scale;         // dV / cm
+  int air_no_self;
+  // derivative mode: scale * dmut(r) * dD/dmu(mu_t(r)) W (lut holds dD/dmu, or the series' derivative)
+  const double* dmut;   // null: the self term itself
+  // complex mu_t = mu_t + i kappa (intensity modulation): W holds (real, imaginary) pairs of rows,
+  // lut_im the imaginary parts of the table (the power series takes the complex mu_t directly)
+  double kappa;
+  const double* lut_im;
+};
+
 struct EpiArgs {
   int N, nx, ny, nz, Cfull, S, nb;  // nb right-hand sides, layout [N][nb][Cfull]
   const double* part;   // [S][N][nb][Cfull]
   const float* partf;   // or FP32 chunk sums of the tile-staged kernel, times N_c here (then part is unused)
-  const double* selfp;  // self-voxel term [N][nb][Cfull] (may be null)
+  SelfArgs self;
   const double* mus;
   int flag_scat;
   double scat[RTE_MAX_L + 1];  // per-l scatter factor (times mu_s of the voxel)
@@ -113,24 +133,6 @@ struct EpiArgs {
   int cplx;             // right-hand sides are (real, imaginary) pairs: odd ones are imaginary parts
 };
 
-struct SelfArgs {
-  int N, nb, Cfull, Cact, K;
-  const double* W;      // [N][nb][Cfull]
-  const double* mut;
-  const int* idx;       // voxel -> row of lut (null: power series)
-  const double* lut;    // [ndistinct][Cfull][Cfull]
-  const double* mom;    // [K][Cfull][Cfull]
-  double scale;         // dV / cm
-  int air_no_self;
-  double* out;          // [N][nb][Cfull]
-  // derivative mode: out = scale * dmut(r) * dD/dmu(mu_t(r)) W (dlut rows, or the series' derivative)
-  const double* dmut;   // null: the self term itself
-  const double* dlut;   // [ndistinct][Cfull][Cfull]
-  // complex mu_t = mu_t + i kappa (intensity modulation): W holds (real, imaginary) pairs of rows,
-  // lut_im the imaginary parts of the table (the power series takes the complex mu_t directly)
-  double kappa;
-  const double* lut_im;
-};
 
 struct ImgArgs {
   int nx, ny, nz, Cfull, L, vstride;
@@ -282,7 +284,6 @@ cudaError_t rte_launch_pair_fp64(const PairArgs& a, int LA, cudaStream_t st);
 cudaError_t rte_launch_store_kernel(const StoreArgs& a, cudaStream_t st, int fp64);
 cudaError_t rte_launch_epilogue(const EpiArgs& a, int LA, cudaStream_t st);
 cudaError_t rte_launch_images(const ImgArgs& a, cudaStream_t st);
-cudaError_t rte_launch_self(const SelfArgs& a, cudaStream_t st);
 // complex basis -> real parts; u1/u2 rows ostride apart (0: C)
 cudaError_t rte_launch_to_real(const double* cplx, double* u1, double* u2, int N, int L, double* red,
                                cudaStream_t st, int ostride = 0);

@@ -391,11 +391,68 @@ __device__ __forceinline__ double stop_weight(int c, bool imag) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Epilogue: add split-K partials, self-voxel term, scatter; write the next term (FP64 and FP32),
-// accumulate the running sum and the norms used by the stop rules.  One thread per (voxel, right-hand
-// side, coefficient) element, grid-stride, so every stream (partials, self term, outputs, running sum)
-// is read and written coalesced; the four norms are reduced per block and added atomically.
-// Self term: computed by k_self into selfp.  Coefficients above (LA+1)^2 are written as 0.
+// Self-voxel term (compute_diagonal_abs, FisherInfo_IO/src/kernels.cu:151-178, and its dV scale) of voxel r,
+// right-hand side b, coefficient c: scale * sum_c' D(mu_t(r))[c][c'] W[r][b][c'].  D is symmetric and read by
+// columns, so neighbouring c load neighbouring entries.  FIM model: voxels with mu_t == 0 (tissue 0) get nothing.
+// Complex mu_t = mu_t + i kappa (the CPU package's (1 - exp(-mu_t beta)) / mu_t, Kernels_selfsub.c:927-946): even b
+// is the real, odd b the imaginary row of a pair.
+__device__ __forceinline__ double self_term(const SelfArgs& a, int r, int b, int c, int nb, int Cfull, int Cact) {
+  const double* w = a.W + ((size_t)r * nb + b) * Cfull;
+  const double mu = a.mut[r];
+  if (a.kappa != 0.0) {
+    const double* w0 = a.W + ((size_t)r * nb + (b & ~1)) * Cfull;
+    const double* w1 = w0 + Cfull;
+    double ur = 0.0, ui = 0.0;
+    if (a.idx) {
+      const size_t row = (size_t)a.idx[r] * Cfull * Cfull + c;
+      const double* Dr = a.lut + row;
+      const double* Di = a.lut_im + row;
+      for (int cp = 0; cp < Cact; ++cp) {
+        const double dr = __ldg(Dr + cp * Cfull), di = __ldg(Di + cp * Cfull), x0 = __ldg(w0 + cp), x1 = __ldg(w1 + cp);
+        ur = fma(dr, x0, fma(-di, x1, ur));
+        ui = fma(dr, x1, fma(di, x0, ui));
+      }
+    } else {  // Horner in the complex mu: u <- mu u + M_k w
+      for (int kk = a.K - 1; kk >= 0; --kk) {
+        const double* M = a.mom + (size_t)kk * Cfull * Cfull + c;
+        double t0 = 0.0, t1 = 0.0;
+        for (int cp = 0; cp < Cact; ++cp) {
+          const double m = __ldg(M + cp * Cfull);
+          t0 = fma(m, __ldg(w0 + cp), t0);
+          t1 = fma(m, __ldg(w1 + cp), t1);
+        }
+        const double nr = mu * ur - a.kappa * ui + t0, ni = mu * ui + a.kappa * ur + t1;
+        ur = nr;
+        ui = ni;
+      }
+    }
+    return a.scale * ((b & 1) ? ui : ur);
+  }
+  if (a.air_no_self && mu == 0.0) return 0.0;
+  double u = 0.0;
+  if (a.idx) {
+    const double* D = a.lut + (size_t)a.idx[r] * Cfull * Cfull + c;
+    for (int cp = 0; cp < Cact; ++cp) u = fma(__ldg(D + cp * Cfull), __ldg(w + cp), u);
+  } else {  // D(mu) = sum_k mu^k M_k; its derivative sum_k k mu^(k-1) M_k, both by Horner
+    const bool der = a.dmut != nullptr;
+    for (int kk = a.K - 1; kk >= (der ? 1 : 0); --kk) {
+      const double* M = a.mom + (size_t)kk * Cfull * Cfull + c;
+      double tk = 0.0;
+      for (int cp = 0; cp < Cact; ++cp) tk = fma(__ldg(M + cp * Cfull), __ldg(w + cp), tk);
+      u = fma(mu, u, der ? (double)kk * tk : tk);
+    }
+  }
+  if (a.dmut) u *= a.dmut[r];
+  return a.scale * u;
+}
+
+// Epilogue: self-voxel term, chunk sums, scatter; write the next term (and its rows for the next pair launch),
+// accumulate the running sum and the norms used by the stop rules.  One thread per (voxel, right-hand side,
+// coefficient) element, grid-stride, so every stream (chunk sums, outputs, running sum) is read and written
+// coalesced; the four norms are reduced per block and added atomically.  Bound by loads of the self-term table
+// (2 C per element, from L1 and L2) and of the chunk sums.  Measured per term, self term and epilogue together: 171 ->
+// 86 us at 33^3 L=5, 448 -> 254 us with four right-hand sides, 310 -> 79 us at 25^3 L=7 against a self-term launch of
+// its own that read rows of D.  Coefficients above (LA+1)^2 are written as 0.
 __global__ void __launch_bounds__(256) k_epilogue(EpiArgs a, int Cact) {
   const int nb = a.nb > 0 ? a.nb : 1;
   const int vstride = nb * a.Cfull;
@@ -403,13 +460,13 @@ __global__ void __launch_bounds__(256) k_epilogue(EpiArgs a, int Cact) {
   const int plane = a.nx * a.ny;
   double w2 = 0.0, s2 = 0.0, lw = 0.0, ls = 0.0;
   for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-    const int r = (int)(t / vstride), e = (int)(t - (size_t)r * vstride);
-    const int b = e / a.Cfull, c = e - b * a.Cfull;
+    const int r = total < (1ull << 32) ? (int)((unsigned)t / (unsigned)vstride) : (int)(t / vstride);
+    const int e = (int)(t - (size_t)r * vstride), b = nb == 1 ? 0 : e / a.Cfull, c = e - b * a.Cfull;
     int l = 0;
     while ((l + 1) * (l + 1) <= c) ++l;
     double x = 0.0;
     if (c < Cact) {
-      x = a.selfp ? a.selfp[t] : 0.0;
+      x = a.self.W ? self_term(a.self, r, b, c, nb, a.Cfull, Cact) : 0.0;
       if (a.partf) {  // FP32 chunk sums of the tile-staged kernel: FP64 sum over the chunks, then N_c
         double u = 0.0;
         for (int q = 0; q < a.S; ++q) u += (double)a.partf[(size_t)q * NV + t];
@@ -457,84 +514,6 @@ __global__ void __launch_bounds__(256) k_epilogue(EpiArgs a, int Cact) {
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) x += red[threadIdx.x][w];
     atomicAdd(a.red + threadIdx.x, x);
   }
-}
-
-// Self-voxel term (compute_diagonal_abs, FisherInfo_IO/src/kernels.cu:151-178, and its dV scale)
-// for every voxel, right-hand side and output coefficient (one thread each):
-//   out[r][b][c] = scale * sum_c' D(mu_t(r))[c][c'] W[r][b][c'],
-// D from a table of the medium's distinct mu_t values (lut/idx), else by the power series
-// D(mu) = sum_k mu^k M_k (Horner).  FIM model: voxels with mu_t == 0 (tissue 0) get nothing.
-__global__ void k_self(SelfArgs a) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = (long long)a.N * a.nb * a.Cact;
-  if (t >= total) return;
-  const int c = (int)(t % a.Cact);
-  const int b = (int)((t / a.Cact) % a.nb);
-  const int r = (int)(t / ((long long)a.Cact * a.nb));
-  const size_t base = (size_t)r * a.nb * a.Cfull + (size_t)b * a.Cfull;
-  const double mu = a.mut[r];
-  double u = 0.0;
-  if (!(a.air_no_self && mu == 0.0)) {
-    const double* w = a.W + base;
-    const bool der = a.dmut != nullptr;
-    if (a.idx) {
-      const double* D = (der ? a.dlut : a.lut) + ((size_t)a.idx[r] * a.Cfull + c) * a.Cfull;
-      for (int cp = 0; cp < a.Cact; ++cp) u = fma(__ldg(D + cp), __ldg(w + cp), u);
-    } else {  // D(mu) = sum_k mu^k M_k; its derivative sum_k k mu^(k-1) M_k, both by Horner
-      for (int kk = a.K - 1; kk >= (der ? 1 : 0); --kk) {
-        const double* M = a.mom + ((size_t)kk * a.Cfull + c) * a.Cfull;
-        double tk = 0.0;
-        for (int cp = 0; cp < a.Cact; ++cp) tk = fma(__ldg(M + cp), __ldg(w + cp), tk);
-        u = fma(mu, u, der ? (double)kk * tk : tk);
-      }
-    }
-    if (der) u *= a.dmut[r];
-  }
-  a.out[base + c] = a.scale * u;
-}
-
-// Self-voxel term with the complex mu_t + i kappa of intensity modulation (the CPU package's
-// (1 - exp(-mu_t beta)) / mu_t with complex mu_t, Kernels_selfsub.c:927-946): W holds (real,
-// imaginary) row pairs; D from the complex table (lut, lut_im) or the power series in the complex
-// mu_t.  One thread per voxel, complex right-hand side and output coefficient.
-__global__ void k_self_cplx(SelfArgs a) {
-  const int npair = a.nb / 2;
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const long long total = (long long)a.N * npair * a.Cact;
-  if (t >= total) return;
-  const int c = (int)(t % a.Cact);
-  const int p = (int)((t / a.Cact) % npair);
-  const int r = (int)(t / ((long long)a.Cact * npair));
-  const size_t base = (size_t)r * a.nb * a.Cfull + (size_t)(2 * p) * a.Cfull;
-  const double* w0 = a.W + base;
-  const double* w1 = w0 + a.Cfull;
-  double ur = 0.0, ui = 0.0;
-  if (a.idx) {
-    const size_t row = ((size_t)a.idx[r] * a.Cfull + c) * a.Cfull;
-    const double* Dr = a.lut + row;
-    const double* Di = a.lut_im + row;
-    for (int cp = 0; cp < a.Cact; ++cp) {
-      const double dr = __ldg(Dr + cp), di = __ldg(Di + cp), x0 = __ldg(w0 + cp), x1 = __ldg(w1 + cp);
-      ur = fma(dr, x0, fma(-di, x1, ur));
-      ui = fma(dr, x1, fma(di, x0, ui));
-    }
-  } else {  // Horner in the complex mu: u <- mu u + M_k w
-    const double mr = a.mut[r], mi = a.kappa;
-    for (int kk = a.K - 1; kk >= 0; --kk) {
-      const double* M = a.mom + ((size_t)kk * a.Cfull + c) * a.Cfull;
-      double t0 = 0.0, t1 = 0.0;
-      for (int cp = 0; cp < a.Cact; ++cp) {
-        const double m = __ldg(M + cp);
-        t0 = fma(m, __ldg(w0 + cp), t0);
-        t1 = fma(m, __ldg(w1 + cp), t1);
-      }
-      const double nr = mr * ur - mi * ui + t0, ni = mr * ui + mi * ur + t1;
-      ur = nr;
-      ui = ni;
-    }
-  }
-  a.out[base + c] = a.scale * ur;
-  a.out[base + a.Cfull + c] = a.scale * ui;
 }
 
 // Exitance images of the z = nZ-1 and z = 0 faces from the m = 0 coefficients
@@ -1249,18 +1228,6 @@ cudaError_t rte_launch_epilogue(const EpiArgs& a, int LA, cudaStream_t st) {
   const size_t total = (size_t)a.N * (a.nb > 0 ? a.nb : 1) * a.Cfull;
   const unsigned blocks = (unsigned)std::min<size_t>((total + 255) / 256, 148 * 16);
   k_epilogue<<<blocks, 256, 0, st>>>(a, (LA + 1) * (LA + 1));
-  return cudaGetLastError();
-}
-
-cudaError_t rte_launch_self(const SelfArgs& a, cudaStream_t st) {
-  if (a.kappa != 0.0) {
-    if (a.nb % 2 || a.dmut) return cudaErrorInvalidValue;
-    const long long total = (long long)a.N * (a.nb / 2) * a.Cact;
-    k_self_cplx<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(a);
-    return cudaGetLastError();
-  }
-  const long long total = (long long)a.N * a.nb * a.Cact;
-  k_self<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(a);
   return cudaGetLastError();
 }
 

@@ -142,7 +142,6 @@ extern "C" int rte_attenuate_noalloc(int nx, int ny, int nz, double dx, double d
     ep.S = S;
     ep.nb = 1;
     ep.part = part;
-    ep.selfp = nullptr;
     ep.mus = d_mut;
     ep.Wout = part_k ? o2 : o1;
     ep.red = red;
