@@ -2444,6 +2444,23 @@ extern "C" int rte_detector_flux(rte_ctx* c, int nsrc, const rte_source* srcs, c
 //   dL/dmu_s(v) += lambda_v . scat_l (A S)_v;   plus the source column and ballistic terms.
 // Arguments of the back-projection passes; the pair-weight buffer (N x ld, FP32 for the mixed
 // precision path, FP64 otherwise) is allocated on first use and kept with the context.
+struct BpBuffer {  // pair weights, then column-order rows of y and S, then the walk's sums (byte offsets)
+  size_t ld, y, S, gcol, bytes;
+  int pitch;
+};
+
+static BpBuffer bp_buffer(const rte_ctx* c) {
+  const size_t es = c->precision == RTE_PREC_MIXED ? sizeof(float) : sizeof(double);
+  BpBuffer b;
+  b.ld = ((size_t)c->N + 31) / 32 * 32;
+  b.pitch = (c->C + 3) / 4 * 4;
+  b.y = ((size_t)c->N * b.ld * es + 255) / 256 * 256;
+  b.S = b.y + ((size_t)c->N * b.pitch * es + 255) / 256 * 256;
+  b.gcol = b.S + ((size_t)c->N * b.pitch * es + 255) / 256 * 256;
+  b.bytes = b.gcol + sizeof(double) * (size_t)c->N;
+  return b;
+}
+
 static BpArgs bp_args(rte_ctx* c, bool accumulate) {
   BpArgs bp;
   memset(&bp, 0, sizeof bp);
@@ -2457,26 +2474,28 @@ static BpArgs bp_args(rte_ctx* c, bool accumulate) {
   bp.dz = c->dz;
   bp.prop_thresh = c->prop_thresh;
   bp.kscale = c->dV / c->cm;
-  bp.perm = c->d_perm;
   bp.islot = c->d_islot;
   bp.mut = c->d_mut;
-  bp.mutf = c->d_mutf;
-  bp.y = c->d_y;
-  bp.S = c->d_S;
   bp.Kmat = c->K_valid && c->d_K ? c->d_K : nullptr;
   bp.Kmat64 = c->K_valid && c->d_K64 ? c->d_K64 : nullptr;
   bp.Kld = c->N;
   bp.nzp = col_dims(c).nzp;
   bp.group = col_dims(c).group;
   bp.g = c->d_gt;
-  bp.Q = c->d_Qbp;
+  const BpBuffer b = bp_buffer(c);
+  char* base = static_cast<char*>(c->d_Qbp);
+  bp.Q = base;
+  bp.ld = b.ld;
+  bp.pitch = b.pitch;
+  bp.y = base + b.y;
+  bp.S = base + b.S;
+  bp.gcol = reinterpret_cast<double*>(base + b.gcol);
   bp.accumulate = accumulate ? 1 : 0;
   return bp;
 }
 
 static int ensure_bp_buffer(rte_ctx* c) {
-  const size_t ld = ((size_t)c->N + 31) / 32 * 32;
-  const size_t need = (size_t)c->N * ld * (c->precision == RTE_PREC_MIXED ? sizeof(float) : sizeof(double));
+  const size_t need = bp_buffer(c).bytes;
   if (c->d_Qbp && c->qbp_bytes >= need) return RTE_OK;
   if (c->d_Qbp) {
     cudaFree(c->d_Qbp);
@@ -2537,7 +2556,10 @@ static int adjoint_source_terms(rte_ctx* c, const rte_source* s, const rte_stop*
   BpArgs bp = bp_args(c, !first);
   {
     ProfScope ps(c, 0);
-    CUDA_TRY(c, (c->launches++, rte_launch_bp_weights(bp, c->L, mixed ? 0 : 1, c->st)));
+    const int f64 = mixed ? 0 : 1;
+    CUDA_TRY(c, (c->launches++, rte_launch_rows(c->d_y, (void*)bp.y, c->d_islot, c->N, 1, bp.pitch, c->C, f64, c->st)));
+    CUDA_TRY(c, (c->launches++, rte_launch_rows(c->d_S, (void*)bp.S, c->d_islot, c->N, 1, bp.pitch, c->C, f64, c->st)));
+    CUDA_TRY(c, (c->launches++, rte_launch_bp_weights(bp, c->L, f64, c->st)));
   }
   GradLocalArgs gl;
   memset(&gl, 0, sizeof gl);
@@ -2606,7 +2628,7 @@ static int adjoint_finish(rte_ctx* c, const std::vector<double>& ga, const std::
   {
     const BpArgs bp = bp_args(c, true);
     ProfScope ps(c, 0);
-    CUDA_TRY(c, (c->launches++, rte_launch_bp_walk(bp, c->precision == RTE_PREC_MIXED ? 0 : 1, c->st)));
+    CUDA_TRY(c, (c->launches += 2, rte_launch_bp_walk(bp, c->precision == RTE_PREC_MIXED ? 0 : 1, c->st)));
   }
   std::vector<double> gt(c->N), gs(c->N);
   CUDA_TRY(c, cudaMemcpyAsync(gt.data(), c->d_gt, sizeof(double) * c->N, cudaMemcpyDeviceToHost, c->st));

@@ -182,23 +182,27 @@ struct FaceArgs {
   double* e;           // adjoint seed field [N][Cfull]
 };
 
+// Back-projection of the gradient (rte_backproject.cu); T is float for mixed contexts, double otherwise.
 struct BpArgs {
   int N, nx, ny, nz, Cfull;
   double dx, dy, dz, prop_thresh, kscale;
-  const int* perm;
   const int* islot;
   const double* mut;
-  const float* mutf;
-  const double* y;     // destination-side field [N][Cfull] (voxel order)
-  const double* S;     // source-side field [N][Cfull] (voxel order)
-  const float* Kmat;   // stored pair kernel (null: recompute the path integral)
-  const double* Kmat64;  // FP64 stored pair kernel (FP64 contexts in stored-kernel mode)
+  const void* y;       // T, destination-side field, column-order rows times N_c (rte_launch_rows), `pitch` apart
+  const void* S;       // T, source-side field, likewise
+  int pitch;
+  const float* Kmat;   // stored pair kernel (both null: recompute the path integral)
+  const double* Kmat64;
   size_t Kld;
   int nzp, group;      // layout of the stored kernel (ColDims)
-  double* g;           // gradient w.r.t. mu_t, accumulated [N]
-  int use_smem;        // per-CTA private accumulator of N entries in shared memory (set by the launcher)
-  void* Q;             // per unordered pair weight [source slot][destination slot] (row stride Kld), T
+  void* Q;             // T, weight of each unordered pair [source slot][destination slot > source slot]
+  size_t ld;
   int accumulate;      // k_bp_weights: add to Q (later sources) instead of overwriting
+  double* gcol;        // [N] column-order sums of the walk (scratch)
+  double* g;           // gradient w.r.t. mu_t, accumulated [N]
+  // set by the launchers: column pairs per chunk (weights) or three times as many (walk), chunks that share what
+  // depends on the displacement, z block, list entries and |dz| rows of a batch, one batch for every displacement
+  int jq, group_ch, zb, cap, rows, single;
 };
 
 struct GradLocalArgs {

@@ -376,8 +376,6 @@ __global__ void k_strided_add(double* dst, const double* a, int astride, const d
   dst[t] = a[(size_t)r * astride + c] + b[t];
 }
 
-#define RTE_KT 64  // slots per side of a back-projection tile
-
 // Weight of real coefficient c in the reference stop rule's layer sum, sum over m of Re(w_lm) in the
 // complex basis (dist.cu:1143-1152): for a real function R_l0 + sqrt2 R_l,m (even m > 0); for the
 // imaginary part f2 of a complex function (w = w1 + i w2, Re(i w2_lm) = -Im(w2_lm)) sqrt2 R_l,-m for
@@ -834,216 +832,10 @@ __global__ void k_y_field(double* y, const double* e, const double* lam, const d
   y[t] = e[t] + (l <= L ? sc.v[l] : 0.0) * mus[r] * lam[t];
 }
 
-// Segments of the centre-to-centre path of path_sum, each length handed to `add(v, len * Q / dist)`.
-template <typename F>
-__device__ __forceinline__ void path_walk(int i, int j, int k, int ip, int jp, int kp, int nx, int plane, int& Q,
-                                          F add) {
-  const int Dz = abs(ip - i), Dy = abs(jp - j), Dx = abs(kp - k);
-  const int mz = max(Dz, 1), my = max(Dy, 1), mx = max(Dx, 1);
-  Q = 2 * mx * my * mz;
-  const int BIG = 0x3fffffff;
-  const int incz = 2 * mx * my, incy = 2 * mx * mz, incx = 2 * my * mz;
-  int Az = Dz ? mx * my : BIG, Ay = Dy ? mx * mz : BIG, Ax = Dx ? my * mz : BIG;
-  const int stz = ip > i ? plane : -plane, sty = jp > j ? nx : -nx, stx = kp > k ? 1 : -1;
-  int v = i * plane + j * nx + k;
-  int prev = 0;
-  const int steps = Dx + Dy + Dz;
-  for (int s = 0; s < steps; ++s) {
-    const int m = min(Az, min(Ay, Ax));
-    if (m > prev) add(v, m - prev);
-    prev = m;
-    const bool bz = Az == m;
-    const bool by = !bz && (Ay == m);
-    const bool bx = !bz && !by;
-    v += bz ? stz : (by ? sty : stx);
-    Az += bz ? incz : 0;
-    Ay += by ? incy : 0;
-    Ax += bx ? incx : 0;
-  }
-  add(v, Q - prev);
-}
-
-// ---------------------------------------------------------------------------------------------
-// Symmetric back-projection.  The path between voxels r and r' is the same set of segments in
-// both directions, so each unordered pair is walked once with the weight of both ordered pairs:
-//   w(r, r') = k [ (y_r . R(w)) (R(w) . S_r') + (y_r' . P R(w)) (P R(w) . S_r) ],
-// w = (r - r') / |r - r'|, P R(w) = R(-w) = (-1)^l R(w).  Pass 1 (k_bp_weights, once per source,
-// summed into Q) evaluates the weights on 64 x 64 tiles of the upper triangle in slot order; pass 2
-// (k_bp_walk, once per gradient) walks every pair with w != 0 and adds -w * length to each voxel on
-// the path, into a shared-memory copy of the whole gradient per CTA when it fits.
 __host__ __device__ constexpr int l_of_c(int c) {
   int l = 0;
   while ((l + 1) * (l + 1) <= c) ++l;
   return l;
-}
-
-__device__ __forceinline__ void tri_tile(long long t, int& bd, int& bs) {
-  bd = (int)((sqrt(8.0 * (double)t + 1.0) - 1.0) / 2.0);
-  while ((long long)(bd + 1) * (bd + 2) / 2 <= t) ++bd;
-  while ((long long)bd * (bd + 1) / 2 > t) --bd;
-  bs = (int)(t - (long long)bd * (bd + 1) / 2);
-}
-
-template <int LA, typename T>
-__global__ void __launch_bounds__(RTE_KT) k_bp_weights(BpArgs a) {
-  constexpr int C = (LA + 1) * (LA + 1);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* ys = reinterpret_cast<T*>(smem_raw);             // [64][C] y of the tile's sources
-  T* Ss = ys + RTE_KT * C;                             // [64][C] S of the tile's sources
-  int* sx = reinterpret_cast<int*>(Ss + RTE_KT * C);   // [64][3] source coordinates
-  // FP32 sums at L >= 6: the destination's own y and S rows live in shared memory ([2][C][64], one
-  // column per thread) instead of 2C registers, which leaves room for the FP64 SH recurrence at L >= 7
-  // (the FP64 kernel keeps them in registers: in shared memory they would halve its CTAs per SM)
-  constexpr bool DST_SMEM = C >= 49 && sizeof(T) == 4;
-  T* sD = reinterpret_cast<T*>(sx + RTE_KT * 3);
-  const int ntile = (a.N + RTE_KT - 1) / RTE_KT;
-  int bd, bs;
-  tri_tile(blockIdx.x, bd, bs);
-  if (bd >= ntile) return;
-  const int tid = threadIdx.x;
-  const int plane = a.nx * a.ny;
-  const int s0 = bs * RTE_KT, d0 = bd * RTE_KT;
-  {
-    const int sl = s0 + tid;
-    const int v = sl < a.N ? a.perm[sl] : 0;
-    sx[tid * 3 + 0] = v % a.nx;
-    sx[tid * 3 + 1] = (v / a.nx) % a.ny;
-    sx[tid * 3 + 2] = v / plane;
-  }
-  for (int e = tid; e < RTE_KT * C; e += RTE_KT) {  // row by row: neighbouring threads, neighbouring c
-    const int q = e / C, c = e % C;
-    const int sl = s0 + q;
-    const size_t off = sl < a.N ? (size_t)a.perm[sl] * a.Cfull + c : 0;
-    ys[e] = sl < a.N ? (T)a.y[off] : T(0);
-    Ss[e] = sl < a.N ? (T)a.S[off] : T(0);
-  }
-  __syncthreads();
-  const int d = d0 + tid;
-  if (d >= a.N) return;
-  const int r = a.perm[d];
-  const int k = r % a.nx, j = (r / a.nx) % a.ny, i = r / plane;
-  T yd[DST_SMEM ? 1 : C], Sd[DST_SMEM ? 1 : C];
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    const T yv = (T)a.y[(size_t)r * a.Cfull + c], Sv = (T)a.S[(size_t)r * a.Cfull + c];
-    if constexpr (DST_SMEM) {
-      sD[c * RTE_KT + tid] = yv;
-      sD[(C + c) * RTE_KT + tid] = Sv;
-    } else {
-      yd[c] = yv;
-      Sd[c] = Sv;
-    }
-  }
-  const T dxf = (T)a.dx, dyf = (T)a.dy, dzf = (T)a.dz, thr = (T)a.prop_thresh, ks = (T)a.kscale;
-  T* Qp = reinterpret_cast<T*>(a.Q);
-  const int qend = bs == bd ? tid : RTE_KT;  // diagonal tile: each unordered pair once (source slot < destination slot)
-  for (int q = 0; q < qend; ++q) {
-    const int sl = s0 + q;
-    if (sl >= a.N) break;
-    const int kp = sx[q * 3 + 0], jp = sx[q * 3 + 1], ip = sx[q * 3 + 2];
-    const T ddx = (T)(k - kp) * dxf, ddy = (T)(j - jp) * dyf, ddz = (T)(i - ip) * dzf;
-    const T d2 = ddx * ddx + ddy * ddy + ddz * ddz;
-    const T dist = sqrt(d2);
-    T w = T(0);
-    if (d2 > T(0) && dist < thr) {
-      T kk;
-      if (a.Kmat64) {
-        kk = (T)__ldg(a.Kmat64 + kmat_index(sl, kmat_pos(d, a.nz, a.nzp), a.Kld, a.group));
-      } else if (a.Kmat) {
-        kk = (T)__ldg(a.Kmat + kmat_index(sl, kmat_pos(d, a.nz, a.nzp), a.Kld, a.group));
-      } else {
-        int Q0;
-        const T ps = path_sum<T, double>(i, j, k, ip, jp, kp, a.mut, a.nx, plane, Q0);
-        kk = exp(-ps * dist / (T)Q0) * ks / d2;
-      }
-      const T inv = T(1) / dist;
-      T R[C];
-      sh_eval_prec<LA, T>(ddx * inv, ddy * inv, ddz * inv, R);
-      const T* yq = ys + q * C;
-      const T* Sq = Ss + q * C;
-      T a1 = T(0), b1 = T(0), a2 = T(0), b2 = T(0);
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        const T Rp = (l_of_c(c) & 1) ? -R[c] : R[c];
-        const T ydc = DST_SMEM ? sD[c * RTE_KT + tid] : yd[DST_SMEM ? 0 : c];
-        const T Sdc = DST_SMEM ? sD[(C + c) * RTE_KT + tid] : Sd[DST_SMEM ? 0 : c];
-        a1 = fma(ydc, R[c], a1);
-        b1 = fma(R[c], Sq[c], b1);
-        a2 = fma(yq[c], Rp, a2);
-        b2 = fma(Rp, Sdc, b2);
-      }
-      w = kk * (a1 * b1 + a2 * b2);
-    }
-    const size_t idx = (size_t)sl * ((a.N + 31) / 32 * 32) + d;
-    Qp[idx] = a.accumulate ? Qp[idx] + w : w;
-  }
-}
-
-__device__ __forceinline__ void group_sync(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-
-#define RTE_BPW_THREADS 512
-template <typename T>
-__global__ void __launch_bounds__(RTE_BPW_THREADS) k_bp_walk(BpArgs a) {
-  constexpr int G = RTE_BPW_THREADS / RTE_KT;  // independent 64-thread groups, one tile each
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  int* sx = reinterpret_cast<int*>(smem_raw);                          // [G][64][3]
-  T* acc = reinterpret_cast<T*>(smem_raw + G * RTE_KT * 3 * sizeof(int));  // [N] when use_smem
-  const int tid = threadIdx.x, grp = tid / RTE_KT, lane = tid % RTE_KT;
-  if (a.use_smem)
-    for (int v = tid; v < a.N; v += RTE_BPW_THREADS) acc[v] = T(0);
-  __syncthreads();
-  const int plane = a.nx * a.ny;
-  const int ntile = (a.N + RTE_KT - 1) / RTE_KT;
-  const long long ntri = (long long)ntile * (ntile + 1) / 2;
-  const T* Qp = reinterpret_cast<const T*>(a.Q);
-  int* gx = sx + grp * RTE_KT * 3;
-  for (long long t = (long long)blockIdx.x * G + grp; t < ntri; t += (long long)gridDim.x * G) {
-    int bd, bs;
-    tri_tile(t, bd, bs);
-    const int s0 = bs * RTE_KT, d0 = bd * RTE_KT;
-    {
-      const int sl = s0 + lane;
-      const int v = sl < a.N ? a.perm[sl] : 0;
-      gx[lane * 3 + 0] = v % a.nx;
-      gx[lane * 3 + 1] = (v / a.nx) % a.ny;
-      gx[lane * 3 + 2] = v / plane;
-    }
-    group_sync(grp + 1, RTE_KT);
-    const int d = d0 + lane;
-    if (d < a.N) {
-      const int r = a.perm[d];
-      const int k = r % a.nx, j = (r / a.nx) % a.ny, i = r / plane;
-      const int qend = bs == bd ? lane : RTE_KT;
-      for (int q = 0; q < qend; ++q) {
-        const int sl = s0 + q;
-        if (sl >= a.N) break;
-        const T w = Qp[(size_t)sl * ((a.N + 31) / 32 * 32) + d];
-        if (w == T(0)) continue;
-        const int kp = gx[q * 3 + 0], jp = gx[q * 3 + 1], ip = gx[q * 3 + 2];
-        const T ddx = (T)(k - kp) * (T)a.dx, ddy = (T)(j - jp) * (T)a.dy, ddz = (T)(i - ip) * (T)a.dz;
-        const T dist = sqrt(ddx * ddx + ddy * ddy + ddz * ddz);
-        const int Dz = abs(ip - i), Dy = abs(jp - j), Dx = abs(kp - k);
-        // lengths arrive scaled by Q / dist, Q = 2 max(Dx,1) max(Dy,1) max(Dz,1)
-        const T coef = -w * dist / (T)(2 * max(Dx, 1) * max(Dy, 1) * max(Dz, 1));
-        int Qw = 1;
-        if (a.use_smem)
-          path_walk(i, j, k, ip, jp, kp, a.nx, plane, Qw, [&](int v, int len) { atomicAdd(acc + v, coef * (T)len); });
-        else
-          path_walk(i, j, k, ip, jp, kp, a.nx, plane, Qw,
-                    [&](int v, int len) { atomicAdd(a.g + v, (double)(coef * (T)len)); });
-      }
-    }
-    group_sync(grp + 1, RTE_KT);  // the group's coordinates are overwritten by its next tile
-  }
-  if (a.use_smem) {
-    __syncthreads();
-    for (int v = tid; v < a.N; v += RTE_BPW_THREADS) {
-      const T x = acc[v];
-      if (x != T(0)) atomicAdd(a.g + v, (double)x);
-    }
-  }
 }
 
 // Per-voxel parts of the gradient: the scatter D (d/dmu_s: lambda . scat_l . (A S)) and the
@@ -1385,58 +1177,6 @@ cudaError_t rte_launch_y_field(double* y, const double* e, const double* lam, co
   const long long n = (long long)N * Cfull;
   k_y_field<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(y, e, lam, mus, sc, N, L, Cfull);
   return cudaGetLastError();
-}
-
-template <int LA, typename T>
-static cudaError_t launch_bpw(const BpArgs& a, cudaStream_t st) {
-  constexpr int C = (LA + 1) * (LA + 1);
-  const size_t smem = (size_t)RTE_KT * C * 2 * sizeof(T) * (C >= 49 && sizeof(T) == 4 ? 2 : 1) + RTE_KT * 3 * sizeof(int);
-  cudaError_t e = allow_smem((const void*)k_bp_weights<LA, T>, smem);
-  if (e != cudaSuccess) return e;
-  const long long nt = (a.N + RTE_KT - 1) / RTE_KT;
-  k_bp_weights<LA, T><<<(unsigned)(nt * (nt + 1) / 2), RTE_KT, smem, st>>>(a);
-  return cudaGetLastError();
-}
-
-template <int LA>
-static cudaError_t launch_bpw_LA(const BpArgs& a, int fp64, cudaStream_t st) {
-  return fp64 ? launch_bpw<LA, double>(a, st) : launch_bpw<LA, float>(a, st);
-}
-
-cudaError_t rte_launch_bp_weights(const BpArgs& a, int LA, int fp64, cudaStream_t st) {
-  switch (LA) {
-    case 0: return launch_bpw_LA<0>(a, fp64, st);
-    case 1: return launch_bpw_LA<1>(a, fp64, st);
-    case 2: return launch_bpw_LA<2>(a, fp64, st);
-    case 3: return launch_bpw_LA<3>(a, fp64, st);
-    case 4: return launch_bpw_LA<4>(a, fp64, st);
-    case 5: return launch_bpw_LA<5>(a, fp64, st);
-    case 6: return launch_bpw_LA<6>(a, fp64, st);
-    case 7: return launch_bpw_LA<7>(a, fp64, st);
-  }
-  return cudaErrorInvalidValue;
-}
-
-template <typename T>
-static cudaError_t launch_walk(BpArgs a, cudaStream_t st) {
-  const size_t base = (size_t)(RTE_BPW_THREADS / RTE_KT) * RTE_KT * 3 * sizeof(int);
-  int dev = 0, maxsm = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  a.use_smem = base + (size_t)a.N * sizeof(T) <= (size_t)maxsm ? 1 : 0;
-  const size_t smem = base + (a.use_smem ? (size_t)a.N * sizeof(T) : 0);
-  cudaError_t e = allow_smem((const void*)k_bp_walk<T>, smem);
-  if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bp_walk<T>, RTE_BPW_THREADS, smem);
-  if (e != cudaSuccess) return e;
-  k_bp_walk<T><<<(unsigned)(std::max(per_sm, 1) * sms), RTE_BPW_THREADS, smem, st>>>(a);
-  return cudaGetLastError();
-}
-
-cudaError_t rte_launch_bp_walk(const BpArgs& a, int fp64, cudaStream_t st) {
-  return fp64 ? launch_walk<double>(a, st) : launch_walk<float>(a, st);
 }
 
 cudaError_t rte_launch_grad_local(const GradLocalArgs& a, cudaStream_t st) {

@@ -23,6 +23,7 @@
 #include <type_traits>
 
 #include "rte_internal.h"
+#include "rte_walk.cuh"
 
 namespace {
 
@@ -150,8 +151,8 @@ __global__ void __launch_bounds__(ST_THREADS, STAGE ? 1 : 2) k_store_lists(Store
         if (a0 > amin) __syncthreads();
         if (!once || ch == ch0)
         for (int da = a0 + wid; da < a1; da += ST_THREADS / 32) {
-          const int mz = max(da, 1), hx = my * mz, hy = mx * mz, hz = mx * my, Q = 2 * mx * hx;
-          const int first = (da - a0) * (sxy + 1) + (da * (da - 1) - a0 * (a0 - 1)) / 2, S = sxy + da;
+          const int Q = 2 * mx * my * max(da, 1);
+          const int first = (da - a0) * (sxy + 1) + (da * (da - 1) - a0 * (a0 - 1)) / 2;
           if (lane == 0) {
             ls[da] = first;
             const T ex = (T)Dx * dxf, ey = (T)Dy * dyf, ez = (T)da * dzf;
@@ -160,25 +161,12 @@ __global__ void __launch_bounds__(ST_THREADS, STAGE ? 1 : 2) k_store_lists(Store
             lf[2 * da] = (T)(-1.4426950408889634 * sqrt(r2) / (double)Q);
             lf[2 * da + 1] = d2 > T(0) && sqrt(d2) < thr ? (T)(a.kscale / r2) : T(0);
           }
-          // crossing n of an axis lies at (2 n + 1) h; ties step z, then y, then x
-          auto before = [](int t, int h, int D, bool ties) { return D ? (t + h - (ties ? 0 : 1)) / (2 * h) : 0; };
-          for (int e = lane; e <= S; e += 32) {
-            int t, cx, cy, cz;  // this crossing, and the crossings of each axis that precede it
-            if (e == S) {
-              t = Q, cx = Dx, cy = Dy, cz = da;
-            } else if (e < Dx) {
-              t = (2 * e + 1) * hx, cx = e, cy = before(t, hy, Dy, true), cz = before(t, hz, da, true);
-            } else if (e < sxy) {
-              t = (2 * (e - Dx) + 1) * hy, cy = e - Dx, cx = before(t, hx, Dx, false), cz = before(t, hz, da, true);
-            } else {
-              t = (2 * (e - sxy) + 1) * hz, cz = e - sxy, cx = before(t, hx, Dx, false), cy = before(t, hy, Dy, false);
-            }
-            const int prev = max(max((2 * cx - 1) * hx, (2 * cy - 1) * hy), max((2 * cz - 1) * hz, 0));
+          path_list(Dx, Dy, da, lane, [&](int k, int cx, int cy, int cz, int len, bool) {
             Entry<T, PACK> v;
             v.set(cx * stx + cy * sty, cz);
-            v.len = (T)(t - prev);
-            ent[first + cx + cy + cz] = v;
-          }
+            v.len = (T)len;
+            ent[first + k] = v;
+          });
         }
         __syncthreads();
         const int npv = cols[2 * a.npair], jq = a.npair / E;  // lane element: (one of jq pairs) x E, z, sign of dz

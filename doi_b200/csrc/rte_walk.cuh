@@ -161,3 +161,31 @@ RTE_WALK_FN A path_sum_box(int i, int j, int k, int ip, int jp, int kp, const MU
   }
   return acc;
 }
+
+#ifdef __CUDACC__
+// The voxels that a path of displacement (Dx, Dy, Dz) >= 0 crosses, made by the lanes of a warp: entry k of
+// Dx + Dy + Dz + 1 lies cx, cy, cz steps from the path's start and is `len` long over Q = 2 max(Dx,1) max(Dy,1)
+// max(Dz,1); `leaves` marks the entries that a crossing in x or y ends.  The crossings of each axis are an arithmetic
+// progression (crossing n at (2 n + 1) h), so rank, steps and length of every crossing follow in closed form.
+// Same order as path_sum: ties step z, then y, then x.
+template <typename F>
+__device__ __forceinline__ void path_list(int Dx, int Dy, int Dz, int lane, F put) {
+  const int mx = max(Dx, 1), my = max(Dy, 1), mz = max(Dz, 1), hx = my * mz, hy = mx * mz, hz = mx * my;
+  const int sxy = Dx + Dy, S = sxy + Dz;
+  auto before = [](int t, int h, int D, bool ties) { return D ? (t + h - (ties ? 0 : 1)) / (2 * h) : 0; };
+  for (int e = lane; e <= S; e += 32) {
+    int t, cx, cy, cz;  // this crossing, and the crossings of each axis that precede it
+    if (e == S) {
+      t = 2 * mx * hx, cx = Dx, cy = Dy, cz = Dz;
+    } else if (e < Dx) {
+      t = (2 * e + 1) * hx, cx = e, cy = before(t, hy, Dy, true), cz = before(t, hz, Dz, true);
+    } else if (e < sxy) {
+      t = (2 * (e - Dx) + 1) * hy, cy = e - Dx, cx = before(t, hx, Dx, false), cz = before(t, hz, Dz, true);
+    } else {
+      t = (2 * (e - sxy) + 1) * hz, cz = e - sxy, cx = before(t, hx, Dx, false), cy = before(t, hy, Dy, false);
+    }
+    const int prev = max(max((2 * cx - 1) * hx, (2 * cy - 1) * hy), max((2 * cz - 1) * hz, 0));
+    put(cx + cy + cz, cx, cy, cz, t - prev, e < sxy);
+  }
+}
+#endif
