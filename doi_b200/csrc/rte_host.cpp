@@ -337,7 +337,7 @@ struct rte_ctx {
   std::vector<double> h_mom;    // host copy of the moments [K][C][C]
   int* d_islot = nullptr;       // voxel -> slot
   float4* d_slot_xyz = nullptr; // slot -> (x, y, z, voxel)
-  int* d_err = nullptr;         // bounded-wait failure flag of the pair kernels
+  int* d_err = nullptr;         // bounded-wait failure flag of the pair kernels; the precompute's unit counter
   void* d_tab[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // angle rows [FP64][transposed] (rte_column.cu)
   double tab_kappa[2][2] = {{0, 0}, {0, 0}};  // the modulation their phases belong to
   // batched solves (several sources on one medium): buffers for up to bcap right-hand sides
@@ -605,7 +605,7 @@ int rte_create(const rte_config* cfg, rte_ctx** out) {
   }
   if (rc == RTE_OK) cu(dalloc(c, &c->d_islot, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_slot_xyz, c->N), "alloc");
-  if (rc == RTE_OK) cu(dalloc(c, &c->d_err, 1), "alloc");
+  if (rc == RTE_OK) cu(dalloc(c, &c->d_err, 2), "alloc");
   if (rc == RTE_OK) cu(cudaMemset(c->d_err, 0, sizeof(int)), "memset");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_cplx, 2 * NC), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_red, 8), "alloc");
@@ -903,6 +903,7 @@ static StoreArgs store_args(const rte_ctx* c, void* K, size_t ld, int col0, int 
   a.group = d.group;
   a.col0 = col0;
   a.col1 = col1;
+  a.counter = c->d_err + 1;
   return a;
 }
 

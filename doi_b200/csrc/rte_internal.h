@@ -58,6 +58,7 @@ struct StoreArgs {
   size_t Kld;
   int nzp, group;
   int col0, col1;
+  int* counter;       // scratch: next unit of work
   int npair, zb, group_ch;  // set by the launcher: column pairs per chunk, z block, chunks that share their lists
 };
 

@@ -12,8 +12,8 @@
 // written both ways.  mu_t is read from shared memory (in column order) when it fits, else through L1.
 //
 // Bound: instruction issue of the path sums (one add, one load, one multiply-add per voxel crossed) and the barriers
-// between lists, sums and write-out.  33^3 FP32: 22.8 ms by a walk per pair (70 % ALU) -> 9.2; FP64 35.3 -> 21;
-// 41^3 FP32: 96 -> 52.
+// between lists, sums and write-out.  33^3 FP32: 22.8 ms by a walk per pair (70 % ALU) -> 8.7; FP64 35.3 -> 21;
+// 41^3 FP32: 96 -> 50; of the 8.7 (50) ms the sums alone take 4.3 (28), the write-out 1.5 (8).
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -27,13 +27,17 @@
 
 namespace {
 
-constexpr int ST_THREADS = 512;
+// Threads of a CTA: 256 with mu_t in shared memory and room for three CTAs per SM, which go through their barriers
+// independently, else 512 (17^3 FP32 270 us with one CTA of 512 and chunks of 12 pairs in fixed turns; 200 with 256
+// threads and units by a counter; 180 with chunks of up to 30).
 // path sums per lane, of E column pairs: one list entry serves them all (33^3 FP32, mu_t in shared memory: 4 per lane
 // 10.1 ms, 6 9.2; 41^3 through L1: 4 50 ms, 6 55)
 template <typename T, bool STAGE>
 __host__ __device__ constexpr int st_e() {
   return sizeof(T) == 4 && STAGE ? 6 : 4;
 }
+constexpr size_t ST_SMALL = 72 * 1024;     // shared memory of a CTA, three per SM
+constexpr int ST_PAIRS = 30;               // most column pairs of a chunk (a warp lays them out)
 constexpr int ST_CAP = 3072;               // list entries per batch (one list has at most 3 * 1023 + 1)
 
 // A voxel of a path: its column offset and z steps from the destination (the sign of z is the pair's), and the
@@ -76,13 +80,13 @@ struct StLayout {
     off_o = off_f + sizeof(T) * 2 * nz;
     off_s = off_o + sizeof(size_t) * 2 * npair * zb;
     off_c = off_s + sizeof(int) * nz;
-    off_mu = (off_c + sizeof(int) * (2 * npair + 1) + 15) / 16 * 16;
+    off_mu = (off_c + sizeof(int) * (2 * npair + 2) + 15) / 16 * 16;
     bytes = off_mu + sizeof(T) * n_mu;
   }
 };
 
-template <typename T, bool STAGE, bool PACK, int G>
-__global__ void __launch_bounds__(ST_THREADS, STAGE ? 1 : 2) k_store_lists(StoreArgs a) {
+template <typename T, bool STAGE, bool PACK, int G, int ST_THREADS>
+__global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1 : 2)) k_store_lists(StoreArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nx = a.nx, ny = a.ny, nz = a.nz, tid = threadIdx.x, wid = tid / 32, lane = tid % 32;
   const StLayout<T, PACK> Sh(a.npair, a.zb, nz, STAGE ? a.N : 0);
@@ -92,6 +96,7 @@ __global__ void __launch_bounds__(ST_THREADS, STAGE ? 1 : 2) k_store_lists(Store
   size_t* so = reinterpret_cast<size_t*>(smem_raw + Sh.off_o);
   int* ls = reinterpret_cast<int*>(smem_raw + Sh.off_s);   // per |dz|: first entry
   int* cols = reinterpret_cast<int*>(smem_raw + Sh.off_c);  // [npair] destination, [npair] source columns, count
+  int& s_unit = cols[2 * a.npair + 1];
   T* smu = reinterpret_cast<T*>(smem_raw + Sh.off_mu);
   constexpr int E = st_e<T, STAGE>();
   const T* gmu = static_cast<const T*>(a.mu);
@@ -103,10 +108,11 @@ __global__ void __launch_bounds__(ST_THREADS, STAGE ? 1 : 2) k_store_lists(Store
   const int maxch = (nx * (y1 - y0 + 1) + a.npair - 1) / a.npair, ngrp = (maxch + a.group_ch - 1) / a.group_ch;
   const int zb = a.zb, nblk = (nz + zb - 1) / zb, pitch = zb | 1;
   const T dxf = (T)a.dx, dyf = (T)a.dy, dzf = (T)a.dz, thr = (T)a.prop_thresh;
-  for (long long w = blockIdx.x; w < (long long)noff * ngrp; w += gridDim.x) {
-    // neighbouring CTAs take neighbouring dx: their runs of destinations meet in L2
-    const int off = (int)(w % noff), ch0 = (int)(w / noff) * a.group_ch;
-    int dx, dy;  // destination minus source column
+  // Units (displacement, group of chunks) differ in size: a counter hands them out, group 0 of every displacement
+  // first.  Thread 0 draws the next one while the CTA works on this one, past those that do not exist.
+  const int nunit = noff * ngrp;
+  auto unit = [&](int u, int& dx, int& dy, int& xa, int& wx, int& ya) {  // destination minus source column; its pairs
+    const int off = u % noff;
     if (whole) {  // dy = 0, dx >= 0, then dy > 0
       dy = off < nx ? 0 : (off - nx) / (2 * nx - 1) + 1;
       dx = off < nx ? off : (off - nx) % (2 * nx - 1) - (nx - 1);
@@ -114,9 +120,23 @@ __global__ void __launch_bounds__(ST_THREADS, STAGE ? 1 : 2) k_store_lists(Store
       dy = off / (2 * nx - 1) - (ny - 1);
       dx = off % (2 * nx - 1) - (nx - 1);
     }
-    const int xa = max(0, -dx), wx = nx - abs(dx), ya = max(y0, -dy), yb = min(y1, ny - 1 - max(dy, 0));
-    const int np = wx * (yb - ya + 1);  // source columns xa.., ya.. of this displacement
-    if (yb < ya || ch0 * a.npair >= np) continue;
+    xa = max(0, -dx), wx = nx - abs(dx), ya = max(y0, -dy);  // source columns xa.., ya.. of this displacement
+    return wx * max(0, min(y1, ny - 1 - max(dy, 0)) - ya + 1);
+  };
+  auto exists = [&](int u) {
+    int q[5];
+    return u / noff * a.group_ch * a.npair < unit(u, q[0], q[1], q[2], q[3], q[4]);
+  };
+  for (int u = blockIdx.x; u < nunit;) {
+    __syncthreads();  // the previous unit's number is read
+    if (tid == 0) {
+      int n;
+      do n = (int)gridDim.x + atomicAdd(a.counter, 1);
+      while (n < nunit && !exists(n));
+      s_unit = n;
+    }
+    int dx, dy, xa, wx, ya;
+    const int np = unit(u, dx, dy, xa, wx, ya), ch0 = u / noff * a.group_ch;
     const int Dx = abs(dx), Dy = abs(dy), sxy = Dx + Dy;
     const int mx = max(Dx, 1), my = max(Dy, 1);
     const int stx = dx > 0 ? -nz : nz, sty = dy > 0 ? -nx * nz : nx * nz;  // steps towards the source
@@ -149,24 +169,24 @@ __global__ void __launch_bounds__(ST_THREADS, STAGE ? 1 : 2) k_store_lists(Store
         int a1 = a0, total = 0;  // lists a0 .. a1 - 1 of this batch
         while (a1 <= amax && total + sxy + a1 + 1 <= ST_CAP) total += sxy + a1++ + 1;
         if (a0 > amin) __syncthreads();
-        if (!once || ch == ch0)
+        if (!once || ch == ch0) {
+        for (int da = a0 + ST_THREADS - 1 - tid; da < a1; da += ST_THREADS) {
+          const T ex = (T)Dx * dxf, ey = (T)Dy * dyf, ez = (T)da * dzf;
+          const T d2 = fma(ex, ex, fma(ey, ey, ez * ez));
+          const double x = Dx * a.dx, y = Dy * a.dy, z = da * a.dz, r2 = x * x + y * y + z * z;
+          lf[2 * da] = (T)(-1.4426950408889634 * sqrt(r2) / (2.0 * mx * my * max(da, 1)));
+          lf[2 * da + 1] = d2 > T(0) && sqrt(d2) < thr ? (T)(a.kscale / r2) : T(0);
+        }
         for (int da = a0 + wid; da < a1; da += ST_THREADS / 32) {
-          const int Q = 2 * mx * my * max(da, 1);
           const int first = (da - a0) * (sxy + 1) + (da * (da - 1) - a0 * (a0 - 1)) / 2;
-          if (lane == 0) {
-            ls[da] = first;
-            const T ex = (T)Dx * dxf, ey = (T)Dy * dyf, ez = (T)da * dzf;
-            const T d2 = fma(ex, ex, fma(ey, ey, ez * ez));
-            const double x = Dx * a.dx, y = Dy * a.dy, z = da * a.dz, r2 = x * x + y * y + z * z;
-            lf[2 * da] = (T)(-1.4426950408889634 * sqrt(r2) / (double)Q);
-            lf[2 * da + 1] = d2 > T(0) && sqrt(d2) < thr ? (T)(a.kscale / r2) : T(0);
-          }
+          if (lane == 0) ls[da] = first;
           path_list(Dx, Dy, da, lane, [&](int k, int cx, int cy, int cz, int len, bool) {
             Entry<T, PACK> v;
             v.set(cx * stx + cy * sty, cz);
             v.len = (T)len;
             ent[first + k] = v;
           });
+        }
         }
         __syncthreads();
         const int npv = cols[2 * a.npair], jq = a.npair / E;  // lane element: (one of jq pairs) x E, z, sign of dz
@@ -195,7 +215,9 @@ __global__ void __launch_bounds__(ST_THREADS, STAGE ? 1 : 2) k_store_lists(Store
             const int pl = __shfl_sync(0xffffffffu, pl_l, l), np_ = __shfl_sync(0xffffffffu, np_l, l);
             const int ml = __shfl_sync(0xffffffffu, ml_l, l), per = np_ + __shfl_sync(0xffffffffu, nm_l, l);
             const bool live = f0 + lane < jq * per;
-            const int f = live ? f0 + lane : 0, js = f / per, r = f - js * per;
+            const int f = live ? f0 + lane : 0;
+            int js = 0, r = f;  // f / per, f % per; js < jq <= 4
+            while (r >= per) r -= per, ++js;
             const bool plus = r < np_;
             const int z = plus ? pl + r : ml + r - np_, sg = plus ? -1 : 1;
             uint32_t base[E];
@@ -269,19 +291,21 @@ __global__ void __launch_bounds__(ST_THREADS, STAGE ? 1 : 2) k_store_lists(Store
                   tile[(j * zb + zs) * pitch + zd];
         }
     }
+    __syncthreads();
+    u = s_unit;
   }
 }
 
-template <typename T, bool STAGE, bool PACK, int G>
-cudaError_t launch(StoreArgs a, int cap, int sms, cudaStream_t st) {
-  void (*kern)(StoreArgs) = k_store_lists<T, STAGE, PACK, G>;
+template <typename T, bool STAGE, bool PACK, int G, int ST_THREADS>
+cudaError_t launch_t(StoreArgs a, int cap, int sms, cudaStream_t st) {
+  void (*kern)(StoreArgs) = k_store_lists<T, STAGE, PACK, G, ST_THREADS>;
   typedef StLayout<T, PACK> Layout;
   const int nblk = (a.nz + 47) / 48;
   a.zb = (a.nz + nblk - 1) / nblk;
-  const size_t budget = STAGE && Layout(8, a.zb, a.nz, a.N).bytes > 110 * 1024 ? (size_t)cap : (size_t)110 * 1024;
+  const size_t budget = ST_THREADS == 256 ? ST_SMALL : STAGE && Layout(8, a.zb, a.nz, a.N).bytes > 110 * 1024 ? (size_t)cap : (size_t)110 * 1024;
   constexpr int E = st_e<T, STAGE>();
   a.npair = E;
-  while (a.npair + E <= 16 && Layout(a.npair + E, a.zb, a.nz, STAGE ? a.N : 0).bytes <= budget) a.npair += E;
+  while (a.npair + E <= ST_PAIRS && Layout(a.npair + E, a.zb, a.nz, STAGE ? a.N : 0).bytes <= budget) a.npair += E;
   const size_t smem = Layout(a.npair, a.zb, a.nz, STAGE ? a.N : 0).bytes;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
   if (e != cudaSuccess) return e;
@@ -294,8 +318,20 @@ cudaError_t launch(StoreArgs a, int cap, int sms, cudaStream_t st) {
   const long long noff = a.col0 == 0 && a.col1 == a.nx * a.ny ? (2 * a.nx - 1) * (a.ny - 1) + a.nx
                                                                : (2ll * a.nx - 1) * (2 * a.ny - 1);
   a.group_ch = (int)std::max<long long>(1, std::min<long long>(8, maxch * noff / (16ll * occ * sms)));
+  e = cudaMemsetAsync(a.counter, 0, sizeof(int), st);
+  if (e != cudaSuccess) return e;
   kern<<<occ * sms, ST_THREADS, smem, st>>>(a);
   return cudaGetLastError();
+}
+
+template <typename T, bool STAGE, bool PACK, int G>
+cudaError_t launch(const StoreArgs& a, int cap, int sms, cudaStream_t st) {
+  if constexpr (STAGE) {
+    const int nblk = (a.nz + 47) / 48, zb = (a.nz + nblk - 1) / nblk;
+    if (StLayout<T, PACK>(2 * st_e<T, STAGE>(), zb, a.nz, a.N).bytes <= ST_SMALL)
+      return launch_t<T, STAGE, PACK, G, 256>(a, cap, sms, st);
+  }
+  return launch_t<T, STAGE, PACK, G, 512>(a, cap, sms, st);
 }
 
 template <int G>
