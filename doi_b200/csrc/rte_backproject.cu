@@ -46,7 +46,9 @@ __device__ __forceinline__ int chunk_columns(int ch, int npair, int np, int nx, 
 // S of both columns once per pair of columns, so a pair of voxels costs four dot products of 2L+1 instead of four
 // of (L+1)^2 and an SH recurrence.  The trigonometric values of the displacements are FP64 values rounded to T.
 // A thread keeps the two contracted rows of one destination and goes through the sources of its column, whose rows
-// every lane reads (broadcast).
+// every lane reads (broadcast).  Bound by the latency of the loads of K and Q and of the contracted rows' making
+// (issue 42 %, shared memory 58 %).  33^3 L=5, per source: 17.8 ms by spherical harmonics per pair on 64 x 64 tiles
+// -> 9.3.
 template <int L>
 __host__ __device__ constexpr int bw_row() {
   return 2 * L + 2;  // (cos k, sin k) k = 1..L, then (k = 0, 0)
@@ -256,7 +258,7 @@ __global__ void __launch_bounds__(BP_THREADS, sizeof(T) == 4 ? (L <= 5 ? 3 : 2) 
 // u the lower end's z.  The rows of weights lie in shared memory one after another, each with |dz| + 1 or more zeros
 // behind its nz - |dz| values, so that entries whose pair does not exist read zeros: no test per entry, one list
 // entry read for 2 E weights, and no atomics but one FP64 addition per lane, pair and step (atomics on a shared
-// copy of the gradient per voxel crossed in their place: BPOLDW).  Lists and rows come in batches of |dz| when the
+// copy of the gradient per voxel crossed in their place: 86.7 ms at 33^3, now 29.1).  Lists and rows come in batches of |dz| when the
 // columns are too long for one.
 constexpr int BP_E = 3;
 constexpr int BP_CAP = 3072;  // most list entries of a batch (one list has at most 3 * 1023 + 1)

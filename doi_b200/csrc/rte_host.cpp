@@ -336,7 +336,6 @@ struct rte_ctx {
   size_t lut_cap = 0;
   std::vector<double> h_mom;    // host copy of the moments [K][C][C]
   int* d_islot = nullptr;       // voxel -> slot
-  float4* d_slot_xyz = nullptr; // slot -> (x, y, z, voxel)
   int* d_err = nullptr;         // bounded-wait failure flag of the pair kernels; the precompute's unit counter
   void* d_tab[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // angle rows [FP64][transposed] (rte_column.cu)
   double tab_kappa[2][2] = {{0, 0}, {0, 0}};  // the modulation their phases belong to
@@ -382,6 +381,7 @@ struct rte_ctx {
   bool fft_graph_failed = false;   // recording the transforms failed once: graphs use the pair kernels
   bool fft_in_graph[5] = {false, false, false, false, false};
   double* d_dmut = nullptr;     // Fisher: parameter direction of mu_t and mu_s [N], tangent dA S [N][C]
+  double* d_dmutc = nullptr;    // ... of mu_t in column order, in the operator's precision
   double* d_dmus = nullptr;
   double* d_T = nullptr;
   int* d_cidx = nullptr;        // source-column voxels and their source derivative
@@ -484,10 +484,10 @@ static void free_all(rte_ctx* c) {
   for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
   void* ps[] = {c->d_perm, c->d_mut, c->d_mus, c->d_mutf, c->d_W, c->d_Wn, c->d_sum, c->d_part, c->d_mom,
                 c->d_aux1, c->d_aux2, c->d_aux3, c->d_aux4, c->d_Wf, c->d_K, c->d_K64, c->d_cplx, c->d_red, c->d_img,
-                c->d_self_idx, c->d_self_lut, c->d_islot, c->d_slot_xyz, c->d_err,
+                c->d_self_idx, c->d_self_lut, c->d_islot, c->d_err,
                 c->d_bW, c->d_bWn, c->d_bsum, c->d_bres, c->d_bball, c->d_bWf, c->d_h, c->d_S, c->d_out,
                 c->d_e, c->d_lam, c->d_y, c->d_gt, c->d_gs, c->d_J, c->d_rho, c->d_dlut, c->d_fball, c->d_q, c->d_bq,
-                c->d_Qbp, c->d_mask, c->d_dmut, c->d_dmus, c->d_mut_self, c->d_mus_src, c->d_T, c->d_cidx, c->d_cval, c->d_self_lut_im,
+                c->d_Qbp, c->d_mask, c->d_dmut, c->d_dmutc, c->d_dmus, c->d_mut_self, c->d_mus_src, c->d_T, c->d_cidx, c->d_cval, c->d_self_lut_im,
                 c->d_fball_im, c->d_mutc, c->d_mutfc, c->d_slab, c->d_tab[0][0], c->d_tab[0][1], c->d_tab[1][0], c->d_tab[1][1]};
   for (void* p : ps)
     if (p) cudaFree(p);
@@ -604,7 +604,6 @@ int rte_create(const rte_config* cfg, rte_ctx** out) {
     if (rc == RTE_OK) cu(cudaMemset(c->d_Wf, 0, sizeof(double) * nrow), "memset");
   }
   if (rc == RTE_OK) cu(dalloc(c, &c->d_islot, c->N), "alloc");
-  if (rc == RTE_OK) cu(dalloc(c, &c->d_slot_xyz, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_err, 2), "alloc");
   if (rc == RTE_OK) cu(cudaMemset(c->d_err, 0, sizeof(int)), "memset");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_cplx, 2 * NC), "alloc");
@@ -616,20 +615,9 @@ int rte_create(const rte_config* cfg, rte_ctx** out) {
   if (rc == RTE_OK) {
     std::vector<int> p = column_perm(c->nx, c->ny, c->nz);
     std::vector<int> inv(c->N);
-    std::vector<float4> xyz(c->N);
-    for (int q = 0; q < c->N; q++) {
-      const int v = p[q];
-      inv[v] = q;
-      int bits;
-      memcpy(&bits, &v, sizeof bits);
-      float w;
-      memcpy(&w, &bits, sizeof w);
-      xyz[q] = make_float4((float)(v % c->nx), (float)((v / c->nx) % c->ny), (float)(v / (c->nx * c->ny)), w);
-    }
+    for (int q = 0; q < c->N; q++) inv[p[q]] = q;
     cu(cudaMemcpy(c->d_perm, p.data(), sizeof(int) * c->N, cudaMemcpyHostToDevice), "perm upload");
     if (rc == RTE_OK) cu(cudaMemcpy(c->d_islot, inv.data(), sizeof(int) * c->N, cudaMemcpyHostToDevice), "upload");
-    if (rc == RTE_OK)
-      cu(cudaMemcpy(c->d_slot_xyz, xyz.data(), sizeof(float4) * c->N, cudaMemcpyHostToDevice), "upload");
   }
   if (rc != RTE_OK) {
     free_all(c);
@@ -907,6 +895,38 @@ static StoreArgs store_args(const rte_ctx* c, void* K, size_t ld, int col0, int 
   return a;
 }
 
+// The workspace for a slab of source columns of the pair kernel (c->slab_cols of them): as many as 1 GB holds, fewer
+// when the device has less left.
+static int ensure_slab(rte_ctx* c) {
+  const int ncol = c->nx * c->ny;
+  const size_t per_col = kernel_cells(c, c->nz) * (c->precision == RTE_PREC_FP64 ? sizeof(double) : sizeof(float));
+  int cols = (int)std::max<size_t>(1, std::min<size_t>(ncol, kSlabBytes / per_col));
+  for (;; cols = (cols + 1) / 2) {
+    if (cols > c->nx && cols < ncol) cols = cols / c->nx * c->nx;  // whole rows of columns
+    const size_t bytes = per_col * cols;
+    if (bytes <= c->slab_bytes) break;
+    if (c->capturing) return fail(c, RTE_ERR_STATE, "the kernel workspace must exist before a graph is recorded");
+    if (c->d_slab) {
+      cudaFree(c->d_slab);
+      c->bytes -= c->slab_bytes;
+      c->d_slab = nullptr;
+      c->slab_bytes = 0;
+    }
+    unsigned char* m = nullptr;
+    const cudaError_t e = dalloc(c, &m, bytes);
+    if (e == cudaErrorMemoryAllocation && cols > 1) {
+      (void)cudaGetLastError();
+      continue;
+    }
+    CUDA_TRY(c, e);
+    c->d_slab = m;
+    c->slab_bytes = bytes;
+    break;
+  }
+  c->slab_cols = cols;
+  return RTE_OK;
+}
+
 // The stored pair kernel: FP32 for the mixed method (store or automatic mode), FP64 for the FP64 method when
 // RTE_KERNEL_STORE asks for it, or in automatic mode when it is no larger than the recompute workspace.
 // *stored = false: the kernel is recomputed in every application, a slab of source columns at a time (the
@@ -930,28 +950,7 @@ static int ensure_pair_kernel(rte_ctx* c, bool* stored) {
       CUDA_TRY(c, dalloc(c, &c->d_K, cells));
     }
   }
-  if (!keep) {
-    const int ncol = c->nx * c->ny;
-    const size_t per_col = kernel_cells(c, c->nz) * esize;
-    int cols = (int)std::max<size_t>(1, std::min<size_t>(ncol, kSlabBytes / per_col));
-    if (cols > c->nx && cols < ncol) cols = cols / c->nx * c->nx;  // whole rows of columns
-    const size_t bytes = per_col * cols;
-    if (bytes > c->slab_bytes) {
-      if (c->capturing) return fail(c, RTE_ERR_STATE, "the kernel workspace must exist before a graph is recorded");
-      if (c->d_slab) {
-        cudaFree(c->d_slab);
-        c->bytes -= c->slab_bytes;
-        c->d_slab = nullptr;
-        c->slab_bytes = 0;
-      }
-      unsigned char* m = nullptr;
-      CUDA_TRY(c, dalloc(c, &m, bytes));
-      c->d_slab = m;
-      c->slab_bytes = bytes;
-    }
-    c->slab_cols = cols;
-    return RTE_OK;
-  }
+  if (!keep) return ensure_slab(c);
   if (!c->K_valid || c->capture_store) {
     const StoreArgs a = store_args(c, f64 ? (void*)c->d_K64 : (void*)c->d_K, c->N, 0, c->nx * c->ny);
     if (c->capturing) {
@@ -975,10 +974,6 @@ static int ensure_pair_kernel(rte_ctx* c, bool* stored) {
 }
 
 static int check_kernel_err(rte_ctx* c);
-
-static inline int split_chunk(int N, int S) {
-  return ((N + S - 1) / S + RTE_PAIR_TS - 1) / RTE_PAIR_TS * RTE_PAIR_TS;
-}
 
 // Angle rows of the column kernels in the context's precision (and for the transposed table model).
 static int ensure_col_table(rte_ctx* c) {
@@ -3137,62 +3132,61 @@ extern "C" int rte_fisher_regions(rte_ctx* c, const rte_source* s, const rte_sto
 // For a parameter direction (dmu_a, dmu_s) per voxel and a converged forward solution
 // S = sum_k (DA)^k xi, out = A S, the discrete model's derivative is
 //   dS = (I - DA)^-1 [ dxi + dD (A S) + D (dA S) ],   d out = A dS + dA S,
-// dA S from k_pair_tangent (path integrals of dmu_t along every pair, the kernel recomputed or read
-// from the stored FP32 copy) plus the self-term derivative; dxi and the ballistic derivative of the
+// dA S by the column kernels on dK = -dtau K (tangent_pairs) plus the self-term derivative; dxi and the ballistic derivative of the
 // collimated beam by a complex step on the host (exact to rounding).  J = d(binned flux)/dtheta and,
 // with Poisson counts, F = J^T diag(1 / flux) J.
 
+
+// Off-diagonal part: the column operator with the derivative of the pair kernel, dK(r, r') = -dtau(r, r') K(r, r'),
+// dtau the path integral of dmu_t, a slab of source columns at a time; K is the stored one or recomputed in the slab.
+// Chunk sums into d_part, *S of them.  17^3 L=5 mixed, K recomputed, per parameter: 2.23 ms by a walk and spherical
+// harmonics per pair -> 0.46.
+static int tangent_pairs(rte_ctx* c, const double* d_in, const std::vector<double>& dmut, int* S) {
+  const int f = c->precision == RTE_PREC_FP64 ? 1 : 0, ncol = c->nx * c->ny, plane = ncol;
+  std::vector<double> col(c->N);  // the direction in column order, in the operator's precision
+  for (int r = 0; r < c->N; r++) {
+    const int slot = r % plane * c->nz + r / plane;
+    if (f)
+      col[slot] = dmut[r];
+    else
+      reinterpret_cast<float*>(col.data())[slot] = (float)dmut[r];
+  }
+  CUDA_TRY(c, cudaMemcpyAsync(c->d_dmutc, col.data(), (f ? sizeof(double) : sizeof(float)) * c->N, cudaMemcpyHostToDevice,
+                              c->st));
+  CUDA_TRY(c, (c->launches++, rte_launch_rows(d_in, rows_of(c, 1), c->d_islot, c->N, 1, col_dims(c).pitch, c->C, f, c->st)));
+  int rc = ensure_slab(c), chunk = 1;
+  if (rc) return rc;
+  const void* stored = !c->K_valid ? nullptr : f ? (const void*)c->d_K64 : (const void*)c->d_K;
+  const int cols = c->slab_cols;
+  const size_t ld = (size_t)cols * c->nz;
+  rc = plan_columns(c, c->L, 1, c->d_slab, ld, cols, &chunk, S);
+  if (rc) return rc;
+  for (int c0 = 0, s0 = 0; c0 < ncol; c0 += cols) {
+    StoreArgs a = store_args(c, c->d_slab, ld, c0, std::min(ncol, c0 + cols));
+    ProfScope ps(c, 0);
+    if (!stored) CUDA_TRY(c, (c->launches++, rte_launch_store_kernel(a, c->st, f)));
+    a.mu = c->d_dmutc;
+    a.Kin = stored ? stored : c->d_slab;
+    a.Kin_ld = stored ? (size_t)c->N : ld;
+    a.kin_slot = stored ? c0 * c->nz : 0;
+    CUDA_TRY(c, (c->launches++, rte_launch_store_kernel(a, c->st, f)));
+    const ColArgs ca = col_args(c, 1, c->d_slab, ld, c0, a.col1, chunk, s0);
+    CUDA_TRY(c, (c->launches++, launch_columns(c, ca, c->L)));
+    s0 += ca.nsplit;
+  }
+  return RTE_OK;
+}
+
 static int tangent_dA(rte_ctx* c, const double* d_in, double* d_outT, const std::vector<double>& dmut) {
   const size_t NC = (size_t)c->N * c->C;
-  int lo[3] = {c->nx, c->ny, c->nz}, hi[3] = {-1, -1, -1};
-  for (int r = 0; r < c->N; r++)
-    if (dmut[r] != 0.0) {
-      const int v[3] = {r % c->nx, (r / c->nx) % c->ny, r / (c->nx * c->ny)};
-      for (int a = 0; a < 3; a++) {
-        lo[a] = std::min(lo[a], v[a]);
-        hi[a] = std::max(hi[a], v[a]);
-      }
-    }
-  if (hi[0] < 0) return cudaMemsetAsync(d_outT, 0, NC * sizeof(double), c->st) == cudaSuccess
-                            ? RTE_OK : fail(c, RTE_ERR_DEVICE, "memset");
+  bool any = false;
+  for (int r = 0; r < c->N && !any; r++) any = dmut[r] != 0.0;
+  if (!any)
+    return cudaMemsetAsync(d_outT, 0, NC * sizeof(double), c->st) == cudaSuccess ? RTE_OK
+                                                                                : fail(c, RTE_ERR_DEVICE, "memset");
   CUDA_TRY(c, cudaMemcpyAsync(c->d_dmut, dmut.data(), sizeof(double) * c->N, cudaMemcpyHostToDevice, c->st));
-  const int tiles = (c->N + RTE_PAIR_THREADS - 1) / RTE_PAIR_THREADS;
-  const int S = std::max(1, std::min(c->max_split, (4 * 148 + tiles - 1) / tiles));
-  PairArgs a;
-  memset(&a, 0, sizeof a);
-  a.N = c->N;
-  a.nx = c->nx;
-  a.ny = c->ny;
-  a.nz = c->nz;
-  a.Cfull = c->C;
-  a.dx = c->dx;
-  a.dy = c->dy;
-  a.dz = c->dz;
-  a.prop_thresh = c->prop_thresh;
-  a.kscale = c->dV / c->cm;
-  a.perm = c->d_perm;
-  a.mut = c->d_mut;
-  a.mutf = c->d_mutf;
-  a.Kld = c->N;
-  a.nzp = col_dims(c).nzp;
-  a.group = col_dims(c).group;
-  a.Win = d_in;
-  a.part = c->d_part;
-  a.chunk = split_chunk(c->N, S);
-  a.nsplit = (c->N + a.chunk - 1) / a.chunk;
-  a.Kmat = c->K_valid && c->d_K ? c->d_K : nullptr;
-  a.Kmat64 = c->K_valid && c->d_K64 ? c->d_K64 : nullptr;
-  a.islot = c->d_islot;
-  a.dmut = c->d_dmut;
-  for (int q = 0; q < 3; q++) {
-    a.box_lo[q] = lo[q];
-    a.box_hi[q] = hi[q];
-  }
-  {
-    ProfScope ps(c, 0);
-    CUDA_TRY(c, (c->launches++, rte_launch_pair_tangent(a, c->L, c->precision == RTE_PREC_MIXED ? 0 : 1,
-                                                         c->model == RTE_MODEL_FIM ? 1 : 0, c->st)));
-  }
+  int S = 1, rc = tangent_pairs(c, d_in, dmut, &S);
+  if (rc) return rc;
   EpiArgs e;
   memset(&e, 0, sizeof e);
   e.N = c->N;
@@ -3200,9 +3194,10 @@ static int tangent_dA(rte_ctx* c, const double* d_in, double* d_outT, const std:
   e.ny = c->ny;
   e.nz = c->nz;
   e.Cfull = c->C;
-  e.S = a.nsplit;
+  e.S = S;
   e.nb = 1;
   e.part = c->d_part;
+  e.partf = c->precision == RTE_PREC_MIXED ? reinterpret_cast<const float*>(c->d_part) : nullptr;
   e.self = self_args(c, d_in);
   e.self.mut = c->d_mut;
   e.self.lut = c->d_dlut;
@@ -3212,7 +3207,6 @@ static int tangent_dA(rte_ctx* c, const double* d_in, double* d_outT, const std:
   e.Wout = d_outT;
   e.islot = c->d_islot;
   e.red = c->d_red;
-  CUDA_TRY(c, cudaMemsetAsync(c->d_red, 0, 4 * sizeof(double), c->st));
   CUDA_TRY(c, (c->launches++, rte_launch_epilogue(e, c->L, c->st)));
   return RTE_OK;
 }
@@ -3240,6 +3234,7 @@ extern "C" int rte_fisher(rte_ctx* c, int nsrc, const rte_source* srcs, const rt
   }
   if (!c->d_dmut) {
     CUDA_TRY(c, dalloc(c, &c->d_dmut, (size_t)c->N));
+    CUDA_TRY(c, dalloc(c, &c->d_dmutc, (size_t)c->N));
     CUDA_TRY(c, dalloc(c, &c->d_dmus, (size_t)c->N));
     CUDA_TRY(c, dalloc(c, &c->d_T, (size_t)std::max(2, nbt) * NC));  // nbt is fixed for a context (L, precision)
     CUDA_TRY(c, dalloc(c, &c->d_cidx, (size_t)std::max(c->nx, std::max(c->ny, c->nz))));

@@ -26,27 +26,17 @@ __host__ __device__ inline int kmat_pos(int slot, int nz, int nzp) { return slot
 // ... of a complex pair's kernel: the same, or one where two sets of sums exceed the registers
 #define RTE_COL_GC(L, fp64) ((L) <= ((fp64) ? 3 : 5) ? RTE_COL_G(L) : 1)
 
+// Plain FP64 pair operator (k_pair_fp64): sums over `chunk` sources per blockIdx.y.
 struct PairArgs {
   int N, nx, ny, nz, Cfull;
   double dx, dy, dz;
   double prop_thresh;
   double kscale;        // dV / cm folded into the pair kernel
-  const int* perm;      // slot -> voxel index (column order)
-  const int* islot;     // voxel -> slot
-  const double* mut;    // mu_t per voxel, FP64
-  const float* mutf;    // mu_t per voxel, FP32
-  float* Kmat;          // FP32 pair kernel, blocked (kmat_index, ld = Kld, columns padded to nzp)
-  double* Kmat64;       // FP64 pair kernel, same layout
-  size_t Kld;
-  int nzp, group;
-  // tangent pass (k_pair_tangent): current term N x Cfull, sums over `chunk` sources per blockIdx.y, derivative
-  // of mu_t along a parameter direction, and the voxel bounding box of its support (pairs whose segment misses
-  // the box have no path derivative)
-  const double* Win;
+  const int* perm;      // thread -> voxel index
+  const double* mut;    // mu_t per voxel
+  const double* Win;    // [N][Cfull]
   double* part;         // partial sums [S][N][Cfull], indexed by voxel
   int chunk, nsplit;
-  const double* dmut;
-  int box_lo[3], box_hi[3];  // (x, y, z) voxel indices
 };
 
 // Pair-kernel precompute (rte_store.cu): rows of the source columns [col0, col1), destinations all.
@@ -58,6 +48,9 @@ struct StoreArgs {
   size_t Kld;
   int nzp, group;
   int col0, col1;
+  const void* Kin;    // derivative mode: K of the same sources, whose slot 0 of this launch is row kin_slot (may be K)
+  size_t Kin_ld;
+  int kin_slot;
   int* counter;       // scratch: next unit of work
   int npair, zb, group_ch;  // set by the launcher: column pairs per chunk, z block, chunks that share their lists
 };
@@ -239,7 +232,6 @@ cudaError_t rte_launch_y_field(double* y, const double* e, const double* lam, co
 // over every unordered pair scattering Q * length into the gradient.
 cudaError_t rte_launch_bp_weights(const BpArgs& a, int LA, int fp64, cudaStream_t st);
 cudaError_t rte_launch_bp_walk(const BpArgs& a, int fp64, cudaStream_t st);
-cudaError_t rte_launch_pair_tangent(const PairArgs& a, int LA, int fp64, int table, cudaStream_t st);
 // q = mus * scat_l * T + dmus * scat_l * out (per voxel and coefficient; q rows qstride apart)
 cudaError_t rte_launch_tangent_rhs(double* q, int qstride, const double* T, const double* out, const double* mus,
                                    const double* dmus, const double* scat, int N, int L, cudaStream_t st);

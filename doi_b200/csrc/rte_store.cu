@@ -11,6 +11,9 @@
 // destinations per source row; over all sources K is symmetric, so half of the displacements are computed and
 // written both ways.  mu_t is read from shared memory (in column order) when it fits, else through L1.
 //
+// DERIV: the derivative of K along a direction of mu_t instead, K times minus the path integral of the direction
+// (mu: the direction, Kin: K of the same sources, which may be the output).
+//
 // Bound: instruction issue of the path sums (one add, one load, one multiply-add per voxel crossed) and the barriers
 // between lists, sums and write-out.  33^3 FP32: 22.8 ms by a walk per pair (70 % ALU) -> 8.7; FP64 35.3 -> 21;
 // 41^3 FP32: 96 -> 50; of the 8.7 (50) ms the sums alone take 4.3 (28), the write-out 1.5 (8).
@@ -85,7 +88,7 @@ struct StLayout {
   }
 };
 
-template <typename T, bool STAGE, bool PACK, int G, int ST_THREADS>
+template <typename T, bool STAGE, bool PACK, int G, int ST_THREADS, bool DERIV>
 __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1 : 2)) k_store_lists(StoreArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nx = a.nx, ny = a.ny, nz = a.nz, tid = threadIdx.x, wid = tid / 32, lane = tid % 32;
@@ -174,7 +177,7 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
           const T ex = (T)Dx * dxf, ey = (T)Dy * dyf, ez = (T)da * dzf;
           const T d2 = fma(ex, ex, fma(ey, ey, ez * ez));
           const double x = Dx * a.dx, y = Dy * a.dy, z = da * a.dz, r2 = x * x + y * y + z * z;
-          lf[2 * da] = (T)(-1.4426950408889634 * sqrt(r2) / (2.0 * mx * my * max(da, 1)));
+          lf[2 * da] = (T)((DERIV ? -1.0 : -1.4426950408889634) * sqrt(r2) / (2.0 * mx * my * max(da, 1)));
           lf[2 * da + 1] = d2 > T(0) && sqrt(d2) < thr ? (T)(a.kscale / r2) : T(0);
         }
         for (int da = a0 + wid; da < a1; da += ST_THREADS / 32) {
@@ -252,7 +255,9 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
 #pragma unroll
             for (int q = 0; q < E; ++q) {
               T k;
-              if constexpr (std::is_same<T, float>::value)
+              if constexpr (DERIV)
+                k = acc[q] * f1;
+              else if constexpr (std::is_same<T, float>::value)
                 k = exp2f(acc[q] * f1) * f2;
               else
                 k = exp2(acc[q] * f1) * f2;
@@ -273,22 +278,31 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
         const unsigned jj = e / zb, zz = e - jj * zb, side = jj >= (unsigned)npv;
         const int col = side ? cols[a.npair + jj - npv] : cols[jj];
         const unsigned p = (unsigned)(col * a.nzp + (side ? s0 : d0)) + zz, o = p % KB;
-        so[(side * a.npair + (side ? jj - npv : jj)) * zb + zz] = (size_t)(p / KB) * a.Kld * KB + o % G * 32 + o / G;
+        size_t& at = so[(side * a.npair + (side ? jj - npv : jj)) * zb + zz];
+        if constexpr (DERIV)
+          at = (size_t)(p / KB) << 32 | (o % G * 32 + o / G);
+        else
+          at = (size_t)(p / KB) * a.Kld * KB + o % G * 32 + o / G;
       }
       __syncthreads();
+      auto put = [&](size_t at, unsigned src, T v) {  // src: source slot from the slab's first
+        if constexpr (DERIV)
+          K[((at >> 32) * a.Kld + src) * KB + (uint32_t)at] =
+              v * static_cast<const T*>(a.Kin)[((at >> 32) * a.Kin_ld + a.kin_slot + src) * KB + (uint32_t)at];
+        else
+          K[at + (size_t)src * KB] = v;
+      };
       for (unsigned e = tid; e < nd * ns; e += ST_THREADS) {
         const unsigned zs = (e * md) >> 20, zd = e - zs * nd;  // e < 48^2
         for (int j = 0; j < npv; ++j)
-          K[so[j * zb + zd] + (size_t)(unsigned)(cols[a.npair + j] * nz + s0 - src0 + (int)zs) * KB] =
-              tile[(j * zb + zs) * pitch + zd];
+          put(so[j * zb + zd], (unsigned)(cols[a.npair + j] * nz + s0 - src0 + (int)zs), tile[(j * zb + zs) * pitch + zd]);
       }
       if (whole)
         for (unsigned e = tid; e < nd * ns; e += ST_THREADS) {
           const unsigned zd = (e * ms) >> 20, zs = e - zd * ns;
           for (int j = 0; j < npv; ++j)
             if (cols[j] != cols[a.npair + j])
-              K[so[(a.npair + j) * zb + zs] + (size_t)(unsigned)(cols[j] * nz + d0 + (int)zd) * KB] =
-                  tile[(j * zb + zs) * pitch + zd];
+              put(so[(a.npair + j) * zb + zs], (unsigned)(cols[j] * nz + d0 + (int)zd), tile[(j * zb + zs) * pitch + zd]);
         }
     }
     __syncthreads();
@@ -296,9 +310,9 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
   }
 }
 
-template <typename T, bool STAGE, bool PACK, int G, int ST_THREADS>
-cudaError_t launch_t(StoreArgs a, int cap, int sms, cudaStream_t st) {
-  void (*kern)(StoreArgs) = k_store_lists<T, STAGE, PACK, G, ST_THREADS>;
+template <typename T, bool STAGE, bool PACK, int G, int ST_THREADS, bool DERIV>
+cudaError_t launch_d(StoreArgs a, int cap, int sms, cudaStream_t st) {
+  void (*kern)(StoreArgs) = k_store_lists<T, STAGE, PACK, G, ST_THREADS, DERIV>;
   typedef StLayout<T, PACK> Layout;
   const int nblk = (a.nz + 47) / 48;
   a.zb = (a.nz + nblk - 1) / nblk;
@@ -322,6 +336,12 @@ cudaError_t launch_t(StoreArgs a, int cap, int sms, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   kern<<<occ * sms, ST_THREADS, smem, st>>>(a);
   return cudaGetLastError();
+}
+
+template <typename T, bool STAGE, bool PACK, int G, int ST_THREADS>
+cudaError_t launch_t(const StoreArgs& a, int cap, int sms, cudaStream_t st) {
+  return a.Kin ? launch_d<T, STAGE, PACK, G, ST_THREADS, true>(a, cap, sms, st)
+               : launch_d<T, STAGE, PACK, G, ST_THREADS, false>(a, cap, sms, st);
 }
 
 template <typename T, bool STAGE, bool PACK, int G>
