@@ -52,7 +52,8 @@ struct StoreArgs {
   size_t Kin_ld;
   int kin_slot;
   int* counter;       // scratch: next unit of work
-  int npair, zb, group_ch;  // set by the launcher: column pairs per chunk, z block, chunks that share their lists
+  // set by the launcher: column pairs per chunk, z block, chunks that share their lists, list entries of a batch
+  int npair, zb, group_ch, cap;
 };
 
 // Column form of the pair operator (rte_column.cu): sources and destinations in column order, one CTA per

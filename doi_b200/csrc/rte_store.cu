@@ -15,8 +15,8 @@
 // (mu: the direction, Kin: K of the same sources, which may be the output).
 //
 // Bound: instruction issue of the path sums (one add, one load, one multiply-add per voxel crossed) and the barriers
-// between lists, sums and write-out.  33^3 FP32: 22.8 ms by a walk per pair (70 % ALU) -> 8.7; FP64 35.3 -> 21;
-// 41^3 FP32: 96 -> 50; of the 8.7 (50) ms the sums alone take 4.3 (28), the write-out 1.5 (8).
+// between lists, sums and write-out.  33^3 FP32: 22.8 ms by a walk per pair (70 % ALU) -> 8.8; FP64 35.3 -> 21;
+// 41^3 FP32: 96 -> 44; of the 8.8 (44) ms the sums alone take about half, the write-out a sixth.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -32,7 +32,8 @@ namespace {
 
 // Threads of a CTA: 256 with mu_t in shared memory and room for three CTAs per SM, which go through their barriers
 // independently, else 512 (17^3 FP32 270 us with one CTA of 512 and chunks of 12 pairs in fixed turns; 200 with 256
-// threads and units by a counter; 180 with chunks of up to 30).
+// threads and units by a counter; 180 with chunks of up to 30; 152 with room for the entries the grid can have,
+// FP64 442 -> 273).
 // path sums per lane, of E column pairs: one list entry serves them all (33^3 FP32, mu_t in shared memory: 4 per lane
 // 10.1 ms, 6 9.2; 41^3 through L1: 4 50 ms, 6 55)
 template <typename T, bool STAGE>
@@ -72,13 +73,13 @@ struct __align__(16) Entry<double, false> {
   __device__ int oz() const { return z; }
 };
 
-// entries | tile [npair][zb][zb | 1] | per list: f1, f2 | per pair and z: kernel offset of the destination and of the
+// entries [cap] | tile [npair][zb][zb | 1] | per list: f1, f2 | per pair and z: kernel offset of the destination and of the
 // source column's position | per list: start | per pair: destination, source column | mu_t
 template <typename T, bool PACK>
 struct StLayout {
   size_t off_tile, off_f, off_o, off_s, off_c, off_mu, bytes;
-  __host__ __device__ StLayout(int npair, int zb, int nz, int n_mu) {
-    off_tile = sizeof(Entry<T, PACK>) * ST_CAP;
+  __host__ __device__ StLayout(int npair, int zb, int nz, int cap, int n_mu) {
+    off_tile = sizeof(Entry<T, PACK>) * cap;
     off_f = (off_tile + sizeof(T) * npair * zb * (zb | 1) + 15) / 16 * 16;
     off_o = off_f + sizeof(T) * 2 * nz;
     off_s = off_o + sizeof(size_t) * 2 * npair * zb;
@@ -92,7 +93,7 @@ template <typename T, bool STAGE, bool PACK, int G, int ST_THREADS, bool DERIV>
 __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1 : 2)) k_store_lists(StoreArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nx = a.nx, ny = a.ny, nz = a.nz, tid = threadIdx.x, wid = tid / 32, lane = tid % 32;
-  const StLayout<T, PACK> Sh(a.npair, a.zb, nz, STAGE ? a.N : 0);
+  const StLayout<T, PACK> Sh(a.npair, a.zb, nz, a.cap, STAGE ? a.N : 0);
   Entry<T, PACK>* ent = reinterpret_cast<Entry<T, PACK>*>(smem_raw);
   T* tile = reinterpret_cast<T*>(smem_raw + Sh.off_tile);
   T* lf = reinterpret_cast<T*>(smem_raw + Sh.off_f);       // per |dz|: log2(e) dist / Q (exp2 argument), dV / (cm dist^2)
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
     const int mx = max(Dx, 1), my = max(Dy, 1);
     const int stx = dx > 0 ? -nz : nz, sty = dy > 0 ? -nx * nz : nx * nz;  // steps towards the source
     // one batch holds all lists of the displacement (ordinary grids): made once for the group's chunks
-    const bool once = nblk == 1 && nz * (sxy + 1) + nz * (nz - 1) / 2 <= ST_CAP;
+    const bool once = nblk == 1 && nz * (sxy + 1) + nz * (nz - 1) / 2 <= a.cap;
     for (int ch = ch0; ch < ch0 + a.group_ch && ch * a.npair < np; ++ch)
     for (int bb = 0; bb < nblk * nblk; ++bb) {
       // destination z in [d0, d1), source z in [s0, s1)
@@ -170,7 +171,7 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
       }
       for (int a0 = amin; a0 <= amax;) {
         int a1 = a0, total = 0;  // lists a0 .. a1 - 1 of this batch
-        while (a1 <= amax && total + sxy + a1 + 1 <= ST_CAP) total += sxy + a1++ + 1;
+        while (a1 <= amax && total + sxy + a1 + 1 <= a.cap) total += sxy + a1++ + 1;
         if (a0 > amin) __syncthreads();
         if (!once || ch == ch0) {
         for (int da = a0 + ST_THREADS - 1 - tid; da < a1; da += ST_THREADS) {
@@ -310,17 +311,25 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
   }
 }
 
+// list entries of a batch: those of all lists of the longest displacement, when they are fewer
+int st_cap(const StoreArgs& a) {
+  const long long all = (long long)a.nz * (a.nx + a.ny - 1) + (long long)a.nz * (a.nz - 1) / 2;
+  return (int)std::min<long long>(ST_CAP, (all + 3) / 4 * 4);
+}
+
 template <typename T, bool STAGE, bool PACK, int G, int ST_THREADS, bool DERIV>
 cudaError_t launch_d(StoreArgs a, int cap, int sms, cudaStream_t st) {
   void (*kern)(StoreArgs) = k_store_lists<T, STAGE, PACK, G, ST_THREADS, DERIV>;
   typedef StLayout<T, PACK> Layout;
   const int nblk = (a.nz + 47) / 48;
   a.zb = (a.nz + nblk - 1) / nblk;
-  const size_t budget = ST_THREADS == 256 ? ST_SMALL : STAGE && Layout(8, a.zb, a.nz, a.N).bytes > 110 * 1024 ? (size_t)cap : (size_t)110 * 1024;
+  a.cap = st_cap(a);
+  const size_t budget = ST_THREADS == 256 ? ST_SMALL
+                        : STAGE && Layout(8, a.zb, a.nz, a.cap, a.N).bytes > 110 * 1024 ? (size_t)cap : (size_t)110 * 1024;
   constexpr int E = st_e<T, STAGE>();
   a.npair = E;
-  while (a.npair + E <= ST_PAIRS && Layout(a.npair + E, a.zb, a.nz, STAGE ? a.N : 0).bytes <= budget) a.npair += E;
-  const size_t smem = Layout(a.npair, a.zb, a.nz, STAGE ? a.N : 0).bytes;
+  while (a.npair + E <= ST_PAIRS && Layout(a.npair + E, a.zb, a.nz, a.cap, STAGE ? a.N : 0).bytes <= budget) a.npair += E;
+  const size_t smem = Layout(a.npair, a.zb, a.nz, a.cap, STAGE ? a.N : 0).bytes;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
   if (e != cudaSuccess) return e;
   int occ = 0;
@@ -348,7 +357,7 @@ template <typename T, bool STAGE, bool PACK, int G>
 cudaError_t launch(const StoreArgs& a, int cap, int sms, cudaStream_t st) {
   if constexpr (STAGE) {
     const int nblk = (a.nz + 47) / 48, zb = (a.nz + nblk - 1) / nblk;
-    if (StLayout<T, PACK>(2 * st_e<T, STAGE>(), zb, a.nz, a.N).bytes <= ST_SMALL)
+    if (StLayout<T, PACK>(2 * st_e<T, STAGE>(), zb, a.nz, st_cap(a), a.N).bytes <= ST_SMALL)
       return launch_t<T, STAGE, PACK, G, 256>(a, cap, sms, st);
   }
   return launch_t<T, STAGE, PACK, G, 512>(a, cap, sms, st);
@@ -358,7 +367,7 @@ template <int G>
 cudaError_t launch_G(const StoreArgs& a, int fp64, int cap, int sms, cudaStream_t st) {
   // mu_t in shared memory when 48 KB and more remain for tiles beside the lists
   const size_t es = fp64 ? sizeof(double) : sizeof(float);
-  const size_t lists = ST_CAP * (fp64 ? sizeof(Entry<double, false>) : sizeof(Entry<float, true>));
+  const size_t lists = st_cap(a) * (fp64 ? sizeof(Entry<double, false>) : sizeof(Entry<float, true>));
   const bool stage = es * a.N + lists + 48 * 1024 <= (size_t)cap;
   if (fp64) return stage ? launch<double, true, false, G>(a, cap, sms, st) : launch<double, false, false, G>(a, cap, sms, st);
   if (stage) return launch<float, true, true, G>(a, cap, sms, st);
