@@ -561,8 +561,7 @@ def run_ours(args):
     src = R.Source(pos_x=0.0, pos_y=0.0, kind=R.SRC_COLUMN)
     stop = R.Stop(R.STOP_FIXED, TERMS)
     # batched form: B of the four collimated z=0 sources at (+-0.825, +-0.825) cm of the adjoint
-    # configuration, solved together on each phantom (each pair's direction, spherical harmonics and
-    # kernel value serve all B sources)
+    # configuration, solved together on each phantom (one pair kernel serves all B sources)
     B = args.batch
     srcs = [R.Source(pos_x=x, pos_y=y, kind=R.SRC_COLUMN) for x, y in
             ((-0.825, -0.825), (0.825, -0.825), (-0.825, 0.825), (0.825, 0.825))][:B] if B > 1 else [src]
@@ -676,8 +675,9 @@ def run_ours(args):
             c64.close()
         avg_pair_ms = st["ms_pair"] / max(st["n_pair"], 1)
         nbk = 1 if B == 1 else (2 if B <= 2 else 4)  # right-hand sides per launch
-        # algorithmic FLOP per launch: per coupled pair 3C (SH) + 4C per right-hand side + 10 (direction)
-        apply_flop = counts["pairs"] * (3 * counts["C"] + 4 * counts["C"] * B + 10)
+        # algorithmic FLOP per launch: per coupled pair and right-hand side 2L+1 multiply-adds in and out (the
+        # coefficients contract onto the meridian of a pair of columns)
+        apply_flop = counts["pairs"] * 4 * (2 * L + 1) * B
         achieved = apply_flop / (avg_pair_ms * 1e-3) / 1e12
         peak = peak32 if prec == R.PREC_MIXED else peak64
         # DRAM bytes of one pair launch from the ncu capture in profiles/ (per pair, scaled to this grid)
@@ -702,8 +702,8 @@ def run_ours(args):
                        "parallelism": f"replicas x{ws}"},
             "roofline": {"bound": "fp32-cuda-core" if prec == R.PREC_MIXED else "fp64-cuda-core",
                          "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-                         "traffic": traffic, "kernel": f"k_pair_mixed_tk<5,{nbk}> (stored FP32 kernel staged by bulk copy)"
-                         if prec == R.PREC_MIXED else "k_pair_fp64<5>", "avg_launch_ms": avg_pair_ms,
+                         "traffic": traffic, "kernel": "k_column<5,float> (stored FP32 kernel staged by bulk copy)"
+                         if prec == R.PREC_MIXED else "k_column<5,double>", "avg_launch_ms": avg_pair_ms,
                          "flop_per_launch": apply_flop, "rhs_per_launch": nbk,
                          "peak_source": ("measured in this run by rte_measure_fma_peak (8 independent FMA chains "
                                          "per thread on every SM), of measured; theoretical FP32 148 SMs x 128 "

@@ -1059,8 +1059,8 @@ static cudaError_t launch_columns(const rte_ctx* c, const ColArgs& a, int LA) {
 
 // Launch-plan autotuner of the column kernels.  The grid is (tiles of 128 threads' destinations x right-hand
 // sides) x (chunks of source columns); more chunks fill the SMs' last wave better and cost chunk sums.
-// Candidates are the chunk sizes that a model of waves and chunk-sum traffic ranks best; in mixed precision on
-// 4096 voxels and more each is launched on the context's own buffers and timed with CUDA events (best of two),
+// Candidates are the chunk sizes that a model of waves and chunk-sum traffic ranks best; on
+// 1024 voxels and more each is launched on the context's own buffers and timed with CUDA events (best of two),
 // and the fastest is kept for the process (every context of that shape on that device reuses it).
 // RTE_AUTOTUNE=0 keeps the model's choice; RTE_NSPLIT forces a split.
 namespace {

@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
             const int v = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += v;
           }
-          const int ntask = __shfl_sync(0xffffffffu, incl, 31);
+          const int ntask = npv > 0 ? __shfl_sync(0xffffffffu, incl, 31) : 0;  // a chunk may miss the slab's columns
           int task = rot;
           for (; task < ntask; task += ST_THREADS / 32) {
             const int l = __ffs(__ballot_sync(0xffffffffu, incl > task)) - 1, da = a1 - 1 - (ab - a0) - l;

@@ -258,9 +258,8 @@ int rte_fisher(rte_ctx* ctx, int nsrc, const rte_source* srcs, const rte_stop* s
                int P, const double* dmua, const double* dmus, double* J, double* F);
 
 /* Batched forward solves (new): nsrc <= 4 sources on the current medium, propagated together so
- * each voxel pair's direction, spherical harmonics and kernel value serve every source.  Outputs
- * are the nsrc single-source results back to back (W_out nsrc*N*C, trans/ref nsrc*nX*nY, each may
- * be NULL).  Stop rule RTE_STOP_FIXED or RTE_STOP_REL_L2 (norms over all sources). */
+ * one pair kernel serves every source.  Outputs are the nsrc single-source results back to back
+ * (W_out nsrc*N*C, trans/ref nsrc*nX*nY, each may be NULL).  Stop rule RTE_STOP_FIXED or RTE_STOP_REL_L2 (norms over all sources). */
 int rte_forward_batch(rte_ctx* ctx, int nsrc, const rte_source* srcs, const rte_stop* stop,
                       rte_cplx* W_out, rte_cplx* trans, rte_cplx* ref, rte_report* report);
 

@@ -50,3 +50,20 @@ def test_recompute_slabs_equal_the_stored_kernel(rte, n, prec, tol):
             ctx.set_medium_voxel(mua, mus)
             out.append(ctx.prop_abs(W, 1, 0))
     assert rel(out[1], out[0]) < tol
+
+
+@pytest.mark.parametrize("nx,nz,prec,tol", [(160, 64, 0, 1e-12), (200, 64, 1, 2e-6)])
+def test_slabs_of_partial_rows_equal_the_stored_kernel(rte, nx, nz, prec, tol):
+    """The workspace holds fewer columns than a row of the grid has, so slabs start and end within rows and some
+    chunks of column pairs have no source in the slab."""
+    rng = np.random.default_rng(nx)
+    N, L = nx * 2 * nz, 1
+    assert N * nz * (8, 4)[prec] * nx > 1 << 30  # one row of source columns is more than the workspace
+    mua, mus = rng.uniform(0.005, 0.1, N), rng.uniform(0.5, 2.0, N)
+    W = real_to_complex(rng.standard_normal((N, 4)), L)
+    out = []
+    for mode in (rte.KERNEL_STORE, rte.KERNEL_RECOMPUTE):
+        with rte.Context(nx, 2, nz, dx=0.1, nL=L, g=0.8, precision=prec, kernel_mode=mode) as ctx:
+            ctx.set_medium_voxel(mua, mus)
+            out.append(ctx.prop_abs(W, 1, 0))
+    assert rel(out[1], out[0]) < tol
