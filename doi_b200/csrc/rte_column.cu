@@ -70,10 +70,10 @@ struct ColLayout {
 };
 
 // columns of tensor memory for the sums of a thread's destinations (a power of two, at least 32)
-template <int L, typename T, int G, bool CPLX>
+template <int L, typename T, int G, int NB>
 __host__ __device__ constexpr int tmem_cols() {
   int n = 32;
-  while (n < (CPLX ? 2 : 1) * G * (L + 1) * (L + 1) * (int)(sizeof(T) / 4)) n *= 2;
+  while (n < NB * G * (L + 1) * (L + 1) * (int)(sizeof(T) / 4)) n *= 2;
   return n;
 }
 
@@ -84,16 +84,17 @@ __host__ __device__ constexpr int tmem_cols() {
 // one new trigonometric row per source serves all G.  The pair kernel is streamed by bulk copies, a ring of
 // stages per warp (each warp's values are contiguous: kmat_index); register prefetch in its place waited on
 // every load (5.9 ms against 2.7 at 33^3 L=5).  The coefficient sums, touched once per source column, live in
-// tensor memory, which leaves the registers of four CTAs per SM.  CPLX: (real, imaginary) rows of one complex
+// tensor memory, which leaves the registers of four CTAs per SM.  NB = 2: two right-hand sides a thread, which
+// share the trigonometric rows, the kernel values and the copies (two CTAs per SM at L >= 4).  CPLX: (real, imaginary) rows of one complex
 // right-hand side, the pair kernel times exp(-i kappa r) (phase tabulated beside the angles).
 // 33^3 L=5 launch, FP32, one right-hand side: 7.40 ms by per-pair spherical harmonics -> 2.36; four: 20.1 -> 9.3;
 // FP64: 24.7 -> 4.3.  Of the 2.4 ms, skipping phases one at a time: pair loop 1.15, contraction 0.25, angle rows
 // 0.2, the kernel stream 0.15, the rest expansion, start of runs and barriers.  All copies are bulk copies by warp 0
 // and by each warp for its own ring (copies by all threads: 2.40, FP64 5.4); deeper rings and a fifth of the
 // registers less did not pay (ring of 3 stages 2.37, four CTAs with 3-row stages 2.50).
-template <int L, typename T, int G, bool CPLX, bool FULL>
+template <int L, typename T, int G, int NB, bool CPLX, bool FULL>
 __device__ __forceinline__ void column_body(const ColArgs& a) {
-  constexpr int C = (L + 1) * (L + 1), NT = nb_row<L>(), NB = CPLX ? 2 : 1, LL = L > 0 ? L : 1;
+  constexpr int C = (L + 1) * (L + 1), NT = nb_row<L>(), LL = L > 0 ? L : 1;
   constexpr bool SUB = G == 1;  // one destination of each thread of the layout's groups
   constexpr bool F32 = std::is_same<T, float>::value;
   constexpr int U = ring_rows<G>(), NST = ring_stages<G>();
@@ -110,7 +111,8 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
   T* sK = sW + Sh.off_k + wid * NST * U * 32 * G;
   uint64_t* kbar = bar + 2 + wid * NST;
   const int tid = threadIdx.x, nz = a.nz, ncol = a.nx * a.ny;
-  const int tile = blockIdx.x / a.nrhs, rhs = CPLX ? 0 : blockIdx.x - tile * a.nrhs;
+  const int nrg = CPLX ? 1 : a.nrhs / NB;  // groups of right-hand sides
+  const int tile = blockIdx.x / nrg, rhs = (blockIdx.x - tile * nrg) * NB;
   const int p0 = tile * T_CTA * G, np = ncol * a.nzp;  // destination positions: columns padded to nzp
   // destination columns of the CTA (SUB: those of the layout's blocks that its warps lie in)
   const int pa = SUB ? p0 / (32 * a.group) * 32 * a.group : p0;
@@ -129,7 +131,7 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (blockIdx.x == 0 && blockIdx.y == 0 && tid < 4 && a.red) a.red[tid] = 0.0;
-  constexpr int TMC = tmem_cols<L, T, G, CPLX>(), W32 = sizeof(T) / 4;
+  constexpr int TMC = tmem_cols<L, T, G, NB>(), W32 = sizeof(T) / 4;
   if (wid == 0) tmem_alloc(stm, TMC);
   tmem_fence_before();
   for (int q = tid; q < ncd; q += T_CTA) sxy[q] = ((c0 + q) / a.nx) << 16 | (c0 + q) % a.nx;
@@ -493,15 +495,16 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
 
 // CTAs per SM to fit the registers to: four warps per scheduler hide the latencies of one another's loads (33^3
 // L=5: 2.77 ms per launch at two CTAs with the sums in registers, 2.41 at four with them in tensor memory)
-template <int L, typename T, bool CPLX>
+template <int L, typename T, int NB, bool CPLX>
 __host__ __device__ constexpr int col_ctas() {
-  if (CPLX) return 2;
+  if (CPLX || (NB == 2 && L >= 4)) return 2;
+  if (NB == 2) return 3;
   return std::is_same<T, float>::value ? (L <= 5 ? 4 : 3) : (L <= 3 ? 2 : 1);
 }
 
-template <int L, typename T, int G, bool CPLX, bool FULL>
-__global__ void __launch_bounds__(T_CTA, col_ctas<L, T, CPLX>()) k_column(ColArgs a) {
-  column_body<L, T, G, CPLX, FULL>(a);
+template <int L, typename T, int G, int NB, bool CPLX, bool FULL>
+__global__ void __launch_bounds__(T_CTA, col_ctas<L, T, NB, CPLX>()) k_column(ColArgs a) {
+  column_body<L, T, G, NB, CPLX, FULL>(a);
 }
 
 // Angle rows: per column displacement (dx, dy) first azn values (cos m phi, sin m phi, m = 1..L), then the polar
@@ -580,11 +583,11 @@ cudaError_t smem_limit(const void* kern, size_t smem) {
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
 }
 
-template <int L, typename T, int G, bool CPLX>
-cudaError_t launch_one(ColArgs a, cudaStream_t st, int* occ) {
-  void (*kern)(ColArgs) = k_column<L, T, G, CPLX, false>;
+template <int L, typename T, int G, int NB, bool CPLX>
+cudaError_t launch_nb(ColArgs a, cudaStream_t st, int* occ) {
+  void (*kern)(ColArgs) = k_column<L, T, G, NB, CPLX, false>;
   if constexpr (L >= RTE_FULL_L && std::is_same<T, float>::value)
-    if (a.nz <= RTE_FULL_NZ) kern = k_column<L, T, G, CPLX, true>;
+    if (a.nz <= RTE_FULL_NZ) kern = k_column<L, T, G, NB, CPLX, true>;
   const int np = a.nx * a.ny * a.nzp;
   // positions a CTA's columns span: its threads' destinations, or (G = 1) the layout blocks of its warps
   const int span = G == 1 ? ((T_CTA / 32 + a.group - 2) / a.group + 1) * 32 * a.group : T_CTA * G;
@@ -593,7 +596,7 @@ cudaError_t launch_one(ColArgs a, cudaStream_t st, int* occ) {
   size_t smem = 0;
   for (int nrun = 1;; ++nrun) {
     a.tz = (a.nz + nrun - 1) / nrun;
-    smem = ColLayout(a.tz, a.pitch, a.azn, a.row - a.azn, a.ncd, (CPLX ? 2 : 1) * nb_row<L>(), CPLX ? 2 : 1,
+    smem = ColLayout(a.tz, a.pitch, a.azn, a.row - a.azn, a.ncd, NB * nb_row<L>(), NB,
                      ring_stages<G>() * ring_rows<G>() * 32 * G, ring_stages<G>(), (int)sizeof(T)).bytes;
     if (smem <= 113 * 1024 || a.tz <= 8) break;
   }
@@ -602,9 +605,21 @@ cudaError_t launch_one(ColArgs a, cudaStream_t st, int* occ) {
   if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, T_CTA, smem);
   const int nblk = (np + 32 * a.group - 1) / (32 * a.group);  // layout blocks: a warp each, or `group` warps for G = 1
   const int warps = G == 1 ? nblk * a.group : nblk;
-  dim3 grid((unsigned)((warps + T_CTA / 32 - 1) / (T_CTA / 32)) * a.nrhs, a.nsplit);
+  dim3 grid((unsigned)((warps + T_CTA / 32 - 1) / (T_CTA / 32)) * (CPLX ? 1 : a.nrhs / NB), a.nsplit);
   kern<<<grid, T_CTA, smem, st>>>(a);
   return cudaGetLastError();
+}
+
+// Right-hand sides of a thread: RTE_COL_NB where the launch has an even number of real ones in FP32.
+template <int L, typename T, int G, bool CPLX>
+cudaError_t launch_one(const ColArgs& a, cudaStream_t st, int* occ) {
+  if constexpr (CPLX) {
+    return launch_nb<L, T, G, 2, true>(a, st, occ);
+  } else {
+    if constexpr (std::is_same<T, float>::value && RTE_COL_NB(L) == 2)
+      if (a.nrhs % 2 == 0) return launch_nb<L, T, G, 2, false>(a, st, occ);
+    return launch_nb<L, T, G, 1, false>(a, st, occ);
+  }
 }
 
 // Destinations per thread: RTE_COL_G; a complex pair's kernel may take one on the same layout (RTE_COL_GC).  A launch of a lower

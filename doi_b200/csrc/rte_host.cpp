@@ -1134,12 +1134,13 @@ static int plan_columns(rte_ctx* c, int LA, int nb, const void* K, size_t ld, in
   CUDA_TRY(c, rte_launch_column(col_args(c, nb, K, ld, 0, cols, cols, 0), LA, f, cplx, c->st, &occ));
   const ColDims d = col_dims(c);
   const int rhs = cplx ? nb / 2 : nb, group = d.tg;
-  const long long tiles = (long long)((ncol * d.nzp + 128 * group - 1) / (128 * group)) * rhs;
+  const int per = !f && !cplx && rhs % 2 == 0 ? RTE_COL_NB(LA) : 1;  // right-hand sides of a CTA
+  const long long tiles = (long long)((ncol * d.nzp + 128 * group - 1) / (128 * group)) * (rhs / per);
   const long long slots = (long long)std::max(occ, 1) * sms;
   const int cap = f ? cols : std::min(cols, kChunkColumns);
   // a wave of resident CTAs takes (chunk + one column of start-up) x the SM's time per column at ~0.6 of the FMA
   // rate; chunk sums are written and read once more each (us)
-  const double col_us = (f ? 2.0 : 1.0) * (cplx ? 2 : 1) * occ * (double)group * c->nz * (4 * LA + 15.0) / (1.9e3 * 0.6);
+  const double col_us = (f ? 2.0 : 1.0) * (cplx ? 2 : per) * occ * (double)group * c->nz * (4 * LA + 15.0) / (1.9e3 * 0.6);
   const double part_us = (double)c->N * c->C * nb * (f ? 8 : 4) * 2 / 5e6;
   std::vector<std::pair<double, int>> rank;
   for (int chunk = 1, last = 0; chunk <= cap; chunk++) {

@@ -67,3 +67,21 @@ def test_slabs_of_partial_rows_equal_the_stored_kernel(rte, nx, nz, prec, tol):
             ctx.set_medium_voxel(mua, mus)
             out.append(ctx.prop_abs(W, 1, 0))
     assert rel(out[1], out[0]) < tol
+
+
+@pytest.mark.parametrize("nx,ny,nz,L", [(5, 4, 7, 1), (3, 2, 1, 2), (2, 1, 33, 3), (4, 3, 5, 4), (7, 6, 5, 5), (1, 2, 49, 5),
+                                        (5, 3, 4, 6), (4, 4, 9, 7)])
+@pytest.mark.parametrize("nsrc", [2, 3, 4])
+def test_batched_right_hand_sides_equal_single_ones(rte, nx, ny, nz, L, nsrc):
+    """Two right-hand sides of a thread against one; the difference is the order of FP32 sums."""
+    rng = np.random.default_rng(nx * 100 + nz + L)
+    N = nx * ny * nz
+    mua, mus = rng.uniform(0.005, 0.1, N), rng.uniform(0.5, 2.0, N)
+    srcs = [rte.Source(pos_x=0.1 * nx * x, kind=rte.SRC_COLUMN, mag=m) for x, m in ((0, 1), (-0.2, 2), (0.2, 0.5), (0.4, 3))][:nsrc]
+    stop = rte.Stop(rte.STOP_FIXED, 4)
+    with rte.Context(nx, ny, nz, dx=0.1, nL=L, g=0.8, precision=rte.PREC_MIXED, kernel_mode=rte.KERNEL_STORE) as ctx:
+        ctx.set_medium_voxel(mua, mus)
+        got = ctx.forward_batch(srcs, stop, want_W=True)["W"]
+        for q, s in enumerate(srcs):
+            want = ctx.forward(s, stop, want_W=True)["W"]
+            assert rel(got[q], want) < 2e-6
