@@ -133,6 +133,7 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
   }
   if (blockIdx.x == 0 && blockIdx.y == 0 && tid < 4 && a.red) a.red[tid] = 0.0;
   constexpr int TMC = tmem_cols<L, T, G, NB>(), W32 = sizeof(T) / 4;
+  __syncwarp();
   if (wid == 0) tmem_alloc(stm, TMC);
   tmem_fence_before();
   for (int q = tid; q < ncd; q += T_CTA) sxy[q] = ((c0 + q) / a.nx) << 16 | (c0 + q) % a.nx;
@@ -223,6 +224,7 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
     uint32_t zero[C * W32];
 #pragma unroll
     for (int c = 0; c < C * W32; ++c) zero[c] = 0u;
+    __syncwarp();
 #pragma unroll
     for (int i = 0; i < NB * G; ++i) tmem_st<C * W32>(tm + i * C * W32, zero);
     tmem_wait_st();
@@ -249,7 +251,10 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
         mbar_wait(&kbar[u_st], u_ph);
         if (++u_st == NST) u_st = 0, u_ph ^= 1;
       }
+      tmem_fence_before();
       __syncthreads();
+      tmem_fence_after();
+      __syncwarp();
       if (wid == 0) tmem_free(*stm, TMC);
       return;
     }
@@ -439,6 +444,7 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
       __syncwarp();
       next_group();
     }
+    __syncwarp();  // one lane's copies, a wait's end
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
@@ -457,7 +463,7 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
         const uint32_t at = tm + (b * G + i) * C * W32;
         T out[C];
         tmem_ld<C * W32>(at, reinterpret_cast<uint32_t*>(out));
-        tmem_wait_ld();
+        tmem_wait_ld<C * W32>(reinterpret_cast<uint32_t*>(out));
         expand_row<L, T>(g, At + j * a.azn, out);
         tmem_st<C * W32>(at, reinterpret_cast<const uint32_t*>(out));
       }
@@ -472,8 +478,9 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
       T out[C];
+      __syncwarp();  // the branch of the previous destination (ragged columns, the last tile)
       tmem_ld<C * W32>(tm + (b * G + i) * C * W32, reinterpret_cast<uint32_t*>(out));
-      tmem_wait_ld();
+      tmem_wait_ld<C * W32>(reinterpret_cast<uint32_t*>(out));
       if (!act || z + i >= nz) continue;
       const size_t r = (size_t)(z + i) * ncol + cd;
       T* o = static_cast<T*>(a.part) + ((size_t)(a.split0 + blockIdx.y) * a.N + r) * a.vstride + (rhs + b) * a.Cfull;
@@ -491,6 +498,7 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
   tmem_fence_before();
   __syncthreads();
   tmem_fence_after();
+  __syncwarp();
   if (wid == 0) tmem_free(*stm, TMC);
 }
 

@@ -134,6 +134,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 
 // Tensor memory as a per-thread accumulator store: 128 lanes x 512 columns of 32 bits per SM; warp w of a CTA owns
 // lanes 32 (w % 4) .. + 31, so each thread of a 128-thread CTA has the CTA's allocated columns of its own lane.
+// All of these are .sync.aligned: a warp executes them converged, with a __syncwarp() behind whatever may have split it.
 template <int N>
 __device__ __forceinline__ void tmem_ld_x(uint32_t addr, uint32_t* v);
 template <int N>
@@ -199,7 +200,14 @@ __device__ __forceinline__ void tmem_st(uint32_t addr, const uint32_t* v) {
   tmem_st_x<P>(addr, v);
   if constexpr (N > P) tmem_st<N - P>(addr + P, v + P);
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// The loaded registers pass through an empty statement behind the wait, so that no arithmetic on them, which depends on
+// registers alone, is scheduled ahead of it.
+template <int N>
+__device__ __forceinline__ void tmem_wait_ld(uint32_t* v) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int q = 0; q < N; ++q) asm volatile("" : "+r"(v[q]));
+}
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // one warp allocates (address to shared memory) and frees
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem, uint32_t cols) {
