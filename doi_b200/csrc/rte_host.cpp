@@ -2909,6 +2909,10 @@ static int run_series_graph(rte_ctx* c, int nb, int nterms, double** d_res) {
     int rc = ensure_fft(c);  // the table spectra of the current medium, outside the graph
     if (rc) return rc;
   }
+  if (!c->fft_in_graph[gi]) {  // angle rows of this modulation: another one's may have taken their buffer
+    int rc = ensure_col_table(c);
+    if (rc) return rc;
+  }
   (void)NC;
   c->launches += 4 * nterms + 4;
   CUDA_TRY(c, cudaGraphLaunch(c->graph[gi], c->st));
