@@ -26,23 +26,10 @@
 #include <type_traits>
 
 #include "rte_internal.h"
+#include "rte_store_plan.h"
 #include "rte_walk.cuh"
 
 namespace {
-
-// Threads of a CTA: 256 with mu_t in shared memory and room for three CTAs per SM, which go through their barriers
-// independently, else 512 (17^3 FP32 270 us with one CTA of 512 and chunks of 12 pairs in fixed turns; 200 with 256
-// threads and units by a counter; 180 with chunks of up to 30; 152 with room for the entries the grid can have,
-// FP64 442 -> 273).
-// path sums per lane, of E column pairs: one list entry serves them all (33^3 FP32, mu_t in shared memory: 4 per lane
-// 10.1 ms, 6 9.2; 41^3 through L1: 4 50 ms, 6 55)
-template <typename T, bool STAGE>
-__host__ __device__ constexpr int st_e() {
-  return sizeof(T) == 4 && STAGE ? 6 : 4;
-}
-constexpr size_t ST_SMALL = 72 * 1024;     // shared memory of a CTA, three per SM
-constexpr int ST_PAIRS = 30;               // most column pairs of a chunk (a warp lays them out)
-constexpr int ST_CAP = 3072;               // list entries per batch (one list has at most 3 * 1023 + 1)
 
 // A voxel of a path: its column offset and z steps from the destination (the sign of z is the pair's), and the
 // length in it.  The packed form holds column offsets of grids below 2^21 voxels.
@@ -73,27 +60,16 @@ struct __align__(16) Entry<double, false> {
   __device__ int oz() const { return z; }
 };
 
-// entries [cap] | tile [npair][zb][zb | 1] | per list: f1, f2 | per pair and z: kernel offset of the destination and of the
-// source column's position | per list: start | per pair: destination, source column | mu_t
-template <typename T, bool PACK>
-struct StLayout {
-  size_t off_tile, off_f, off_o, off_s, off_c, off_mu, bytes;
-  __host__ __device__ StLayout(int npair, int zb, int nz, int cap, int n_mu) {
-    off_tile = sizeof(Entry<T, PACK>) * cap;
-    off_f = (off_tile + sizeof(T) * npair * zb * (zb | 1) + 15) / 16 * 16;
-    off_o = off_f + sizeof(T) * 2 * nz;
-    off_s = off_o + sizeof(size_t) * 2 * npair * zb;
-    off_c = off_s + sizeof(int) * nz;
-    off_mu = (off_c + sizeof(int) * (2 * npair + 2) + 15) / 16 * 16;
-    bytes = off_mu + sizeof(T) * n_mu;
-  }
-};
+static_assert(sizeof(Entry<float, true>) == st_entry_bytes(false, true) &&
+                  sizeof(Entry<float, false>) == st_entry_bytes(false, false) &&
+                  sizeof(Entry<double, false>) == st_entry_bytes(true, false),
+              "list entries as the plan counts them");
 
 template <typename T, bool STAGE, bool PACK, int G, int ST_THREADS, bool DERIV>
 __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1 : 2)) k_store_lists(StoreArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nx = a.nx, ny = a.ny, nz = a.nz, tid = threadIdx.x, wid = tid / 32, lane = tid % 32;
-  const StLayout<T, PACK> Sh(a.npair, a.zb, nz, a.cap, STAGE ? a.N : 0);
+  const StLayout Sh(sizeof(T), sizeof(Entry<T, PACK>), a.npair, a.zb, nz, a.cap, STAGE ? a.N : 0);
   Entry<T, PACK>* ent = reinterpret_cast<Entry<T, PACK>*>(smem_raw);
   T* tile = reinterpret_cast<T*>(smem_raw + Sh.off_tile);
   T* lf = reinterpret_cast<T*>(smem_raw + Sh.off_f);       // per |dz|: log2(e) dist / Q (exp2 argument), dV / (cm dist^2)
@@ -102,7 +78,7 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
   int* cols = reinterpret_cast<int*>(smem_raw + Sh.off_c);  // [npair] destination, [npair] source columns, count
   int& s_unit = cols[2 * a.npair + 1];
   T* smu = reinterpret_cast<T*>(smem_raw + Sh.off_mu);
-  constexpr int E = st_e<T, STAGE>();
+  constexpr int E = st_pairs_per_lane(sizeof(T) == 8, STAGE);
   const T* gmu = static_cast<const T*>(a.mu);
   if constexpr (STAGE)
     for (int q = tid; q < a.N; q += ST_THREADS) smu[q] = gmu[q];
@@ -311,29 +287,16 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
   }
 }
 
-// list entries of a batch: those of all lists of the longest displacement, when they are fewer
-int st_cap(const StoreArgs& a) {
-  const long long all = (long long)a.nz * (a.nx + a.ny - 1) + (long long)a.nz * (a.nz - 1) / 2;
-  return (int)std::min<long long>(ST_CAP, (all + 3) / 4 * 4);
-}
-
 template <typename T, bool STAGE, bool PACK, int G, int ST_THREADS, bool DERIV>
-cudaError_t launch_d(StoreArgs a, int cap, int sms, cudaStream_t st) {
+cudaError_t launch_d(StoreArgs a, const StPlan& p, int cap, int sms, cudaStream_t st) {
   void (*kern)(StoreArgs) = k_store_lists<T, STAGE, PACK, G, ST_THREADS, DERIV>;
-  typedef StLayout<T, PACK> Layout;
-  const int nblk = (a.nz + 47) / 48;
-  a.zb = (a.nz + nblk - 1) / nblk;
-  a.cap = st_cap(a);
-  const size_t budget = ST_THREADS == 256 ? ST_SMALL
-                        : STAGE && Layout(8, a.zb, a.nz, a.cap, a.N).bytes > 110 * 1024 ? (size_t)cap : (size_t)110 * 1024;
-  constexpr int E = st_e<T, STAGE>();
-  a.npair = E;
-  while (a.npair + E <= ST_PAIRS && Layout(a.npair + E, a.zb, a.nz, a.cap, STAGE ? a.N : 0).bytes <= budget) a.npair += E;
-  const size_t smem = Layout(a.npair, a.zb, a.nz, a.cap, STAGE ? a.N : 0).bytes;
+  a.zb = p.zb;
+  a.cap = p.cap;
+  a.npair = p.npair;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
   if (e != cudaSuccess) return e;
   int occ = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, ST_THREADS, smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, ST_THREADS, p.bytes);
   if (e != cudaSuccess) return e;
   if (occ < 1) return cudaErrorInvalidConfiguration;
   // chunks of column pairs that share one set of lists: as many as leave a few groups for every CTA
@@ -343,35 +306,30 @@ cudaError_t launch_d(StoreArgs a, int cap, int sms, cudaStream_t st) {
   a.group_ch = (int)std::max<long long>(1, std::min<long long>(8, maxch * noff / (16ll * occ * sms)));
   e = cudaMemsetAsync(a.counter, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
-  kern<<<occ * sms, ST_THREADS, smem, st>>>(a);
+  kern<<<occ * sms, ST_THREADS, p.bytes, st>>>(a);
   return cudaGetLastError();
 }
 
 template <typename T, bool STAGE, bool PACK, int G, int ST_THREADS>
-cudaError_t launch_t(const StoreArgs& a, int cap, int sms, cudaStream_t st) {
-  return a.Kin ? launch_d<T, STAGE, PACK, G, ST_THREADS, true>(a, cap, sms, st)
-               : launch_d<T, STAGE, PACK, G, ST_THREADS, false>(a, cap, sms, st);
+cudaError_t launch_t(const StoreArgs& a, const StPlan& p, int cap, int sms, cudaStream_t st) {
+  return a.Kin ? launch_d<T, STAGE, PACK, G, ST_THREADS, true>(a, p, cap, sms, st)
+               : launch_d<T, STAGE, PACK, G, ST_THREADS, false>(a, p, cap, sms, st);
 }
 
 template <typename T, bool STAGE, bool PACK, int G>
-cudaError_t launch(const StoreArgs& a, int cap, int sms, cudaStream_t st) {
-  if constexpr (STAGE) {
-    const int nblk = (a.nz + 47) / 48, zb = (a.nz + nblk - 1) / nblk;
-    if (StLayout<T, PACK>(2 * st_e<T, STAGE>(), zb, a.nz, st_cap(a), a.N).bytes <= ST_SMALL)
-      return launch_t<T, STAGE, PACK, G, 256>(a, cap, sms, st);
-  }
-  return launch_t<T, STAGE, PACK, G, 512>(a, cap, sms, st);
+cudaError_t launch(const StoreArgs& a, const StPlan& p, int cap, int sms, cudaStream_t st) {
+  if constexpr (STAGE)
+    if (p.threads == 256) return launch_t<T, STAGE, PACK, G, 256>(a, p, cap, sms, st);
+  return launch_t<T, STAGE, PACK, G, 512>(a, p, cap, sms, st);
 }
 
 template <int G>
 cudaError_t launch_G(const StoreArgs& a, int fp64, int cap, int sms, cudaStream_t st) {
-  // mu_t in shared memory when 48 KB and more remain for tiles beside the lists
-  const size_t es = fp64 ? sizeof(double) : sizeof(float);
-  const size_t lists = st_cap(a) * (fp64 ? sizeof(Entry<double, false>) : sizeof(Entry<float, true>));
-  const bool stage = es * a.N + lists + 48 * 1024 <= (size_t)cap;
-  if (fp64) return stage ? launch<double, true, false, G>(a, cap, sms, st) : launch<double, false, false, G>(a, cap, sms, st);
-  if (stage) return launch<float, true, true, G>(a, cap, sms, st);
-  return a.N < (1 << 21) ? launch<float, false, true, G>(a, cap, sms, st) : launch<float, false, false, G>(a, cap, sms, st);
+  const StPlan p = st_plan(a.nx, a.ny, a.nz, fp64 != 0, cap);
+  if (fp64)
+    return p.stage ? launch<double, true, false, G>(a, p, cap, sms, st) : launch<double, false, false, G>(a, p, cap, sms, st);
+  if (p.stage) return launch<float, true, true, G>(a, p, cap, sms, st);
+  return p.pack ? launch<float, false, true, G>(a, p, cap, sms, st) : launch<float, false, false, G>(a, p, cap, sms, st);
 }
 
 }  // namespace
