@@ -380,6 +380,7 @@ struct rte_ctx {
   bool fft_capture_ready = false;  // a graph recording may capture the transforms
   bool fft_graph_failed = false;   // recording the transforms failed once: graphs use the pair kernels
   bool fft_in_graph[5] = {false, false, false, false, false};
+  bool store_in_graph[5] = {false, false, false, false, false};  // the graph fills the stored pair kernel
   double* d_dmut = nullptr;     // Fisher: parameter direction of mu_t and mu_s [N], tangent dA S [N][C]
   double* d_dmutc = nullptr;    // ... of mu_t in column order, in the operator's precision
   double* d_dmus = nullptr;
@@ -944,10 +945,12 @@ static int ensure_pair_kernel(rte_ctx* c, bool* stored) {
       if (c->kernel_mode == RTE_KERNEL_STORE)
         return fail(c, RTE_ERR_NOMEM, "pair kernel needs %.1f GB, %.1f GB free", need / 1e9, fr / 1e9);
       keep = false;  // auto: recompute
-    } else if (f64) {
-      CUDA_TRY(c, dalloc(c, &c->d_K64, cells));
     } else {
-      CUDA_TRY(c, dalloc(c, &c->d_K, cells));
+      if (f64)
+        CUDA_TRY(c, dalloc(c, &c->d_K64, cells));
+      else
+        CUDA_TRY(c, dalloc(c, &c->d_K, cells));
+      c->K_valid = false;
     }
   }
   if (!keep) return ensure_slab(c);
@@ -2871,6 +2874,7 @@ static int run_series_graph(rte_ctx* c, int nb, int nterms, double** d_res) {
     c->capturing = true;
     cudaGraph_t g = nullptr;
     CUDA_TRY(c, cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
+    c->store_in_graph[gi] = stored;
     if (stored) {  // the precompute for whatever medium is set when the graph is replayed
       c->capture_store = true;
       rc = ensure_pair_kernel(c, &stored);
@@ -2916,7 +2920,7 @@ static int run_series_graph(rte_ctx* c, int nb, int nterms, double** d_res) {
   (void)NC;
   c->launches += 4 * nterms + 4;
   CUDA_TRY(c, cudaGraphLaunch(c->graph[gi], c->st));
-  if (!c->fft_in_graph[gi]) c->K_valid = true;  // the graph recomputed the stored kernel
+  if (c->store_in_graph[gi]) c->K_valid = true;
   *d_res = res;
   return RTE_OK;
 }
