@@ -330,6 +330,7 @@ struct rte_ctx {
   void* d_slab = nullptr;       // recompute workspace: pair-kernel rows of slab_cols source columns
   size_t slab_bytes = 0;
   int slab_cols = 0;
+  bool slab_short = false;      // the device had no room for all that a workspace may take
   int* d_self_idx = nullptr;    // voxel -> distinct mu_t
   double* d_self_lut = nullptr; // [ndistinct][C][C]
   bool self_lut_ok = false;
@@ -896,34 +897,43 @@ static StoreArgs store_args(const rte_ctx* c, void* K, size_t ld, int col0, int 
   return a;
 }
 
-// The workspace for a slab of source columns of the pair kernel (c->slab_cols of them): as many as 1 GB holds, fewer
-// when the device has less left.
+// The workspace for a slab of source columns of the pair kernel (c->slab_cols of them): as many as 1 GB holds, and no
+// more than half of the memory that is free (angle rows and chunk sums need the rest).  A workspace that was cut short
+// stays as it is, so that solves do not allocate in every term and recorded graphs keep their buffer.
 static int ensure_slab(rte_ctx* c) {
   const int ncol = c->nx * c->ny;
   const size_t per_col = kernel_cells(c, c->nz) * (c->precision == RTE_PREC_FP64 ? sizeof(double) : sizeof(float));
-  int cols = (int)std::max<size_t>(1, std::min<size_t>(ncol, kSlabBytes / per_col));
-  for (;; cols = (cols + 1) / 2) {
-    if (cols > c->nx && cols < ncol) cols = cols / c->nx * c->nx;  // whole rows of columns
-    const size_t bytes = per_col * cols;
-    if (bytes <= c->slab_bytes) break;
-    if (c->capturing) return fail(c, RTE_ERR_STATE, "the kernel workspace must exist before a graph is recorded");
-    if (c->d_slab) {
-      cudaFree(c->d_slab);
-      c->bytes -= c->slab_bytes;
-      c->d_slab = nullptr;
-      c->slab_bytes = 0;
-    }
-    unsigned char* m = nullptr;
-    const cudaError_t e = dalloc(c, &m, bytes);
-    if (e == cudaErrorMemoryAllocation && cols > 1) {
-      (void)cudaGetLastError();
-      continue;
-    }
-    CUDA_TRY(c, e);
-    c->d_slab = m;
-    c->slab_bytes = bytes;
-    break;
+  auto whole_rows = [&](size_t cols) {
+    const int n = (int)std::max<size_t>(1, std::min<size_t>(cols, ncol));
+    return n > c->nx && n < ncol ? n / c->nx * c->nx : n;
+  };
+  int cols = whole_rows(kSlabBytes / per_col);
+  const size_t have = c->slab_bytes / per_col;
+  if (have >= (size_t)cols || ((c->slab_short || c->capturing) && have > 0)) {
+    c->slab_cols = std::min(cols, whole_rows(have));
+    return RTE_OK;
   }
+  if (c->capturing) return fail(c, RTE_ERR_STATE, "the kernel workspace must exist before a graph is recorded");
+  if (c->d_slab) {
+    cudaFree(c->d_slab);
+    c->bytes -= c->slab_bytes;
+    c->d_slab = nullptr;
+    c->slab_bytes = 0;
+  }
+  size_t fr = 0, tot = 0;
+  CUDA_TRY(c, cudaMemGetInfo(&fr, &tot));
+  const int want = cols;
+  cols = std::min(cols, whole_rows(fr / 2 / per_col));
+  unsigned char* m = nullptr;
+  for (;; cols = whole_rows(cols / 2)) {
+    const cudaError_t e = dalloc(c, &m, per_col * cols);
+    if (e == cudaSuccess) break;
+    if (e != cudaErrorMemoryAllocation || cols == 1) CUDA_TRY(c, e);
+    (void)cudaGetLastError();
+  }
+  c->d_slab = m;
+  c->slab_bytes = per_col * cols;
+  c->slab_short = cols < want;
   c->slab_cols = cols;
   return RTE_OK;
 }
@@ -2824,7 +2834,7 @@ static std::vector<uintptr_t> graph_signature(const rte_ctx* c, int nb) {
   return {u(std::min(W, Wn)), u(std::max(W, Wn)), u(nb == 1 ? c->d_sum : c->d_bsum),
           u(nb == 1 ? c->d_aux2 : c->d_bres), u(nb == 1 ? c->d_Wf : c->d_bWf),
           u(c->d_part), u(c->d_self_idx), u(c->d_self_lut), u(c->d_mom), (uintptr_t)c->K,
-          (uintptr_t)c->self_lut_ok, u(c->d_K), u(c->d_K64), u(c->d_slab), u(c->d_mut), u(c->d_mutf), u(c->d_mus),
+          (uintptr_t)c->self_lut_ok, u(c->d_K), u(c->d_K64), u(c->d_slab), (uintptr_t)c->slab_bytes, u(c->d_mut), u(c->d_mutf), u(c->d_mus),
           u(c->d_tab[0][0]), u(c->d_tab[1][0]), u(c->d_red), u(c->d_err), (uintptr_t)c->bcap, (uintptr_t)(fft_eligible(c) && !c->fft_graph_failed),
           rte_fft_signature(c->fft)};
 }

@@ -41,3 +41,29 @@ def test_kernel_stored_after_a_graph_that_kept_none(rte, prec):
         a = ctx.forward_graph([src], T)
         b = ctx.forward(src, stop, want_W=False)
         assert rel(a[0][0], b["trans"]) < 1e-9 and rel(a[1][0], b["ref"]) < 1e-9
+
+
+@pytest.mark.parametrize("n,prec,tol", [(23, 0, 1e-12), (27, 1, 2e-6)])
+def test_workspace_cut_short(rte, n, prec, tol):
+    """The workspace wants 1 GB and gets at most half of 700 MB: it stays where it is from solve to solve (the memory
+    comes free after the first), a graph can be recorded on it, and a Fisher matrix of a mixed context shares it with
+    its FP64 solves.  The sums of more slabs come in another order: tolerances as the slab tests of the operator."""
+    T = 3
+    src, stop, det = rte.Source(kind=rte.SRC_COLUMN), rte.Stop(rte.STOP_FIXED, T), rte.Detector(nbins=2, faces=63)
+    mua, mus, _ = rte.sphere_phantom(n, nspheres=2, seed=2, rmin=0.15, rmax=0.3)
+    out = []
+    for short in (False, True):
+        with rte.Context(n, n, n, dx=0.1, nL=1, g=0.8, precision=prec, kernel_mode=rte.KERNEL_RECOMPUTE) as ctx:
+            with _left(700 << 20) if short else contextlib.nullcontext():
+                ctx.set_medium_voxel(mua, mus)
+                a = ctx.forward(src, stop)
+                size = ctx.device_bytes()
+            assert not short or size < 600 << 20
+            g = [ctx.forward_graph([src], T) for _ in range(2)]
+            assert ctx.device_bytes() == size
+            F, J = ctx.fisher([src], stop, det, mua, 0 * mus, want_J=True)
+            g.append(ctx.forward_graph([src], T))
+            for tr, rf, _ in g:
+                assert rel(tr[0], a["trans"]) < 1e-9 and rel(rf[0], a["ref"]) < 1e-9
+            out.append((a["W"], J))
+    assert rel(out[1][0], out[0][0]) < tol and rel(out[1][1], out[0][1]) < tol
