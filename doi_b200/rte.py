@@ -343,7 +343,7 @@ class Context:
         if any(len(t) != n for t in tabs):
             raise ValueError("the four tables must have the same length")
         self._check(self.lib.rte_set_medium_tissue_split(self.h, _ptr(tiss), n, *[_ptr(t) for t in tabs]),
-                    "rte_set_medium_tissue_split", "rte_prop_abs_adjoint")
+                    "rte_set_medium_tissue_split")
 
     def set_modulation(self, modulation):
         """Intensity modulation: mu_a -> mu_a + i*modulation/(c/n) (the reference's [Source] modulation);
