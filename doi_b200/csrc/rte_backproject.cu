@@ -91,14 +91,15 @@ __global__ void __launch_bounds__(BP_THREADS, sizeof(T) == 4 ? (L <= 5 ? 3 : 2) 
   const T* rows[2] = {static_cast<const T*>(a.S), static_cast<const T*>(a.y)};
   T* Q = static_cast<T*>(a.Q);
   const int kb = 32 * a.group;
-  for (long long w = blockIdx.x; w < (long long)noff * ngrp; w += gridDim.x) {
+  for (long long w = blockIdx.x; w < (long long)noff * ngrp * a.nparts; w += gridDim.x) {
     int dx, dy;
     half_plane((int)(w % noff), nx, dx, dy);
-    const int ch0 = (int)(w / noff) * a.group_ch, np = (nx - abs(dx)) * (ny - dy);
+    const int part = (int)(w / noff % a.nparts), ch0 = (int)(w / noff / a.nparts) * a.group_ch;
+    const int np = (nx - abs(dx)) * (ny - dy);
     if (ch0 * npair >= np) continue;
     const bool same = dx == 0 && dy == 0;
     const double ex = dx * a.dx, ey = dy * a.dy, rho = sqrt(ex * ex + ey * ey);
-    for (int bb = 0; bb < nblk * nblk; ++bb) {
+    for (int bb = part; bb < nblk * nblk; bb += a.nparts) {
       const int d0 = bb / nblk * zb, d1 = min(nz, d0 + zb), s0 = bb % nblk * zb, s1 = min(nz, s0 + zb);
       const int nd = d1 - d0, ns = s1 - s0, e0 = d0 - s1 + 1;  // displacements e0 .. d1 - 1 - s0
       if (same && s0 >= d1) continue;
@@ -258,8 +259,8 @@ __global__ void __launch_bounds__(BP_THREADS, sizeof(T) == 4 ? (L <= 5 ? 3 : 2) 
 // u the lower end's z.  The rows of weights lie in shared memory one after another, each with |dz| + 1 or more zeros
 // behind its nz - |dz| values, so that entries whose pair does not exist read zeros: no test per entry, one list
 // entry read for 2 E weights, and no atomics but one FP64 addition per lane, pair and step (atomics on a shared
-// copy of the gradient per voxel crossed in their place: 86.7 ms at 33^3, now 29.1).  Lists and rows come in batches of |dz| when the
-// columns are too long for one.
+// copy of the gradient per voxel crossed in their place: 86.7 ms at 33^3, now 29.1).  Where the columns are too long for
+// one batch of lists and rows, a batch of |dz| is a unit of work of its own.
 constexpr int BP_E = 3;
 constexpr int BP_CAP = 3072;  // most list entries of a batch (one list has at most 3 * 1023 + 1)
 
@@ -299,17 +300,19 @@ __global__ void __launch_bounds__(BP_THREADS) k_bp_walk(BpArgs a) {
   const T* Q = static_cast<const T*>(a.Q);
   for (int e = tid; e < ntile; e += BP_THREADS) tile[e] = T(0);
   int rot = wid;
-  for (long long w = blockIdx.x; w < (long long)noff * ngrp; w += gridDim.x) {
+  for (long long w = blockIdx.x; w < (long long)noff * ngrp * a.nparts; w += gridDim.x) {
     int dx, dy;
     half_plane((int)(w % noff), nx, dx, dy);
-    const int ch0 = (int)(w / noff) * a.group_ch, np = (nx - abs(dx)) * (ny - dy);
+    const int part = (int)(w / noff % a.nparts), ch0 = (int)(w / noff / a.nparts) * a.group_ch;
+    const int np = (nx - abs(dx)) * (ny - dy);
     if (ch0 * npair >= np) continue;
     const bool same = dx == 0 && dy == 0;
+    const int A1 = a.single ? nz : min(nz, (part + 1) * rows);  // this unit's |dz|: all, or one batch of rows
     const int Dx = abs(dx), Dy = dy, sxy = Dx + Dy, stx = dx > 0 ? -1 : 1, sty = -nx;  // steps towards the source
     for (int ch = ch0; ch < ch0 + a.group_ch && ch * npair < np; ++ch)
-      for (int a0 = 0; a0 < nz;) {
+      for (int a0 = a.single ? 0 : part * rows; a0 < A1;) {
         int a1 = a0, total = 0;  // lists a0 .. a1 - 1 of this batch
-        while (a1 < nz && a1 - a0 < rows && total + sxy + a1 + 1 <= a.cap) total += sxy + a1++ + 1;
+        while (a1 < A1 && total + sxy + a1 + 1 <= a.cap) total += sxy + a1++ + 1;
         __syncthreads();  // the previous batch's rows, lists and columns are done with
         const int npv = chunk_columns(ch, npair, np, nx, dx, dy, cols);
         if (!a.single || ch == ch0)
@@ -335,9 +338,16 @@ __global__ void __launch_bounds__(BP_THREADS) k_bp_walk(BpArgs a) {
           for (int e = tid; e < ntile; e += BP_THREADS) tile[e] = T(0);
         }
         __syncthreads();
-        for (int e = tid; e < nz * nz; e += BP_THREADS) {
-          const int zs = e / nz, zd = e - zs * nz, da = abs(zd - zs);
-          if (da < a0 || da >= a1) continue;
+        // a single batch: the pairs of a column pair in the order they lie in; else only those of the batch
+        const int nel = a.single ? nz * nz : 2 * nz * (a1 - a0);
+        for (int e = tid; e < nel; e += BP_THREADS) {
+          int zs = e / nz, zd = e - zs * nz;
+          if (!a.single) {
+            const int d = a0 + zs / 2, up = zs & 1, u = zd;
+            if (u + d >= nz || (up && d == 0)) continue;
+            zs = up ? u + d : u, zd = up ? u : u + d;
+          }
+          const int da = abs(zd - zs);
           T* to = tile + pitch + ((zd < zs ? rows : 0) + da - a0) * pitch + min(zs, zd);
           const bool on = !same || zs < zd;
           for (int p = 0; p < npv; ++p)
@@ -400,7 +410,10 @@ struct Device {
 
 // one wave of CTAs over the (displacement, group of chunks) units, chunks per group as many as leave several
 // groups for every CTA
-cudaError_t launch_units(void (*kern)(BpArgs), BpArgs a, int npair, size_t smem, const Device& d, cudaStream_t st) {
+// nparts: into how many parts a unit's |dz| or blocks of z can be divided; `split` does it only where the units leave
+// CTAs without work (few columns, tall ones: the weights of 1x1x600 by one CTA)
+cudaError_t launch_units(void (*kern)(BpArgs), BpArgs a, int npair, size_t smem, int nparts, bool split, const Device& d,
+                         cudaStream_t st) {
   cudaError_t e = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, d.cap);
   if (e != cudaSuccess) return e;
   int occ = 0;
@@ -409,7 +422,8 @@ cudaError_t launch_units(void (*kern)(BpArgs), BpArgs a, int npair, size_t smem,
   if (occ < 1) return cudaErrorInvalidConfiguration;
   const long long maxch = ((long long)a.nx * a.ny + npair - 1) / npair, noff = (2ll * a.nx - 1) * (a.ny - 1) + a.nx;
   a.group_ch = (int)std::max<long long>(1, std::min<long long>(8, maxch * noff / (16ll * occ * d.sms)));
-  const long long units = noff * ((maxch + a.group_ch - 1) / a.group_ch);
+  a.nparts = split && maxch * noff >= 4ll * occ * d.sms ? 1 : nparts;
+  const long long units = noff * ((maxch + a.group_ch - 1) / a.group_ch) * a.nparts;
   kern<<<(unsigned)std::min<long long>(units, (long long)occ * d.sms), BP_THREADS, smem, st>>>(a);
   return cudaGetLastError();
 }
@@ -423,7 +437,7 @@ cudaError_t launch_weights(BpArgs a, cudaStream_t st) {
   // column pairs per chunk: up to 256 destinations, two or three CTAs per SM
   a.jq = 1;
   while (a.jq * a.zb < 256 && BwLayout<L, T>(a.jq + 1, a.zb).bytes <= 72 * 1024) ++a.jq;
-  return launch_units(k_bp_weights<L, T>, a, a.jq, BwLayout<L, T>(a.jq, a.zb).bytes, d, st);
+  return launch_units(k_bp_weights<L, T>, a, a.jq, BwLayout<L, T>(a.jq, a.zb).bytes, nblk * nblk, true, d, st);
 }
 
 template <int L>
@@ -455,7 +469,7 @@ cudaError_t launch_walk(BpArgs a, cudaStream_t st) {
   const size_t smem = WalkLayout<T>(BP_E * a.jq, a.rows, a.nz, a.cap, nxy).bytes;
   if (smem > (size_t)d.cap) return cudaErrorInvalidValue;
   a.single = a.rows == a.nz && all <= a.cap;
-  e = launch_units(k_bp_walk<T>, a, BP_E * a.jq, smem, d, st);
+  e = launch_units(k_bp_walk<T>, a, BP_E * a.jq, smem, a.single ? 1 : (a.nz + a.rows - 1) / a.rows, false, d, st);
   if (e != cudaSuccess) return e;
   k_bp_add<<<(a.N + 255) / 256, 256, 0, st>>>(a.gcol, a.islot, a.g, a.N);
   return cudaGetLastError();

@@ -57,8 +57,9 @@ struct StoreArgs {
   size_t Kin_ld;
   int kin_slot;
   int* counter;       // scratch: next unit of work
-  // set by the launcher: column pairs per chunk, z block, chunks that share their lists, list entries of a batch
-  int npair, zb, group_ch, cap;
+  // set by the launcher: column pairs per chunk, z block, chunks that share their lists, list entries of a batch,
+  // blocks of z as units of their own
+  int npair, zb, group_ch, cap, zsplit;
 };
 
 // Column form of the pair operator (rte_column.cu): sources and destinations in column order, one CTA per
@@ -201,8 +202,9 @@ struct BpArgs {
   double* gcol;        // [N] column-order sums of the walk (scratch)
   double* g;           // gradient w.r.t. mu_t, accumulated [N]
   // set by the launchers: column pairs per chunk (weights) or three times as many (walk), chunks that share what
-  // depends on the displacement, z block, list entries and |dz| rows of a batch, one batch for every displacement
-  int jq, group_ch, zb, cap, rows, single;
+  // depends on the displacement, z block, list entries and |dz| rows of a batch, one batch for every displacement,
+  // parts of a unit's z blocks or |dz| that are units of their own
+  int jq, group_ch, zb, cap, rows, single, nparts;
 };
 
 struct GradLocalArgs {

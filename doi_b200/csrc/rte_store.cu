@@ -88,9 +88,10 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
   const int maxch = (nx * (y1 - y0 + 1) + a.npair - 1) / a.npair, ngrp = (maxch + a.group_ch - 1) / a.group_ch;
   const int zb = a.zb, nblk = (nz + zb - 1) / zb, pitch = zb | 1;
   const T dxf = (T)a.dx, dyf = (T)a.dy, dzf = (T)a.dz, thr = (T)a.prop_thresh;
-  // Units (displacement, group of chunks) differ in size: a counter hands them out, group 0 of every displacement
-  // first.  Thread 0 draws the next one while the CTA works on this one, past those that do not exist.
-  const int nunit = noff * ngrp;
+  // Units (displacement, group of chunks, on few columns also block of z) differ in size: a counter hands them out,
+  // group 0 of every displacement first.  Thread 0 draws the next one while the CTA works on this one, past those that
+  // do not exist.
+  const int nparts = a.zsplit ? nblk * nblk : 1, nunit = noff * ngrp * nparts;
   auto unit = [&](int u, int& dx, int& dy, int& xa, int& wx, int& ya) {  // destination minus source column; its pairs
     const int off = u % noff;
     if (whole) {  // dy = 0, dx >= 0, then dy > 0
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
   };
   auto exists = [&](int u) {
     int q[5];
-    return u / noff * a.group_ch * a.npair < unit(u, q[0], q[1], q[2], q[3], q[4]);
+    return u / noff / nparts * a.group_ch * a.npair < unit(u, q[0], q[1], q[2], q[3], q[4]);
   };
   for (int u = blockIdx.x; u < nunit;) {
     __syncthreads();  // the previous unit's number is read
@@ -116,16 +117,18 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
       s_unit = n;
     }
     int dx, dy, xa, wx, ya;
-    const int np = unit(u, dx, dy, xa, wx, ya), ch0 = u / noff * a.group_ch;
+    const int np = unit(u, dx, dy, xa, wx, ya), part = u / noff % nparts, ch0 = u / noff / nparts * a.group_ch;
     const int Dx = abs(dx), Dy = abs(dy), sxy = Dx + Dy;
     const int mx = max(Dx, 1), my = max(Dy, 1);
     const int stx = dx > 0 ? -nz : nz, sty = dy > 0 ? -nx * nz : nx * nz;  // steps towards the source
     // one batch holds all lists of the displacement (ordinary grids): made once for the group's chunks
     const bool once = nblk == 1 && nz * (sxy + 1) + nz * (nz - 1) / 2 <= a.cap;
     for (int ch = ch0; ch < ch0 + a.group_ch && ch * a.npair < np; ++ch)
-    for (int bb = 0; bb < nblk * nblk; ++bb) {
+    for (int bb = part; bb < (a.zsplit ? part + 1 : nblk * nblk); ++bb) {
       // destination z in [d0, d1), source z in [s0, s1)
       const int d0 = bb / nblk * zb, d1 = min(nz, d0 + zb), s0 = bb % nblk * zb, s1 = min(nz, s0 + zb);
+      const bool same = whole && dx == 0 && dy == 0;  // a column with itself: blocks below the diagonal by symmetry
+      if (same && s0 > d0) continue;
       const int amin = max(0, max(d0 - s1 + 1, s0 - d1 + 1)), amax = max(d1 - 1 - s0, s1 - 1 - d0);
       __syncthreads();  // the previous tile, lists and columns are done with (and mu_t is staged)
       if (wid == 0) {  // the chunk's column pairs, those of the slab's columns
@@ -169,80 +172,91 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
         }
         }
         __syncthreads();
-        const int npv = cols[2 * a.npair], jq = a.npair / E;  // lane element: (one of jq pairs) x E, z, sign of dz
-        for (int ab = a0, rot = wid; ab < a1; ab += 32) {
-          // lane l holds list a1 - 1 - (ab - a0) - l, the longest first: the pairs of z at dz = +|dz| and -|dz| and its tasks of 32 elements
-          const int da_l = a1 - 1 - (ab - a0) - lane;
-          int pl_l = 0, np_l = 0, ml_l = 0, nm_l = 0;
-          if (da_l >= a0) {
-            pl_l = max(d0, s0 + da_l);
-            np_l = max(0, min(d1, s1 + da_l) - pl_l);
-            ml_l = max(d0, s0 - da_l);
-            nm_l = da_l > 0 ? max(0, min(d1, s1 - da_l) - ml_l) : 0;
-          }
-          int incl = (jq * (np_l + nm_l) + 31) / 32;
-          const int own = incl;
-#pragma unroll
-          for (int o = 1; o < 32; o *= 2) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-          }
-          const int ntask = npv > 0 ? __shfl_sync(0xffffffffu, incl, 31) : 0;  // a chunk may miss the slab's columns
-          int task = rot;
-          for (; task < ntask; task += ST_THREADS / 32) {
-            const int l = __ffs(__ballot_sync(0xffffffffu, incl > task)) - 1, da = a1 - 1 - (ab - a0) - l;
-            const int f0 = (task - __shfl_sync(0xffffffffu, incl - own, l)) * 32;
-            const int pl = __shfl_sync(0xffffffffu, pl_l, l), np_ = __shfl_sync(0xffffffffu, np_l, l);
-            const int ml = __shfl_sync(0xffffffffu, ml_l, l), per = np_ + __shfl_sync(0xffffffffu, nm_l, l);
-            const bool live = f0 + lane < jq * per;
-            const int f = live ? f0 + lane : 0;
-            int js = 0, r = f;  // f / per, f % per; js < jq <= 4
-            while (r >= per) r -= per, ++js;
-            const bool plus = r < np_;
-            const int z = plus ? pl + r : ml + r - np_, sg = plus ? -1 : 1;
-            uint32_t base[E];
-            T acc[E];
-#pragma unroll
-            for (int q = 0; q < E; ++q) {
-              base[q] = (uint32_t)(cols[min(q * jq + js, npv - 1)] * nz + z);
-              if constexpr (STAGE) base[q] = (uint32_t)Sh.off_mu + base[q] * (uint32_t)sizeof(T);  // byte offset: one add per load
-              acc[q] = T(0);
+        const int npv = cols[2 * a.npair];
+        // lane element: (one of jq pairs) x EE, z, sign of dz; the last chunk of a displacement and grids of few columns
+        // have fewer pairs than E
+        auto sums = [&](auto ec, int jq) {
+          constexpr int EE = decltype(ec)::value;
+          for (int ab = a0, rot = wid; ab < a1; ab += 32) {
+            // lane l holds list a1 - 1 - (ab - a0) - l, the longest first: the pairs of z at dz = +|dz| and -|dz| and its tasks of 32 elements
+            const int da_l = a1 - 1 - (ab - a0) - lane;
+            int pl_l = 0, np_l = 0, ml_l = 0, nm_l = 0;
+            if (da_l >= a0) {
+              pl_l = max(d0, s0 + da_l);
+              np_l = max(0, min(d1, s1 + da_l) - pl_l);
+              ml_l = max(d0, s0 - da_l);
+              nm_l = da_l > 0 ? max(0, min(d1, s1 - da_l) - ml_l) : 0;
             }
-            const T f1 = lf[2 * da], f2 = lf[2 * da + 1];
-            if (f2 != T(0)) {
-              const Entry<T, PACK>* le = ent + ls[da];
-              const int S = sxy + da;
-#pragma unroll 2
-              for (int e = 0; e <= S; ++e) {
-                const Entry<T, PACK> v = le[e];
-                const uint32_t at = (uint32_t)(v.oc() + sg * v.oz()) * (STAGE ? (uint32_t)sizeof(T) : 1u);
+            int incl = (jq * (np_l + nm_l) + 31) / 32;
+            const int own = incl;
 #pragma unroll
-                for (int q = 0; q < E; ++q) {
-                  T mu;
-                  if constexpr (STAGE)
-                    mu = *reinterpret_cast<const T*>(smem_raw + (base[q] + at));
-                  else
-                    mu = __ldg(gmu + (base[q] + at));
-                  acc[q] = fma(mu, v.len, acc[q]);
+            for (int o = 1; o < 32; o *= 2) {
+              const int v = __shfl_up_sync(0xffffffffu, incl, o);
+              if (lane >= o) incl += v;
+            }
+            const int ntask = npv > 0 ? __shfl_sync(0xffffffffu, incl, 31) : 0;  // a chunk may miss the slab's columns
+            int task = rot;
+            for (; task < ntask; task += ST_THREADS / 32) {
+              const int l = __ffs(__ballot_sync(0xffffffffu, incl > task)) - 1, da = a1 - 1 - (ab - a0) - l;
+              const int f0 = (task - __shfl_sync(0xffffffffu, incl - own, l)) * 32;
+              const int pl = __shfl_sync(0xffffffffu, pl_l, l), np_ = __shfl_sync(0xffffffffu, np_l, l);
+              const int ml = __shfl_sync(0xffffffffu, ml_l, l), per = np_ + __shfl_sync(0xffffffffu, nm_l, l);
+              const bool live = f0 + lane < jq * per;
+              const int f = live ? f0 + lane : 0;
+              int js = 0, r = f;  // f / per, f % per; js < jq <= 7
+              while (r >= per) r -= per, ++js;
+              const bool plus = r < np_;
+              const int z = plus ? pl + r : ml + r - np_, sg = plus ? -1 : 1;
+              uint32_t base[EE];
+              T acc[EE];
+#pragma unroll
+              for (int q = 0; q < EE; ++q) {
+                base[q] = (uint32_t)(cols[min(q * jq + js, npv - 1)] * nz + z);
+                if constexpr (STAGE) base[q] = (uint32_t)Sh.off_mu + base[q] * (uint32_t)sizeof(T);  // byte offset: one add per load
+                acc[q] = T(0);
+              }
+              const T f1 = lf[2 * da], f2 = lf[2 * da + 1];
+              if (f2 != T(0)) {
+                const Entry<T, PACK>* le = ent + ls[da];
+                const int S = sxy + da;
+#pragma unroll (EE < E ? 8 : 2)
+                for (int e = 0; e <= S; ++e) {
+                  const Entry<T, PACK> v = le[e];
+                  const uint32_t at = (uint32_t)(v.oc() + sg * v.oz()) * (STAGE ? (uint32_t)sizeof(T) : 1u);
+#pragma unroll
+                  for (int q = 0; q < EE; ++q) {
+                    T mu;
+                    if constexpr (STAGE)
+                      mu = *reinterpret_cast<const T*>(smem_raw + (base[q] + at));
+                    else
+                      mu = __ldg(gmu + (base[q] + at));
+                    acc[q] = fma(mu, v.len, acc[q]);
+                  }
                 }
               }
-            }
-            if (!live) continue;
-            T* to = tile + (js * zb + (z + sg * da - s0)) * pitch + z - d0;  // [pair][source z][destination z]
+              if (!live) continue;
+              T* to = tile + (js * zb + (z + sg * da - s0)) * pitch + z - d0;  // [pair][source z][destination z]
 #pragma unroll
-            for (int q = 0; q < E; ++q) {
-              T k;
-              if constexpr (DERIV)
-                k = acc[q] * f1;
-              else if constexpr (std::is_same<T, float>::value)
-                k = exp2f(acc[q] * f1) * f2;
-              else
-                k = exp2(acc[q] * f1) * f2;
-              to[q * jq * zb * pitch] = k;
+              for (int q = 0; q < EE; ++q) {
+                T k;
+                if constexpr (DERIV)
+                  k = acc[q] * f1;
+                else if constexpr (std::is_same<T, float>::value)
+                  k = exp2f(acc[q] * f1) * f2;
+                else
+                  k = exp2(acc[q] * f1) * f2;
+                to[q * jq * zb * pitch] = k;
+              }
             }
+            rot = task - ntask;
           }
-          rot = task - ntask;
-        }
+        };
+        if (npv <= 1)
+          sums(std::integral_constant<int, 1>{}, 1);
+        else if (npv <= E / 2)
+          sums(std::integral_constant<int, E / 2>{}, 1);
+        else
+          sums(std::integral_constant<int, E>{}, (npv + E - 1) / E);
         a0 = a1;
       }
       __syncthreads();
@@ -278,7 +292,7 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
         for (unsigned e = tid; e < nd * ns; e += ST_THREADS) {
           const unsigned zd = (e * ms) >> 20, zs = e - zd * ns;
           for (int j = 0; j < npv; ++j)
-            if (cols[j] != cols[a.npair + j])
+            if (!same || s0 != d0)
               put(so[(a.npair + j) * zb + zs], (unsigned)(cols[j] * nz + d0 + (int)zd), tile[(j * zb + zs) * pitch + zd]);
         }
     }
@@ -304,6 +318,9 @@ cudaError_t launch_d(StoreArgs a, const StPlan& p, int cap, int sms, cudaStream_
   const long long noff = a.col0 == 0 && a.col1 == a.nx * a.ny ? (2 * a.nx - 1) * (a.ny - 1) + a.nx
                                                                : (2ll * a.nx - 1) * (2 * a.ny - 1);
   a.group_ch = (int)std::max<long long>(1, std::min<long long>(8, maxch * noff / (16ll * occ * sms)));
+  // few columns, tall ones: the blocks of z are units of their own where the displacements leave CTAs without work
+  // (1x1x1000 FP32 1.58 s in seven applications by one CTA)
+  a.zsplit = p.zb < a.nz && maxch * noff < 4ll * occ * sms;
   e = cudaMemsetAsync(a.counter, 0, sizeof(int), st);
   if (e != cudaSuccess) return e;
   kern<<<occ * sms, ST_THREADS, p.bytes, st>>>(a);
