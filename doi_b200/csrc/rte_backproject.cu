@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(BP_THREADS, sizeof(T) == 4 ? (L <= 5 ? 3 : 2) 
     if (ch0 * npair >= np) continue;
     const bool same = dx == 0 && dy == 0;
     const double ex = dx * a.dx, ey = dy * a.dy, rho = sqrt(ex * ex + ey * ey);
+    const bool far = rho >= a.prop_thresh;  // no coupling, and the stored kernel may not hold these pairs
     for (int bb = part; bb < nblk * nblk; bb += a.nparts) {
       const int d0 = bb / nblk * zb, d1 = min(nz, d0 + zb), s0 = bb % nblk * zb, s1 = min(nz, s0 + zb);
       const int nd = d1 - d0, ns = s1 - s0, e0 = d0 - s1 + 1;  // displacements e0 .. d1 - 1 - s0
@@ -188,7 +189,9 @@ __global__ void __launch_bounds__(BP_THREADS, sizeof(T) == 4 ? (L <= 5 ? 3 : 2) 
             T kk = T(0), old = T(0);
             if (on) {
               if (a.accumulate) old = q[(size_t)zs * a.ld];
-              if (a.Kmat64)
+              if (far)
+                kk = T(0);
+              else if (a.Kmat64)
                 kk = (T)__ldg(a.Kmat64 + k0 + (size_t)(sl0 + zs) * kb);
               else if (a.Kmat)
                 kk = (T)__ldg(a.Kmat + k0 + (size_t)(sl0 + zs) * kb);

@@ -123,7 +123,10 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
   const int p = min(pt, np - G);
   const bool act = pt < np;
   const int cd = p / a.nzp, z = p - cd * a.nzp, j = cd - c0;
-  const int cb = a.col0 + blockIdx.y * a.chunk, ce = min(a.col1, cb + a.chunk);
+  // this CTA's sources; none from rows too far from all of its destinations (33^3 L=1 recomputed, coupling over 2.5
+  // voxels: see rte_store.cu)
+  const int cb = max(a.col0 + (int)blockIdx.y * a.chunk, (c0 / a.nx - a.ry) * a.nx);
+  const int ce = min(min(a.col1, a.col0 + ((int)blockIdx.y + 1) * a.chunk), ((c0 + ncd - 1) / a.nx + a.ry + 1) * a.nx);
   const int nrun = (nz + a.tz - 1) / a.tz, ntile = max(ce - cb, 0) * nrun;
   if (tid == 0) {
     mbar_init(&bar[0], 1);  // a run's source rows and azimuth values
@@ -672,6 +675,11 @@ ColDims rte_col_dims(int C, int L, int nz, int fp64, int cplx) {
   d.cls = (nz + d.nzp + d.tg - 1) / d.tg;
   d.row = (d.azn + d.tg * d.cls * d.csn + unit - 1) / unit * unit;
   return d;
+}
+
+int rte_col_reach(int nx, int nzp, int group, int ry) {
+  const int ncd = (T_CTA * group + nzp - 2) / nzp + 1;  // columns of a CTA at most, and the rows they lie in
+  return ry + (ncd + nx - 2) / nx;
 }
 
 cudaError_t rte_launch_column(const ColArgs& a, int LA, int fp64, int cplx, cudaStream_t st, int* occ) {

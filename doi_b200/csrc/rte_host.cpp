@@ -872,6 +872,12 @@ static size_t kernel_cells(const rte_ctx* c, size_t rows) {
 // Workspace of the forms that recompute the pair kernel: slabs of source columns, at most this much at a time.
 static const size_t kSlabBytes = 1ull << 30;
 
+// Rows of columns within which voxels couple (prop_thresh, a little more for its comparison in FP32).
+static int coupled_rows(const rte_ctx* c) {
+  const double rows = c->prop_thresh * 1.00001 / c->dy;
+  return rows < c->ny ? (int)std::max(rows, 0.0) : c->ny;
+}
+
 // Arguments of the pair-kernel precompute for source columns [col0, col1) into K.
 static StoreArgs store_args(const rte_ctx* c, void* K, size_t ld, int col0, int col1) {
   StoreArgs a;
@@ -893,6 +899,7 @@ static StoreArgs store_args(const rte_ctx* c, void* K, size_t ld, int col0, int 
   a.group = d.group;
   a.col0 = col0;
   a.col1 = col1;
+  a.ry = rte_col_reach(c->nx, d.nzp, d.group, coupled_rows(c));
   a.counter = c->d_err + 1;
   return a;
 }
@@ -1061,6 +1068,7 @@ static ColArgs col_args(const rte_ctx* c, int nb, const void* K, size_t ld, int 
   a.chunk = chunk;
   a.nsplit = (col1 - col0 + chunk - 1) / chunk;
   a.split0 = split0;
+  a.ry = coupled_rows(c);
   a.err = c->d_err;
   a.red = c->d_red;
   return a;

@@ -53,6 +53,7 @@ struct StoreArgs {
   size_t Kld;
   int nzp, group;
   int col0, col1;
+  int ry;             // rows of columns up to which pairs are computed; what lies beyond is not read (rte_col_reach)
   const void* Kin;    // derivative mode: K of the same sources, whose slot 0 of this launch is row kin_slot (may be K)
   size_t Kin_ld;
   int kin_slot;
@@ -79,6 +80,7 @@ struct ColArgs {
   int vstride;
   int split0;         // first chunk-sum slice
   int col0, col1;     // source columns [col0, col1), `chunk` columns per blockIdx.y
+  int ry;             // rows of columns within which voxels couple
   int chunk, nsplit;
   int* err;
   double* red;        // the epilogue's four norms, zeroed here for it
@@ -301,6 +303,8 @@ cudaError_t rte_launch_layer_sums(const double* W, const double* S, int N, int n
 cudaError_t rte_launch_rows(const double* w, void* rows, const int* islot, int N, int nb, int pitch, int Cfull,
                             int fp64, cudaStream_t st);
 ColDims rte_col_dims(int C, int L, int nz, int fp64, int cplx);
+// rows of columns beyond its own that a launch reads the pair kernel of, where voxels couple over ry rows
+int rte_col_reach(int nx, int nzp, int group, int ry);
 cudaError_t rte_launch_col_table(const ColTabArgs& a, void* tab, int fp64, cudaStream_t st);
 // launches, or with occ != null only reports the CTAs per SM
 cudaError_t rte_launch_column(const ColArgs& a, int LA, int fp64, int cplx, cudaStream_t st, int* occ = nullptr);

@@ -11,6 +11,9 @@
 // destinations per source row; over all sources K is symmetric, so half of the displacements are computed and
 // written both ways.  mu_t is read from shared memory (in column order) when it fits, else through L1.
 //
+// Where voxels couple over a short distance only, displacements of more rows than the column kernels read are left out
+// (33^3 L=1 FP64 recomputed, coupling over 2.5 voxels, six terms: all displacements 103 ms; a walk per coupled pair 24).
+//
 // DERIV: the derivative of K along a direction of mu_t instead, K times minus the path integral of the direction
 // (mu: the direction, Kin: K of the same sources, which may be the output).
 //
@@ -83,7 +86,7 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
   if constexpr (STAGE)
     for (int q = tid; q < a.N; q += ST_THREADS) smu[q] = gmu[q];
   const bool whole = a.col0 == 0 && a.col1 == nx * ny;
-  const int noff = whole ? (2 * nx - 1) * (ny - 1) + nx : (2 * nx - 1) * (2 * ny - 1);
+  const int ry = min(a.ry, ny - 1), noff = whole ? (2 * nx - 1) * ry + nx : (2 * nx - 1) * (2 * ry + 1);
   const int y0 = a.col0 / nx, y1 = (a.col1 - 1) / nx;  // source rows
   const int maxch = (nx * (y1 - y0 + 1) + a.npair - 1) / a.npair, ngrp = (maxch + a.group_ch - 1) / a.group_ch;
   const int zb = a.zb, nblk = (nz + zb - 1) / zb, pitch = zb | 1;
@@ -98,7 +101,7 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
       dy = off < nx ? 0 : (off - nx) / (2 * nx - 1) + 1;
       dx = off < nx ? off : (off - nx) % (2 * nx - 1) - (nx - 1);
     } else {
-      dy = off / (2 * nx - 1) - (ny - 1);
+      dy = off / (2 * nx - 1) - ry;
       dx = off % (2 * nx - 1) - (nx - 1);
     }
     xa = max(0, -dx), wx = nx - abs(dx), ya = max(y0, -dy);  // source columns xa.., ya.. of this displacement
@@ -148,7 +151,15 @@ __global__ void __launch_bounds__(ST_THREADS, ST_THREADS == 256 ? 3 : (STAGE ? 1
         }
         if (lane == 0) cols[2 * a.npair] = __popc(m);
       }
-      for (int a0 = amin; a0 <= amax;) {
+      int a0 = amin;
+      {  // columns farther apart than voxels couple: zeros, no lists (|dz| only adds to the distance)
+        const T hx = (T)Dx * dxf, hy = (T)Dy * dyf, h2 = fma(hx, hx, hy * hy);
+        if (h2 > T(0) && !(sqrt(h2) < thr)) {
+          for (int e = tid; e < a.npair * zb * pitch; e += ST_THREADS) tile[e] = T(0);
+          a0 = amax + 1;
+        }
+      }
+      while (a0 <= amax) {
         int a1 = a0, total = 0;  // lists a0 .. a1 - 1 of this batch
         while (a1 <= amax && total + sxy + a1 + 1 <= a.cap) total += sxy + a1++ + 1;
         if (a0 > amin) __syncthreads();
@@ -315,8 +326,8 @@ cudaError_t launch_d(StoreArgs a, const StPlan& p, int cap, int sms, cudaStream_
   if (occ < 1) return cudaErrorInvalidConfiguration;
   // chunks of column pairs that share one set of lists: as many as leave a few groups for every CTA
   const long long rows = (a.col1 - 1) / a.nx - a.col0 / a.nx + 1, maxch = (a.nx * rows + a.npair - 1) / a.npair;
-  const long long noff = a.col0 == 0 && a.col1 == a.nx * a.ny ? (2 * a.nx - 1) * (a.ny - 1) + a.nx
-                                                               : (2ll * a.nx - 1) * (2 * a.ny - 1);
+  const int ry = std::min(a.ry, a.ny - 1);
+  const long long noff = a.col0 == 0 && a.col1 == a.nx * a.ny ? (2 * a.nx - 1) * ry + a.nx : (2ll * a.nx - 1) * (2 * ry + 1);
   a.group_ch = (int)std::max<long long>(1, std::min<long long>(8, maxch * noff / (16ll * occ * sms)));
   // few columns, tall ones: the blocks of z are units of their own where the displacements leave CTAs without work
   // (1x1x1000 FP32 1.58 s in seven applications by one CTA)
