@@ -200,8 +200,8 @@ __global__ void __launch_bounds__(BP_THREADS, sizeof(T) == 4 ? (L <= 5 ? 3 : 2) 
                 const T d2 = fx * fx + fy * fy + fz * fz, dist = sqrt(d2);
                 if (dist < (T)a.prop_thresh) {
                   int Q0;
-                  const T ps = path_sum<T, double>(d0 + zd, cd / nx, cd % nx, s0 + zs, cs / nx, cs % nx, a.mut, nx,
-                                                   nx * ny, Q0);
+                  const T ps = path_sum<T, double>(cd / nx, cd % nx, d0 + zd, cs / nx, cs % nx, s0 + zs, a.mut, nz,
+                                                   nx * nz, Q0);
                   kk = exp(-ps * dist / (T)Q0) * (T)a.kscale / d2;
                 }
               }

@@ -303,6 +303,13 @@ struct rte_ctx {
   rte_config cfg;
   int nx, ny, nz, N, L, C;
   double dx, dy, dz, dV, cm, prop_thresh;
+  // frame of the column kernels: columns along z (ax 0), x (1) or y (2), its grid and spacing; rte_flat.cu
+  int ax = 0, cx, cy, cz;
+  double cdx, cdy, cdz;
+  bool dirs = false;            // pair-by-pair form (the table model's flat grids)
+  double* d_exch = nullptr;     // coefficients of the exchanged frame [C][C]
+  double* d_flat = nullptr;     // sums back in the grid's frame [N][nb][C]
+  size_t flat_cap = 0;
   int model, precision, kernel_mode;
   std::string err;
   cudaStream_t st = nullptr;
@@ -310,7 +317,6 @@ struct rte_ctx {
   ShTables sh;
   SelfQuad quad;
   int K = 0;  // moments in use
-  int* d_perm = nullptr;
   double *d_mut = nullptr, *d_mus = nullptr;
   float* d_mutf = nullptr;
   double* d_mutc = nullptr;     // mu_t in column order
@@ -484,13 +490,13 @@ static void free_all(rte_ctx* c) {
       cudaEventDestroy(p.second);
     }
   for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
-  void* ps[] = {c->d_perm, c->d_mut, c->d_mus, c->d_mutf, c->d_W, c->d_Wn, c->d_sum, c->d_part, c->d_mom,
+  void* ps[] = {c->d_mut, c->d_mus, c->d_mutf, c->d_W, c->d_Wn, c->d_sum, c->d_part, c->d_mom,
                 c->d_aux1, c->d_aux2, c->d_aux3, c->d_aux4, c->d_Wf, c->d_K, c->d_K64, c->d_cplx, c->d_red, c->d_img,
                 c->d_self_idx, c->d_self_lut, c->d_islot, c->d_err,
                 c->d_bW, c->d_bWn, c->d_bsum, c->d_bres, c->d_bball, c->d_bWf, c->d_h, c->d_S, c->d_out,
                 c->d_e, c->d_lam, c->d_y, c->d_gt, c->d_gs, c->d_J, c->d_rho, c->d_dlut, c->d_fball, c->d_q, c->d_bq,
                 c->d_Qbp, c->d_mask, c->d_dmut, c->d_dmutc, c->d_dmus, c->d_mut_self, c->d_mus_src, c->d_T, c->d_cidx, c->d_cval, c->d_self_lut_im,
-                c->d_fball_im, c->d_mutc, c->d_mutfc, c->d_slab, c->d_tab[0][0], c->d_tab[0][1], c->d_tab[1][0], c->d_tab[1][1]};
+                c->d_fball_im, c->d_exch, c->d_flat, c->d_mutc, c->d_mutfc, c->d_slab, c->d_tab[0][0], c->d_tab[0][1], c->d_tab[1][0], c->d_tab[1][1]};
   for (void* p : ps)
     if (p) cudaFree(p);
   if (c->ev0) cudaEventDestroy(c->ev0);
@@ -500,17 +506,63 @@ static void free_all(rte_ctx* c) {
 
 // Column order (x, y columns, z fastest): the order of the column kernels, which take one column of sources
 // against the destinations of a few columns at a time (rte_column.cu).
-static std::vector<int> column_perm(int nx, int ny, int nz) {
-  std::vector<int> p((size_t)nx * ny * nz);
-  size_t q = 0;
-  for (int col = 0; col < nx * ny; col++)
-    for (int i = 0; i < nz; i++) p[q++] = i * nx * ny + col;
-  return p;
+// voxel of the grid -> slot, in the frame whose columns run along axis c->ax
+static int slot_of(const rte_ctx* c, int r) {
+  const int x = r % c->nx, y = r / c->nx % c->ny, z = r / (c->nx * c->ny);
+  if (c->ax == 1) return (y * c->cx + z) * c->cz + x;
+  if (c->ax == 2) return (x * c->cx + z) * c->cz + y;
+  return (y * c->cx + x) * c->cz + z;
+}
+
+// Axis of the columns: z, or (1, 2) the longer of x and y on grids of few layers, where z columns share little
+// (rte_flat.cu).  Forward solves of six terms, mixed, kernel stored / recomputed, columns along z -> along x:
+// 110x110x1 L=3 195 / 940 -> 5.2 / 17 ms, 36x36x9 L=1 5.1 / 12.6 -> 3.2 / 9.0, 20x20x9 L=1 1.32 / 2.06 -> 1.34 / 1.91,
+// 14x14x6 (196 z columns) 0.96 / 1.11 -> 1.21 / 1.35.  From ten layers on z columns are no slower than a walk and
+// spherical harmonics per pair were (35x35x10 L=1 5.0 / 12.4 ms, those 5.2 / 44) and stay.  The table model's
+// pair-by-pair form: 70x70x2 L=3 31 / 80 -> 6.4 / 14, 50x50x4 L=2 9.8 / 22 -> 5.5 / 12 (FP64 15 / 68 -> 6.9 / 16), but
+// 45x45x6 L=5 10 / 20 -> 17 / 23.
+static int column_axis(const rte_ctx* c) {
+  const int layers = c->model != RTE_MODEL_FIM ? 9 : (c->L <= 5 ? 4 : 3);
+  if (c->nz > layers || std::max(c->nx, c->ny) < 2 * c->nz || c->nx * c->ny < 32 * c->nz + 96) return 0;
+  return c->nx >= c->ny ? 1 : 2;
+}
+
+// Coefficients in the frame with the axes exchanged: R_c(P u) = sum M[c][c'] R_c'(u), P u the direction u in that frame,
+// by a quadrature that is exact for the products (Gauss-Legendre in z, equal steps in the azimuth).
+static std::vector<double> exchange_matrix(const rte_ctx* c) {
+  const int C = c->C, n = RTE_MAX_L + 1, np = 2 * RTE_MAX_L + 2;
+  std::vector<double> M((size_t)C * C, 0.0), R(64), Rp(64);
+  for (int q = 0; q < n; q++) {
+    double z = cos(M_PI * (q + 0.75) / (n + 0.5)), dp = 1.0;
+    for (int it = 0; it < 100; it++) {  // root of P_n by Newton's method
+      double p0 = 1.0, p1 = z;
+      for (int k = 2; k <= n; k++) {
+        const double p2 = ((2 * k - 1) * z * p1 - (k - 1) * p0) / k;
+        p0 = p1;
+        p1 = p2;
+      }
+      dp = n * (z * p1 - p0) / (z * z - 1.0);
+      z -= p1 / dp;
+      if (fabs(p1 / dp) < 1e-16) break;
+    }
+    const double w = 2.0 / ((1.0 - z * z) * dp * dp) * 2.0 * M_PI / np, s = sqrt(1.0 - z * z);
+    for (int f = 0; f < np; f++) {
+      const double x = s * cos(2.0 * M_PI * f / np), y = s * sin(2.0 * M_PI * f / np);
+      sh_real_host(c->sh, c->L, x, y, z, R.data());
+      if (c->ax == 1)
+        sh_real_host(c->sh, c->L, z, y, x, Rp.data());
+      else
+        sh_real_host(c->sh, c->L, z, x, y, Rp.data());
+      for (int a = 0; a < C; a++)
+        for (int b = 0; b < C; b++) M[(size_t)a * C + b] += w * Rp[a] * R[b];
+    }
+  }
+  return M;
 }
 
 // Layout of the column kernels' source and angle rows in the context's precision.
 static ColDims col_dims(const rte_ctx* c) {
-  return rte_col_dims(c->C, c->L, c->nz, c->precision == RTE_PREC_FP64 ? 1 : 0, c->kappa != 0.0 ? 1 : 0);
+  return rte_col_dims(c->C, c->L, c->cz, c->precision == RTE_PREC_FP64 ? 1 : 0, c->kappa != 0.0 ? 1 : 0);
 }
 
 extern "C" {
@@ -560,6 +612,14 @@ int rte_create(const rte_config* cfg, rte_ctx** out) {
     return fail(nullptr, RTE_ERR_ARG, "voxel size must be positive");
   }
   c->dV = c->dx * c->dy * c->dz;
+  c->ax = column_axis(c);
+  c->cx = c->ax ? c->nz : c->nx;
+  c->cy = c->ax == 2 ? c->nx : c->ny;
+  c->cz = c->ax == 1 ? c->nx : (c->ax == 2 ? c->ny : c->nz);
+  c->cdx = c->ax ? c->dz : c->dx;
+  c->cdy = c->ax == 2 ? c->dx : c->dy;
+  c->cdz = c->ax == 1 ? c->dx : (c->ax == 2 ? c->dy : c->dz);
+  c->dirs = c->ax && c->model == RTE_MODEL_FIM;
   c->sh = make_sh_tables();
   int rc = RTE_OK;
   auto cu = [&](cudaError_t e, const char* what) {
@@ -582,7 +642,6 @@ int rte_create(const rte_config* cfg, rte_ctx** out) {
   }
   const size_t NC = (size_t)c->N * c->C;
   if (const char* e = getenv("RTE_MAX_SPLIT")) c->max_split = std::max(1, std::min(32, atoi(e)));
-  if (rc == RTE_OK) cu(dalloc(c, &c->d_perm, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_mut, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_mus, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_mutf, c->N), "alloc");
@@ -599,7 +658,7 @@ int rte_create(const rte_config* cfg, rte_ctx** out) {
   c->part_cap = NC * c->max_split;
   if (rc == RTE_OK) cu(dalloc(c, &c->d_self_idx, c->N), "alloc");
   {  // room for FP64 rows in either precision (rte_fisher runs FP64 solves in mixed contexts)
-    const size_t nrow = (size_t)c->N * rte_col_dims(c->C, c->L, c->nz, 1, 0).pitch;
+    const size_t nrow = (size_t)c->N * rte_col_dims(c->C, c->L, c->cz, 1, 0).pitch;
     double* rows = nullptr;
     if (rc == RTE_OK) cu(dalloc(c, &rows, nrow), "alloc");
     c->d_Wf = rows;
@@ -615,11 +674,14 @@ int rte_create(const rte_config* cfg, rte_ctx** out) {
   if (rc == RTE_OK) cu(dalloc(c, &c->d_fball, npix), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_q, NC), "alloc");
   if (rc == RTE_OK) {
-    std::vector<int> p = column_perm(c->nx, c->ny, c->nz);
-    std::vector<int> inv(c->N);
-    for (int q = 0; q < c->N; q++) inv[p[q]] = q;
-    cu(cudaMemcpy(c->d_perm, p.data(), sizeof(int) * c->N, cudaMemcpyHostToDevice), "perm upload");
-    if (rc == RTE_OK) cu(cudaMemcpy(c->d_islot, inv.data(), sizeof(int) * c->N, cudaMemcpyHostToDevice), "upload");
+    std::vector<int> slot(c->N);
+    for (int r = 0; r < c->N; r++) slot[r] = slot_of(c, r);
+    cu(cudaMemcpy(c->d_islot, slot.data(), sizeof(int) * c->N, cudaMemcpyHostToDevice), "upload");
+  }
+  if (rc == RTE_OK && c->ax && !c->dirs) {
+    const std::vector<double> M = exchange_matrix(c);
+    cu(dalloc(c, &c->d_exch, M.size()), "alloc");
+    if (rc == RTE_OK) cu(cudaMemcpy(c->d_exch, M.data(), sizeof(double) * M.size(), cudaMemcpyHostToDevice), "upload");
   }
   if (rc != RTE_OK) {
     free_all(c);
@@ -865,7 +927,7 @@ static void scatter_factors(const rte_ctx* c, int flag, double* s) {
 // Cells of the pair kernel over `rows` source slots (whole blocks of destinations, kmat_index).
 static size_t kernel_cells(const rte_ctx* c, size_t rows) {
   const ColDims d = col_dims(c);
-  const size_t np = (size_t)c->nx * c->ny * d.nzp, kb = 32 * (size_t)d.group;
+  const size_t np = (size_t)c->cx * c->cy * d.nzp, kb = 32 * (size_t)d.group;
   return (np + kb - 1) / kb * kb * rows;
 }
 
@@ -874,8 +936,8 @@ static const size_t kSlabBytes = 1ull << 30;
 
 // Rows of columns within which voxels couple (prop_thresh, a little more for its comparison in FP32).
 static int coupled_rows(const rte_ctx* c) {
-  const double rows = c->prop_thresh * 1.00001 / c->dy;
-  return rows < c->ny ? (int)std::max(rows, 0.0) : c->ny;
+  const double rows = c->prop_thresh * 1.00001 / c->cdy;
+  return rows < c->cy ? (int)std::max(rows, 0.0) : c->cy;
 }
 
 // Arguments of the pair-kernel precompute for source columns [col0, col1) into K.
@@ -884,12 +946,12 @@ static StoreArgs store_args(const rte_ctx* c, void* K, size_t ld, int col0, int 
   memset(&a, 0, sizeof a);
   const ColDims d = col_dims(c);
   a.N = c->N;
-  a.nx = c->nx;
-  a.ny = c->ny;
-  a.nz = c->nz;
-  a.dx = c->dx;
-  a.dy = c->dy;
-  a.dz = c->dz;
+  a.nx = c->cx;
+  a.ny = c->cy;
+  a.nz = c->cz;
+  a.dx = c->cdx;
+  a.dy = c->cdy;
+  a.dz = c->cdz;
   a.prop_thresh = c->prop_thresh;
   a.kscale = c->dV / c->cm;
   a.mu = c->precision == RTE_PREC_FP64 ? (const void*)c->d_mutc : (const void*)c->d_mutfc;
@@ -899,7 +961,7 @@ static StoreArgs store_args(const rte_ctx* c, void* K, size_t ld, int col0, int 
   a.group = d.group;
   a.col0 = col0;
   a.col1 = col1;
-  a.ry = rte_col_reach(c->nx, d.nzp, d.group, coupled_rows(c));
+  a.ry = rte_col_reach(c->cx, d.nzp, d.group, coupled_rows(c));
   a.counter = c->d_err + 1;
   return a;
 }
@@ -908,11 +970,11 @@ static StoreArgs store_args(const rte_ctx* c, void* K, size_t ld, int col0, int 
 // more than half of the memory that is free (angle rows and chunk sums need the rest).  A workspace that was cut short
 // stays as it is, so that solves do not allocate in every term and recorded graphs keep their buffer.
 static int ensure_slab(rte_ctx* c) {
-  const int ncol = c->nx * c->ny;
-  const size_t per_col = kernel_cells(c, c->nz) * (c->precision == RTE_PREC_FP64 ? sizeof(double) : sizeof(float));
+  const int ncol = c->cx * c->cy;
+  const size_t per_col = kernel_cells(c, c->cz) * (c->precision == RTE_PREC_FP64 ? sizeof(double) : sizeof(float));
   auto whole_rows = [&](size_t cols) {
     const int n = (int)std::max<size_t>(1, std::min<size_t>(cols, ncol));
-    return n > c->nx && n < ncol ? n / c->nx * c->nx : n;
+    return n > c->cx && n < ncol ? n / c->cx * c->cx : n;
   };
   int cols = whole_rows(kSlabBytes / per_col);
   const size_t have = c->slab_bytes / per_col;
@@ -972,7 +1034,7 @@ static int ensure_pair_kernel(rte_ctx* c, bool* stored) {
   }
   if (!keep) return ensure_slab(c);
   if (!c->K_valid || c->capture_store) {
-    const StoreArgs a = store_args(c, f64 ? (void*)c->d_K64 : (void*)c->d_K, c->N, 0, c->nx * c->ny);
+    const StoreArgs a = store_args(c, f64 ? (void*)c->d_K64 : (void*)c->d_K, c->N, 0, c->cx * c->cy);
     if (c->capturing) {
       CUDA_TRY(c, rte_launch_store_kernel(a, c->st, f64 ? 1 : 0));
     } else {
@@ -1001,24 +1063,31 @@ static int ensure_col_table(rte_ctx* c) {
   void** p = &c->d_tab[f][tr];
   if (*p && c->tab_kappa[f][tr] == c->kappa) return RTE_OK;
   if (c->capturing) return fail(c, RTE_ERR_STATE, "angle rows must exist before a graph is recorded");
+  if (c->dirs) {
+    unsigned char* m = nullptr;
+    CUDA_TRY(c, dalloc(c, &m, rte_dirs_bytes(c->nx, c->ny, c->nz, c->L, f)));
+    *p = m;
+    CUDA_TRY(c, (c->launches++, rte_launch_dirs_table(c->nx, c->ny, c->nz, c->dx, c->dy, c->dz, tr, c->L, f, *p, c->st)));
+    return RTE_OK;
+  }
   const ColDims d = col_dims(c);
   const size_t esize = f ? sizeof(double) : sizeof(float);
   if (!*p) {  // room for the phases of a modulated context
-    const size_t row = rte_col_dims(c->C, c->L, c->nz, f, 1).row;
+    const size_t row = rte_col_dims(c->C, c->L, c->cz, f, 1).row;
     unsigned char* m = nullptr;
-    CUDA_TRY(c, dalloc(c, &m, (size_t)(2 * c->nx - 1) * (2 * c->ny - 1) * row * esize));
+    CUDA_TRY(c, dalloc(c, &m, (size_t)(2 * c->cx - 1) * (2 * c->cy - 1) * row * esize));
     *p = m;
   }
   ColTabArgs a;
   memset(&a, 0, sizeof a);
-  a.nx = c->nx;
-  a.ny = c->ny;
-  a.nz = c->nz;
+  a.nx = c->cx;
+  a.ny = c->cy;
+  a.nz = c->cz;
   a.nzp = d.nzp;
   a.L = c->L;
-  a.dx = c->dx;
-  a.dy = c->dy;
-  a.dz = c->dz;
+  a.dx = c->cdx;
+  a.dy = c->cdy;
+  a.dz = c->cdz;
   a.kappa = c->kappa;
   a.table = c->model == RTE_MODEL_FIM ? 1 : 0;
   a.transpose = tr;
@@ -1042,9 +1111,9 @@ static ColArgs col_args(const rte_ctx* c, int nb, const void* K, size_t ld, int 
   const int f = c->precision == RTE_PREC_FP64 ? 1 : 0;
   const ColDims d = col_dims(c);
   a.N = c->N;
-  a.nx = c->nx;
-  a.ny = c->ny;
-  a.nz = c->nz;
+  a.nx = c->cx;
+  a.ny = c->cy;
+  a.nz = c->cz;
   a.Cfull = c->C;
   a.nzp = d.nzp;
   a.group = d.group;
@@ -1053,7 +1122,7 @@ static ColArgs col_args(const rte_ctx* c, int nb, const void* K, size_t ld, int 
   a.pitch = d.pitch;
   a.K = K;
   a.Kld = ld;
-  a.kslot0 = col0 * c->nz;
+  a.kslot0 = col0 * c->cz;
   a.tab = c->d_tab[f][c->transpose ? 1 : 0];
   a.row = d.row;
   a.azn = d.azn;
@@ -1069,13 +1138,22 @@ static ColArgs col_args(const rte_ctx* c, int nb, const void* K, size_t ld, int 
   a.nsplit = (col1 - col0 + chunk - 1) / chunk;
   a.split0 = split0;
   a.ry = coupled_rows(c);
+  if (c->dirs) {
+    const int mx = 2 * c->nx - 1, mxy = mx * (2 * c->ny - 1);
+    a.d0 = (c->nz - 1) * mxy + (c->ny - 1) * mx + c->nx - 1;
+    a.dsx = mxy;
+    a.dsy = c->ax == 1 ? mx : 1;
+    a.dsz = c->ax == 1 ? 1 : mx;
+  }
   a.err = c->d_err;
   a.red = c->d_red;
   return a;
 }
 
-static cudaError_t launch_columns(const rte_ctx* c, const ColArgs& a, int LA) {
-  return rte_launch_column(a, LA, c->precision == RTE_PREC_FP64 ? 1 : 0, c->kappa != 0.0 ? 1 : 0, c->st);
+static cudaError_t launch_columns(const rte_ctx* c, const ColArgs& a, int LA, int* occ = nullptr) {
+  const int f = c->precision == RTE_PREC_FP64 ? 1 : 0;
+  if (c->dirs) return rte_launch_pair_dirs(a, LA, f, c->st, occ);
+  return rte_launch_column(a, LA, f, c->kappa != 0.0 ? 1 : 0, c->st, occ);
 }
 
 // Launch-plan autotuner of the column kernels.  The grid is (tiles of 128 threads' destinations x right-hand
@@ -1138,11 +1216,15 @@ static int plan_columns(rte_ctx* c, int LA, int nb, const void* K, size_t ld, in
   const int cplx = c->kappa != 0.0 ? 1 : 0, f = c->precision == RTE_PREC_FP64 ? 1 : 0;
   int rc = ensure_col_table(c);
   if (rc) return rc;
-  const int ncol = c->nx * c->ny;
+  const int ncol = c->cx * c->cy;
   auto total = [&](int chunk) {  // slices over all slabs of `cols` columns
     const int full = ncol / cols, rest = ncol % cols;
     return full * ((cols + chunk - 1) / chunk) + (rest + chunk - 1) / chunk;
   };
+  if (c->ax) {
+    rc = grow(c, &c->d_flat, c->flat_cap, (size_t)c->N * c->C * nb);
+    if (rc) return rc;
+  }
   const int key = (((LA * 8 + nb) * 2 + f) * 2 + cplx) * 2 + (cols == ncol ? 1 : 0);
   for (auto& e : c->splits)
     if (e[0] == key && e[1] == cols) {
@@ -1152,7 +1234,7 @@ static int plan_columns(rte_ctx* c, int LA, int nb, const void* K, size_t ld, in
     }
   int sms = 0, occ = 0;
   CUDA_TRY(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
-  CUDA_TRY(c, rte_launch_column(col_args(c, nb, K, ld, 0, cols, cols, 0), LA, f, cplx, c->st, &occ));
+  CUDA_TRY(c, launch_columns(c, col_args(c, nb, K, ld, 0, cols, cols, 0), LA, &occ));
   const ColDims d = col_dims(c);
   const int rhs = cplx ? nb / 2 : nb, group = d.tg;
   const int per = !f && !cplx && rhs % 2 == 0 ? RTE_COL_NB(LA) : 1;  // right-hand sides of a CTA
@@ -1161,7 +1243,7 @@ static int plan_columns(rte_ctx* c, int LA, int nb, const void* K, size_t ld, in
   const int cap = f ? cols : std::min(cols, kChunkColumns);
   // a wave of resident CTAs takes (chunk + one column of start-up) x the SM's time per column at ~0.6 of the FMA
   // rate; chunk sums are written and read once more each (us)
-  const double col_us = (f ? 2.0 : 1.0) * (cplx ? 2 : per) * occ * (double)group * c->nz * (4 * LA + 15.0) / (1.9e3 * 0.6);
+  const double col_us = (f ? 2.0 : 1.0) * (cplx ? 2 : per) * occ * (double)group * c->cz * (4 * LA + 15.0) / (1.9e3 * 0.6);
   const double part_us = (double)c->N * c->C * nb * (f ? 8 : 4) * 2 / 5e6;
   std::vector<std::pair<double, int>> rank;
   for (int chunk = 1, last = 0; chunk <= cap; chunk++) {
@@ -1178,7 +1260,7 @@ static int plan_columns(rte_ctx* c, int LA, int nb, const void* K, size_t ld, in
   const char* at = getenv("RTE_AUTOTUNE");
   const bool tune = !forced && !(at && at[0] == '0') && !c->capturing && c->N >= 1024 && rank.size() > 1;
   if (forced) chunk = std::max(1, std::min(cap, (cols + std::max(1, atoi(forced)) - 1) / std::max(1, atoi(forced))));
-  const TuneKey tk{c->cfg.device, c->nx, c->ny, c->nz, LA, nb, c->precision, cplx, cols};
+  const TuneKey tk{c->cfg.device, c->cx, c->cy, c->cz, LA, nb, c->precision, cplx, cols};
   bool have = false;
   if (tune) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -1219,7 +1301,7 @@ static int pair_term(rte_ctx* c, int LA, int nb, int* S) {
   bool stored = false;
   int rc = ensure_pair_kernel(c, &stored), chunk = 1;
   if (rc) return rc;
-  const int f = c->precision == RTE_PREC_FP64 ? 1 : 0, ncol = c->nx * c->ny;
+  const int f = c->precision == RTE_PREC_FP64 ? 1 : 0, ncol = c->cx * c->cy;
   if (stored) {
     const void* K = f ? (const void*)c->d_K64 : (const void*)c->d_K;
     rc = plan_columns(c, LA, nb, K, c->N, ncol, &chunk, S);
@@ -1229,11 +1311,11 @@ static int pair_term(rte_ctx* c, int LA, int nb, int* S) {
     return RTE_OK;
   }
   const int cols = c->slab_cols;
-  rc = plan_columns(c, LA, nb, c->d_slab, (size_t)cols * c->nz, cols, &chunk, S);
+  rc = plan_columns(c, LA, nb, c->d_slab, (size_t)cols * c->cz, cols, &chunk, S);
   if (rc) return rc;
   for (int c0 = 0, s0 = 0; c0 < ncol; c0 += cols) {
     const int c1 = std::min(ncol, c0 + cols);
-    const size_t ld = (size_t)cols * c->nz;
+    const size_t ld = (size_t)cols * c->cz;
     {
       ProfScope ps(c, 1);
       CUDA_TRY(c, rte_launch_store_kernel(store_args(c, c->d_slab, ld, c0, c1), c->st, f));
@@ -1300,6 +1382,47 @@ static SelfArgs self_args(const rte_ctx* c, const double* W) {
 
 static void* rows_of(const rte_ctx* c, int nb) { return nb == 1 ? c->d_Wf : c->d_bWf; }
 
+// Rows of the column kernels from a distribution in voxel order.
+static int make_rows(rte_ctx* c, const double* w, void* rows, int nb, int pitch) {
+  const int f = c->precision == RTE_PREC_FP64 ? 1 : 0;
+  if (c->d_exch)
+    CUDA_TRY(c, (c->launches++, rte_launch_rows_rot(w, rows, c->d_exch, c->d_islot, c->N, nb, pitch, c->C, f, c->st)));
+  else
+    CUDA_TRY(c, (c->launches++, rte_launch_rows(w, rows, c->d_islot, c->N, nb, pitch, c->C, f, c->st)));
+  return RTE_OK;
+}
+
+// The epilogue's view of S chunk sums of the pair operator (e->nb right-hand sides), brought back to the grid's frame.
+static int pair_sums(rte_ctx* c, int LA, int S, bool f32part, EpiArgs* e) {
+  if (!c->ax) {
+    e->S = S;
+    e->part = c->d_part;
+    e->partf = f32part ? reinterpret_cast<const float*>(c->d_part) : nullptr;
+    return RTE_OK;
+  }
+  FlatArgs a;
+  memset(&a, 0, sizeof a);
+  a.N = c->N;
+  a.nx = c->nx;
+  a.ny = c->ny;
+  a.nz = c->nz;
+  a.Cfull = c->C;
+  a.S = S;
+  a.nb = e->nb;
+  const int plane = c->cx * c->cy;
+  a.sx = c->ax == 1 ? plane : c->cx;
+  a.sy = c->ax == 1 ? c->cx : plane;
+  a.sz = 1;
+  a.part = c->d_part;
+  a.M = c->d_exch;
+  a.out = c->d_flat;
+  CUDA_TRY(c, (c->launches++, rte_launch_sums_rot(a, LA, f32part ? 0 : 1, c->st)));
+  e->S = 1;
+  e->part = c->d_flat;
+  e->partf = nullptr;
+  return RTE_OK;
+}
+
 static int apply_term(rte_ctx* c, const double* in64, double* out, double* sum, int flag, int flag_scat, int nb = 1,
                       bool rows_ready = false, bool keep_rows = false) {
   const int LA = flag ? c->L : 0;
@@ -1312,9 +1435,10 @@ static int apply_term(rte_ctx* c, const double* in64, double* out, double* sum, 
     ProfScope ps(c, 0);
     CUDA_TRY(c, (c->launches += 5, rte_fft_apply(c->fft, in64, nb * c->C, c->C, LA, nb, c->d_part, c->st)));
   } else {
-    if (!rows_ready)
-      CUDA_TRY(c, (c->launches++, rte_launch_rows(in64, rows_of(c, nb), c->d_islot, c->N, nb, col_dims(c).pitch, c->C,
-                                                  c->precision == RTE_PREC_FP64 ? 1 : 0, c->st)));
+    if (!rows_ready || c->ax) {
+      rc = make_rows(c, in64, rows_of(c, nb), nb, col_dims(c).pitch);
+      if (rc) return rc;
+    }
     rc = pair_term(c, LA, nb, &S);
     if (rc) return rc;
     f32part = c->precision == RTE_PREC_MIXED;
@@ -1327,17 +1451,21 @@ static int apply_term(rte_ctx* c, const double* in64, double* out, double* sum, 
   e.ny = c->ny;
   e.nz = c->nz;
   e.Cfull = c->C;
-  e.S = S;
   e.nb = nb;
-  e.part = c->d_part;
-  e.partf = f32part ? reinterpret_cast<const float*>(c->d_part) : nullptr;
+  if (fft_active(c)) {
+    e.S = S;
+    e.part = c->d_part;
+  } else {
+    rc = pair_sums(c, LA, S, f32part, &e);
+    if (rc) return rc;
+  }
   e.self = self_args(c, in64);
   e.self.lut = c->d_self_lut;
   e.mus = c->d_mus;
   e.flag_scat = flag_scat;
   scatter_factors(c, flag, e.scat);
   e.Wout = out;
-  e.rows = keep_rows && !fft_active(c) ? rows_of(c, nb) : nullptr;
+  e.rows = keep_rows && !fft_active(c) && !c->ax ? rows_of(c, nb) : nullptr;
   e.rows64 = c->precision == RTE_PREC_FP64 ? 1 : 0;
   e.islot = c->d_islot;
   e.pitch = col_dims(c).pitch;
@@ -2154,8 +2282,8 @@ static int ensure_batch(rte_ctx* c, int nb) {
   if (c->d_bWf) cudaFree(c->d_bWf);
   c->d_bWf = nullptr;
   {  // FP32 rows of nb right-hand sides, or FP64 rows of a complex pair
-    const size_t pf = nb * rte_col_dims(c->C, c->L, c->nz, 0, 0).pitch * sizeof(float),
-                 pd = 2 * rte_col_dims(c->C, c->L, c->nz, 1, 0).pitch * sizeof(double);
+    const size_t pf = nb * rte_col_dims(c->C, c->L, c->cz, 0, 0).pitch * sizeof(float),
+                 pd = 2 * rte_col_dims(c->C, c->L, c->cz, 1, 0).pitch * sizeof(double);
     unsigned char* rows = nullptr;
     CUDA_TRY(c, dalloc(c, &rows, (size_t)c->N * std::max(pf, pd)));
     c->d_bWf = rows;
@@ -2483,17 +2611,17 @@ static BpArgs bp_args(rte_ctx* c, bool accumulate) {
   BpArgs bp;
   memset(&bp, 0, sizeof bp);
   bp.N = c->N;
-  bp.nx = c->nx;
-  bp.ny = c->ny;
-  bp.nz = c->nz;
+  bp.nx = c->cx;
+  bp.ny = c->cy;
+  bp.nz = c->cz;
   bp.Cfull = c->C;
-  bp.dx = c->dx;
-  bp.dy = c->dy;
-  bp.dz = c->dz;
+  bp.dx = c->cdx;
+  bp.dy = c->cdy;
+  bp.dz = c->cdz;
   bp.prop_thresh = c->prop_thresh;
   bp.kscale = c->dV / c->cm;
   bp.islot = c->d_islot;
-  bp.mut = c->d_mut;
+  bp.mut = c->d_mutc;
   bp.Kmat = c->K_valid && c->d_K ? c->d_K : nullptr;
   bp.Kmat64 = c->K_valid && c->d_K64 ? c->d_K64 : nullptr;
   bp.Kld = c->N;
@@ -2575,8 +2703,9 @@ static int adjoint_source_terms(rte_ctx* c, const rte_source* s, const rte_stop*
   {
     ProfScope ps(c, 0);
     const int f64 = mixed ? 0 : 1;
-    CUDA_TRY(c, (c->launches++, rte_launch_rows(c->d_y, (void*)bp.y, c->d_islot, c->N, 1, bp.pitch, c->C, f64, c->st)));
-    CUDA_TRY(c, (c->launches++, rte_launch_rows(c->d_S, (void*)bp.S, c->d_islot, c->N, 1, bp.pitch, c->C, f64, c->st)));
+    int rr = make_rows(c, c->d_y, (void*)bp.y, 1, bp.pitch);
+    if (!rr) rr = make_rows(c, c->d_S, (void*)bp.S, 1, bp.pitch);
+    if (rr) return rr;
     CUDA_TRY(c, (c->launches++, rte_launch_bp_weights(bp, c->L, f64, c->st)));
   }
   GradLocalArgs gl;
@@ -2843,7 +2972,7 @@ static std::vector<uintptr_t> graph_signature(const rte_ctx* c, int nb) {
           u(nb == 1 ? c->d_aux2 : c->d_bres), u(nb == 1 ? c->d_Wf : c->d_bWf),
           u(c->d_part), u(c->d_self_idx), u(c->d_self_lut), u(c->d_mom), (uintptr_t)c->K,
           (uintptr_t)c->self_lut_ok, u(c->d_K), u(c->d_K64), u(c->d_slab), (uintptr_t)c->slab_bytes, u(c->d_mut), u(c->d_mutf), u(c->d_mus),
-          u(c->d_tab[0][0]), u(c->d_tab[1][0]), u(c->d_red), u(c->d_err), (uintptr_t)c->bcap, (uintptr_t)(fft_eligible(c) && !c->fft_graph_failed),
+          u(c->d_tab[0][0]), u(c->d_tab[1][0]), u(c->d_flat), u(c->d_red), u(c->d_err), (uintptr_t)c->bcap, (uintptr_t)(fft_eligible(c) && !c->fft_graph_failed),
           rte_fft_signature(c->fft)};
 }
 
@@ -2877,10 +3006,10 @@ static int run_series_graph(rte_ctx* c, int nb, int nterms, double** d_res) {
       rc = ensure_pair_kernel(c, &stored);
       if (rc) return rc;
       const void* K = stored ? (c->precision == RTE_PREC_FP64 ? (const void*)c->d_K64 : (const void*)c->d_K) : c->d_slab;
-      const int cols = stored ? c->nx * c->ny : c->slab_cols;
+      const int cols = stored ? c->cx * c->cy : c->slab_cols;
       int chunk, S;
-      rc = plan_columns(c, c->L, nb, K, (size_t)cols * c->nz, cols, &chunk, &S);
-      if (!rc && flag_l == 0) rc = plan_columns(c, 0, nb, K, (size_t)cols * c->nz, cols, &chunk, &S);
+      rc = plan_columns(c, c->L, nb, K, (size_t)cols * c->cz, cols, &chunk, &S);
+      if (!rc && flag_l == 0) rc = plan_columns(c, 0, nb, K, (size_t)cols * c->cz, cols, &chunk, &S);
     }
     if (rc) return rc;
     c->fft_in_graph[gi] = use_fft;
@@ -3169,10 +3298,10 @@ extern "C" int rte_fisher_regions(rte_ctx* c, const rte_source* s, const rte_sto
 // Chunk sums into d_part, *S of them.  17^3 L=5 mixed, K recomputed, per parameter: 2.23 ms by a walk and spherical
 // harmonics per pair -> 0.46.
 static int tangent_pairs(rte_ctx* c, const double* d_in, const std::vector<double>& dmut, int* S) {
-  const int f = c->precision == RTE_PREC_FP64 ? 1 : 0, ncol = c->nx * c->ny, plane = ncol;
+  const int f = c->precision == RTE_PREC_FP64 ? 1 : 0, ncol = c->cx * c->cy;
   std::vector<double> col(c->N);  // the direction in column order, in the operator's precision
   for (int r = 0; r < c->N; r++) {
-    const int slot = r % plane * c->nz + r / plane;
+    const int slot = slot_of(c, r);
     if (f)
       col[slot] = dmut[r];
     else
@@ -3180,12 +3309,12 @@ static int tangent_pairs(rte_ctx* c, const double* d_in, const std::vector<doubl
   }
   CUDA_TRY(c, cudaMemcpyAsync(c->d_dmutc, col.data(), (f ? sizeof(double) : sizeof(float)) * c->N, cudaMemcpyHostToDevice,
                               c->st));
-  CUDA_TRY(c, (c->launches++, rte_launch_rows(d_in, rows_of(c, 1), c->d_islot, c->N, 1, col_dims(c).pitch, c->C, f, c->st)));
-  int rc = ensure_slab(c), chunk = 1;
+  int rc = make_rows(c, d_in, rows_of(c, 1), 1, col_dims(c).pitch), chunk = 1;
+  if (!rc) rc = ensure_slab(c);
   if (rc) return rc;
   const void* stored = !c->K_valid ? nullptr : f ? (const void*)c->d_K64 : (const void*)c->d_K;
   const int cols = c->slab_cols;
-  const size_t ld = (size_t)cols * c->nz;
+  const size_t ld = (size_t)cols * c->cz;
   rc = plan_columns(c, c->L, 1, c->d_slab, ld, cols, &chunk, S);
   if (rc) return rc;
   for (int c0 = 0, s0 = 0; c0 < ncol; c0 += cols) {
@@ -3195,7 +3324,7 @@ static int tangent_pairs(rte_ctx* c, const double* d_in, const std::vector<doubl
     a.mu = c->d_dmutc;
     a.Kin = stored ? stored : c->d_slab;
     a.Kin_ld = stored ? (size_t)c->N : ld;
-    a.kin_slot = stored ? c0 * c->nz : 0;
+    a.kin_slot = stored ? c0 * c->cz : 0;
     CUDA_TRY(c, (c->launches++, rte_launch_store_kernel(a, c->st, f)));
     const ColArgs ca = col_args(c, 1, c->d_slab, ld, c0, a.col1, chunk, s0);
     CUDA_TRY(c, (c->launches++, launch_columns(c, ca, c->L)));
@@ -3221,10 +3350,9 @@ static int tangent_dA(rte_ctx* c, const double* d_in, double* d_outT, const std:
   e.ny = c->ny;
   e.nz = c->nz;
   e.Cfull = c->C;
-  e.S = S;
   e.nb = 1;
-  e.part = c->d_part;
-  e.partf = c->precision == RTE_PREC_MIXED ? reinterpret_cast<const float*>(c->d_part) : nullptr;
+  rc = pair_sums(c, c->L, S, c->precision == RTE_PREC_MIXED, &e);
+  if (rc) return rc;
   e.self = self_args(c, d_in);
   e.self.mut = c->d_mut;
   e.self.lut = c->d_dlut;

@@ -84,6 +84,8 @@ struct ColArgs {
   int chunk, nsplit;
   int* err;
   double* red;        // the epilogue's four norms, zeroed here for it
+  // pair-by-pair form of flat grids (rte_flat.cu; tab: directions): entry of displacement 0, steps per column axis
+  int d0, dsx, dsy, dsz;
   int tz, ncd;        // set by the launcher: sources per run, destination columns per CTA at most
 };
 struct ColDims {
@@ -92,6 +94,15 @@ struct ColDims {
   int row, azn, csn, nk, pho;       // angle rows: entries of csn values in tg residue classes of cls
   int tg, cls;
 };
+// chunk sums of a flat grid's exchanged frame (rte_flat.cu)
+struct FlatArgs {
+  int N, nx, ny, nz, Cfull, S, nb;
+  int sx, sy, sz;       // voxel steps of the exchanged frame along the grid's axes
+  const void* part;     // chunk sums [S][N][nb][Cfull] (ColArgs)
+  const double* M;      // coefficients of the exchanged frame [Cfull][Cfull] (null: the same)
+  double* out;          // [N][nb][Cfull]
+};
+
 struct ColTabArgs {
   int nx, ny, nz, nzp, L;
   double dx, dy, dz, kappa;
@@ -190,7 +201,7 @@ struct BpArgs {
   int N, nx, ny, nz, Cfull;
   double dx, dy, dz, prop_thresh, kscale;
   const int* islot;
-  const double* mut;
+  const double* mut;   // column order
   const void* y;       // T, destination-side field, column-order rows times N_c (rte_launch_rows), `pitch` apart
   const void* S;       // T, source-side field, likewise
   int pitch;
@@ -303,6 +314,13 @@ cudaError_t rte_launch_layer_sums(const double* W, const double* S, int N, int n
 cudaError_t rte_launch_rows(const double* w, void* rows, const int* islot, int N, int nb, int pitch, int Cfull,
                             int fp64, cudaStream_t st);
 ColDims rte_col_dims(int C, int L, int nz, int fp64, int cplx);
+cudaError_t rte_launch_rows_rot(const double* w, void* rows, const double* M, const int* islot, int N, int nb, int pitch,
+                                int Cfull, int fp64, cudaStream_t st);
+cudaError_t rte_launch_sums_rot(const FlatArgs& a, int LA, int fp64, cudaStream_t st);
+size_t rte_dirs_bytes(int nx, int ny, int nz, int L, int fp64);
+cudaError_t rte_launch_dirs_table(int nx, int ny, int nz, double dx, double dy, double dz, int transpose, int L, int fp64,
+                                  void* tab, cudaStream_t st);
+cudaError_t rte_launch_pair_dirs(const ColArgs& a, int LA, int fp64, cudaStream_t st, int* occ = nullptr);
 // rows of columns beyond its own that a launch reads the pair kernel of, where voxels couple over ry rows
 int rte_col_reach(int nx, int nzp, int group, int ry);
 cudaError_t rte_launch_col_table(const ColTabArgs& a, void* tab, int fp64, cudaStream_t st);

@@ -65,3 +65,11 @@ def test_limited_coupling(rte, prec):
     n = (33, 33, 33)
     a = _forward(rte, n, prec, rte.KERNEL_RECOMPUTE, thresh=0.25)
     assert a < 0.25 * _forward(rte, n, prec, rte.KERNEL_RECOMPUTE)
+
+
+@pytest.mark.parametrize("prec", [0, 1])
+@pytest.mark.parametrize("mode", [1, 2])
+def test_flat_grid(rte, prec, mode):
+    """110x110x1 against 23^3: 50 and 150 times its time with z columns (kernel stored, recomputed), 1 to 7 now."""
+    a = _forward(rte, (110, 110, 1), prec, mode)
+    assert a < 20 * _forward(rte, (23, 23, 23), prec, mode)
