@@ -462,9 +462,11 @@ static int fail(rte_ctx* c, int code, const char* fmt, ...) {
   return code;
 }
 
+// a failed allocation also stays behind as the runtime's last error, which the next launch would report as its own
 #define CUDA_TRY(ctx, call)                                                                       \
   do {                                                                                            \
     cudaError_t e_ = (call);                                                                      \
+    if (e_ == cudaErrorMemoryAllocation) (void)cudaGetLastError();                                \
     if (e_ != cudaSuccess)                                                                        \
       return fail(ctx, e_ == cudaErrorMemoryAllocation ? RTE_ERR_NOMEM : RTE_ERR_DEVICE,          \
                   "%s: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__);           \
@@ -788,6 +790,7 @@ static int build_self_lut(rte_ctx* c) {
         cudaFree(c->d_self_lut_im);
         c->bytes -= c->lut_im_cap * sizeof(double);
         c->d_self_lut_im = nullptr;
+        c->lut_im_cap = 0;
       }
       const size_t cap = std::max(lut_im.size(), (size_t)16 * C * C);
       CUDA_TRY(c, dalloc(c, &c->d_self_lut_im, cap));
@@ -803,6 +806,7 @@ static int build_self_lut(rte_ctx* c) {
         cudaFree(c->d_dlut);
         c->bytes -= c->dlut_cap * sizeof(double);
         c->d_dlut = nullptr;
+        c->dlut_cap = 0;
       }
       const size_t cap = std::max(dlut.size(), (size_t)16 * C * C);  // headroom: fewer reallocations
       CUDA_TRY(c, dalloc(c, &c->d_dlut, cap));
@@ -816,6 +820,7 @@ static int build_self_lut(rte_ctx* c) {
       cudaFree(c->d_self_lut);
       c->bytes -= c->lut_cap * sizeof(double);
       c->d_self_lut = nullptr;
+      c->lut_cap = 0;
     }
     const size_t cap = std::max(lut.size(), (size_t)16 * C * C);
     CUDA_TRY(c, dalloc(c, &c->d_self_lut, cap));
@@ -832,6 +837,7 @@ static int build_self_lut(rte_ctx* c) {
 
 // mu_t, mu_s (and the FP32 mu_t) from device arrays; the pair kernel becomes stale.
 static int medium_from_device(rte_ctx* c, const double* d_mua, const double* d_mus) {
+  c->medium_set = false;  // until its self-voxel tables are there
   CUDA_TRY(c, cudaMemsetAsync(c->d_red + 6, 0, sizeof(double), c->st));
   CUDA_TRY(c, (c->launches++, rte_launch_medium(d_mua, d_mus, c->d_mut, c->d_mus, c->d_mutf, c->d_mutc, c->d_mutfc,
                                                    c->d_islot, c->N, c->d_red + 6, c->st)));
@@ -839,12 +845,12 @@ static int medium_from_device(rte_ctx* c, const double* d_mua, const double* d_m
   CUDA_TRY(c, cudaMemcpyAsync(&mumax, c->d_red + 6, sizeof(double), cudaMemcpyDeviceToHost, c->st));
   CUDA_TRY(c, cudaStreamSynchronize(c->st));
   c->K_valid = false;
-  c->medium_set = true;
   c->split = false;
   c->mumax = mumax;
   int rc = ensure_moments(c, std::hypot(mumax, c->kappa));
-  if (rc) return rc;
-  return build_self_lut(c);
+  if (!rc) rc = build_self_lut(c);
+  c->medium_set = rc == RTE_OK;
+  return rc;
 }
 
 extern "C" int rte_set_medium_voxel(rte_ctx* c, const double* mua, const double* mus) {
@@ -1230,7 +1236,8 @@ static int plan_columns(rte_ctx* c, int LA, int nb, const void* K, size_t ld, in
     if (e[0] == key && e[1] == cols) {
       *chunk_out = e[2];
       *total_out = total(e[2]);
-      return RTE_OK;
+      const size_t cells = (size_t)c->N * c->C * nb * *total_out;
+      return grow(c, &c->d_part, c->part_cap, f ? cells : (cells + 1) / 2);
     }
   int sms = 0, occ = 0;
   CUDA_TRY(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->cfg.device));
@@ -2256,6 +2263,7 @@ static int grow(rte_ctx* c, T** p, size_t& cap, size_t n) {
     cudaFree(*p);
     c->bytes -= cap * sizeof(T);
     *p = nullptr;
+    cap = 0;  // also if the allocation fails
   }
   CUDA_TRY(c, dalloc(c, p, n));
   cap = n;
@@ -2266,6 +2274,7 @@ static int ensure_batch(rte_ctx* c, int nb) {
   const size_t NC = (size_t)c->N * c->C;
   int rc = grow(c, &c->d_part, c->part_cap, NC * nb * c->max_split);
   if (rc || nb <= c->bcap) return rc;
+  c->bcap = 0;  // also if an allocation fails
   double** bufs[] = {&c->d_bW, &c->d_bWn, &c->d_bsum, &c->d_bres};
   for (double** b : bufs) {
     if (*b) cudaFree(*b);
@@ -2437,17 +2446,18 @@ static void face_weights(rte_ctx* c) {
 }
 
 static int ensure_detector_buffers(rte_ctx* c) {
-  if (c->d_h) return RTE_OK;
+  if (c->d_rho) return RTE_OK;  // the last one below
   const size_t NC = (size_t)c->N * c->C;
   const size_t npix = 2 * ((size_t)c->nx * c->ny + (size_t)c->nz * c->nx + (size_t)c->nz * c->ny);
   face_weights(c);
-  CUDA_TRY(c, dalloc(c, &c->d_h, c->h_h.size()));
+  if (!c->d_h) CUDA_TRY(c, dalloc(c, &c->d_h, c->h_h.size()));
   CUDA_TRY(c, cudaMemcpy(c->d_h, c->h_h.data(), sizeof(double) * c->h_h.size(), cudaMemcpyHostToDevice));
   double** bufs[] = {&c->d_S, &c->d_out, &c->d_e, &c->d_lam, &c->d_y};
-  for (double** b : bufs) CUDA_TRY(c, dalloc(c, b, NC));
-  CUDA_TRY(c, dalloc(c, &c->d_gt, c->N));
-  CUDA_TRY(c, dalloc(c, &c->d_gs, c->N));
-  CUDA_TRY(c, dalloc(c, &c->d_J, npix));
+  for (double** b : bufs)
+    if (!*b) CUDA_TRY(c, dalloc(c, b, NC));
+  if (!c->d_gt) CUDA_TRY(c, dalloc(c, &c->d_gt, c->N));
+  if (!c->d_gs) CUDA_TRY(c, dalloc(c, &c->d_gs, c->N));
+  if (!c->d_J) CUDA_TRY(c, dalloc(c, &c->d_J, npix));
   CUDA_TRY(c, dalloc(c, &c->d_rho, npix));
   return RTE_OK;
 }
@@ -3387,13 +3397,14 @@ extern "C" int rte_fisher(rte_ctx* c, int nsrc, const rte_source* srcs, const rt
     rc = ensure_batch(c, nbt);
     if (rc) return rc;
   }
-  if (!c->d_dmut) {
-    CUDA_TRY(c, dalloc(c, &c->d_dmut, (size_t)c->N));
-    CUDA_TRY(c, dalloc(c, &c->d_dmutc, (size_t)c->N));
-    CUDA_TRY(c, dalloc(c, &c->d_dmus, (size_t)c->N));
-    CUDA_TRY(c, dalloc(c, &c->d_T, (size_t)std::max(2, nbt) * NC));  // nbt is fixed for a context (L, precision)
-    CUDA_TRY(c, dalloc(c, &c->d_cidx, (size_t)std::max(c->nx, std::max(c->ny, c->nz))));
-    CUDA_TRY(c, dalloc(c, &c->d_cval, (size_t)std::max(c->nx, std::max(c->ny, c->nz)) * c->C));
+  {
+    const size_t longest = (size_t)std::max(c->nx, std::max(c->ny, c->nz));
+    if (!c->d_dmut) CUDA_TRY(c, dalloc(c, &c->d_dmut, (size_t)c->N));
+    if (!c->d_dmutc) CUDA_TRY(c, dalloc(c, &c->d_dmutc, (size_t)c->N));
+    if (!c->d_dmus) CUDA_TRY(c, dalloc(c, &c->d_dmus, (size_t)c->N));
+    if (!c->d_T) CUDA_TRY(c, dalloc(c, &c->d_T, (size_t)std::max(2, nbt) * NC));  // nbt is fixed for a context (precision)
+    if (!c->d_cidx) CUDA_TRY(c, dalloc(c, &c->d_cidx, longest));
+    if (!c->d_cval) CUDA_TRY(c, dalloc(c, &c->d_cval, longest * c->C));
   }
   std::vector<double> mut(c->N), mus(c->N);
   CUDA_TRY(c, cudaMemcpy(mut.data(), c->d_mut, sizeof(double) * c->N, cudaMemcpyDeviceToHost));

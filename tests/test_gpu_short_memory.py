@@ -2,6 +2,7 @@
 over to storing it when memory comes free."""
 import contextlib
 
+import numpy as np
 import pytest
 import torch
 
@@ -67,3 +68,38 @@ def test_workspace_cut_short(rte, n, prec, tol):
                 assert rel(tr[0], a["trans"]) < 1e-9 and rel(rf[0], a["ref"]) < 1e-9
             out.append((a["W"], J))
     assert rel(out[1][0], out[0][0]) < tol and rel(out[1][1], out[0][1]) < tol
+
+
+@pytest.mark.parametrize("left", [2, 8, 20, 40, 70])
+def test_context_after_a_failed_allocation(rte, left):
+    """A batch, a gradient and a Fisher matrix that find no room fail with an error; the context keeps nothing of what it
+    freed or half made: a single solve, and with room the refused calls, give what they gave before."""
+    n, T = 21, 3
+    srcs = [rte.Source(pos_x=0.2 * q, kind=rte.SRC_COLUMN) for q in (-1, 0, 1)]
+    stop, det = rte.Stop(rte.STOP_FIXED, T), rte.Detector(nbins=2, faces=63)
+    mua, mus, _ = rte.sphere_phantom(n, nspheres=2, seed=2, rmin=0.15, rmax=0.3)
+
+    def calls(ctx):
+        return (lambda: [ctx.forward_batch(srcs, stop)["W"]],
+                lambda: list(ctx.gradient(srcs[:1], stop, det, np.zeros((1, 6, 2, 2)))[1:]),
+                lambda: list(ctx.fisher(srcs[:1], stop, det, mua, 0 * mus, want_J=True)))
+
+    with rte.Context(n, n, n, dx=0.1, nL=5, g=0.8, precision=rte.PREC_MIXED, kernel_mode=rte.KERNEL_STORE) as ctx:
+        ctx.set_medium_voxel(mua, mus)
+        want = [f() for f in calls(ctx)]
+        one = ctx.forward(srcs[0], stop)["W"]
+    with rte.Context(n, n, n, dx=0.1, nL=5, g=0.8, precision=rte.PREC_MIXED, kernel_mode=rte.KERNEL_STORE) as ctx:
+        ctx.set_medium_voxel(mua, mus)
+        ctx.forward(srcs[0], stop)
+        refused = 0
+        with _left(left << 20):
+            for f in calls(ctx):
+                try:
+                    f()
+                except rte.RteError:
+                    refused += 1
+                assert rel(ctx.forward(srcs[0], stop)["W"], one) < 2e-6
+        assert refused > 0
+        for f, w in zip(calls(ctx), want):
+            for a, b in zip(f(), w):
+                assert rel(a, b) < 1e-5
