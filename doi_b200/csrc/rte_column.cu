@@ -11,9 +11,10 @@
 // the sums g_k of one source column expand to the (L+1)^2 destination coefficients once per column pair:
 // 22 multiply-adds per pair and right-hand side at L = 5 instead of 72, and no SH recurrence per pair.
 // The trigonometric values come from (cos theta, sin theta) per displacement, tabulated in FP64 once per
-// context (rte_launch_col_table), by double-angle and addition steps; for FP32 sums at L >= 7 the whole
-// row cos k theta, sin k theta is tabulated in FP64 and rounded, so that the angular functions there are
-// FP64 values as in the other kernels.  The reference's snapped direction table (FisherInfo_IO) fits the
+// context (rte_launch_col_table), by double-angle and addition steps; for FP32 sums at L >= 7 they are FP64 values
+// rounded: the whole row cos k theta, sin k theta is tabulated, or, in columns too long for that, made in FP64 from
+// the FP64 pair.  (The contraction onto them is FP32 there too.  Against FP64, 25^3 L=7, six terms: 1.5e-7 with the
+// kernel stored; per-pair functions evaluated in FP64, 6.5e-7 stored and 2.0e-7 recomputed, there 2.3e-7 now.)  The reference's snapped direction table (FisherInfo_IO) fits the
 // same form: its azimuth index depends on (dx, dy) alone.
 #include <cuda_runtime.h>
 #include <math.h>
@@ -317,6 +318,12 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
       if constexpr (FULL) {
 #pragma unroll
         for (int k = 0; k < L; ++k) tr[q][k] = reinterpret_cast<const f2_t*>(an)[k];
+      } else if constexpr (F32 && L >= RTE_FULL_L) {
+        double ck[L], sk[L];
+        const double2 v = *reinterpret_cast<const double2*>(an);
+        trig_pairs<L, double>(v.x, v.y, fma(v.x, v.x, -(v.y * v.y)), 2.0 * v.x * v.y, ck, sk);
+#pragma unroll
+        for (int k = 0; k < L; ++k) tr[q][k] = f2_pack((float)ck[k], (float)sk[k]);
       } else if constexpr (L > 0) {
         T ck[L], sk[L];
         if constexpr (F32) {
@@ -521,8 +528,8 @@ __global__ void __launch_bounds__(T_CTA, col_ctas<L, T, NB, CPLX>()) k_column(Co
 
 // Angle rows: per column displacement (dx, dy) first azn values (cos m phi, sin m phi, m = 1..L), then the polar
 // entries of dz = e - nz, e = 0..nz+nzp-1, csn values each, entry e at (e % tg) * cls + e / tg: (cos theta,
-// sin theta), for FP32 also (cos 2theta, sin 2theta), for FP32 at L >= 7 every (cos k theta, sin k theta), and
-// with kappa != 0 the phase (cos kappa r, sin kappa r) at offset pho.  One thread per (dx, dy, dz).
+// sin theta), for FP32 also (cos 2theta, sin 2theta), for FP32 at L >= 7 every (cos k theta, sin k theta) or, in long
+// columns, (cos theta, sin theta) in FP64, and with kappa != 0 the phase (cos kappa r, sin kappa r) at offset pho.  One thread per (dx, dy, dz).
 template <typename T>
 __global__ void k_col_table(ColTabArgs a, T* tab) {
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -560,7 +567,8 @@ __global__ void k_col_table(ColTabArgs a, T* tab) {
   }
   T* p = row + a.azn + ((size_t)(iz % a.tg) * a.cls + iz / a.tg) * a.csn;
   double c = 1.0, s = 0.0;
-  for (int k = 1; k <= a.nk; ++k) {
+  if (a.wide) *reinterpret_cast<double2*>(p) = make_double2(ct, st);  // in the place of two FP32 pairs
+  for (int k = 1; k <= (a.wide ? 0 : a.nk); ++k) {
     const double n = c * ct - s * st;
     s = c * st + s * ct;
     c = n;
@@ -604,20 +612,27 @@ cudaError_t launch_nb(ColArgs a, cudaStream_t st, int* occ) {
   // positions a CTA's columns span: its threads' destinations, or (G = 1) the layout blocks of its warps
   const int span = G == 1 ? ((T_CTA / 32 + a.group - 2) / a.group + 1) * 32 * a.group : T_CTA * G;
   a.ncd = (span + a.nzp - 2) / a.nzp + 1;
-  // the whole column as one run when two CTAs fit an SM's shared memory, else equal runs
-  size_t smem = 0;
-  for (int nrun = 1;; ++nrun) {
-    a.tz = (a.nz + nrun - 1) / nrun;
-    smem = ColLayout(a.tz, a.pitch, a.azn, a.row - a.azn, a.ncd, NB * nb_row<L>(), NB,
+  const int nblk = (np + 32 * a.group - 1) / (32 * a.group);  // layout blocks: a warp each, or `group` warps for G = 1
+  const int warps = G == 1 ? nblk * a.group : nblk;
+  dim3 grid((unsigned)((warps + T_CTA / 32 - 1) / (T_CTA / 32)) * (CPLX ? 1 : a.nrhs / NB), a.nsplit);
+  // the whole column as one run when two CTAs fit an SM's shared memory, else equal runs; runs that the angle rows of
+  // two CTAs would cut below 16 sources take the shared memory of one, up to 64 sources (1x1x500 L=7 mixed, six terms and
+  // the final application 3.8 ms in runs of 8 -> 3.2; FP32 sums of 512 sources 2.1e-7 from FP64, of 64 1.5e-7)
+  auto bytes = [&](int tz) {
+    return ColLayout(tz, a.pitch, a.azn, a.row - a.azn, a.ncd, NB * nb_row<L>(), NB,
                      ring_stages<G>() * ring_rows<G>() * 32 * G, ring_stages<G>(), (int)sizeof(T)).bytes;
-    if (smem <= 113 * 1024 || a.tz <= 8) break;
+  };
+  const bool one = bytes(std::min(a.nz, 16)) > 113 * 1024;
+  const size_t limit = (one ? 227 : 113) * 1024;
+  size_t smem = 0;
+  for (int nrun = one ? (a.nz + 63) / 64 : 1;; ++nrun) {
+    a.tz = (a.nz + nrun - 1) / nrun;
+    smem = bytes(a.tz);
+    if (smem <= limit || a.tz <= 8) break;
   }
   cudaError_t e = smem_limit((const void*)kern, smem);
   if (e != cudaSuccess) return e;
   if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, T_CTA, smem);
-  const int nblk = (np + 32 * a.group - 1) / (32 * a.group);  // layout blocks: a warp each, or `group` warps for G = 1
-  const int warps = G == 1 ? nblk * a.group : nblk;
-  dim3 grid((unsigned)((warps + T_CTA / 32 - 1) / (T_CTA / 32)) * (CPLX ? 1 : a.nrhs / NB), a.nsplit);
   kern<<<grid, T_CTA, smem, st>>>(a);
   return cudaGetLastError();
 }
@@ -666,9 +681,10 @@ ColDims rte_col_dims(int C, int L, int nz, int fp64, int cplx) {
   d.nzp = (nz + d.group - 1) / d.group * d.group;
   d.azn = up4(2 * L);
   // FP32 at L >= 7 tabulates whole trigonometric rows, an odd number of 8-byte units apart (conflict-free);
-  // columns so long that two of them no longer fit shared memory keep the two pairs
+  // columns so long that two of them no longer fit shared memory keep the FP64 pair in the place of two FP32 ones
   const bool full = !fp64 && L >= RTE_FULL_L && nz <= RTE_FULL_NZ;
   d.nk = fp64 ? 1 : (full ? L : 2);
+  d.wide = !fp64 && L >= RTE_FULL_L && !full;
   d.pho = cplx ? 2 * d.nk : 0;
   d.csn = 2 * d.nk + (cplx ? (fp64 ? 2 : 4) : 0);
   d.tg = cplx ? RTE_COL_GC(L, fp64) : d.group;

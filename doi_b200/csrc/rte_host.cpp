@@ -1104,6 +1104,7 @@ static int ensure_col_table(rte_ctx* c) {
   a.pho = d.pho;
   a.tg = d.tg;
   a.cls = d.cls;
+  a.wide = d.wide;
   CUDA_TRY(c, (c->launches++, rte_launch_col_table(a, *p, f, c->st)));
   c->tab_kappa[f][tr] = c->kappa;
   return RTE_OK;

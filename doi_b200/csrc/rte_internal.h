@@ -93,6 +93,7 @@ struct ColDims {
   int group, nzp;                   // destinations per thread, destination positions per column
   int row, azn, csn, nk, pho;       // angle rows: entries of csn values in tg residue classes of cls
   int tg, cls;
+  int wide;                         // FP32 rows whose entries hold (cos theta, sin theta) in FP64
 };
 // chunk sums of a flat grid's exchanged frame (rte_flat.cu)
 struct FlatArgs {
@@ -107,7 +108,7 @@ struct ColTabArgs {
   int nx, ny, nz, nzp, L;
   double dx, dy, dz, kappa;
   int table, transpose;
-  int row, azn, csn, nk, pho, tg, cls;
+  int row, azn, csn, nk, pho, tg, cls, wide;
 };
 
 // Self-voxel term of the epilogue: scale * D(mu_t(r)) W[r], D symmetric, from a table of the medium's distinct mu_t
