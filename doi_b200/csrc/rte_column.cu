@@ -632,7 +632,14 @@ cudaError_t launch_nb(ColArgs a, cudaStream_t st, int* occ) {
   }
   cudaError_t e = smem_limit((const void*)kern, smem);
   if (e != cudaSuccess) return e;
-  if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, T_CTA, smem);
+  if (occ) {  // by registers, shared and tensor memory (the runtime's query answers 1 for kernels that use the latter)
+    cudaFuncAttributes at;
+    e = cudaFuncGetAttributes(&at, (const void*)kern);
+    if (e != cudaSuccess) return e;
+    const size_t regs = (size_t)(at.numRegs * 32 + 255) / 256 * 256 * (T_CTA / 32);
+    *occ = (int)std::min<size_t>(std::min<size_t>(65536 / regs, 228 * 1024 / (smem + 1024)), 512 / tmem_cols<L, T, G, NB>());
+    return cudaSuccess;
+  }
   kern<<<grid, T_CTA, smem, st>>>(a);
   return cudaGetLastError();
 }

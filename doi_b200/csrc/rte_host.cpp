@@ -1165,8 +1165,9 @@ static cudaError_t launch_columns(const rte_ctx* c, const ColArgs& a, int LA, in
 
 // Launch-plan autotuner of the column kernels.  The grid is (tiles of 128 threads' destinations x right-hand
 // sides) x (chunks of source columns); more chunks fill the SMs' last wave better and cost chunk sums.
-// Candidates are the chunk sizes that a model of waves and chunk-sum traffic ranks best; on
-// 1024 voxels and more each is launched on the context's own buffers and timed with CUDA events (best of two),
+// A model of waves and chunk-sum traffic ranks the chunk sizes.  FP64 launches and grids below 4096 voxels take its
+// choice, so that the order of their sums, and with it the last bits of a result, does not depend on a timing.  Mixed
+// launches on 4096 voxels and more try the best six on the context's own buffers, timed with CUDA events (best of two),
 // and the fastest is kept for the process (every context of that shape on that device reuses it).
 // RTE_AUTOTUNE=0 keeps the model's choice; RTE_NSPLIT forces a split.
 namespace {
@@ -1249,24 +1250,33 @@ static int plan_columns(rte_ctx* c, int LA, int nb, const void* K, size_t ld, in
   const long long tiles = (long long)((ncol * d.nzp + 128 * group - 1) / (128 * group)) * (rhs / per);
   const long long slots = (long long)std::max(occ, 1) * sms;
   const int cap = f ? cols : std::min(cols, kChunkColumns);
-  // a wave of resident CTAs takes (chunk + one column of start-up) x the SM's time per column at ~0.6 of the FMA
-  // rate; chunk sums are written and read once more each (us)
-  const double col_us = (f ? 2.0 : 1.0) * (cplx ? 2 : per) * occ * (double)group * c->cz * (4 * LA + 15.0) / (1.9e3 * 0.6);
+  // CTAs take their columns one after another, each at a rate that falls little with the CTAs on its SM (they wait for
+  // their own phases most of the time); chunk sums are written and read once more each (us).  Over 61 launches at
+  // 10^3-33^3 this picks a chunk within 1.3 % (FP64) and 6 % (FP32) of the fastest on average, 9 and 17 % at worst.
+  const double col_us = (f ? 2.0 : 1.0) * (cplx ? 2 : per) * (double)group * c->cz * (4 * LA + 15.0) / (1.9e3 * 0.6);
+  auto slowed = [&](long long ctas) { return 1.0 + (f ? 0.33 : 0.05) * (double)((ctas + sms - 1) / sms - 1); };
   const double part_us = (double)c->N * c->C * nb * (f ? 8 : 4) * 2 / 5e6;
   std::vector<std::pair<double, int>> rank;
   for (int chunk = 1, last = 0; chunk <= cap; chunk++) {
     const int S = (cols + chunk - 1) / chunk;
     if (S == last) continue;  // the smallest chunk of each split count
     last = S;
-    const double waves = ceil((double)tiles * S / (double)slots);
-    rank.push_back({waves * (chunk + 1) * col_us + S * part_us, chunk});
+    // whole waves, then a last one of what is left and the shorter last chunks
+    const int rest = cols % chunk;
+    const long long n = tiles * (cols / chunk), left = n % slots, tail = left + (rest ? tiles : 0);
+    double t = (double)(n / slots) * chunk * slowed(slots);
+    if (left && tail > slots)
+      t += chunk * slowed(slots) + rest * slowed(tail - slots);
+    else if (tail)
+      t += (left ? chunk : rest) * slowed(tail);
+    rank.push_back({t * col_us + S * part_us, chunk});
   }
   std::sort(rank.begin(), rank.end());
   if (rank.size() > 6) rank.resize(6);
   int chunk = rank[0].second;
   const char* forced = getenv("RTE_NSPLIT");
   const char* at = getenv("RTE_AUTOTUNE");
-  const bool tune = !forced && !(at && at[0] == '0') && !c->capturing && c->N >= 1024 && rank.size() > 1;
+  const bool tune = !forced && !(at && at[0] == '0') && !c->capturing && !f && c->N >= 4096 && rank.size() > 1;
   if (forced) chunk = std::max(1, std::min(cap, (cols + std::max(1, atoi(forced)) - 1) / std::max(1, atoi(forced))));
   const TuneKey tk{c->cfg.device, c->cx, c->cy, c->cz, LA, nb, c->precision, cplx, cols};
   bool have = false;
