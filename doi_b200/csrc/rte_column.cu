@@ -85,7 +85,8 @@ __host__ __device__ constexpr int tmem_cols() {
 // one new trigonometric row per source serves all G.  The pair kernel is streamed by bulk copies, a ring of
 // stages per warp (each warp's values are contiguous: kmat_index); register prefetch in its place waited on
 // every load (5.9 ms against 2.7 at 33^3 L=5).  The coefficient sums, touched once per source column, live in
-// tensor memory, which leaves the registers of four CTAs per SM.  NB = 2: two right-hand sides a thread, which
+// tensor memory, which leaves the registers of four CTAs per SM (at 33^3 L=5 the
+// layout's 58 KB admit three).  NB = 2: two right-hand sides a thread, which
 // share the trigonometric rows, the kernel values and the copies (two CTAs per SM at L >= 4).  CPLX: (real, imaginary) rows of one complex
 // right-hand side, the pair kernel times exp(-i kappa r) (phase tabulated beside the angles).
 // 33^3 L=5 launch, FP32, one right-hand side: 7.40 ms by per-pair spherical harmonics -> 2.36; four: 20.1 -> 9.3,
@@ -512,8 +513,9 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
   if (wid == 0) tmem_free(*stm, TMC);
 }
 
-// CTAs per SM to fit the registers to: four warps per scheduler hide the latencies of one another's loads (33^3
-// L=5: 2.77 ms per launch at two CTAs with the sums in registers, 2.41 at four with them in tensor memory)
+// CTAs per SM to fit the registers to (shared memory may admit fewer, three at 33^3 L=5): their warps hide the latencies
+// of one another's loads (33^3 L=5: 2.77 ms per launch at two CTAs with the sums in registers, 2.41 with them in tensor
+// memory and the registers of four)
 template <int L, typename T, int NB, bool CPLX>
 __host__ __device__ constexpr int col_ctas() {
   if (CPLX || (NB == 2 && L >= 4)) return 2;
@@ -594,6 +596,9 @@ __global__ void k_rows(const double* w, T* rows, const int* islot, int N, int nb
   rows[((size_t)rhs * N + islot[r]) * pitch + c] = (T)(w[t] * kMonic.N[c]);
 }
 
+// Dynamic shared memory above 48 KB: the attribute is set to the device's opt-in maximum, the same value from every host
+// thread, not to one launch's size: the server launches the same instantiation from several worker threads with sizes
+// that depend on the context, and per-launch values let one thread lower the limit between another's set and launch.
 cudaError_t smem_limit(const void* kern, size_t smem) {
   int dev = 0, cap = 0;
   cudaError_t e = cudaGetDevice(&dev);

@@ -23,9 +23,7 @@ __device__ __forceinline__ f2_t f2_fma(f2_t a, f2_t b, f2_t c) {
   return d;
 }
 
-// Compile-time copies of the SH recurrence coefficients (the same formulas as the host tables in
-// rte_host.cpp), so the unrolled FP32 recurrence multiplies by immediates and the l = m+1 steps
-// carry no B term.
+// Compile-time copies of the SH recurrence coefficients (the same formulas as the host tables in rte_host.cpp).
 struct ShConstTab {
   double A[64], B[64], Q0[RTE_MAX_L + 1];
 };
@@ -54,11 +52,10 @@ constexpr ShConstTab make_sh_const() {
   }
   return t;
 }
-__device__ constexpr ShConstTab kShConst = make_sh_const();
 
 // Monic form of the SH recurrence.  With q_l^m = s_lm u_l^m, s_mm = Q0[m] and s_lm = A_lm s_{l-1,m}, the
 // polynomials u satisfy u_l = z u_{l-1} - beta_lm u_{l-2} (beta_lm = B_lm s_{l-2,m} / s_lm), so R_c = N_c U_c with
-// U_{l,+-m} = u_l^m Re/Im((x+iy)^m) and N_c = s_lm.  The pair kernels work with U: the factors N_c are applied
+// U_{l,+-m} = u_l^m Re/Im((x+iy)^m) and N_c = s_lm.  The column kernels work with U: the factors N_c are applied
 // once per source row (the rows hold N_c W_c) and once per destination.
 struct MonicTab {
   double beta[64];  // index l*(l+1)/2 + m

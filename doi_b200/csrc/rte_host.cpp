@@ -318,7 +318,6 @@ struct rte_ctx {
   SelfQuad quad;
   int K = 0;  // moments in use
   double *d_mut = nullptr, *d_mus = nullptr;
-  float* d_mutf = nullptr;
   double* d_mutc = nullptr;     // mu_t in column order
   float* d_mutfc = nullptr;
   double *d_W = nullptr, *d_Wn = nullptr, *d_sum = nullptr, *d_part = nullptr, *d_mom = nullptr;
@@ -492,7 +491,7 @@ static void free_all(rte_ctx* c) {
       cudaEventDestroy(p.second);
     }
   for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
-  void* ps[] = {c->d_mut, c->d_mus, c->d_mutf, c->d_W, c->d_Wn, c->d_sum, c->d_part, c->d_mom,
+  void* ps[] = {c->d_mut, c->d_mus, c->d_W, c->d_Wn, c->d_sum, c->d_part, c->d_mom,
                 c->d_aux1, c->d_aux2, c->d_aux3, c->d_aux4, c->d_Wf, c->d_K, c->d_K64, c->d_cplx, c->d_red, c->d_img,
                 c->d_self_idx, c->d_self_lut, c->d_islot, c->d_err,
                 c->d_bW, c->d_bWn, c->d_bsum, c->d_bres, c->d_bball, c->d_bWf, c->d_h, c->d_S, c->d_out,
@@ -646,7 +645,6 @@ int rte_create(const rte_config* cfg, rte_ctx** out) {
   if (const char* e = getenv("RTE_MAX_SPLIT")) c->max_split = std::max(1, std::min(32, atoi(e)));
   if (rc == RTE_OK) cu(dalloc(c, &c->d_mut, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_mus, c->N), "alloc");
-  if (rc == RTE_OK) cu(dalloc(c, &c->d_mutf, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_mutc, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_mutfc, c->N), "alloc");
   if (rc == RTE_OK) cu(dalloc(c, &c->d_W, NC), "alloc");
@@ -835,11 +833,11 @@ static int build_self_lut(rte_ctx* c) {
   return RTE_OK;
 }
 
-// mu_t, mu_s (and the FP32 mu_t) from device arrays; the pair kernel becomes stale.
+// mu_t, mu_s (and mu_t in column order) from device arrays; the pair kernel becomes stale.
 static int medium_from_device(rte_ctx* c, const double* d_mua, const double* d_mus) {
   c->medium_set = false;  // until its self-voxel tables are there
   CUDA_TRY(c, cudaMemsetAsync(c->d_red + 6, 0, sizeof(double), c->st));
-  CUDA_TRY(c, (c->launches++, rte_launch_medium(d_mua, d_mus, c->d_mut, c->d_mus, c->d_mutf, c->d_mutc, c->d_mutfc,
+  CUDA_TRY(c, (c->launches++, rte_launch_medium(d_mua, d_mus, c->d_mut, c->d_mus, c->d_mutc, c->d_mutfc,
                                                    c->d_islot, c->N, c->d_red + 6, c->st)));
   double mumax = 0.0;
   CUDA_TRY(c, cudaMemcpyAsync(&mumax, c->d_red + 6, sizeof(double), cudaMemcpyDeviceToHost, c->st));
@@ -1517,7 +1515,6 @@ static int check_kernel_err(rte_ctx* c) {
 static int neumann_real(rte_ctx* c, const double* W0, const double* S0, double* res, int flag, const rte_stop* stop,
                         int force_terms, int* nterms, double* last_rel) {
   const size_t NC = (size_t)c->N * c->C;
-  const bool mixed = c->precision == RTE_PREC_MIXED;
   CUDA_TRY(c, cudaMemcpyAsync(c->d_sum, S0, NC * sizeof(double), cudaMemcpyDeviceToDevice, c->st));
   int terms = 0;
   double rel = 0.0;
@@ -1627,7 +1624,6 @@ static int download_pair(rte_ctx* c, const double* d_pair, rte_cplx* h) {
 // (row pairs); A * sum to d_bres.  Stop rules as neumann_real (the reference rule on the real parts
 // of the complex-basis layer sums, as StopIteration takes creal, Kernels_selfsub.c:1184-1220).
 static int neumann_cplx(rte_ctx* c, int flag, const rte_stop* stop, int* nterms, double* last_rel) {
-  const bool mixed = c->precision == RTE_PREC_MIXED;
   int terms = 0;
   double rel = 0.0;
   if (flag) {
@@ -1738,7 +1734,6 @@ extern "C" int rte_prop_abs(rte_ctx* c, const rte_cplx* in, rte_cplx* out, int f
   int rc = upload_cplx(c, in, c->d_aux1, c->d_aux2, &has2);
   if (rc) return rc;
   const size_t NC = (size_t)c->N * c->C;
-  const bool mixed = c->precision == RTE_PREC_MIXED;
   // part 1 -> d_W, part 2 -> d_sum (both scratch here)
   rc = apply_term(c, c->d_aux1, c->d_W, nullptr, flag, flag_scat);
   if (rc) return rc;
@@ -1761,7 +1756,7 @@ extern "C" int rte_prop_abs_adjoint(rte_ctx* c, const rte_cplx* in, rte_cplx* ou
   bool has2 = false;
   int rc = upload_cplx(c, in, c->d_aux1, c->d_aux2, &has2);
   if (rc) return rc;
-  const bool mixed = c->precision == RTE_PREC_MIXED, table = c->model == RTE_MODEL_FIM;
+  const bool table = c->model == RTE_MODEL_FIM;
   double* parts[2] = {c->d_aux1, c->d_aux2};
   double* res[2] = {c->d_W, c->d_sum};
   for (int k = 0; k < (has2 ? 2 : 1) && !rc; k++) {
@@ -2992,7 +2987,7 @@ static std::vector<uintptr_t> graph_signature(const rte_ctx* c, int nb) {
   return {u(std::min(W, Wn)), u(std::max(W, Wn)), u(nb == 1 ? c->d_sum : c->d_bsum),
           u(nb == 1 ? c->d_aux2 : c->d_bres), u(nb == 1 ? c->d_Wf : c->d_bWf),
           u(c->d_part), u(c->d_self_idx), u(c->d_self_lut), u(c->d_mom), (uintptr_t)c->K,
-          (uintptr_t)c->self_lut_ok, u(c->d_K), u(c->d_K64), u(c->d_slab), (uintptr_t)c->slab_bytes, u(c->d_mut), u(c->d_mutf), u(c->d_mus),
+          (uintptr_t)c->self_lut_ok, u(c->d_K), u(c->d_K64), u(c->d_slab), (uintptr_t)c->slab_bytes, u(c->d_mut), u(c->d_mus),
           u(c->d_tab[0][0]), u(c->d_tab[1][0]), u(c->d_flat), u(c->d_red), u(c->d_err), (uintptr_t)c->bcap, (uintptr_t)(fft_eligible(c) && !c->fft_graph_failed),
           rte_fft_signature(c->fft)};
 }

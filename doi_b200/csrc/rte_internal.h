@@ -1,5 +1,5 @@
 // rte_internal.h -- shared declarations between the host context (rte_host.cpp) and the
-// sm_100a kernels (rte_kernels.cu).  Not part of the public ABI (include/rte_b200.h).
+// sm_100a kernels (rte_*.cu).  Not part of the public ABI (include/rte_b200.h).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -133,7 +133,7 @@ struct SelfArgs {
 struct EpiArgs {
   int N, nx, ny, nz, Cfull, S, nb;  // nb right-hand sides, layout [N][nb][Cfull]
   const double* part;   // [S][N][nb][Cfull]
-  const float* partf;   // or FP32 chunk sums of the tile-staged kernel, times N_c here (then part is unused)
+  const float* partf;   // or FP32 chunk sums, times N_c here (then part is unused)
   SelfArgs self;
   const double* mus;
   int flag_scat;
@@ -268,7 +268,7 @@ cudaError_t rte_launch_grad_local(const GradLocalArgs& a, cudaStream_t st);
 __attribute__((visibility("hidden"))) void rte_set_global_error(const char* msg);
 cudaError_t rte_launch_source(const SrcArgs& a, cudaStream_t st);
 // mutc / mutfc: mu_t in column order (islot), FP64 and FP32
-cudaError_t rte_launch_medium(const double* mua, const double* mus, double* mut, double* mus_out, float* mutf,
+cudaError_t rte_launch_medium(const double* mua, const double* mus, double* mut, double* mus_out,
                               double* mutc, float* mutfc, const int* islot, int N, double* red_max, cudaStream_t st);
 cudaError_t rte_launch_fma_peak(int fp64, int iters, float* sink, cudaStream_t st, int blocks);
 cudaError_t rte_upload_sh_tables(const ShTables& t);

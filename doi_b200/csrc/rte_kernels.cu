@@ -10,8 +10,9 @@
 //   w = (r - r')/|r - r'|,  k = exp(-tau(r,r')) dV / (cm |r - r'|^2),
 //
 // then D multiplies coefficient (l,m) by scat[l] * mu_s(r).  The sum over pairs is in rte_column.cu, k in
-// rte_store.cu; the pair sums arrive here as chunk sums that the epilogue adds in a fixed order, so results are
-// deterministic.
+// rte_store.cu; the pair sums arrive here as chunk sums that the epilogue adds in a fixed order.  The chunks are a rule
+// of the grid and the order for FP64 and small grids, which makes results reproducible bit for bit; mixed launches on
+// 4096 voxels and more take theirs from a timing once per process (plan_columns).
 //
 // Path integrals follow mu_int (FisherInfo_IO/src/kernels.cu:50-148): a Siddon walk
 // between voxel centres whose axis crossings are ordered here with exact integer
@@ -34,55 +35,27 @@ struct ScatTab {
 };
 
 __constant__ ShTables c_sh;
-__constant__ float c_shAf[64];
-__constant__ float c_shBf[64];
-__constant__ float c_shQ0f[RTE_MAX_L + 1];
-
-cudaError_t rte_upload_sh_tables(const ShTables& t) {
-  float af[64], bf[64], qf[RTE_MAX_L + 1];
-  for (int i = 0; i < 64; i++) {
-    af[i] = (float)t.A[i];
-    bf[i] = (float)t.B[i];
-  }
-  for (int i = 0; i <= RTE_MAX_L; i++) qf[i] = (float)t.Q0[i];
-  cudaError_t e = cudaMemcpyToSymbol(c_sh, &t, sizeof(ShTables));
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_shAf, af, sizeof af);
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_shBf, bf, sizeof bf);
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_shQ0f, qf, sizeof qf);
-  return e;
-}
-
-template <typename T> __device__ __forceinline__ T shA(int i);
-template <typename T> __device__ __forceinline__ T shB(int i);
-template <typename T> __device__ __forceinline__ T shQ0(int i);
-template <> __device__ __forceinline__ double shA<double>(int i) { return c_sh.A[i]; }
-template <> __device__ __forceinline__ double shB<double>(int i) { return c_sh.B[i]; }
-template <> __device__ __forceinline__ double shQ0<double>(int i) { return c_sh.Q0[i]; }
-template <> __device__ __forceinline__ float shA<float>(int i) { return c_shAf[i]; }
-template <> __device__ __forceinline__ float shB<float>(int i) { return c_shBf[i]; }
-template <> __device__ __forceinline__ float shQ0<float>(int i) { return c_shQ0f[i]; }
+cudaError_t rte_upload_sh_tables(const ShTables& t) { return cudaMemcpyToSymbol(c_sh, &t, sizeof(ShTables)); }
 
 // Real orthonormal SH R_lm at the unit direction (x, y, z), index l*l + l + m.
 // R_l0 = q_l^0(z), R_l,+m = q_l^m(z) Re((x+iy)^m), R_l,-m = q_l^m(z) Im((x+iy)^m), with the
 // normalised associated-Legendre polynomials q (Condon-Shortley phase included) from the
-// upward recurrence in l.  No trigonometric calls.  FP64 reads the uploaded tables; FP32 uses
-// the compile-time copies.
-template <int L, typename T>
-__device__ __forceinline__ void sh_eval(T x, T y, T z, T* R) {
-  constexpr bool F32 = std::is_same<T, float>::value;
-  T cmv = T(1), smv = T(0);
+// upward recurrence in l.  No trigonometric calls.
+template <int L>
+__device__ __forceinline__ void sh_eval(double x, double y, double z, double* R) {
+  double cmv = 1.0, smv = 0.0;
 #pragma unroll
   for (int m = 0; m <= L; ++m) {
     if (m == 1) {
       cmv = x;
       smv = y;
     } else if (m > 1) {
-      T c2 = cmv * x - smv * y;
-      T s2 = cmv * y + smv * x;
+      double c2 = cmv * x - smv * y;
+      double s2 = cmv * y + smv * x;
       cmv = c2;
       smv = s2;
     }
-    T q2 = T(0), q1 = F32 ? (T)kShConst.Q0[m] : shQ0<T>(m);
+    double q2 = 0.0, q1 = c_sh.Q0[m];
     if (m == 0) {
       R[0] = q1;
     } else {
@@ -92,13 +65,12 @@ __device__ __forceinline__ void sh_eval(T x, T y, T z, T* R) {
 #pragma unroll
     for (int l = m + 1; l <= L; ++l) {
       const int id = l * (l + 1) / 2 + m;
-      const T A = F32 ? (T)kShConst.A[id] : shA<T>(id);
-      T q;
+      const double A = c_sh.A[id];
+      double q;
       if (l == m + 1) {
         q = (A * z) * q1;
       } else {
-        const T B = F32 ? (T)kShConst.B[id] : shB<T>(id);
-        q = (A * z) * q1 - B * q2;
+        q = (A * z) * q1 - c_sh.B[id] * q2;
       }
       q2 = q1;
       q1 = q;
@@ -107,54 +79,6 @@ __device__ __forceinline__ void sh_eval(T x, T y, T z, T* R) {
       } else {
         R[l * l + l + m] = q * cmv;
         R[l * l + l - m] = q * smv;
-      }
-    }
-  }
-}
-
-// The monic recurrence, each coefficient handed to emit(index, value) as it is made (the index is a
-// compile-time constant once the loops unroll).
-template <int L, typename T, typename Emit>
-__device__ __forceinline__ void sh_monic_recurrence(T x, T y, T z, Emit emit) {
-  T cmv = T(1), smv = T(0);
-#pragma unroll
-  for (int m = 0; m <= L; ++m) {
-    if (m == 1) {
-      cmv = x;
-      smv = y;
-    } else if (m > 1) {
-      const T c2 = cmv * x - smv * y;
-      const T s2 = cmv * y + smv * x;
-      cmv = c2;
-      smv = s2;
-    }
-    T c1 = cmv, s1 = smv, c0 = T(0), s0 = T(0);
-    if (m == 0) {
-      emit(0, T(1));
-    } else {
-      emit(m * m + 2 * m, cmv);
-      emit(m * m, smv);
-    }
-#pragma unroll
-    for (int l = m + 1; l <= L; ++l) {
-      T cn, sn = T(0);
-      if (l == m + 1) {
-        cn = m == 0 ? z : z * c1;
-        if (m > 0) sn = z * s1;
-      } else {
-        const T b = (T)kMonic.beta[l * (l + 1) / 2 + m];
-        cn = fma(z, c1, -b * c0);
-        if (m > 0) sn = fma(z, s1, -b * s0);
-      }
-      c0 = c1;
-      c1 = cn;
-      s0 = s1;
-      s1 = sn;
-      if (m == 0) {
-        emit(l * l + l, cn);
-      } else {
-        emit(l * l + l + m, cn);
-        emit(l * l + l - m, sn);
       }
     }
   }
@@ -199,7 +123,7 @@ __global__ void __launch_bounds__(RTE_PAIR_THREADS) k_pair_fp64(PairArgs a) {
         if (dist < a.prop_thresh) {
           const double inv = 1.0 / dist;
           double R[C];
-          sh_eval<LA, double>(ddx * inv, ddy * inv, ddz * inv, R);
+          sh_eval<LA>(ddx * inv, ddy * inv, ddz * inv, R);
           double S = 0.0;
 #pragma unroll
           for (int c = 0; c < C; ++c) S = fma(R[c], sW[sv * C + c], S);
@@ -341,7 +265,7 @@ __global__ void __launch_bounds__(256) k_epilogue(EpiArgs a, int Cact) {
     double x = 0.0;
     if (c < Cact) {
       x = a.self.W ? self_term(a.self, r, b, c, nb, a.Cfull, Cact) : 0.0;
-      if (a.partf) {  // FP32 chunk sums of the tile-staged kernel: FP64 sum over the chunks, then N_c
+      if (a.partf) {  // FP32 chunk sums: FP64 sum over the chunks, then N_c
         double u = 0.0;
         for (int q = 0; q < a.S; ++q) u += (double)a.partf[(size_t)q * NV + t];
         x = fma(u, kMonic.N[c], x);
@@ -351,7 +275,7 @@ __global__ void __launch_bounds__(256) k_epilogue(EpiArgs a, int Cact) {
       if (a.flag_scat) x *= a.scat[l] * a.mus[r];
     }
     a.Wout[t] = x;
-    // the pair kernels read N_c W_c (monic SH, sh_eval_monic)
+    // the column kernels read N_c W_c (rte_trig.cuh)
     if (a.rows) {
       const size_t o = ((size_t)b * a.N + a.islot[r]) * a.pitch + c;
       if (a.rows64)
@@ -517,16 +441,15 @@ __global__ void k_source(SrcArgs a) {
   if (a.fball_im) a.fball_im[off[ef] + p] = bi;
 }
 
-// mu_t = mu_a + mu_s (FP64 and FP32 copies, in voxel and column order), mu_s copy, and max(mu_t) into red_max (>= 0 values,
+// mu_t = mu_a + mu_s (FP64 in voxel and column order, FP32 in column order), mu_s copy, and max(mu_t) into red_max (>= 0 values,
 // so the bit pattern orders like the value).
-__global__ void k_medium(const double* mua, const double* mus, double* mut, double* mus_out, float* mutf, double* mutc,
+__global__ void k_medium(const double* mua, const double* mus, double* mut, double* mus_out, double* mutc,
                          float* mutfc, const int* islot, int N, double* red_max) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   double m = 0.0;
   if (r < N) {
     m = mua[r] + mus[r];
     mut[r] = m;
-    mutf[r] = (float)m;
     mutc[islot[r]] = m;
     mutfc[islot[r]] = (float)m;
     if (mus_out != mus) mus_out[r] = mus[r];
@@ -860,21 +783,6 @@ __global__ void k_layer_sums(const double* W, const double* S, int N, int nx, in
 // ---------------------------------------------------------------------------------------------
 // launchers
 
-// Dynamic shared memory above 48 KB for a kernel: the attribute is set to the device's opt-in maximum,
-// the same value from every host thread, not to one launch's size.  The size a launch needs can depend
-// on the context (the lower-order passes of a pair kernel size their source rows by the context's own
-// order), and the server launches the same instantiation from several worker threads; per-launch values
-// let one thread lower the limit between another thread's set and launch, which fails that launch with
-// an invalid-argument error.  Each launch still asks for its own size.
-static cudaError_t allow_smem(const void* kern, size_t smem) {
-  int dev = 0, cap = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&cap, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (e != cudaSuccess) return e;
-  if (smem > (size_t)cap) return cudaErrorInvalidValue;
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, cap);
-}
-
 cudaError_t rte_launch_pair_fp64(const PairArgs& a, int LA, cudaStream_t st) {
   dim3 grid((a.N + RTE_PAIR_THREADS - 1) / RTE_PAIR_THREADS, a.nsplit);
   switch (LA) {
@@ -931,9 +839,8 @@ cudaError_t rte_launch_source(const SrcArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-cudaError_t rte_launch_medium(const double* mua, const double* mus, double* mut, double* mus_out, float* mutf,
-                              double* mutc, float* mutfc, const int* islot, int N, double* red_max, cudaStream_t st) {
-  k_medium<<<(N + 127) / 128, 128, 0, st>>>(mua, mus, mut, mus_out, mutf, mutc, mutfc, islot, N, red_max);
+cudaError_t rte_launch_medium(const double* mua, const double* mus, double* mut, double* mus_out, double* mutc, float* mutfc, const int* islot, int N, double* red_max, cudaStream_t st) {
+  k_medium<<<(N + 127) / 128, 128, 0, st>>>(mua, mus, mut, mus_out, mutc, mutfc, islot, N, red_max);
   return cudaGetLastError();
 }
 
@@ -1066,7 +973,7 @@ __global__ void k_fft_table(FftTabArgs a, double* T, size_t M) {
       uy = ddy / dist;
       uz = ddz / dist;
     }
-    sh_eval<LA, double>(ux, uy, uz, R);
+    sh_eval<LA>(ux, uy, uz, R);
   }
   int p = 0;
 #pragma unroll 1

@@ -1,6 +1,6 @@
-// Exact path integrals along voxel-centre segments (host and device): the walks the pair kernels,
-// the kernel precompute and the tangent kernel share.  Host builds (the CPU checks of the walks) read
-// the medium through plain loads.
+// Exact path integrals along voxel-centre segments (host and device): the walk of the plain FP64 pair operator and of
+// the gradient's weights, and the closed-form path lists of the kernel precompute and the gradient's walk.  Host
+// builds (the CPU checks) read the medium through plain loads.
 #pragma once
 #include <cmath>
 #include <cstdlib>
@@ -107,7 +107,7 @@ RTE_WALK_FN A path_sum(int i, int j, int k, int ip, int jp, int kp, const MU* __
 // the last crossing at or before the path enters the box and stops where it leaves, so the segments it
 // skips are exactly the zero terms of the whole walk and the sum is the same, bit for bit (the entry and
 // exit parameters are found per axis from the crossing counts, crossing n of axis a lying at
-// (2n + 1) h_a).  0 when the path never has all three coordinates inside the box.
+// (2n + 1) h_a).  0 when the path never has all three coordinates inside the box.  No kernel walks it.
 template <typename A, typename MU>
 RTE_WALK_FN A path_sum_box(int i, int j, int k, int ip, int jp, int kp, const MU* __restrict__ mu, int nx,
                            int plane, const int* lo, const int* hi, int& Q) {
@@ -162,15 +162,14 @@ RTE_WALK_FN A path_sum_box(int i, int j, int k, int ip, int jp, int kp, const MU
   return acc;
 }
 
-#ifdef __CUDACC__
 // The voxels that a path of displacement (Dx, Dy, Dz) >= 0 crosses, made by the lanes of a warp: entry k of
 // Dx + Dy + Dz + 1 lies cx, cy, cz steps from the path's start and is `len` long over Q = 2 max(Dx,1) max(Dy,1)
 // max(Dz,1); `leaves` marks the entries that a crossing in x or y ends.  The crossings of each axis are an arithmetic
 // progression (crossing n at (2 n + 1) h), so rank, steps and length of every crossing follow in closed form.
 // Same order as path_sum: ties step z, then y, then x.
 template <typename F>
-__device__ __forceinline__ void path_list(int Dx, int Dy, int Dz, int lane, F put) {
-  const int mx = max(Dx, 1), my = max(Dy, 1), mz = max(Dz, 1), hx = my * mz, hy = mx * mz, hz = mx * my;
+RTE_WALK_FN void path_list(int Dx, int Dy, int Dz, int lane, F put) {
+  const int mx = rte_walk_max(Dx, 1), my = rte_walk_max(Dy, 1), mz = rte_walk_max(Dz, 1), hx = my * mz, hy = mx * mz, hz = mx * my;
   const int sxy = Dx + Dy, S = sxy + Dz;
   auto before = [](int t, int h, int D, bool ties) { return D ? (t + h - (ties ? 0 : 1)) / (2 * h) : 0; };
   for (int e = lane; e <= S; e += 32) {
@@ -184,8 +183,7 @@ __device__ __forceinline__ void path_list(int Dx, int Dy, int Dz, int lane, F pu
     } else {
       t = (2 * (e - sxy) + 1) * hz, cz = e - sxy, cx = before(t, hx, Dx, false), cy = before(t, hy, Dy, false);
     }
-    const int prev = max(max((2 * cx - 1) * hx, (2 * cy - 1) * hy), max((2 * cz - 1) * hz, 0));
+    const int prev = rte_walk_max(rte_walk_max((2 * cx - 1) * hx, (2 * cy - 1) * hy), rte_walk_max((2 * cz - 1) * hz, 0));
     put(cx + cy + cz, cx, cy, cz, t - prev, e < sxy);
   }
 }
-#endif

@@ -15,7 +15,12 @@ pytestmark = pytest.mark.gpu
 def _left(nbytes):
     """About nbytes of device memory left."""
     torch.cuda.init()
-    held = torch.empty(max(0, torch.cuda.mem_get_info()[0] - nbytes), dtype=torch.uint8, device="cuda")
+    held, n = None, max(0, torch.cuda.mem_get_info()[0] - nbytes)
+    while held is None:
+        try:
+            held = torch.empty(n, dtype=torch.uint8, device="cuda")
+        except torch.cuda.OutOfMemoryError:  # the last pages may not be had in one piece
+            n -= 4 << 20
     try:
         yield
     finally:
