@@ -620,21 +620,22 @@ cudaError_t launch_nb(ColArgs a, cudaStream_t st, int* occ) {
   const int nblk = (np + 32 * a.group - 1) / (32 * a.group);  // layout blocks: a warp each, or `group` warps for G = 1
   const int warps = G == 1 ? nblk * a.group : nblk;
   dim3 grid((unsigned)((warps + T_CTA / 32 - 1) / (T_CTA / 32)) * (CPLX ? 1 : a.nrhs / NB), a.nsplit);
-  // the whole column as one run when two CTAs fit an SM's shared memory, else equal runs; runs that the angle rows of
-  // two CTAs would cut below 16 sources take the shared memory of one, up to 64 sources (1x1x500 L=7 mixed, six terms and
+  // the whole column as one run when two CTAs fit an SM's shared memory, else equal runs; where the angle rows leave no
+  // room for two CTAs at runs of 8, the shared memory of one and up to 64 sources (1x1x500 L=7 mixed, six terms and
   // the final application 3.8 ms in runs of 8 -> 3.2; FP32 sums of 512 sources 2.1e-7 from FP64, of 64 1.5e-7)
   auto bytes = [&](int tz) {
     return ColLayout(tz, a.pitch, a.azn, a.row - a.azn, a.ncd, NB * nb_row<L>(), NB,
                      ring_stages<G>() * ring_rows<G>() * 32 * G, ring_stages<G>(), (int)sizeof(T)).bytes;
   };
-  const bool one = bytes(std::min(a.nz, 16)) > 113 * 1024;
-  const size_t limit = (one ? 227 : 113) * 1024;
   size_t smem = 0;
-  for (int nrun = one ? (a.nz + 63) / 64 : 1;; ++nrun) {
-    a.tz = (a.nz + nrun - 1) / nrun;
-    smem = bytes(a.tz);
-    if (smem <= limit || a.tz <= 8) break;
-  }
+  auto runs = [&](int nrun, size_t limit) {
+    do {
+      a.tz = (a.nz + nrun - 1) / nrun++;
+      smem = bytes(a.tz);
+    } while (smem > limit && a.tz > 8);
+    return smem <= limit;
+  };
+  if (!runs(1, 113 * 1024)) runs((a.nz + 63) / 64, 227 * 1024);
   cudaError_t e = smem_limit((const void*)kern, smem);
   if (e != cudaSuccess) return e;
   if (occ) {  // by registers, shared and tensor memory (the runtime's query answers 1 for kernels that use the latter)
