@@ -125,11 +125,6 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
   const int p = min(pt, np - G);
   const bool act = pt < np;
   const int cd = p / a.nzp, z = p - cd * a.nzp, j = cd - c0;
-  // this CTA's sources; none from rows too far from all of its destinations (33^3 L=1 recomputed, coupling over 2.5
-  // voxels: see rte_store.cu)
-  const int cb = max(a.col0 + (int)blockIdx.y * a.chunk, (c0 / a.nx - a.ry) * a.nx);
-  const int ce = min(min(a.col1, a.col0 + ((int)blockIdx.y + 1) * a.chunk), ((c0 + ncd - 1) / a.nx + a.ry + 1) * a.nx);
-  const int nrun = (nz + a.tz - 1) / a.tz, ntile = max(ce - cb, 0) * nrun;
   if (tid == 0) {
     mbar_init(&bar[0], 1);  // a run's source rows and azimuth values
     mbar_init(&bar[1], 1);  // its polar values
@@ -144,6 +139,11 @@ __device__ __forceinline__ void column_body(const ColArgs& a) {
   for (int q = tid; q < ncd; q += T_CTA) sxy[q] = ((c0 + q) / a.nx) << 16 | (c0 + q) % a.nx;
   __syncthreads();
   tmem_fence_after();
+  // this CTA's sources; none from rows too far from all of its destinations (rte_store.cu).  Read back from shared memory:
+  // derived from c0 they cost 48 more bytes of spills at L = 7 (25^3, four right-hand sides 4.57 ms a launch, 4.46 here)
+  const int cb = max(a.col0 + (int)blockIdx.y * a.chunk, ((sxy[0] >> 16) - a.ry) * a.nx);
+  const int ce = min(min(a.col1, a.col0 + ((int)blockIdx.y + 1) * a.chunk), ((sxy[ncd - 1] >> 16) + a.ry + 1) * a.nx);
+  const int nrun = (nz + a.tz - 1) / a.tz, ntile = max(ce - cb, 0) * nrun;
   const uint32_t tm = *stm + ((uint32_t)(wid * 32) << 16);  // this warp's lanes, column 0
   const T* gW = static_cast<const T*>(a.W) + (size_t)rhs * a.N * a.pitch;
   const T* gT = static_cast<const T*>(a.tab);

@@ -1169,7 +1169,7 @@ static cudaError_t launch_columns(const rte_ctx* c, const ColArgs& a, int LA, in
 // and the fastest is kept for the process (every context of that shape on that device reuses it).
 // RTE_AUTOTUNE=0 keeps the model's choice; RTE_NSPLIT forces a split.
 namespace {
-using TuneKey = std::tuple<int, int, int, int, int, int, int, int, int>;  // device, grid, LA, nb, precision, cplx, columns
+using TuneKey = std::tuple<int, int, int, int, int, int, int, int, int>;  // device, grid, LA, nb, precision, cplx or pair by pair, columns
 std::mutex g_tune_mu;
 std::map<TuneKey, int> g_tuned;  // source columns per chunk
 }  // namespace
@@ -1276,7 +1276,7 @@ static int plan_columns(rte_ctx* c, int LA, int nb, const void* K, size_t ld, in
   const char* at = getenv("RTE_AUTOTUNE");
   const bool tune = !forced && !(at && at[0] == '0') && !c->capturing && !f && c->N >= 4096 && rank.size() > 1;
   if (forced) chunk = std::max(1, std::min(cap, (cols + std::max(1, atoi(forced)) - 1) / std::max(1, atoi(forced))));
-  const TuneKey tk{c->cfg.device, c->cx, c->cy, c->cz, LA, nb, c->precision, cplx, cols};
+  const TuneKey tk{c->cfg.device, c->cx, c->cy, c->cz, LA, nb, c->precision, cplx + 2 * (c->dirs ? 1 : 0), cols};
   bool have = false;
   if (tune) {
     std::lock_guard<std::mutex> lk(g_tune_mu);

@@ -38,16 +38,17 @@ extern "C" {
 #define RTE_MODEL_FIM 1   /* FisherInfo_IO kernels as shipped: 100x100 SH table, g truncated ... */
 #define RTE_MODEL_CPU 2   /* CPU package (uniform medium) discretisation */
 
-#define RTE_PREC_FP64 0  /* plain FP64 method: every pair recomputed in FP64 each term */
-#define RTE_PREC_MIXED 1 /* FP32 path integrals + SH projection, FP64 sums and norms */
+#define RTE_PREC_FP64 0  /* plain FP64 method: every pair in FP64 (recomputed each term or kept: kernel mode) */
+#define RTE_PREC_MIXED 1 /* FP32 path integrals, SH projection and sums over a chunk of sources; FP64 sums of the
+                            chunks, running sum, self term, scatter and norms */
 
 #define RTE_KERNEL_AUTO 0      /* mixed precision: store the voxel-pair kernel when it fits, else recompute;
                                   FP64: recompute (the plain method), keeping the kernel while it is no
                                   larger than the recompute workspace (1 GB) */
 #define RTE_KERNEL_STORE 1     /* store exp(-tau)/r^2 per voxel pair in HBM (FP32 for mixed precision,
                                   FP64 for the FP64 method: 8 N^2 bytes) */
-#define RTE_KERNEL_RECOMPUTE 2 /* recompute path integrals every term, in a workspace of at most 1 GB or one
-                                  column of sources */
+#define RTE_KERNEL_RECOMPUTE 2 /* recompute path integrals every term, in a workspace of at most 1 GB and half of the
+                                  free memory, or one column of sources */
 
 #define RTE_SRC_COLUMN 0 /* collimated pencil on the z=0 face, column containing (pos_x,pos_y) */
 #define RTE_SRC_FIM 1    /* FisherInfo_IO rule: column x == nX/2.0 && y == nY/2.0 (even grids only) */
