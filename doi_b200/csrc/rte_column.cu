@@ -89,9 +89,8 @@ __host__ __device__ constexpr int tmem_cols() {
 // layout's 58 KB admit three).  NB = 2: two right-hand sides a thread, which
 // share the trigonometric rows, the kernel values and the copies (two CTAs per SM at L >= 4).  CPLX: (real, imaginary) rows of one complex
 // right-hand side, the pair kernel times exp(-i kappa r) (phase tabulated beside the angles).
-// 33^3 L=5 launch, FP32, one right-hand side: 7.40 ms by per-pair spherical harmonics -> 2.36; four: 20.1 -> 9.3,
-// two a thread 8.3;
-// FP64: 24.7 -> 4.3.  Of the 2.4 ms, skipping phases one at a time: pair loop 1.15, contraction 0.25, angle rows
+// 33^3 L=5 launch, FP32, one right-hand side: 7.40 ms by per-pair spherical harmonics -> 2.37; four: 20.1 -> 9.3, two a
+// thread 8.2; FP64: 24.7 -> 4.2.  Of the 2.4 ms, skipping phases one at a time: pair loop 1.15, contraction 0.25, angle rows
 // 0.2, the kernel stream 0.15, the rest expansion, start of runs and barriers.  All copies are bulk copies by warp 0
 // and by each warp for its own ring (copies by all threads: 2.40, FP64 5.4); deeper rings and a fifth of the
 // registers less did not pay (ring of 3 stages 2.37, four CTAs with 3-row stages 2.50).

@@ -27,8 +27,8 @@ __host__ __device__ inline int kmat_pos(int slot, int nz, int nzp) { return slot
 #define RTE_COL_GC(L, fp64) ((L) <= ((fp64) ? 3 : 5) ? RTE_COL_G(L) : 1)
 // real right-hand sides per thread of an FP32 launch with an even number of them.  Two share the
 // trigonometric rows, the kernel values and the copies, but take the registers of half the CTAs at L >= 4.  Solves of
-// four sources, one -> two a thread: L=1 57 -> 41 ms, L=2 69 -> 59, L=3 (33^3) 138 -> 119, L=5 (33^3) 214 -> 191; L=4
-// 81.1 -> 82.5, L=6 53 -> 58, L=7 83 -> 79 with longer first passes, so these keep one.
+// four sources and 20 terms, one -> two a thread: 33^3 L=1 92 -> 62 ms, L=2 111 -> 95, L=3 128 -> 111, L=5 203 -> 182;
+// 29^3 L=4 79 -> 81, 25^3 L=6 76 -> 78, so these keep one.  (L = 7 would gain: 25^3 99.9 -> 96.9, 17^3 18.3 -> 17.2.)
 #define RTE_COL_NB(L) (((L) >= 1 && (L) <= 3) || (L) == 5 ? 2 : 1)
 
 // Plain FP64 pair operator (k_pair_fp64): sums over `chunk` sources per blockIdx.y.

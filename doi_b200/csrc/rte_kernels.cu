@@ -248,8 +248,8 @@ __device__ __forceinline__ double self_term(const SelfArgs& a, int r, int b, int
 // accumulate the running sum and the norms used by the stop rules.  One thread per (voxel, right-hand side,
 // coefficient) element, grid-stride, so every stream (chunk sums, outputs, running sum) is read and written
 // coalesced; the four norms are reduced per block and added atomically.  Bound by loads of the self-term table
-// (2 C per element, from L1 and L2) and of the chunk sums.  Measured per term, self term and epilogue together: 171 ->
-// 86 us at 33^3 L=5, 448 -> 254 us with four right-hand sides, 310 -> 79 us at 25^3 L=7 against a self-term launch of
+// (2 C per element, from L1 and L2) and of the chunk sums.  Measured per term, self term and epilogue together (by the
+// number of chunks): 171 -> 90 us at 33^3 L=5, 448 -> 290 us with four right-hand sides, 310 -> 79 us at 25^3 L=7 against a self-term launch of
 // its own that read rows of D.  Coefficients above (LA+1)^2 are written as 0.
 __global__ void __launch_bounds__(256) k_epilogue(EpiArgs a, int Cact) {
   const int nb = a.nb > 0 ? a.nb : 1;

@@ -12,14 +12,15 @@
 // written both ways.  mu_t is read from shared memory (in column order) when it fits, else through L1.
 //
 // Where voxels couple over a short distance only, displacements of more rows than the column kernels read are left out
-// (33^3 L=1 FP64 recomputed, coupling over 2.5 voxels, six terms: all displacements 103 ms; a walk per coupled pair 24).
+// (33^3 L=1 FP64 recomputed, coupling over 2.5 voxels, six terms: all displacements 103 ms, a walk per coupled pair 24,
+// now 18).
 //
 // DERIV: the derivative of K along a direction of mu_t instead, K times minus the path integral of the direction
 // (mu: the direction, Kin: K of the same sources, which may be the output).
 //
 // Bound: instruction issue of the path sums (one add, one load, one multiply-add per voxel crossed) and the barriers
-// between lists, sums and write-out.  33^3 FP32: 22.8 ms by a walk per pair (70 % ALU) -> 8.8; FP64 35.3 -> 21;
-// 41^3 FP32: 96 -> 44; of the 8.8 (44) ms the sums alone take about half, the write-out a sixth.
+// between lists, sums and write-out.  33^3 FP32: 22.8 ms by a walk per pair (70 % ALU) -> 8.5; FP64 35.3 -> 19;
+// 41^3 FP32: 96 -> 46; the sums alone take about half, the write-out a sixth.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
