@@ -20,7 +20,7 @@ CC="${RTE_CC:-gcc}"
 
 "$CXX" -O2 -std=c++17 -fopenmp -fPIC -shared -o "$HERE/liboracle.so" "$HERE/rte_oracle.cpp"
 
-if [ ! -d "$REF" ]; then
+if [ ! -f "$REF/CPU package/src/RTE_uniform.c" ]; then  # absent, or a directory without the sources
   echo "oracle/build.sh: reference tree not present; built liboracle.so only"
   exit 0
 fi
