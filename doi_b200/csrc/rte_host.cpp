@@ -515,15 +515,21 @@ static int slot_of(const rte_ctx* c, int r) {
   return (y * c->cx + x) * c->cz + z;
 }
 
+// Workspace of the forms that recompute the pair kernel: slabs of source columns, at most this much at a time.
+static const size_t kSlabBytes = 1ull << 30;
+
 // Axis of the columns: z, or (1, 2) the longer of x and y on grids of few layers, where z columns share little
 // (rte_flat.cu).  Forward solves of six terms, mixed, kernel stored / recomputed, columns along z -> along x:
 // 110x110x1 L=3 195 / 940 -> 5.2 / 17 ms, 36x36x9 L=1 5.1 / 12.6 -> 3.2 / 9.0, 20x20x9 L=1 1.32 / 2.06 -> 1.34 / 1.91,
-// 14x14x6 (196 z columns) 0.96 / 1.11 -> 1.21 / 1.35.  From ten layers on z columns are no slower than a walk and
-// spherical harmonics per pair were (35x35x10 L=1 5.0 / 12.4 ms, those 5.2 / 44) and stay.  The table model's
+// 14x14x6 (196 z columns) 0.96 / 1.11 -> 1.21 / 1.35.  Ten to twelve layers exchange axes where
+// the kernel is kept (four sources 221x4x12 L=1, ten terms: per pair 3.9 ms, z 5.8, x 3.6); recomputed, z columns are
+// faster there (60x20x12 L=1 23 ms, x 24.5; FP64 63 and 78).  The table model's
 // pair-by-pair form: 70x70x2 L=3 31 / 80 -> 6.4 / 14, 50x50x4 L=2 9.8 / 22 -> 5.5 / 12 (FP64 15 / 68 -> 6.9 / 16), but
 // 45x45x6 L=5 10 / 20 -> 17 / 23.
 static int column_axis(const rte_ctx* c) {
-  const int layers = c->model != RTE_MODEL_FIM ? 9 : (c->L <= 5 ? 4 : 3);
+  const bool f64 = c->precision == RTE_PREC_FP64, kept = c->kernel_mode == RTE_KERNEL_STORE ||
+      (c->kernel_mode == RTE_KERNEL_AUTO && (!f64 || sizeof(double) * (size_t)c->N * c->N <= kSlabBytes));
+  const int layers = c->model == RTE_MODEL_FIM ? (c->L <= 5 ? 4 : 3) : (kept ? 12 : 9);
   if (c->nz > layers || std::max(c->nx, c->ny) < 2 * c->nz || c->nx * c->ny < 32 * c->nz + 96) return 0;
   return c->nx >= c->ny ? 1 : 2;
 }
@@ -934,9 +940,6 @@ static size_t kernel_cells(const rte_ctx* c, size_t rows) {
   const size_t np = (size_t)c->cx * c->cy * d.nzp, kb = 32 * (size_t)d.group;
   return (np + kb - 1) / kb * kb * rows;
 }
-
-// Workspace of the forms that recompute the pair kernel: slabs of source columns, at most this much at a time.
-static const size_t kSlabBytes = 1ull << 30;
 
 // Rows of columns within which voxels couple (prop_thresh, a little more for its comparison in FP32).
 static int coupled_rows(const rte_ctx* c) {

@@ -13,7 +13,7 @@ from conftest import real_to_complex, rel
 
 pytestmark = pytest.mark.gpu
 
-GRIDS = [(64, 4, 1, 3), (4, 65, 1, 5), (129, 2, 2, 7), (3, 90, 6, 2), (30, 9, 9, 1), (1, 256, 1, 4), (300, 1, 1, 6), (20, 13, 3, 0)]
+GRIDS = [(64, 4, 1, 3), (4, 65, 1, 5), (129, 2, 2, 7), (3, 90, 6, 2), (30, 9, 9, 1), (1, 256, 1, 4), (300, 1, 1, 6), (20, 13, 3, 0), (64, 8, 12, 2)]
 _REF = {}
 
 
